@@ -98,6 +98,26 @@ def test_brick_list_build_writes_the_same_lists(gpu):
         assert np.array_equal(x, y)
 
 
+@pytest.mark.parametrize("n_side", [8, 50, 51])
+def test_warp_and_thread_list_builds_write_the_same_lists(gpu, n_side):
+    # up to 131,072 atoms one warp builds an atom's list, above one thread;
+    # variant 8's brick build is the independent count, variant 5 the full
+    # list of the same builds
+    cfg, u = _lattice(n_side, temperature=200.0, coul=True)
+    out = []
+    for variant in (6, 8, 5):
+        h = _handle(cfg, variant)
+        h.set_universe(u)
+        st = h.step(6)
+        out.append((h.get_state(), st, h.list_stats(), h.list_rebuilds()))
+        h.close()
+    assert out[0][2] == out[1][2] and out[0][2][0] > 0 and out[0][3] >= 2
+    for o in out[1:]:
+        assert np.array_equal(out[0][1], o[1])
+        for x, y in zip(out[0][0], o[0]):
+            assert np.array_equal(x, y)
+
+
 @pytest.mark.parametrize("thermo", [False, True])
 def test_trajectory_follows_per_tick_variant(gpu, thermo):
     cfg, u = _lattice(16, temperature=120.0, coul=True)
