@@ -5,7 +5,7 @@
 #include <cstring>
 #include <string>
 
-#include "gx_internal.cuh"
+#include "gx_nlist.cuh"
 
 namespace gx {
 int upload_pair_table_f64(gx_handle* h);
@@ -341,9 +341,10 @@ int commit_lambda(gx_handle* h) {
 int step_error(gx_handle* h, uint32_t e) {
     if (!e) return GX_OK;
     cudaMemset(h->derr, 0, sizeof(uint32_t));
+    if (e & kErrTimeout) nl_after_timeout(h);
     if (e & kErrNonFinite) return set_err(h, GX_ERR_NONFINITE, "non-finite force in the pair pass");
     if (e & kErrSaturation) return set_err(h, GX_ERR_SATURATION, "fixed-point force saturated");
-    if (e & kErrTimeout) return set_err(h, GX_ERR_TIMEOUT, "shared-memory staging wait timed out");
+    if (e & kErrTimeout) return set_err(h, GX_ERR_TIMEOUT, "a bounded device wait timed out");
     return set_err(h, GX_ERR_CUDA, "unknown device error");
 }
 
@@ -905,7 +906,9 @@ int step_impl(gx_handle* h, int nsteps, gx_tick_stats* stats, int use_graph, boo
         h->launches = l0;
         return GX_OK;
     };
-    for (int s = 0; s < nsteps; ++s) {
+    const bool one_launch = graph && use_nl && nl_ticks_eligible(h);  // a small universe: no graph at all
+    if (one_launch && nsteps > 0 && (rc = nl_ticks(h, nsteps, drec, thermo, tau, kpart, spart))) return rc;
+    for (int s = one_launch ? nsteps : 0; s < nsteps; ++s) {
         if (!graph) {
             if ((rc = tick(false))) return rc;
             continue;
@@ -969,7 +972,7 @@ int step_impl(gx_handle* h, int nsteps, gx_tick_stats* stats, int use_graph, boo
     }
     if (use_nl) h->sorted = false;  // buf[cur] is ordered by the list grid, not the force grid
     h->nl_fresh = nsteps > 0 ? (use_nl && h->nl_valid) : fresh0;
-    h->last_tick_nl = use_nl;
+    h->last_tick_nl = use_nl && !one_launch;  // whether the tick recorded io_ev[3]
     if (defer) return GX_OK;
     if (drec) {
         GX_CUDA(h, cudaMemcpyAsync(stats, drec, (size_t)nsteps * sizeof(gx_tick_stats), cudaMemcpyDeviceToHost,
@@ -1028,6 +1031,7 @@ int gx_autotune(gx_handle* h, int reps, int* best, double* ms) {
     // passes leave the state bit-identical whichever variant runs.
     const int cand[4] = {4, 1, 3, 2};
     int pick = 4;
+    bool automatic = false;  // the one-launch tick of a small universe won
     double best_ms = 1e300;
     const int saved = h->kernel_variant;
     for (int v : cand) {
@@ -1150,13 +1154,27 @@ int gx_autotune(gx_handle* h, int reps, int* best, double* ms) {
                     int r2 = tick_ms(&best_t);  // restores the snapshot after the tick above
                     if (!rc) rc = r2;
                 }
+                // a small universe's automatic tick is one launch (gx_nltick.cu)
+                if (!rc && n <= kTickMaxAtoms) {
+                    int lanes = 0, block = 0, slots = 0, brick = 0;
+                    nl_shape(h, &lanes, &block, &slots, &brick);
+                    double t = 1e300;
+                    h->kernel_variant = 0;
+                    nl_clear_shape(h);
+                    rc = tick_ms(&t);
+                    automatic = !rc && t < best_t;
+                    if (!automatic) {
+                        nl_set_tpp(h, lanes);
+                        nl_set_block(h, block);
+                    }
+                }
             }
             cudaFree(snap);
         }
     }
-    h->kernel_variant = rc ? saved : pick;
+    h->kernel_variant = rc ? saved : (automatic ? 0 : pick);
     invalidate_graphs(h);
-    if (best) *best = h->kernel_variant;
+    if (best) *best = automatic ? 6 : h->kernel_variant;  // the automatic variant walks the half list of 6
     return rc;
 }
 

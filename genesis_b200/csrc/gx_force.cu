@@ -229,51 +229,22 @@ __global__ void k_bonds(GridGeom g, StateBuf b, const uint32_t* __restrict__ key
     double vb = 0.0;
     for (size_t t = (size_t)blockIdx.x * kForceThreads + threadIdx.x; t < nbonds;
          t += (size_t)gridDim.x * kForceThreads) {
-        uint32_t ia = pos_of_slot[bonds[2 * t]], ib = pos_of_slot[bonds[2 * t + 1]];
-        double dx = min_image1(xsub(b.x[ia], b.x[ib]), L.box[0]);
-        double dy = min_image1(xsub(b.y[ia], b.y[ib]), L.box[1]);
-        double dz = min_image1(xsub(b.z[ia], b.z[ib]), L.box[2]);
-        double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
-        double d = xsqrt(d2);
-        if (d2 < L.rc2 && d > kEpsF64) {
-            int ta = b.elem[ia], tb = b.elem[ib];
-            double sg = psig[ta * kNElem + tb], ep = peps[ta * kNElem + tb];
-            double r_eq = xmul(sg, r_eq_factor);
-            double rc_bond = xmul(k_bind, sg);
-            if (d < rc_bond) {
-                double kk = xdiv(xmul(curv_factor, ep), xmul(sg, sg));
-                double dr = xsub(d, r_eq);
-                double m = xmul(-kk, dr);
-                double v = xmul(xmul(xmul(0.5, kk), dr), dr);
-                double sw, dsw;
-                smooth_f64(d, r_eq, rc_bond, sw, dsw);
-                double fm = xsub(xmul(m, sw), xmul(v, dsw));
-                double vv = xmul(v, sw);
-                int mult = key ? pair_multiplicity(g, key[ia], key[ib]) : 1;
-                double inv = xdiv(1.0, d);
-                double nx = xmul(dx, inv), ny = xmul(dy, inv), nz = xmul(dz, inv);
-                for (int r = 0; r < mult; ++r) {
-                    vb = xadd(vb, vv);
-                    if (fm == 0.0) continue;
-                    if (mixed) {
-                        long long qx = __double2ll_rn(xmul(xmul(nx, fm), kFixScale));
-                        long long qy = __double2ll_rn(xmul(xmul(ny, fm), kFixScale));
-                        long long qz = __double2ll_rn(xmul(xmul(nz, fm), kFixScale));
-                        atomicAdd((unsigned long long*)&F[ia], (unsigned long long)qx);
-                        atomicAdd((unsigned long long*)&F[fstride + ia], (unsigned long long)qy);
-                        atomicAdd((unsigned long long*)&F[2 * fstride + ia], (unsigned long long)qz);
-                        atomicAdd((unsigned long long*)&F[ib], (unsigned long long)(-qx));
-                        atomicAdd((unsigned long long*)&F[fstride + ib], (unsigned long long)(-qy));
-                        atomicAdd((unsigned long long*)&F[2 * fstride + ib], (unsigned long long)(-qz));
-                    } else {
-                        atomicAdd(&b.ax[ia], xmul(xmul(nx, fm), b.inv_mass[ia]));
-                        atomicAdd(&b.ay[ia], xmul(xmul(ny, fm), b.inv_mass[ia]));
-                        atomicAdd(&b.az[ia], xmul(xmul(nz, fm), b.inv_mass[ia]));
-                        atomicAdd(&b.ax[ib], xmul(xmul(nx, -fm), b.inv_mass[ib]));
-                        atomicAdd(&b.ay[ib], xmul(xmul(ny, -fm), b.inv_mass[ib]));
-                        atomicAdd(&b.az[ib], xmul(xmul(nz, -fm), b.inv_mass[ib]));
-                    }
-                }
+        const uint32_t ia = pos_of_slot[bonds[2 * t]], ib = pos_of_slot[bonds[2 * t + 1]];
+        double nx, ny, nz, fm, vv;
+        if (!bond_f64(L, b, ia, ib, psig, peps, k_bind, r_eq_factor, curv_factor, nx, ny, nz, fm, vv)) continue;
+        const int mult = key ? pair_multiplicity(g, key[ia], key[ib]) : 1;
+        for (int r = 0; r < mult; ++r) {
+            vb = xadd(vb, vv);
+            if (fm == 0.0) continue;
+            if (mixed) {
+                bond_to_fixed(F, fstride, ia, ib, nx, ny, nz, fm);
+            } else {
+                atomicAdd(&b.ax[ia], xmul(xmul(nx, fm), b.inv_mass[ia]));
+                atomicAdd(&b.ay[ia], xmul(xmul(ny, fm), b.inv_mass[ia]));
+                atomicAdd(&b.az[ia], xmul(xmul(nz, fm), b.inv_mass[ia]));
+                atomicAdd(&b.ax[ib], xmul(xmul(nx, -fm), b.inv_mass[ib]));
+                atomicAdd(&b.ay[ib], xmul(xmul(ny, -fm), b.inv_mass[ib]));
+                atomicAdd(&b.az[ib], xmul(xmul(nz, -fm), b.inv_mass[ib]));
             }
         }
     }

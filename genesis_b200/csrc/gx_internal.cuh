@@ -347,10 +347,15 @@ bool nl_eligible(gx_handle* h);
 int nl_prepare(gx_handle* h, bool* graphs_stale);
 int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, int* nblocks, bool energy);
 int nl_rebuilds(gx_handle* h, uint64_t* out);
+// The ticks of a small universe in one cooperative launch (gx_nltick.cu).
+bool nl_ticks_eligible(gx_handle* h);
+int nl_ticks(gx_handle* h, int nticks, gx_tick_stats* rec, bool thermo, double tau, double* kpart, double* spart);
+void nl_after_timeout(gx_handle* h);
 int nl_set_skin(gx_handle* h, double skin);
 int nl_tune_tpp(gx_handle* h, int reps);
 int nl_config(gx_handle* h, double* skin, int* tpp);
 int nl_set_tpp(gx_handle* h, int tpp);
+void nl_clear_shape(gx_handle* h);  // threads per atom and far-end block back to automatic
 int nl_set_slots(gx_handle* h, int slots);
 int nl_set_brick(gx_handle* h, int cells);
 int nl_set_block(gx_handle* h, int block);

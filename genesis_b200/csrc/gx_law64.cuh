@@ -75,6 +75,52 @@ __device__ __forceinline__ void pair_f64(const LawF64& L, double d, double sg, d
     pair_f64_e24(L, d, sg, ep, xdiv(xmul(24.0, ep), sg), qa, qb, ma, mb, fmag, V);
 }
 
+// One observed bond's spring (src/systems/forces.rs:305-317,
+// bond_harmonic_raw forces.rs:290-293), exact: the unit normal, the force
+// magnitude and the energy.  False when the pair is out of the spring's reach.
+__device__ __forceinline__ bool bond_f64(const LawF64& L, const StateBuf& b, uint32_t ia, uint32_t ib,
+                                         const double* psig, const double* peps, double k_bind, double r_eq_factor,
+                                         double curv_factor, double& nx, double& ny, double& nz, double& fm,
+                                         double& vv) {
+    const double dx = min_image1(xsub(b.x[ia], b.x[ib]), L.box[0]);
+    const double dy = min_image1(xsub(b.y[ia], b.y[ib]), L.box[1]);
+    const double dz = min_image1(xsub(b.z[ia], b.z[ib]), L.box[2]);
+    const double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
+    const double d = xsqrt(d2);
+    if (!(d2 < L.rc2 && d > kEpsF64)) return false;
+    const int ta = b.elem[ia], tb = b.elem[ib];
+    const double sg = psig[ta * kNElem + tb], ep = peps[ta * kNElem + tb];
+    const double r_eq = xmul(sg, r_eq_factor);
+    const double rc_bond = xmul(k_bind, sg);
+    if (!(d < rc_bond)) return false;
+    const double kk = xdiv(xmul(curv_factor, ep), xmul(sg, sg));
+    const double dr = xsub(d, r_eq);
+    const double m = xmul(-kk, dr);
+    const double v = xmul(xmul(xmul(0.5, kk), dr), dr);
+    double sw, dsw;
+    smooth_f64(d, r_eq, rc_bond, sw, dsw);
+    fm = xsub(xmul(m, sw), xmul(v, dsw));
+    vv = xmul(v, sw);
+    const double inv = xdiv(1.0, d);
+    nx = xmul(dx, inv);
+    ny = xmul(dy, inv);
+    nz = xmul(dz, inv);
+    return true;
+}
+
+// The spring's force quantised into the mixed path's fixed-point sums.
+__device__ __forceinline__ void bond_to_fixed(long long* F, size_t fstride, uint32_t ia, uint32_t ib, double nx,
+                                              double ny, double nz, double fm) {
+    const long long q[3] = {__double2ll_rn(xmul(xmul(nx, fm), kFixScale)),
+                            __double2ll_rn(xmul(xmul(ny, fm), kFixScale)),
+                            __double2ll_rn(xmul(xmul(nz, fm), kFixScale))};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        atomicAdd((unsigned long long*)&F[c * fstride + ia], (unsigned long long)q[c]);
+        atomicAdd((unsigned long long*)&F[c * fstride + ib], (unsigned long long)(-q[c]));
+    }
+}
+
 inline LawF64 make_law64(const gx_handle* h) {
     LawF64 L;
     L.lj_rc = h->fs.lj_rc;

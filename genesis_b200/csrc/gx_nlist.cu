@@ -39,35 +39,9 @@
 #include <cstring>
 
 #include "gx_law64.cuh"
-#include "gx_pair_f32.cuh"
+#include "gx_nlist.cuh"
 
 namespace gx {
-
-struct NlState {
-    GridGeom lg{};            // list grid: cells >= r_c + skin
-    double skin = -1.0;       // < 0: default (0.1 r_c)
-    double skin_used = 0.0;
-    int half = -1;            // list kind built: 0 full, 1 half (variant 6)
-    int tpp = 1;              // threads per atom in the list pass (1, 2, 4, 8)
-    int slots = 16;           // variant 7: stash slots per thread (8 or 16)
-    int brick = 1;            // variant 8: 0 = bricks of 4 cells (1024 staged atoms), 1 = 8 cells (2048)
-    int block = 0;            // variant 6, one lane per atom: 0 = far ends always global, 128 or 256 = far
-                              // ends inside a block of that many atoms summed in shared memory
-    int cap_nb = 0;           // list entries per atom
-    size_t cap = 0;           // atoms the buffers hold
-    uint32_t* list = nullptr; // entry e of atom p at list[e * cap + p]
-    uint32_t* cnt = nullptr;  // entries per atom (> cap_nb: overflowed)
-    float4* ref = nullptr;    // home-frame positions at the last rebuild
-    uint32_t* flag = nullptr; // [0] rebuild requested, [1] rebuilds done, [2] half-box translations since (mod 2),
-                              // [3] runs of a captured rebuild body
-    CellList cl;
-    // A captured tick puts the rebuild in the body of a conditional (IF)
-    // graph node, set from flag[0], so that a tick without a rebuild does
-    // not launch it at all.  The body is captured from a second stream.
-    cudaStream_t side = nullptr;
-    uint64_t body_kernels = 0;  // kernels in the body (counted when it runs)
-    uint32_t body_runs_seen = 0;
-};
 
 namespace {
 
@@ -76,49 +50,13 @@ constexpr int kNlBuildThreads = 128;
 constexpr int kNlBuildUnroll = 4;
 constexpr uint32_t kNlBuildWarpMax = 131072;  // atoms up to which a list is built by one warp per atom (k_nl_build_warp)
 constexpr int kRedThreads = 256;
-constexpr uint32_t kIdxMask = (1u << 27) - 1u;
 
 inline unsigned nblk(size_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 __device__ __forceinline__ bool gated_off(const uint32_t* gate) { return gate && *gate == 0u; }
 
-// Offset of a coordinate from its home cell's origin in the frame of the
-// last rebuild (`shift` = the translation to undo, 0 or L/2), unwrapped
-// across the periodic boundary (the atom may have left its home cell).
-__device__ __forceinline__ double home_local(double v, double L, double c, uint32_t i, double shift) {
-    double u = xsub(rem_euclid(xadd(xadd(v, xmul(0.5, L)), shift), L), xmul((double)i, c));
-    if (u > 0.5 * L) u = xsub(u, L);
-    else if (u < -0.5 * L) u = xadd(u, L);
-    return u;
-}
-
-__device__ __forceinline__ float4 stage_one(const GridGeom& g, const StateBuf& b, uint32_t home, uint32_t i,
-                                            double x, double y, double z, bool half) {
-    uint32_t ix, iy, iz;
-    decode(g, home, ix, iy, iz);
-    return make_float4((float)home_local(x, g.L[0], g.cell[0], ix, half ? xmul(0.5, g.L[0]) : 0.0),
-                       (float)home_local(y, g.L[1], g.cell[1], iy, half ? xmul(0.5, g.L[1]) : 0.0),
-                       (float)home_local(z, g.L[2], g.cell[2], iz, half ? xmul(0.5, g.L[2]) : 0.0),
-                       __int_as_float((int)b.kind[i]));
-}
-
-// Neighbour-cell code: (ox+1) + 3(oy+1) + 9(oz+1); 13 is the home cell.
-__device__ __forceinline__ void code_shift(const GridGeom& g, uint32_t code, float& sx, float& sy, float& sz) {
-    int ox = (int)(code % 3u) - 1, oy = (int)((code / 3u) % 3u) - 1, oz = (int)(code / 9u) - 1;
-    sx = -(float)ox * g.cellf[0];
-    sy = -(float)oy * g.cellf[1];
-    sz = -(float)oz * g.cellf[2];
-}
-
-__device__ __forceinline__ uint32_t cell_at(const GridGeom& g, uint32_t cx, uint32_t cy, uint32_t cz, uint32_t code) {
-    int ox = (int)(code % 3u) - 1, oy = (int)((code / 3u) % 3u) - 1, oz = (int)(code / 9u) - 1;
-    return encode(g, wrap_add(cx, ox, g.n[0]), wrap_add(cy, oy, g.n[1]), wrap_add(cz, oz, g.n[2]));
-}
-
-// Kick (integrate.rs:38-45, with the pending scale of thermostat.rs:68-70),
-// drift (integrate.rs:62-66), wrap (boundary.rs:28-34) with the same exact
-// FP64 operations as k_kick/k_drift/k_wrap; then the home-frame staging and
-// the displacement test against the last rebuild.
+// nl_advance_one over the universe, the force sums of the half-list pass
+// zeroed beside it; the flag is raised once per warp.
 __global__ void __launch_bounds__(256) k_nl_advance(StateBuf b, uint32_t n, const double* __restrict__ lambda,
                                                      double half_dt, double dt, double hx, double hy, double hz,
                                                      int wrap, GridGeom g, const uint32_t* __restrict__ home,
@@ -127,7 +65,6 @@ __global__ void __launch_bounds__(256) k_nl_advance(StateBuf b, uint32_t n, cons
                                                      uint32_t* __restrict__ err, long long* __restrict__ F,
                                                      size_t fstride) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool over = false;
     if (F && i < n) {  // the half-list pass accumulates into F: zero it here, not in a separate memset
         F[i] = 0;
         F[fstride + i] = 0;
@@ -135,40 +72,8 @@ __global__ void __launch_bounds__(256) k_nl_advance(StateBuf b, uint32_t n, cons
     }
     // translations since the rebuild, this tick's wrap included
     const bool half = ((flag[2] + (wrap ? 1u : 0u)) & 1u) != 0u;
-    if (i < n) {
-        double vx = b.vx[i], vy = b.vy[i], vz = b.vz[i];
-        if (lambda) {
-            double l = *lambda;
-            vx = xmul(vx, l);
-            vy = xmul(vy, l);
-            vz = xmul(vz, l);
-        }
-        vx = xadd(vx, xmul(b.ax[i], half_dt));
-        vy = xadd(vy, xmul(b.ay[i], half_dt));
-        vz = xadd(vz, xmul(b.az[i], half_dt));
-        double x = xadd(b.x[i], xmul(vx, dt)), y = xadd(b.y[i], xmul(vy, dt)), z = xadd(b.z[i], xmul(vz, dt));
-        if (wrap) {
-            x = xsub(rem_euclid(x, xmul(2.0, hx)), hx);
-            y = xsub(rem_euclid(y, xmul(2.0, hy)), hy);
-            z = xsub(rem_euclid(z, xmul(2.0, hz)), hz);
-        }
-        b.vx[i] = vx;
-        b.vy[i] = vy;
-        b.vz[i] = vz;
-        b.x[i] = x;
-        b.y[i] = y;
-        b.z[i] = z;
-        if (!(isfinite(x) && isfinite(y) && isfinite(z))) {
-            atomicOr(err, kErrNonFinite);
-            over = true;
-        } else {
-            float4 p = stage_one(g, b, home[i], i, x, y, z, half);
-            pos4[i] = p;
-            float4 r = ref[i];
-            float dx = p.x - r.x, dy = p.y - r.y, dz = p.z - r.z;
-            over = !(dx * dx + dy * dy + dz * dz <= lim2);
-        }
-    }
+    const bool over =
+        i < n && nl_advance_one(b, i, lambda, half_dt, dt, hx, hy, hz, wrap, g, home, pos4, ref, lim2, half, err);
     if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(flag, 1u);
 }
 
@@ -256,19 +161,6 @@ __global__ void __launch_bounds__(kNlBuildThreads) k_nl_build(GridGeom g, const 
     cnt[p] = m;
 }
 
-// The same lists from one warp per atom.  Lane k < 27 looks up neighbour
-// cell k (skipped or out of reach: no candidates), a warp scan of the 27
-// counts turns the candidates into one run t = 0 .. total - 1, and the lanes
-// take it 32 at a time, each finding its candidate's cell by a binary search
-// over the scan and its place in the list from the ballot: the candidates,
-// the test and the order are k_nl_build's, so the lists are the same words.
-// A small build is bound by the serial walk of one atom's ~150 candidates
-// (one thread per atom leaves most of the chip idle), a large one by
-// instructions, of which the searches and shuffles here take twice as many.
-// Microseconds per build, half list, warp / thread per atom: 11 / 78 at
-// 4,096 atoms, 25 / 78 at 32,768, 37 / 73 at 59,319, 72 / 83 at 125,000,
-// 142 / 100 at 262,144; full list (FP64): 13 / 99, 37 / 94, 54 / 86,
-// 107 / 104, 217 / 171.
 template <bool HALF>
 __global__ void __launch_bounds__(kNlBuildThreads) k_nl_build_warp(GridGeom g, const float4* __restrict__ pos4,
                                                                const uint32_t* __restrict__ home,
@@ -278,60 +170,7 @@ __global__ void __launch_bounds__(kNlBuildThreads) k_nl_build_warp(GridGeom g, c
                                                                const uint32_t* __restrict__ gate) {
     if (gated_off(gate)) return;
     const uint32_t p = (blockIdx.x * kNlBuildThreads + threadIdx.x) / 32u;
-    if (p >= n) return;  // whole warps leave
-    const uint32_t lane = threadIdx.x & 31u;
-    const float4 pi = pos4[p];
-    const uint32_t c = home[p];
-    uint32_t cx, cy, cz;
-    decode(g, c, cx, cy, cz);
-    float qx = pi.x, qy = pi.y, qz = pi.z;  // the atom in this lane's cell frame
-    uint32_t lo = 0, len = 0;
-    if (lane < 27) {
-        const int ox = (int)(lane % 3u) - 1, oy = (int)((lane / 3u) % 3u) - 1, oz = (int)(lane / 9u) - 1;
-        const uint32_t B = cell_at(g, cx, cy, cz, lane);
-        const float slack = 1e-3f;  // as k_nl_build
-        const float mx = fmaxf((ox > 0 ? g.cellf[0] - pi.x : (ox < 0 ? pi.x : 0.f)) - slack, 0.f);
-        const float my = fmaxf((oy > 0 ? g.cellf[1] - pi.y : (oy < 0 ? pi.y : 0.f)) - slack, 0.f);
-        const float mz = fmaxf((oz > 0 ? g.cellf[2] - pi.z : (oz < 0 ? pi.z : 0.f)) - slack, 0.f);
-        if (!(HALF && B < c) && dist2(mx, my, mz) < rl2) {
-            lo = HALF && B == c ? p + 1 : start[B];
-            len = start[B + 1] - lo;
-        }
-        float sx, sy, sz;
-        code_shift(g, lane, sx, sy, sz);
-        qx = fadd(pi.x, sx);
-        qy = fadd(pi.y, sy);
-        qz = fadd(pi.z, sz);
-    }
-    uint32_t end = len;  // inclusive scan: the candidates of cells 0 .. lane
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
-        if (lane >= (uint32_t)o) end += v;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, end, 31);
-    const uint32_t base = lo - (end - len);  // candidate t of this cell is atom base + t
-    uint32_t m = 0;
-    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
-        const uint32_t t = t0 + lane;
-        uint32_t k = 0;  // the first cell whose scan exceeds t
-#pragma unroll
-        for (uint32_t step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(0xffffffffu, end, k + step - 1) <= t) k += step;
-        const uint32_t q = __shfl_sync(0xffffffffu, base, k) + t;
-        const float x = __shfl_sync(0xffffffffu, qx, k), y = __shfl_sync(0xffffffffu, qy, k),
-                    z = __shfl_sync(0xffffffffu, qz, k);
-        bool hit = false;
-        if (t < total && (HALF || q != p)) {
-            const float4 pj = __ldg(pos4 + q);
-            hit = dist2(fsub(x, pj.x), fsub(y, pj.y), fsub(z, pj.z)) < rl2;
-        }
-        const uint32_t found = __ballot_sync(0xffffffffu, hit);
-        const uint32_t e = m + __popc(found & ((1u << lane) - 1u));
-        if (hit && e < (uint32_t)cap_nb) list[(size_t)e * stride + p] = q | (k << 27);
-        m += __popc(found);
-    }
-    if (lane == 0) cnt[p] = m;
+    if (p < n) nl_build_warp_one<HALF>(g, pos4, home, start, p, rl2, list, stride, cap_nb, cnt);  // whole warps
 }
 
 // The rebuild body's condition: the flag k_nl_advance raised.
@@ -351,22 +190,6 @@ __global__ void k_nl_end(uint32_t* flag, int wrap, unsigned long long* __restric
     } else if (wrap) {
         flag[2] ^= 1u;
     }
-}
-
-template <int BS>
-__device__ __forceinline__ unsigned long long block_sum_u(unsigned long long v, unsigned long long* sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    v = (threadIdx.x < BS / 32) ? sh[threadIdx.x] : 0ull;
-    if (wid == 0) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    }
-    __syncthreads();
-    return v;
 }
 
 // The half-list pass with one lane per atom and the far end's force kept in
@@ -1151,22 +974,6 @@ __global__ void k_nl_fix_to_double(const unsigned long long* __restrict__ v, dou
     *zero = 0.0;
 }
 
-template <int BS>
-__device__ __forceinline__ double block_sum_d(double v, double* sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    v = (threadIdx.x < BS / 32) ? sh[threadIdx.x] : 0.0;
-    if (wid == 0) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    }
-    __syncthreads();
-    return v;
-}
-
 // a = F 2^-32 (1/m) (as k_fix_to_acc), v += a dt/2 (as k_kick), and with
 // THERMO >= 1 the kinetic-energy partials of the new v with k_kinetic's block
 // mapping and operation order, so lambda is bit-identical to the unfused tick;
@@ -1186,21 +993,8 @@ __global__ void __launch_bounds__(kRedThreads) k_nl_finish(StateBuf b, const lon
     }
     double ks = 0.0, ss = 0.0;
     for (uint32_t i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
-        double im = b.inv_mass[i];
-        double ax = xmul(xmul(__ll2double_rn(F[i]), kFixInv), im);
-        double ay = xmul(xmul(__ll2double_rn(F[fstride + i]), kFixInv), im);
-        double az = xmul(xmul(__ll2double_rn(F[2 * fstride + i]), kFixInv), im);
-        b.ax[i] = ax;
-        b.ay[i] = ay;
-        b.az[i] = az;
-        double vx = xadd(b.vx[i], xmul(ax, half_dt));
-        double vy = xadd(b.vy[i], xmul(ay, half_dt));
-        double vz = xadd(b.vz[i], xmul(az, half_dt));
-        b.vx[i] = vx;
-        b.vy[i] = vy;
-        b.vz[i] = vz;
+        const double l2 = nl_finish_one(b, F, fstride, i, half_dt);
         if (THERMO) {
-            double l2 = xadd(xadd(xmul(vx, vx), xmul(vy, vy)), xmul(vz, vz));
             ks = xadd(ks, xmul(xmul(0.5, b.mass[i]), l2));
             if (THERMO == 2) ss = xadd(ss, xsqrt(l2));
         }
@@ -1328,6 +1122,13 @@ NlState* nl_of(gx_handle* h) {
     return static_cast<NlState*>(h->nl);
 }
 
+// Threads per atom of the list pass: as set or tuned, else by the size (the
+// far-end blocks, the stash and the bricks take one thread per atom).
+int nl_lanes(const NlState* s, uint32_t n) {
+    if (s->tpp > 0) return s->tpp;
+    return s->block > 0 ? 1 : nl_auto_lanes(n);
+}
+
 double skin_of(const gx_handle* h, const NlState* s) { return s->skin >= 0.0 ? s->skin : 0.1 * h->fs.rc; }
 
 }  // namespace
@@ -1339,6 +1140,7 @@ void nl_free(gx_handle* h) {
     cudaFree(s->cnt);
     cudaFree(s->ref);
     cudaFree(s->flag);
+    cudaFree(s->tick_sync);
     cells_free(s->cl);
     if (s->side) cudaStreamDestroy(s->side);
     delete s;
@@ -1528,9 +1330,9 @@ int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, in
                   psig + kNElem * kNElem, s->list, s->cap, s->cap_nb, s->cnt, vpart, h->dcount + 0);
         launch_sum_rows(h, vpart, (int)fb, h->dscal + 2);
     } else if (halfl) {
-        launch_nl_force<true>(h, s->tpp, g, s, n, L, energy);
+        launch_nl_force<true>(h, nl_lanes(s, n), g, s, n, L, energy);
     } else {
-        launch_nl_force<false>(h, s->tpp, g, s, n, L, energy);
+        launch_nl_force<false>(h, nl_lanes(s, n), g, s, n, L, energy);
     }
     prof_end(h, "force_nl");
     const bool spring = bonds_on(h);
@@ -1598,7 +1400,7 @@ int nl_tune_tpp(gx_handle* h, int reps) {
     int pick = 0;
     int launches = reps;
     for (int k = 0; k < ncand; ++k) {
-        int tpp = s->tpp;
+        int tpp = nl_lanes(s, n);
         if (stash) s->slots = k == 0 ? 8 : 16;
         else if (brick) s->brick = k;
         else if (s->half == 1) {
@@ -1689,13 +1491,13 @@ int nl_stats(gx_handle* h, uint64_t* entries, uint64_t* overflowed) {
 int nl_config(gx_handle* h, double* skin, int* tpp) {
     NlState* s = nl_of(h);
     if (skin) *skin = skin_of(h, s);
-    if (tpp) *tpp = s->tpp;
+    if (tpp) *tpp = nl_lanes(s, (uint32_t)h->n);
     return GX_OK;
 }
 
 int nl_shape(gx_handle* h, int* tpp, int* block, int* stash, int* brick) {
     const NlState* s = nl_of(h);
-    *tpp = s->tpp;
+    *tpp = nl_lanes(s, (uint32_t)h->n);
     *block = s->block;
     *stash = s->slots;
     *brick = s->brick == 0 ? 4 : 8;
@@ -1712,6 +1514,7 @@ int nl_set_block(gx_handle* h, int block) {
     if (block != 0 && block != 128 && block != 256)
         return set_err(h, GX_ERR_ARG, "list block must be 0 (far ends in global memory), 128 or 256");
     nl_of(h)->block = block;
+    nl_of(h)->shape_set = true;
     return GX_OK;
 }
 
@@ -1724,7 +1527,14 @@ int nl_set_slots(gx_handle* h, int slots) {
 int nl_set_tpp(gx_handle* h, int tpp) {
     if (tpp != 1 && tpp != 2 && tpp != 4 && tpp != 8) return set_err(h, GX_ERR_ARG, "threads per atom must be 1, 2, 4 or 8");
     nl_of(h)->tpp = tpp;
+    nl_of(h)->shape_set = true;
     return GX_OK;
+}
+
+void nl_clear_shape(gx_handle* h) {
+    NlState* s = nl_of(h);
+    s->tpp = s->block = 0;
+    s->shape_set = false;
 }
 
 int nl_set_skin(gx_handle* h, double skin) {
@@ -1732,6 +1542,10 @@ int nl_set_skin(gx_handle* h, double skin) {
     s->skin = skin;
     h->nl_valid = false;
     return GX_OK;
+}
+
+void nl_after_timeout(gx_handle* h) {
+    if (h->nl) static_cast<NlState*>(h->nl)->tick_sync_dirty = true;
 }
 
 bool nl_view(const gx_handle* h, NlView* v) {

@@ -1,0 +1,274 @@
+// gx_nlist.cuh -- the persistent neighbour list's state and the device
+// functions that the per-kernel tick (gx_nlist.cu) and the one-launch tick of
+// small universes (gx_nltick.cu) share.
+#pragma once
+
+#include "gx_pair_f32.cuh"
+
+namespace gx {
+
+// Device words of the one-launch ticks (gx_nltick.cu).
+struct TickSync {
+    uint32_t arrived, left;        // grid barrier arrivals, blocks that left the launch
+    uint32_t request[2];           // rebuild requested, by tick parity
+    unsigned long long acc[2][4];  // by tick parity: potential, pair count, bond energy
+    uint32_t tile[64];             // scan tile totals of a rebuild
+};
+
+struct NlState {
+    GridGeom lg{};            // list grid: cells >= r_c + skin
+    double skin = -1.0;       // < 0: default (0.1 r_c)
+    double skin_used = 0.0;
+    int half = -1;            // list kind built: 0 full, 1 half (variant 6)
+    int tpp = 0;              // threads per atom in the list pass (1, 2, 4, 8; 0: nl_auto_lanes)
+    bool shape_set = false;   // the work shape was set or tuned: it is the per-kernel tick's
+    int slots = 16;           // variant 7: stash slots per thread (8 or 16)
+    int brick = 1;            // variant 8: 0 = bricks of 4 cells (1024 staged atoms), 1 = 8 cells (2048)
+    int block = 0;            // variant 6, one lane per atom: 0 = far ends always global, 128 or 256 = far
+                              // ends inside a block of that many atoms summed in shared memory
+    int cap_nb = 0;           // list entries per atom
+    size_t cap = 0;           // atoms the buffers hold
+    uint32_t* list = nullptr; // entry e of atom p at list[e * cap + p]
+    uint32_t* cnt = nullptr;  // entries per atom (> cap_nb: overflowed)
+    float4* ref = nullptr;    // home-frame positions at the last rebuild
+    uint32_t* flag = nullptr; // [0] rebuild requested, [1] rebuilds done, [2] half-box translations since (mod 2),
+                              // [3] runs of a captured rebuild body
+    CellList cl;
+    // A captured tick puts the rebuild in the body of a conditional (IF)
+    // graph node, set from flag[0], so that a tick without a rebuild does
+    // not launch it at all.  The body is captured from a second stream.
+    cudaStream_t side = nullptr;
+    uint64_t body_kernels = 0;  // kernels in the body (counted when it runs)
+    uint32_t body_runs_seen = 0;
+    TickSync* tick_sync = nullptr;
+    bool tick_sync_dirty = false;  // a launch gave up: clear the words before the next one
+    int tick_blocks[2] = {0, 0};   // resident blocks of the one-launch tick, without / with records
+};
+
+// Universes up to this size run their ticks in one launch (gx_nltick.cu, where
+// both sides' times stand).
+constexpr size_t kTickMaxAtoms = 65536;
+// Ticks of one launch at most, so that a long call stays a queue of launches.
+constexpr int kTicksPerLaunch = 256;
+
+// Lanes per atom of the half-list pass where none were set: enough to fill
+// the chip, two while that shortens the tail of long lists, one above.
+// Microseconds per pass with 1 / 2 / 4 / 8 lanes: 29 / 21 / 14 / 10 at 4,096
+// atoms, 29 / 21 / 14 / 12 at 13,824, 29 / 23 / 19 / 21 at 32,768,
+// 35 / 27 / 29 / 29 at 59,319, 47 / 47 / 45 / 49 at 125,000,
+// 86 / 80 / 82 / 98 at 262,144, 145 / 143 / 154 / 191 at 512,000,
+// 256 / 256 / 289 / 379 at 1,000,000, 502 / 518 / 590 / 758 at 2,097,152.
+inline int nl_auto_lanes(uint32_t n) {
+    if (n > (1u << 20)) return 1;
+    return n <= 16384 ? 8 : (n <= 32768 ? 4 : 2);
+}
+
+constexpr uint32_t kIdxMask = (1u << 27) - 1u;  // a list word: 27-bit neighbour position, 5-bit neighbour-cell code
+
+// Offset of a coordinate from its home cell's origin in the frame of the
+// last rebuild (`shift` = the translation to undo, 0 or L/2), unwrapped
+// across the periodic boundary (the atom may have left its home cell).
+__device__ __forceinline__ double home_local(double v, double L, double c, uint32_t i, double shift) {
+    double u = xsub(rem_euclid(xadd(xadd(v, xmul(0.5, L)), shift), L), xmul((double)i, c));
+    if (u > 0.5 * L) u = xsub(u, L);
+    else if (u < -0.5 * L) u = xadd(u, L);
+    return u;
+}
+
+__device__ __forceinline__ float4 stage_one(const GridGeom& g, const StateBuf& b, uint32_t home, uint32_t i,
+                                            double x, double y, double z, bool half) {
+    uint32_t ix, iy, iz;
+    decode(g, home, ix, iy, iz);
+    return make_float4((float)home_local(x, g.L[0], g.cell[0], ix, half ? xmul(0.5, g.L[0]) : 0.0),
+                       (float)home_local(y, g.L[1], g.cell[1], iy, half ? xmul(0.5, g.L[1]) : 0.0),
+                       (float)home_local(z, g.L[2], g.cell[2], iz, half ? xmul(0.5, g.L[2]) : 0.0),
+                       __int_as_float((int)b.kind[i]));
+}
+
+// The Berendsen scale (thermostat.rs:58-71) of n atoms with kinetic energy K.
+__device__ __forceinline__ double berendsen_scale(double K, uint32_t n, double k, double target, double tau) {
+    if (n == 0) return 1.0;
+    const double t = xdiv(xmul(2.0 / 3.0, xdiv(K, (double)n)), k);
+    if (!(isfinite(t) && t > 0.0)) return 1.0;
+    return xsqrt(fmax(xadd(1.0, xmul(xdiv(1.0, tau), xsub(xdiv(target, t), 1.0))), 0.0));
+}
+
+// Neighbour-cell code: (ox+1) + 3(oy+1) + 9(oz+1); 13 is the home cell.
+__device__ __forceinline__ void code_shift(const GridGeom& g, uint32_t code, float& sx, float& sy, float& sz) {
+    int ox = (int)(code % 3u) - 1, oy = (int)((code / 3u) % 3u) - 1, oz = (int)(code / 9u) - 1;
+    sx = -(float)ox * g.cellf[0];
+    sy = -(float)oy * g.cellf[1];
+    sz = -(float)oz * g.cellf[2];
+}
+
+__device__ __forceinline__ uint32_t cell_at(const GridGeom& g, uint32_t cx, uint32_t cy, uint32_t cz, uint32_t code) {
+    int ox = (int)(code % 3u) - 1, oy = (int)((code / 3u) % 3u) - 1, oz = (int)(code / 9u) - 1;
+    return encode(g, wrap_add(cx, ox, g.n[0]), wrap_add(cy, oy, g.n[1]), wrap_add(cz, oz, g.n[2]));
+}
+
+// Kick (integrate.rs:38-45, with the pending scale of thermostat.rs:68-70),
+// drift (integrate.rs:62-66), wrap (boundary.rs:28-34) of one atom with the
+// same exact FP64 operations as k_kick/k_drift/k_wrap; then the home-frame
+// staging.  True when the atom moved too far since the last rebuild.
+__device__ __forceinline__ bool nl_advance_one(const StateBuf& b, uint32_t i, const double* lambda, double half_dt,
+                                               double dt, double hx, double hy, double hz, int wrap,
+                                               const GridGeom& g, const uint32_t* home, float4* pos4,
+                                               const float4* ref, float lim2, bool half, uint32_t* err) {
+    double vx = b.vx[i], vy = b.vy[i], vz = b.vz[i];
+    if (lambda) {
+        double l = *lambda;
+        vx = xmul(vx, l);
+        vy = xmul(vy, l);
+        vz = xmul(vz, l);
+    }
+    vx = xadd(vx, xmul(b.ax[i], half_dt));
+    vy = xadd(vy, xmul(b.ay[i], half_dt));
+    vz = xadd(vz, xmul(b.az[i], half_dt));
+    double x = xadd(b.x[i], xmul(vx, dt)), y = xadd(b.y[i], xmul(vy, dt)), z = xadd(b.z[i], xmul(vz, dt));
+    if (wrap) {
+        x = xsub(rem_euclid(x, xmul(2.0, hx)), hx);
+        y = xsub(rem_euclid(y, xmul(2.0, hy)), hy);
+        z = xsub(rem_euclid(z, xmul(2.0, hz)), hz);
+    }
+    b.vx[i] = vx;
+    b.vy[i] = vy;
+    b.vz[i] = vz;
+    b.x[i] = x;
+    b.y[i] = y;
+    b.z[i] = z;
+    if (!(isfinite(x) && isfinite(y) && isfinite(z))) {
+        atomicOr(err, kErrNonFinite);
+        return true;
+    }
+    const float4 p = stage_one(g, b, home[i], i, x, y, z, half);
+    pos4[i] = p;
+    const float4 r = ref[i];
+    const float dx = p.x - r.x, dy = p.y - r.y, dz = p.z - r.z;
+    return !(dx * dx + dy * dy + dz * dz <= lim2);
+}
+
+// The same lists from one warp per atom.  Lane k < 27 looks up neighbour
+// cell k (skipped or out of reach: no candidates), a warp scan of the 27
+// counts turns the candidates into one run t = 0 .. total - 1, and the lanes
+// take it 32 at a time, each finding its candidate's cell by a binary search
+// over the scan and its place in the list from the ballot: the candidates,
+// the test and the order are k_nl_build's, so the lists are the same words.
+// A small build is bound by the serial walk of one atom's ~150 candidates
+// (one thread per atom leaves most of the chip idle), a large one by
+// instructions, of which the searches and shuffles here take twice as many.
+// Microseconds per build, half list, warp / thread per atom: 11 / 78 at
+// 4,096 atoms, 25 / 78 at 32,768, 37 / 73 at 59,319, 72 / 83 at 125,000,
+// 142 / 100 at 262,144; full list (FP64): 13 / 99, 37 / 94, 54 / 86,
+// 107 / 104, 217 / 171.
+template <bool HALF>
+__device__ __forceinline__ void nl_build_warp_one(const GridGeom& g, const float4* pos4, const uint32_t* home,
+                                                  const uint32_t* start, uint32_t p, float rl2, uint32_t* list,
+                                                  size_t stride, int cap_nb, uint32_t* cnt) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const float4 pi = pos4[p];
+    const uint32_t c = home[p];
+    uint32_t cx, cy, cz;
+    decode(g, c, cx, cy, cz);
+    float qx = pi.x, qy = pi.y, qz = pi.z;  // the atom in this lane's cell frame
+    uint32_t lo = 0, len = 0;
+    if (lane < 27) {
+        const int ox = (int)(lane % 3u) - 1, oy = (int)((lane / 3u) % 3u) - 1, oz = (int)(lane / 9u) - 1;
+        const uint32_t B = cell_at(g, cx, cy, cz, lane);
+        const float slack = 1e-3f;  // as k_nl_build
+        const float mx = fmaxf((ox > 0 ? g.cellf[0] - pi.x : (ox < 0 ? pi.x : 0.f)) - slack, 0.f);
+        const float my = fmaxf((oy > 0 ? g.cellf[1] - pi.y : (oy < 0 ? pi.y : 0.f)) - slack, 0.f);
+        const float mz = fmaxf((oz > 0 ? g.cellf[2] - pi.z : (oz < 0 ? pi.z : 0.f)) - slack, 0.f);
+        if (!(HALF && B < c) && dist2(mx, my, mz) < rl2) {
+            lo = HALF && B == c ? p + 1 : start[B];
+            len = start[B + 1] - lo;
+        }
+        float sx, sy, sz;
+        code_shift(g, lane, sx, sy, sz);
+        qx = fadd(pi.x, sx);
+        qy = fadd(pi.y, sy);
+        qz = fadd(pi.z, sz);
+    }
+    uint32_t end = len;  // inclusive scan: the candidates of cells 0 .. lane
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= (uint32_t)o) end += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, end, 31);
+    const uint32_t base = lo - (end - len);  // candidate t of this cell is atom base + t
+    uint32_t m = 0;
+    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+        const uint32_t t = t0 + lane;
+        uint32_t k = 0;  // the first cell whose scan exceeds t
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xffffffffu, end, k + step - 1) <= t) k += step;
+        const uint32_t q = __shfl_sync(0xffffffffu, base, k) + t;
+        const float x = __shfl_sync(0xffffffffu, qx, k), y = __shfl_sync(0xffffffffu, qy, k),
+                    z = __shfl_sync(0xffffffffu, qz, k);
+        bool hit = false;
+        if (t < total && (HALF || q != p)) {
+            const float4 pj = pos4[q];
+            hit = dist2(fsub(x, pj.x), fsub(y, pj.y), fsub(z, pj.z)) < rl2;
+        }
+        const uint32_t found = __ballot_sync(0xffffffffu, hit);
+        const uint32_t e = m + __popc(found & ((1u << lane) - 1u));
+        if (hit && e < (uint32_t)cap_nb) list[(size_t)e * stride + p] = q | (k << 27);
+        m += __popc(found);
+    }
+    if (lane == 0) cnt[p] = m;
+}
+
+template <int BS>
+__device__ __forceinline__ unsigned long long block_sum_u(unsigned long long v, unsigned long long* sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) sh[wid] = v;
+    __syncthreads();
+    v = (threadIdx.x < BS / 32) ? sh[threadIdx.x] : 0ull;
+    if (wid == 0) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    }
+    __syncthreads();
+    return v;
+}
+
+template <int BS>
+__device__ __forceinline__ double block_sum_d(double v, double* sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (lane == 0) sh[wid] = v;
+    __syncthreads();
+    v = (threadIdx.x < BS / 32) ? sh[threadIdx.x] : 0.0;
+    if (wid == 0) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    }
+    __syncthreads();
+    return v;
+}
+
+// a = F 2^-32 (1/m) (as k_fix_to_acc) and v += a dt/2 (as k_kick) of one
+// atom; returns |v|^2.
+__device__ __forceinline__ double nl_finish_one(const StateBuf& b, const long long* F, size_t fstride, uint32_t i,
+                                                double half_dt) {
+    const double im = b.inv_mass[i];
+    const double ax = xmul(xmul(__ll2double_rn(F[i]), kFixInv), im);
+    const double ay = xmul(xmul(__ll2double_rn(F[fstride + i]), kFixInv), im);
+    const double az = xmul(xmul(__ll2double_rn(F[2 * fstride + i]), kFixInv), im);
+    b.ax[i] = ax;
+    b.ay[i] = ay;
+    b.az[i] = az;
+    const double vx = xadd(b.vx[i], xmul(ax, half_dt));
+    const double vy = xadd(b.vy[i], xmul(ay, half_dt));
+    const double vz = xadd(b.vz[i], xmul(az, half_dt));
+    b.vx[i] = vx;
+    b.vy[i] = vy;
+    b.vz[i] = vz;
+    return xadd(xadd(xmul(vx, vx), xmul(vy, vy)), xmul(vz, vz));
+}
+
+}  // namespace gx

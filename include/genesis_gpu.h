@@ -105,7 +105,8 @@ const char* gx_last_error(const gx_handle* h);
 const char* gx_status_string(int status);
 int gx_set_precision(gx_handle* h, int precision);
 /* Tuning knob of the mixed pair pass: 0 = automatic (6 where it applies,
- * else 4), 1 = one thread per atom over the canonical half shell,
+ * else 4; up to 65,536 atoms with no work shape set, the ticks of a gx_step
+ * call with use_graph run in one launch, the same bits), 1 = one thread per atom over the canonical half shell,
  * 2 = warp-tiled cell pairs with ballot compaction, 3 = thread per atom with
  * staged rows, 4 = thread per atom with per-thread candidate lists (all
  * four re-sort the atoms by the force grid every tick, as the reference
@@ -148,7 +149,8 @@ int gx_autotune(gx_handle* h, int reps, int* best, double* ms);
  * (default 0.1 r_c); 0 rebuilds every tick. */
 int gx_set_list_skin(gx_handle* h, double skin);
 /* Threads per atom of the variant-5/6 list pass: 1, 2, 4 or 8 lanes share
- * one atom's list (default 1; the autotuner picks the fastest).  Every
+ * one atom's list (default: by the atom count; the autotuner picks the
+ * fastest).  Every
  * choice gives the same bits (integer sums).  No counterpart in the
  * reference. */
 int gx_set_list_threads(gx_handle* h, int threads_per_atom);
@@ -227,8 +229,9 @@ int gx_stats(gx_handle* h, double* kinetic, double* speed_sum);
 /* nsteps ticks of the whole chain: kick, drift, [wrap], forces, kick,
  * [thermostat] -- Universe::tick with the force schedule
  * (src/universe/mod.rs:141-159, 356-369).  stats may be NULL, else it
- * receives nsteps entries.  Runs as one captured CUDA graph per tick
- * shape when use_graph != 0. */
+ * receives nsteps entries.  With use_graph != 0 the ticks replay captured
+ * CUDA graphs, or run in one cooperative launch for a small universe on the
+ * automatic pair pass (gx_set_kernel_variant). */
 int gx_step(gx_handle* h, int nsteps, gx_tick_stats* stats, int use_graph);
 
 /* ---- parity probes and lenses ---------------------------------------- */

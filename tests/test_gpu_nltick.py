@@ -1,0 +1,97 @@
+"""The one-launch ticks of small universes (automatic variant, captured or
+one-launch step) against the per-kernel ticks of the same handle settings
+(eager step): the same sums in the same order, so the same bits."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from genesis_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(cfg, u, ticks, bonds=None, skin=None, precision="mixed"):
+    from genesis_b200._lib import Handle
+    out = []
+    for graph in (True, False):
+        h = Handle(cfg, precision)
+        h.set_universe(u)
+        if bonds is not None:
+            h.set_bonds(bonds)
+        if skin is not None:
+            h.set_list_skin(skin)
+        l0 = h.launches
+        st = [h.step(k, stats=rec, graph=graph) for k, rec in ticks]
+        out.append((st, h.get_state(), h.list_rebuilds(), h.stats(), h.launches - l0))
+        h.close()
+    (sa, xa, ra, ka, la), (sb, xb, rb, kb, lb) = out
+    assert la < lb  # the two paths are not the same one
+    assert ra == rb
+    assert ka == kb
+    for a, b in zip(xa, xb):
+        assert np.array_equal(a, b)
+    for a, b in zip(sa, sb):
+        assert (a is None) == (b is None) and (a is None or np.array_equal(a, b))
+    return ra
+
+
+@pytest.mark.parametrize("n_side,coul,target", [(8, False, 0.0), (9, True, 40.0), (16, False, 0.0), (16, True, 40.0),
+                                                (25, True, 0.0), (40, True, 300.0)])
+def test_one_launch_ticks_match_the_per_kernel_ticks(gpu, n_side, coul, target):
+    wl = W.Workload("tick check", n_side=n_side, temperature=200.0, steps=10, electrostatics=coul,
+                    thermostat=target > 0.0, thermostat_temperature=target if target > 0.0 else 300.0)
+    rebuilds = _pair(wl.config(), wl.generate(), [(1, True), (2, False), (7, True), (1, False), (9, True)])
+    assert rebuilds >= 2
+
+
+def test_one_launch_gravity_and_no_walls(gpu):
+    wl = W.Workload("tick check", n_side=11, temperature=100.0, steps=10, electrostatics=True)
+    cfg = wl.config()
+    cfg.enable_gravity, cfg.gravity_constant = True, 1e-3
+    _pair(cfg, wl.generate(), [(6, True), (3, False)])
+    cfg.enable_boundaries = False
+    _pair(cfg, wl.generate(), [(6, True), (3, False)])
+
+
+def test_one_launch_spring_and_zero_skin(gpu):
+    wl = W.C2.scaled(10)
+    cfg, u = wl.config(), wl.generate()
+    i = np.arange(0, u.n - 1, 2, dtype=np.uint32)
+    bonds = np.stack([i, i + 1], 1)  # neighbours along the lattice's fastest axis
+    _pair(cfg, u, [(5, True), (4, False)], bonds=bonds)
+    assert _pair(cfg, u, [(3, True), (3, False)], skin=0.0) >= 5
+
+
+def test_one_launch_sparse_box_and_overflowing_clump(gpu):
+    # more list cells than one scan tile, and atoms whose lists overflow
+    wl = W.Workload("tick check", n_side=10, temperature=20.0, steps=10)
+    cfg, u = wl.config(), wl.generate()
+    L = 110.0
+    cfg.size = (L, L, L)
+    u.box[:] = L
+    rng = np.random.default_rng(3)
+    u.pos[:300] = rng.normal(scale=2.5, size=(300, 3))
+    u.pos[300:] = rng.uniform(-0.5 * L, 0.5 * L, size=(700, 3))
+    u.vel[:] *= 0.01
+    _pair(cfg, u, [(3, True), (1, False)])
+
+
+def test_one_launch_tick_reports_and_recovers_from_a_non_finite_velocity(gpu):
+    from genesis_b200._lib import GxError, Handle
+    wl = W.C1.scaled(9)
+    cfg, u = wl.config(), wl.generate()
+    bad = u.vel.copy()
+    bad[5, 1] = np.nan
+    with Handle(cfg, "mixed") as h:
+        h.set_universe(u)
+        h.step(2, graph=True)
+        h.set_dynamic(u.pos, bad, np.zeros_like(u.pos))
+        with pytest.raises(GxError):
+            h.step(2, graph=True)
+        h.set_dynamic(u.pos, u.vel, np.zeros_like(u.pos))
+        st = h.step(3, graph=True)
+    with Handle(cfg, "mixed") as h:
+        h.set_universe(u)
+        want = h.step(3, graph=True)
+    assert np.array_equal(st["potential"], want["potential"])
