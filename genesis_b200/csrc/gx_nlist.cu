@@ -48,6 +48,7 @@ namespace {
 constexpr int kNlThreads = 128;
 constexpr int kNlBuildThreads = 128;
 constexpr int kNlBuildUnroll = 4;
+constexpr double kListRoomBytes = 512.0 * (1 << 20);  // of one universe's list, beyond what twice the mean takes
 constexpr uint32_t kNlBuildWarpMax = 131072;  // atoms up to which a list is built by one warp per atom (k_nl_build_warp)
 constexpr int kRedThreads = 256;
 
@@ -1172,9 +1173,15 @@ int nl_prepare(gx_handle* h, bool* stale) {
     const double vol = h->p.box[0] * h->p.box[1] * h->p.box[2];
     const double rl = h->fs.rc + skin;
     const double expect = (double)h->n / vol * (4.0 / 3.0) * 3.14159265358979 * rl * rl * rl;
-    int cap_nb = (int)std::ceil(2.0 * expect) + 32;
+    // Twice the mean, and up to four times it within 512 MB: the core of a
+    // condensed state is that much denser, and one overflowed atom, scanning
+    // its 27 cells, holds a whole pass up (13,824 atoms after 4,000 ticks of
+    // condensation: 2 of them overflowed, 108 us a tick; none, 51 us).
+    const double room = kListRoomBytes / (sizeof(uint32_t) * (double)h->cap);
+    int cap_nb = (int)std::ceil(std::max(2.0 * expect + 32.0, std::min(4.0 * expect, room)));
     cap_nb = (cap_nb + 7) & ~7;
     if (cap_nb > 1024) cap_nb = 1024;
+    s->expect = expect;
     if (!s->flag) {
         GX_CUDA(h, cudaMalloc(&s->flag, 4 * sizeof(uint32_t)));
         GX_CUDA(h, cudaMemsetAsync(s->flag, 0, 4 * sizeof(uint32_t), h->stream));

@@ -27,6 +27,7 @@ struct NlState {
     int block = 0;            // variant 6, one lane per atom: 0 = far ends always global, 128 or 256 = far
                               // ends inside a block of that many atoms summed in shared memory
     int cap_nb = 0;           // list entries per atom
+    double expect = 0.0;      // neighbours within r_c + skin at the mean density
     size_t cap = 0;           // atoms the buffers hold
     uint32_t* list = nullptr; // entry e of atom p at list[e * cap + p]
     uint32_t* cnt = nullptr;  // entries per atom (> cap_nb: overflowed)
@@ -45,22 +46,27 @@ struct NlState {
     int tick_blocks[2] = {0, 0};   // resident blocks of the one-launch tick, without / with records
 };
 
-// Universes up to this size run their ticks in one launch (gx_nltick.cu, where
-// both sides' times stand).
+// Universes up to this many atoms and expected half-list entries run their
+// ticks in one launch (gx_nltick.cu, where both sides' times stand).
 constexpr size_t kTickMaxAtoms = 65536;
+constexpr double kTickMaxEntries = 1.7e6;
 // Ticks of one launch at most, so that a long call stays a queue of launches.
 constexpr int kTicksPerLaunch = 256;
 
 // Lanes per atom of the half-list pass where none were set: enough to fill
-// the chip, two while that shortens the tail of long lists, one above.
-// Microseconds per pass with 1 / 2 / 4 / 8 lanes: 29 / 21 / 14 / 10 at 4,096
-// atoms, 29 / 21 / 14 / 12 at 13,824, 29 / 23 / 19 / 21 at 32,768,
-// 35 / 27 / 29 / 29 at 59,319, 47 / 47 / 45 / 49 at 125,000,
-// 86 / 80 / 82 / 98 at 262,144, 145 / 143 / 154 / 191 at 512,000,
-// 256 / 256 / 289 / 379 at 1,000,000, 502 / 518 / 590 / 758 at 2,097,152.
+// the chip and to share the long lists of a condensed state, one where the
+// gathers of a homogeneous one set the time.  Microseconds per pass with
+// 1 / 2 / 4 / 8 lanes on the lattice: 29 / 21 / 14 / 10 at 4,096 atoms,
+// 29 / 23 / 19 / 21 at 32,768, 35 / 27 / 29 / 29 at 59,319, 47 / 47 / 45 / 49
+// at 125,000, 86 / 80 / 82 / 98 at 262,144, 145 / 143 / 154 / 191 at 512,000,
+// 256 / 256 / 289 / 379 at 1,000,000, 502 / 518 / 590 / 758 at 2,097,152; per
+// tick after 1,000 ticks of condensation with charges and gravity:
+// 96 / 73 / 60 / 59 at 32,768, 107 / 89 / 82 / 77 at 59,319,
+// 263 / 234 / 223 / 232 at 262,144.
 inline int nl_auto_lanes(uint32_t n) {
-    if (n > (1u << 20)) return 1;
-    return n <= 16384 ? 8 : (n <= 32768 ? 4 : 2);
+    if (n <= 98304) return 8;
+    if (n <= 327680) return 4;
+    return n <= (1u << 20) ? 2 : 1;
 }
 
 constexpr uint32_t kIdxMask = (1u << 27) - 1u;  // a list word: 27-bit neighbour position, 5-bit neighbour-cell code

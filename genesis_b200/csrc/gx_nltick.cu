@@ -29,10 +29,11 @@
 // A phase is bound by the latency of its few dependent accesses and the
 // barrier, not by bytes or operations.  Microseconds per recorded NVE tick,
 // rebuilds included, here / as a graph of kernels: 16 / 32 at 512 atoms,
-// 20 / 35 at 4,096, 26 / 40 at 13,824, 43 / 48 at 32,768, 56 / 62 at 59,319;
-// from about 90,000 atoms the kernels win (77 / 77, 98 / 93 at 125,000,
-// 202 / 143 at 262,144): their pair pass keeps more warps resident than the
-// one kernel that holds every phase.
+// 19 / 33 at 4,096, 25 / 40 at 13,824, 41 / 48 at 32,768, 54 / 63 at 59,319;
+// from about 1.7 M list entries the kernels win (73 / 73 at 2.6 M, 98 / 93 at
+// 3.4 M, 202 / 143 at 7.1 M): their pair pass keeps more warps resident than
+// the one kernel that holds every phase.  Four blocks per SM (64 registers):
+// 54 us at 59,319 atoms, against 55 with three and 57 with five.
 #include <algorithm>
 
 #include "gx_law64.cuh"
@@ -170,7 +171,7 @@ __device__ __forceinline__ void take_record(const TickArgs& a, int tick, double 
 }
 
 template <bool REC>
-__global__ void __launch_bounds__(kTickThreads) k_nl_ticks(const __grid_constant__ TickArgs a) {
+__global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_constant__ TickArgs a) {
     __shared__ PairF st[kMaxKinds * kMaxKinds];
     __shared__ float4 s_shift[27];
     __shared__ double sh[kTickThreads / 32];
@@ -435,7 +436,8 @@ bool nl_ticks_eligible(gx_handle* h) {
     if (h->n == 0 || h->n > kTickMaxAtoms || h->precision != GX_MIXED || h->kernel_variant != 0) return false;
     if (h->p.enable_collisions || h->prof_on || h->pass_timing) return false;
     const NlState* s = static_cast<const NlState*>(h->nl);
-    return s && !s->shape_set && s->half == 1 && s->lg.ncell < kTickTile * kTickMaxTiles;
+    if (!s || 0.5 * s->expect * (double)h->n > kTickMaxEntries) return false;
+    return !s->shape_set && s->half == 1 && s->lg.ncell < kTickTile * kTickMaxTiles;
 }
 
 // nticks ticks with the records (may be null) at rec[0 .. nticks).
