@@ -13,6 +13,7 @@
 // canonical half shell.  Distance tests use the reference's FP64 operation
 // order, so the pair multiset (including the repeats the reference produces
 // on axes with exactly two cells) is identical to the reference's.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -27,6 +28,7 @@ struct AuxSet {
     uint32_t* key;  // aux-grid cell of each sorted aux atom
     const uint32_t* start;
     uint32_t m;
+    float4* loc = nullptr;  // offset from the cell's origin; w: element, cell along x << 8 (for k_gr)
 };
 
 }  // namespace gx
@@ -39,6 +41,7 @@ struct AuxPool {
     double* xyz = nullptr;  // 6 * cap: staging xyz + sorted xyz
     uint8_t* elem = nullptr;  // 2 * cap
     uint32_t* u32 = nullptr;  // 6 * cap: slot, slot_sorted, key, key_sorted, perm, sel
+    float4* loc = nullptr;    // cap
     size_t cap = 0;
     CellList cl;
     uint32_t* parent = nullptr;
@@ -52,7 +55,7 @@ struct AuxPool {
 
 void pool_release(AuxPool* P) {
     if (!P) return;
-    void* ps[] = {P->xyz, P->elem, P->u32, P->parent, P->cnt, P->counts};
+    void* ps[] = {P->xyz, P->elem, P->u32, P->loc, P->parent, P->cnt, P->counts};
     for (void* q : ps) cudaFree(q);
     cells_free(P->cl);
     delete P;
@@ -71,10 +74,12 @@ int ensure_pool(gx_handle* h, AuxPool& P, size_t m, size_t natoms) {
         cudaFree(P.xyz);
         cudaFree(P.elem);
         cudaFree(P.u32);
+        cudaFree(P.loc);
         size_t cap = m < 1024 ? 1024 : m;
         GX_CUDA(h, cudaMalloc(&P.xyz, 6 * cap * sizeof(double)));
         GX_CUDA(h, cudaMalloc(&P.elem, 2 * cap));
         GX_CUDA(h, cudaMalloc(&P.u32, 6 * cap * sizeof(uint32_t)));
+        GX_CUDA(h, cudaMalloc(&P.loc, cap * sizeof(float4)));
         P.cap = cap;
     }
     if (natoms > P.ucap) {
@@ -111,16 +116,27 @@ __global__ void k_select(GridGeom g, StateBuf b, const uint32_t* __restrict__ se
 
 __global__ void k_aux_gather(const uint32_t* __restrict__ perm, uint32_t m, const double* tx, const double* ty,
                              const double* tz, const uint8_t* te, const uint32_t* tslot, const uint32_t* key,
-                             AuxSet a) {
+                             AuxSet a, GridGeom g) {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= m) return;
     uint32_t q = perm[p];
-    a.x[p] = tx[q];
-    a.y[p] = ty[q];
-    a.z[p] = tz[q];
+    const double x = tx[q], y = ty[q], z = tz[q];
+    const uint32_t c = key[q];
+    a.x[p] = x;
+    a.y[p] = y;
+    a.z[p] = z;
     a.elem[p] = te[q];
     a.slot[p] = tslot[q];
-    a.key[p] = key[q];
+    a.key[p] = c;
+    if (a.loc) {
+        uint32_t cx, cy, cz;
+        decode(g, c, cx, cy, cz);
+        // far outside the box the FP64 differences round too: no offset, so that every pair is taken exactly
+        const bool near = fabs(x) <= 1024.0 * g.L[0] && fabs(y) <= 1024.0 * g.L[1] && fabs(z) <= 1024.0 * g.L[2];
+        a.loc[p] = make_float4(near ? (float)cell_local(x, g.L[0], g.cell[0], cx) : __int_as_float(0x7fffffff),
+                               (float)cell_local(y, g.L[1], g.cell[1], cy),
+                               (float)cell_local(z, g.L[2], g.cell[2], cz), __int_as_float((int)te[q] | (int)(cx << 8)));
+    }
 }
 
 // The bond grid for the observation: every atom's cell, counted as it is
@@ -256,6 +272,158 @@ struct GrVisit {
             atomicAdd(&counts[bi], 1ull);
     }
 };
+
+// g(r) where the reference's grid (cells >= r_max) has at least 3 cells per
+// axis.  The atoms are binned on cells of r_max / sub (at least 2 sub + 1 per
+// axis): finer cells leave fewer candidates beyond r_max.  A warp owns TI
+// consecutive sorted atoms; for each run of them in one cell it takes the
+// candidates of the half space around the cell, row by row (cells along x are
+// one range of sorted atoms, two where the row wraps), as one run of 32 at a
+// time (a scan of the rows' counts, then a binary search per candidate, so
+// that crowded and nearly empty cells cost the same per candidate), and tests
+// each against the run's atoms.  Where the general pass needs an FP64
+// distance, root and division per pair, here the bin coordinate d / dr is
+// taken in FP32 from offsets in the cells' frames.  Its error is below
+// `slack`: two offsets (2 cell), the cell edge and the shift (2 sub cell), the
+// shifted offset and the difference (2 (sub + 1) cell) round by 2^-24 of
+// these per axis, 6.93 (sub + 1) cell 2^-24 in d, and the root and product by
+// 2^-20 of the bin number; a pair within `slack` of a bin's edge (r_max is
+// one) goes through the exact arithmetic of k_pairs and GrVisit, so every
+// count is the same.  A pair within r_max <= L/3 has its minimum image in the
+// cell offset that finds it, and its other images lie beyond r_max.
+// Milliseconds, 256 bins to 17.25, this / one FP64 thread per atom: 0.018 /
+// 0.38 for a sample of 8,192 of 59,319 atoms, 1.1 / 4.0 for all of 262,144
+// (134 M pairs in range).  Instruction issue bounds it: about 30 warp
+// instructions per 32 candidate pairs, of which a third lie in range.
+constexpr int kGrThreads = 128;
+constexpr unsigned kGrBlocks = 148 * 12;
+constexpr size_t kGrWideAtoms = 65536;  // atoms from which a warp takes 8 at a time, 2 below
+constexpr int kGrMaxSub = 3;            // 25 rows of the half space: one per lane
+
+template <int TI, bool BETWEEN>
+__global__ void __launch_bounds__(kGrThreads, 8) k_gr(GridGeom g, int sub, AuxSet a, double box0, double box1,
+                                                   double box2, double cd2, float reach2, float inv_dr, float slack,
+                                                   GrVisit visit) {
+    constexpr int kGroup = TI < 4 ? TI : 4;
+    visit.begin();  // clears the block's histogram and synchronises
+    unsigned* hist = visit.local();
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warps = gridDim.x * (kGrThreads / 32), warp = blockIdx.x * (kGrThreads / 32) + threadIdx.x / 32;
+    const float inner = 0.5f - slack, beyond = (float)visit.nbins + slack;
+    // this lane's row of the half space: lane 0 the own row, then z = 0, then z > 0
+    const int rows = sub + sub * (2 * sub + 1);
+    int oy = 0, oz = 0;
+    if (lane > 0 && (int)lane <= sub) {
+        oy = (int)lane;
+    } else if ((int)lane > sub) {
+        const int r = (int)lane - 1 - sub;
+        oz = 1 + r / (2 * sub + 1);
+        oy = r % (2 * sub + 1) - sub;
+    }
+    const float my = (float)max(abs(oy) - 1, 0) * g.cellf[1], mz = (float)max(oz - 1, 0) * g.cellf[2];
+    const float left = reach2 - my * my - mz * mz;  // what the row leaves for x
+    const int kx = (int)lane <= rows && left > 0.f ? min(sub, (int)(sqrtf(left) / g.cellf[0]) + 1) : -1;
+    const float sy = (float)oy * g.cellf[1], sz = (float)oz * g.cellf[2];
+    const int nx = (int)g.n[0];
+    for (uint32_t i0 = warp * TI; i0 < a.m; i0 += warps * TI) {
+        const uint32_t iend = min(i0 + TI, a.m);
+        for (uint32_t r0 = i0; r0 < iend;) {
+            const uint32_t c = a.key[r0];
+            const uint32_t r1 = min(iend, a.start[c + 1]);  // this run: atoms r0 .. r1 - 1 of cell c
+            const int run = (int)(r1 - r0);
+            float4 pi[TI];
+#pragma unroll
+            for (int k = 0; k < TI; ++k) pi[k] = a.loc[min(r0 + k, r1 - 1)];
+            uint32_t cx, cy, cz;
+            decode(g, c, cx, cy, cz);
+            const int x = (int)cx;
+            const uint32_t row = encode(g, 0, wrap_add(cy, oy, g.n[1]), wrap_add(cz, oz, g.n[2]));
+            for (int part = 0; part < 2; ++part) {  // the row itself, then what wraps around x
+                uint32_t lo = 0, len = 0;
+                int xo = -x;  // x offset of a candidate: its cell + xo
+                if (kx >= 0) {
+                    int xa = lane == 0 ? x : max(x - kx, 0), xb = min(x + kx, nx - 1);
+                    if (part == 1) {
+                        if (x + kx >= nx) {
+                            xa = 0;
+                            xb = x + kx - nx;
+                            xo += nx;
+                        } else if (lane > 0 && x - kx < 0) {
+                            xa = nx + x - kx;
+                            xb = nx - 1;
+                            xo -= nx;
+                        } else {
+                            xb = xa - 1;
+                        }
+                    }
+                    if (xb >= xa) {
+                        lo = part == 0 && lane == 0 ? r0 + 1 : a.start[row + xa];  // own cell: after r0
+                        len = a.start[row + xb + 1] - lo;
+                    }
+                }
+                uint32_t end = len;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
+                    if (lane >= (uint32_t)o) end += v;
+                }
+                const uint32_t total = __shfl_sync(0xffffffffu, end, 31);
+                const uint32_t base = lo - (end - len);
+                for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+                    const uint32_t t = t0 + lane;
+                    uint32_t k = 0;  // the first row whose scan exceeds t
+#pragma unroll
+                    for (uint32_t step = 16; step > 0; step >>= 1)
+                        if (__shfl_sync(0xffffffffu, end, k + step - 1) <= t) k += step;
+                    const uint32_t j = __shfl_sync(0xffffffffu, base, k) + t;
+                    const int jx = __shfl_sync(0xffffffffu, xo, k);
+                    const float hy = __shfl_sync(0xffffffffu, sy, k), hz = __shfl_sync(0xffffffffu, sz, k);
+                    if (t >= total) continue;
+                    const float4 pj = a.loc[j];
+                    const int w = __float_as_int(pj.w);  // the element, then the cell along x
+                    const float qx = pj.x + (float)((w >> 8) + jx) * g.cellf[0], qy = pj.y + hy, qz = pj.z + hz;
+                    const int last = (int)((k == 0 && part == 0 ? min(j, r1) : r1) - r0);  // own cell: atoms before j
+#pragma unroll
+                    for (int v = 0; v < TI; v += kGroup) {
+                        if (v >= run) break;
+                        uint32_t edge = 0;  // the pairs of this group to take exactly
+#pragma unroll
+                        for (int u = v; u < v + kGroup; ++u) {
+                            const float dx = pi[u].x - qx, dy = pi[u].y - qy, dz = pi[u].z - qz;
+                            const float d2 = dx * dx + dy * dy + dz * dz;
+                            const float f = d2 * rsqrtf(d2) * inv_dr;
+                            // the nearest integer to f - 1/2 from the sum's low bits: the bin, and how far f is into it
+                            const float up = (f - 0.5f) + 12582912.f;
+                            const uint32_t bin = __float_as_uint(up) - 0x4b400000u;
+                            const bool inside = fabsf((f - (up - 12582912.f)) - 0.5f) < inner;
+                            bool valid = u < last;
+                            if (BETWEEN) {
+                                const int ei = __float_as_int(pi[u].w) & 255, ej = w & 255;
+                                valid = valid && ((ei == visit.ta && ej == visit.tb) || (ei == visit.tb && ej == visit.ta));
+                            }
+                            if (valid && inside && bin < visit.nbins) atomicAdd(&hist[bin], 1u);
+                            // a zero or non-finite f is not inside
+                            edge |= valid && !inside && !(f > beyond) ? 1u << u : 0u;
+                        }
+                        for (; edge; edge &= edge - 1u) {
+                            const uint32_t i = r0 + (uint32_t)__ffs(edge) - 1u;
+                            const double ex = near_image1(xsub(a.x[i], a.x[j]), box0);
+                            const double ey = near_image1(xsub(a.y[i], a.y[j]), box1);
+                            const double ez = near_image1(xsub(a.z[i], a.z[j]), box2);
+                            const double e2 = xadd(xadd(xmul(ex, ex), xmul(ey, ey)), xmul(ez, ez));
+                            if (e2 >= cd2) continue;
+                            const double d = xsqrt(e2);
+                            if (d <= kEpsF64) continue;
+                            visit(a, i, j, d);
+                        }
+                    }
+                }
+            }
+            r0 = r1;
+        }
+    }
+    visit.end();
+}
 
 __device__ __forceinline__ uint32_t uf_root(uint32_t* par, uint32_t x) {
     uint32_t cur = par[x];
@@ -607,11 +775,17 @@ __global__ void k_iota(uint32_t* p, uint32_t n) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = i;
 }
+// The size of every component.  A condensed state has one component of most
+// atoms, so a warp first adds up its atoms of the same root: one atomic per
+// root and warp instead of one per atom on the same word (262,144 atoms:
+// 8 us instead of 163).
 __global__ void k_fof_finish(uint32_t* par, uint32_t* size, uint32_t n) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t live = __ballot_sync(0xffffffffu, i < n);
     if (i >= n) return;
-    uint32_t r = uf_root(par, i);
-    atomicAdd(&size[r], 1u);
+    const uint32_t r = uf_root(par, i);
+    const uint32_t same = __match_any_sync(live, r);
+    if ((int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&size[r], (uint32_t)__popc(same));
 }
 __global__ void k_fof_labels(uint32_t* par, uint32_t n) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -635,7 +809,9 @@ __global__ void k_cell_assign(GridGeom g, StateBuf b, uint32_t n, uint32_t* out)
 
 // Builds the aux grid over m selected atoms (sel = sorted positions, or
 // nullptr for all atoms).
-int build_aux(gx_handle* h, AuxPool& P, const GridGeom& g, const uint32_t* sel, uint32_t m, AuxSet& a) {
+int build_aux(gx_handle* h, AuxPool& P, const GridGeom& g, const uint32_t* sel, uint32_t m, AuxSet& a,
+              bool local = false) {
+    a.loc = local ? P.loc : nullptr;
     size_t cap = P.cap;
     double* tx = P.xyz;
     double* ty = tx + cap;
@@ -654,7 +830,7 @@ int build_aux(gx_handle* h, AuxPool& P, const GridGeom& g, const uint32_t* sel, 
     if (m) GX_LAUNCH(h, k_select, nblk(m, 256), 256, g, h->buf[h->cur], sel, m, tx, ty, tz, te, tslot, key);
     int rc = counting_sort(h, P.cl, g.ncell, key, m, perm);
     if (rc) return rc;
-    if (m) GX_LAUNCH(h, k_aux_gather, nblk(m, 256), 256, perm, m, tx, ty, tz, te, tslot, key, a);
+    if (m) GX_LAUNCH(h, k_aux_gather, nblk(m, 256), 256, perm, m, tx, ty, tz, te, tslot, key, a, g);
     a.start = P.cl.start;
     return GX_OK;
 }
@@ -700,12 +876,45 @@ int gr_common(gx_handle* h, int ta, int tb, double r_max_in, size_t nbins_in, si
     GridGeom g = make_grid(box, r_max, &ok);
     if (!ok) return set_err(h, GX_ERR_UNSUPPORTED, "g(r) grid too large");
     AuxSet a;
-    if ((rc = build_aux(h, P, g, sel, (uint32_t)m, a))) return rc;
+    bool fast = nbins <= kGrLocalBins && g.n[0] >= 3 && g.n[1] >= 3 && g.n[2] >= 3 && g.n[0] < (1u << 23);
+    int sub = 1;
+    if (fast) {
+        // The finest cells that still hold four atoms.  Microseconds with
+        // cells of r_max / 1, / 2, / 3: 123 / 85 / 61 for 8,000 atoms (296 in
+        // a cell of r_max), 572 / 254 / 190 for 29,791 (238), 1790 / 1262 /
+        // 1125 for 262,144 (262); samples of 8,192 atoms: 24 / 18 / 19 (38 in
+        // a cell), 14.3 / 14.8 / 16.7 (8), 13.5 / 14.2 / 14.8 (1).
+        const double per_cell = (double)m / ((double)g.n[0] * g.n[1] * g.n[2]);
+        for (int s = kGrMaxSub; s > 1; --s) {
+            int ok2 = 0;
+            const GridGeom f = make_grid(box, r_max / s, &ok2);
+            const uint32_t least = 2 * (uint32_t)s + 1;
+            if (!ok2 || f.n[0] < least || f.n[1] < least || f.n[2] < least) continue;
+            if (per_cell < 4.0 * s * s * s) continue;
+            sub = s;
+            g = f;
+            break;
+        }
+    }
+    if ((rc = build_aux(h, P, g, sel, (uint32_t)m, a, fast))) return rc;
     GX_CUDA(h, cudaMemsetAsync(P.counts, 0, nbins * sizeof(uint64_t), h->stream));
     GX_CUDA(h, cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream));
     GrVisit v{r_max, dr, (unsigned long long*)P.counts, (uint32_t)nbins, ta, tb, h->derr};
     prof_begin(h, "gr_pairs");
-    if (m) GX_LAUNCH(h, k_pairs, nblk(m, 128), 128, g, a, box[0], box[1], box[2], r_max * r_max, v);
+    if (m && fast) {
+        const double cell = std::fmax(std::fmax(g.cell[0], g.cell[1]), g.cell[2]);
+        // the bound on the error of the FP32 bin coordinate (k_gr)
+        const float slack = (float)(10.0 * (sub + 1) * cell * std::ldexp(1.0, -24) / dr + (double)nbins * std::ldexp(1.0, -20));
+        const float reach2 = (float)(r_max * r_max * (1.0 + 1e-4));
+        const bool wide = m >= kGrWideAtoms;
+        const size_t warps = wide ? (m + 7) / 8 : (m + 1) / 2;
+        const unsigned grid = (unsigned)std::min<size_t>(nblk(warps, kGrThreads / 32), kGrBlocks);
+        auto kern = ta >= 0 ? (wide ? k_gr<8, true> : k_gr<2, true>) : (wide ? k_gr<8, false> : k_gr<2, false>);
+        GX_LAUNCH(h, kern, grid, kGrThreads, g, sub, a, box[0], box[1], box[2], r_max * r_max, reach2,
+                  (float)(1.0 / dr), slack, v);
+    } else if (m) {
+        GX_LAUNCH(h, k_pairs, nblk(m, 128), 128, g, a, box[0], box[1], box[2], r_max * r_max, v);
+    }
     prof_end(h, "gr_pairs");
     uint32_t e = 0;
     GX_CUDA(h, cudaMemcpyAsync(counts, P.counts, nbins * sizeof(uint64_t), cudaMemcpyDeviceToHost, h->stream));
