@@ -7,14 +7,13 @@
 // Gaussian-kernel pair distribution averaged over sampled ticks.
 //
 // Forward.  The trajectory is recomputed in slot order (atoms never move
-// between arrays; a per-tick counting sort gives the cell list as an index),
-// in FP64 with the reference's per-pair arithmetic (pair_f64).  On a handle
-// of mixed precision the forward is the mixed method instead: the FP32 pair
-// law of the list passes (pair_f32) on the FP64 minimum-image displacement
-// rounded to FP32, the per-atom force summed in 2^-32 fixed point, and FP64
-// positions, velocities and observables; the backward below stays FP64,
-// linearised on that trajectory.  A checkpoint of (x, v, a) is kept every K
-// ticks.
+// between arrays) in FP64 with the reference's per-pair arithmetic
+// (pair_f64).  On a handle of mixed precision the forward is the mixed method
+// instead: the FP32 pair law of the list passes (pair_f32) on the FP64
+// minimum-image displacement rounded to FP32, the per-atom force summed in
+// 2^-32 fixed point, and FP64 positions, velocities and observables; the
+// backward below stays FP64, linearised on that trajectory.  A checkpoint of
+// (x, v, a) is kept every K ticks.
 //
 // Backward.  Per segment: restore the checkpoint, recompute the segment's
 // positions, then walk the ticks backwards.  With adjoints (Lx, Lv, La) of
@@ -26,29 +25,49 @@
 // and (da/dx)^T W is the pairwise Hessian-vector product: with
 // a_i = sum_j f(d_ij) n_ij / m_i, u = W_i/m_i - W_j/m_j and rho = n.u, the
 // pair adds  f'(d) rho n + (f/d) (u - rho n)  to Lx_i (and the opposite to
-// Lx_j).  One thread owns one atom and gathers its full neighbourhood, so
-// every sum is over a fixed order: the result is deterministic and needs no
-// atomics.  Parameter partials are accumulated per atom (the own end of each
+// Lx_j).  Parameter partials are accumulated per atom (the own end of each
 // visit takes half of the pair's derivative) and reduced per element once at
 // the end.
+//
+// Launches.  A horizon is hundreds of ticks of a few thousand atoms, each a
+// few microseconds of work: one cooperative launch runs the ticks of a chunk
+// (k_adj_ticks), one the reverse sweep of a segment (k_adj_reverse), with one
+// grid barrier per tick.  Eight lanes own one atom: partner j belongs to lane
+// lane_of(j), and a lane visits its partners in ascending slot order, so each
+// sum's order depends on the pairs in range alone, not on when the list was
+// built: recomputed ticks reproduce the forward pass for any checkpoint
+// spacing.  The lists hold the pairs within rc + skin and are rebuilt, inside
+// the launch, on the ticks on which an atom may have moved skin/2 since.
+// What bounds a tick is latency: 13 warps per SM walk lists of ten to twenty
+// partners, each a chain of dependent FP64 operations.  8,000 atoms, 200
+// ticks, mixed forward, both losses: 29.4 ms, where a sort, a staging and a
+// pair pass over 27 cells per tick, one kernel each, took 143 ms; per tick
+// 13 us for the recomputed pair pass, 17 / 30 for the reverse pass without /
+// with g(r), 40 for a list rebuild every ten ticks.  Lists of rc + 0.2 rc:
+// 31.4 ms where 0.1 takes 33.8, 0.15 32.3 and 0.25 33.5; sixteen lanes per
+// atom 36.3 where eight take 34.7.
 //
 // The cutoffs are multiples of max sigma; their derivative goes to the
 // lowest-index element attaining the max.  The hard-core clamp
 // r = max(d, sigma/2) and the Coulomb/gravity clamp r = max(d, 0.5) are
 // differentiated on the side the value takes; the periodic wrap and the
 // minimum image have derivative one.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
 
+#include "gx_gridsync.cuh"
 #include "gx_law64.cuh"
 #include "gx_pair_f32.cuh"
 
 namespace gx {
 namespace {
 
-constexpr int kAdjThreads = 128;
-constexpr int kAdjLanes = 8;  // lanes per atom in the pair kernels: each takes every 8th neighbour cell
+constexpr int kAdjThreads = 256;
+constexpr int kAdjLanes = 8;              // lanes per atom
+constexpr double kAdjSkin = 0.2;          // list skin in units of the cutoff
+constexpr int kAdjTicksPerLaunch = 256;
 constexpr int kAdjMaxBins = 512;
 constexpr double kRonFrac = 0.9;  // r_on = 0.9 rc for every switched term (forces.rs:237, systems/forces.rs:118-124)
 constexpr double kHistScale = 4294967296.0;
@@ -67,6 +86,7 @@ struct Vec3Field {
 struct GrSpec {
     int bins;
     double dr, width, reach, c2;  // bin width, kernel width, truncation radius, -1/(2 w^2)
+    double step;                  // exp(2 c2 dr^2): how the ratio of neighbouring bins' kernels changes per bin
 };
 
 // Switch S(r) of smooth_cutoff (forces.rs:302-318) with its first two
@@ -103,10 +123,11 @@ struct PairG {
     double frc[3], Urc[3];    // d/drc of the LJ, Coulomb and gravity terms
 };
 
-__device__ __forceinline__ void central_term(double q, double d, double ron, double rc, PairG& o, int slot) {
+__device__ __forceinline__ void central_term(double q, double d, double inv_d, double ron, double rc, PairG& o,
+                                             int slot) {
     bool clamped = d < 0.5;  // r = max(d, 0.5), systems/forces.rs:283,293
-    double r = clamped ? 0.5 : d, rd = clamped ? 0.0 : 1.0;
-    double ir = 1.0 / r;
+    double rd = clamped ? 0.0 : 1.0;
+    double ir = clamped ? 2.0 : inv_d;
     double v = q * ir, m = v * ir;
     double mr = -2.0 * m * ir, vr = -m;
     SwD w = switch_d(d, ron, rc);  // the switch is evaluated at d, not r
@@ -117,8 +138,9 @@ __device__ __forceinline__ void central_term(double q, double d, double ron, dou
     o.Urc[slot] = v * w.Src;
 }
 
-__device__ __forceinline__ PairG pair_grad(const LawF64& L, double d, double sg, double ep, double qa, double qb,
-                                           double ma, double mb) {
+// inv_d = 1 / d; is = 1 / sg (a table of the element pairs).
+__device__ __forceinline__ PairG pair_grad(const LawF64& L, double d, double inv_d, double sg, double is, double ep,
+                                           double qa, double qb, double ma, double mb) {
     PairG o;
     o.f = o.fd = o.Ud = o.fs = o.Us = o.fe = o.Ue = 0.0;
     for (int k = 0; k < 3; ++k) o.frc[k] = o.Urc[k] = 0.0;
@@ -127,8 +149,7 @@ __device__ __forceinline__ PairG pair_grad(const LawF64& L, double d, double sg,
         double half = 0.5 * sg;
         bool clamped = d < half;
         double r = clamped ? half : d, rd = clamped ? 0.0 : 1.0, rs = clamped ? 0.5 : 0.0;
-        double is = 1.0 / sg;
-        double s = sg / r, s2 = s * s, s6 = s2 * s2 * s2, s12 = s6 * s6;
+        double s = clamped ? 2.0 : sg * inv_d, s2 = s * s, s6 = s2 * s2 * s2, s12 = s6 * s6;
         double v1 = 4.0 * (s12 - s6);                            // V / eps
         double m1 = 24.0 * is * s * (2.0 * s12 - s6);            // -dV/dr / eps
         double m1r = 24.0 * is * is * (7.0 * s6 * s2 - 26.0 * s12 * s2);
@@ -148,8 +169,8 @@ __device__ __forceinline__ PairG pair_grad(const LawF64& L, double d, double sg,
         o.frc[0] = ep * (m1 * w.Src - v1 * w.S1rc);
         o.Urc[0] = ep * v1 * w.Src;
     }
-    if (L.coul && d < L.coul_rc) central_term(L.k_e * qa * qb, d, L.coul_ron, L.coul_rc, o, 1);
-    if (L.grav && d < L.grav_rc) central_term(-L.G * ma * mb, d, L.grav_ron, L.grav_rc, o, 2);
+    if (L.coul && d < L.coul_rc) central_term(L.k_e * qa * qb, d, inv_d, L.coul_ron, L.coul_rc, o, 1);
+    if (L.grav && d < L.grav_rc) central_term(-L.G * ma * mb, d, inv_d, L.grav_ron, L.grav_rc, o, 2);
     return o;
 }
 
@@ -167,14 +188,6 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     }
     __syncthreads();
     return v;
-}
-
-// Neighbour cell `k` of cell (cx, cy, cz); k = -1 is the cell itself.
-__device__ __forceinline__ uint32_t visit_cell(const GridGeom& g, uint32_t c, uint32_t cx, uint32_t cy, uint32_t cz,
-                                               int k) {
-    if (k < 0) return c;
-    return encode(g, wrap_add(cx, g.full[k][0], g.n[0]), wrap_add(cy, g.full[k][1], g.n[1]),
-                  wrap_add(cz, g.full[k][2], g.n[2]));
 }
 
 // min_image1 for |d| <= 0.49 L without the division: the rounded quotient
@@ -223,285 +236,626 @@ __global__ void k_adj_import(StateBuf b, uint32_t n, Vec3Field x, Vec3Field v, V
     kind[s] = b.kind[p];
 }
 
-// First kick, drift, wrap (integrate.rs:39-43, 62-66; boundary.rs:28-34) and
-// the cell key of the new position; optionally saves the position.
-__global__ void k_adj_kick_drift(GridGeom g, uint32_t n, Vec3Field x, Vec3Field v, Vec3Field a, double half_dt,
-                                 double dt, double hx, double hy, double hz, int wrap, uint32_t* key, Vec3Field xsave,
-                                 uint32_t* err) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double hb[3] = {hx, hy, hz};
-    double p[3];
-    for (int k = 0; k < 3; ++k) {
-        double vk = xadd(v.c(k, i), xmul(a.c(k, i), half_dt));
-        double xk = xadd(x.c(k, i), xmul(vk, dt));
-        if (wrap) xk = xsub(rem_euclid(xk, xmul(2.0, hb[k])), hb[k]);
-        v.c(k, i) = vk;
-        x.c(k, i) = xk;
-        p[k] = xk;
-        if (xsave.p) xsave.c(k, i) = xk;
+// The lane that visits partner j: neighbours in space are mostly runs of
+// neighbouring slots, which this deals out evenly.
+__device__ __forceinline__ uint32_t lane_of(uint32_t j) { return j % kAdjLanes; }
+constexpr uint32_t kAdjFound = 256;  // partners of one atom that a rebuild can hold
+constexpr uint32_t kAdjQueue = 128;  // distances that a warp collects for the histogram
+
+// A rebuild's words of one warp: the partners found, as (lane, slot) keys
+// padded to whole vectors, and how many each lane has.
+struct __align__(16) AdjFound {
+    uint32_t key[kAdjFound + 4];
+    uint32_t count[kAdjLanes];
+};
+
+struct AdjArgs {
+    GridGeom lg;  // list grid: cells >= rc + skin
+    GridGeom fg;  // force grid: its axes of two cells repeat pairs
+    int two;      // the force grid has such an axis
+    int plain;    // at least three force cells per axis, positions wrapped
+    double half_box[3], inv_box[3];
+    uint32_t n;
+    size_t cap;
+    LawF64 L;
+    LawF32 L32;
+    const PairF* tabf;
+    const double *psig, *peps, *epsk;  // pair tables, epsilon_k
+    const uint8_t *elem, *kind;
+    const double *charge, *mass, *inv_mass;
+    double* S;            // x, v, a: nine rows of cap
+    double* ck;           // checkpoints of S, or null
+    double* slabs;        // positions of a tick: (x, y, z, packed) per atom, 4 cap doubles each
+    int first, last;      // ticks of this launch
+    int K;
+    int keep;             // tick t's positions stay in slab t - first; else two slabs take turns
+    int obs;              // record the observables
+    uint32_t* list;       // entry k of lane e = i * kAdjLanes + l at [k * kAdjLanes * cap + e], ascending slots
+    uint32_t* cnt;
+    int cap_l;
+    double* ref;          // positions at the last rebuild, three rows
+    double* sorted;       // a rebuild's cell-sorted (x, y, z, slot)
+    uint32_t *key, *count, *start, *fill;
+    GridSync* sync;
+    uint32_t* err;
+    double *vpart, *pot;  // block partials (two turns), V_t
+    unsigned long long* ghist;  // two turns of bins
+    double* hacc;
+    GrSpec gs;
+    int every;
+    double half_dt, dt, rl2, lim2;
+    int wrap;
+    // reverse sweep
+    double *Ladj, *P;     // adjoints of x, v, a (nine rows); parameter partials (five rows)
+    double* W;            // two turns of (W/m, -) per atom, 4 cap doubles each
+    const double *alpha, *bw;
+    int gr;
+};
+
+__device__ __forceinline__ double4 load_slab(const double* X, uint32_t j) {
+    const double2* p = reinterpret_cast<const double2*>(X) + 2 * (size_t)j;
+    const double2 u = p[0], w = p[1];
+    return make_double4(u.x, u.y, w.x, w.y);
+}
+// The packed word of a slab: element, kind << 8, force cell << 32 (with `two`).
+__device__ __forceinline__ uint32_t packed_elem(double w) { return (uint32_t)__double_as_longlong(w) & 255u; }
+__device__ __forceinline__ uint32_t packed_kind(double w) { return ((uint32_t)__double_as_longlong(w) >> 8) & 255u; }
+__device__ __forceinline__ uint32_t packed_cell(double w) { return (uint32_t)((unsigned long long)__double_as_longlong(w) >> 32); }
+
+// Whether an atom may have left its list: the squared displacement of
+// component l (of lanes 0 .. 2 of its group) since the rebuild, summed over
+// the group.  `odd`: half-box translations of the wrap since then (mod 2).
+__device__ __forceinline__ double moved2(const AdjArgs& a, uint32_t i, uint32_t l, bool live, double x, bool odd) {
+    double d = 0.0;
+    if (live && l < 3) {
+        const double L = a.L.box[l];
+        d = x - a.ref[l * a.cap + i] - (odd ? 0.5 * L : 0.0);
+        d -= L * rint(d * a.inv_box[l]);
+        d *= d;
     }
-    if (!(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]))) atomicOr(err, kErrNonFinite);
-    key[i] = cell_of(g, p[0], p[1], p[2]);
+    return lane_sum(d);
 }
 
-__global__ void k_adj_keys(GridGeom g, uint32_t n, Vec3Field x, uint32_t* key) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    key[i] = cell_of(g, x.c(0, i), x.c(1, i), x.c(2, i));
+// A minimum image to rounding, for the lists' tests, which have the skin's
+// room: no division and no branch.
+__device__ __forceinline__ double list_image(const AdjArgs& a, double d, int k) {
+    return d - a.L.box[k] * rint(d * a.inv_box[k]);
 }
 
-// Cell-sorted copies of what the pair loops read (p = sorted position).
-// With an adjoint, also W/m = (La + half_dt Lv) / m per atom.
-__global__ void k_adj_stage(uint32_t n, const uint32_t* __restrict__ perm, const uint32_t* __restrict__ key,
-                            Vec3Field x, const uint8_t* __restrict__ elem, const double* __restrict__ charge,
-                            const double* __restrict__ mass, const double* __restrict__ inv_mass, Vec3Field xs,
-                            uint8_t* es, double* qs, double* ms, uint32_t* ks, Vec3Field Lv, Vec3Field La,
-                            double half_dt, Vec3Field ws, const uint8_t* __restrict__ kind, uint8_t* kinds) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    uint32_t i = perm[p];
-    for (int k = 0; k < 3; ++k) xs.c(k, p) = x.c(k, i);
-    es[p] = elem[i];
-    if (kinds) kinds[p] = kind[i];
-    qs[p] = charge[i];
-    ms[p] = mass[i];
-    ks[p] = key[i];
-    if (ws.p) {
-        double im = inv_mass[i];
-        for (int k = 0; k < 3; ++k) ws.c(k, p) = (La.c(k, i) + half_dt * Lv.c(k, i)) * im;
+// Lists of the pairs within rc + skin of the positions X, by lane; their
+// reference positions.  False when a barrier gave up.
+__device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target, int* s_ok, uint32_t* s_warp,
+                            uint32_t* s_off, AdjFound* s_found) {
+    const uint32_t tid = threadIdx.x, gt = blockIdx.x * kAdjThreads + tid, gs = gridDim.x * kAdjThreads;
+    const uint32_t n = a.n, m = a.lg.ncell + 1, ntiles = (m + kScanTileCells - 1) / kScanTileCells;
+    for (uint32_t i = gt; i < n; i += gs) {
+        const double4 p = load_slab(X, i);
+        const uint32_t c = cell_of(a.lg, p.x, p.y, p.z);
+        a.key[i] = c;
+        atomicAdd(&a.count[c], 1u);
     }
-}
-
-// Forward force pass + second kick.  kAdjLanes lanes own atom perm[p]: lane
-// l visits the neighbour cells l - 1, l - 1 + kAdjLanes, ... (the atom's own
-// cell first) in the reference's per-pair FP64 arithmetic, and lane_sum
-// combines their accelerations; the potential and the smoothed histogram
-// take each pair-list entry once (canonical half-shell visits, or j > p
-// within a cell).  One histogram per warp in shared memory, integer counts.
-// F32: the mixed method's pair law (pair_f32 on the FP64 displacement
-// rounded to FP32, the kinds' FP32 pair table) with the force summed in
-// 2^-32 fixed point and a = F 2^-32 / m as the list path's finish takes it;
-// the potential sums the FP32 pair energies in FP64.
-template <bool OBS, bool GR, bool F32>
-__global__ void __launch_bounds__(kAdjThreads)
-    k_adj_force(GridGeom g, uint32_t n, LawF64 L, const double* __restrict__ psig, const double* __restrict__ peps,
-                const uint32_t* __restrict__ start, const uint32_t* __restrict__ ks, Vec3Field xs,
-                const uint8_t* __restrict__ es, const double* __restrict__ qs, const double* __restrict__ ms,
-                const uint32_t* __restrict__ perm, const double* __restrict__ inv_mass, Vec3Field v, Vec3Field a,
-                double half_dt, double* __restrict__ vpart, GrSpec gs, double* __restrict__ hpart, LawF32 L32,
-                const PairF* __restrict__ tabf, const uint8_t* __restrict__ kinds, uint32_t* __restrict__ err) {
-    constexpr int kWarps = kAdjThreads / 32;
-    __shared__ double shd[kWarps];
-    __shared__ unsigned long long hist[GR ? kWarps : 1][GR ? kAdjMaxBins : 1];
-    if (GR)
-        for (int k = threadIdx.x; k < kWarps * gs.bins; k += kAdjThreads) hist[k / gs.bins][k % gs.bins] = 0ull;
-    if (GR) __syncthreads();
-    unsigned long long* wh = hist[GR ? threadIdx.x / 32 : 0];
-    const uint32_t t = blockIdx.x * kAdjThreads + threadIdx.x;
-    const uint32_t p = t / kAdjLanes;
-    const int lane = (int)(t % kAdjLanes);
-    double V = 0.0;
-    double ax = 0.0, ay = 0.0, az = 0.0;
-    long long fx = 0, fy = 0, fz = 0;
-    if (p < n) {
-        uint32_t c = ks[p], cx, cy, cz;
-        decode(g, c, cx, cy, cz);
-        double xi = xs.c(0, p), yi = xs.c(1, p), zi = xs.c(2, p);
-        int ti = es[p];
-        const int kti = F32 ? (int)kinds[p] * L32.nkinds : 0;
-        double qi = qs[p], mi = ms[p];
-        double inv_mi = inv_mass[perm[p]];
-        for (int k = lane - 1; k < g.nfull; k += kAdjLanes) {
-            uint32_t B = visit_cell(g, c, cx, cy, cz, k);
-            bool half = k < g.nhalf;
-            uint32_t lo = start[B], hi = start[B + 1];
-            for (uint32_t q = lo; q < hi; ++q) {
-                if (q == p) continue;
-                double dx = near_image(xsub(xi, xs.c(0, q)), L.box[0]);
-                double dy = near_image(xsub(yi, xs.c(1, q)), L.box[1]);
-                double dz = near_image(xsub(zi, xs.c(2, q)), L.box[2]);
-                double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
-                if (d2 >= L.rc2) continue;
-                double d = xsqrt(d2);
-                if (d <= kEpsF64) continue;
-                bool count = (k < 0) ? (q > p) : half;
-                double fmag = 0.0, Vij = 0.0;
-                if (F32) {
-                    const float fdx = (float)dx, fdy = (float)dy, fdz = (float)dz;
-                    float fs, vf;
-                    pair_f32(L32, tabf[kti + kinds[q]], dist2(fdx, fdy, fdz), fs, vf);
-                    long long qx, qy, qz;
-                    quant3(fmul(fdx, fs), fmul(fdy, fs), fmul(fdz, fs), qx, qy, qz, err);
-                    fx += qx;
-                    fy += qy;
-                    fz += qz;
-                    Vij = (double)vf;
-                } else {
-                    int tj = es[q];
-                    pair_f64(L, d, psig[ti * kNElem + tj], peps[ti * kNElem + tj], qi, qs[q], mi, ms[q], fmag, Vij);
+    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
+    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x)
+        scan_tile<kAdjThreads>(a.count, t, m, &a.sync->tile[t], s_warp);
+    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
+    if (tid < ntiles) {
+        uint32_t run = 0;
+        for (uint32_t t = 0; t < tid; ++t) run += a.sync->tile[t];
+        s_off[tid] = run;
+    }
+    __syncthreads();
+    for (uint32_t c = gt; c < m; c += gs) a.start[c] = a.count[c] + s_off[c / kScanTileCells];
+    for (uint32_t i = gt; i < n; i += gs) {
+        const uint32_t c = a.key[i];
+        const double4 p = load_slab(X, i);
+        double2* to = reinterpret_cast<double2*>(a.sorted) +
+                      2 * (size_t)(a.count[c] + s_off[c / kScanTileCells] + atomicAdd(&a.fill[c], 1u));
+        to[0] = make_double2(p.x, p.y);
+        to[1] = make_double2(p.z, __longlong_as_double((long long)i));
+    }
+    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
+    for (uint32_t c = gt; c < m; c += gs) a.count[c] = a.fill[c] = 0u;  // for the next rebuild
+    // A warp per atom: lane k < 27 looks up neighbour cell k (every distinct
+    // one: both sides of an axis only from three cells on), a scan of the
+    // counts turns the candidates into one run taken 32 at a time, and the
+    // partners found go to shared memory.  A partner's place in its lane's
+    // list is the number of that lane's partners with smaller slots.
+    constexpr int kAhead = 4;  // candidates of a lane in flight
+    const size_t stride = (size_t)kAdjLanes * a.cap;
+    const uint32_t lane = tid & 31u;
+    AdjFound& found = s_found[tid / 32];
+    const int ox = (int)(lane % 3u) - 1, oy = (int)((lane / 3u) % 3u) - 1, oz = (int)(lane / 9u) - 1;
+    const bool distinct = lane < 27 && (ox == 0 || a.lg.n[0] >= 3 || (ox > 0 && a.lg.n[0] == 2)) &&
+                          (oy == 0 || a.lg.n[1] >= 3 || (oy > 0 && a.lg.n[1] == 2)) &&
+                          (oz == 0 || a.lg.n[2] >= 3 || (oz > 0 && a.lg.n[2] == 2));
+    for (uint32_t i = gt / 32u; i < n; i += gs / 32u) {
+        const double4 pi = load_slab(X, i);
+        if (lane < 3) a.ref[lane * a.cap + i] = lane == 0 ? pi.x : (lane == 1 ? pi.y : pi.z);
+        uint32_t lo = 0, len = 0;
+        if (distinct) {
+            uint32_t cx, cy, cz;
+            decode(a.lg, a.key[i], cx, cy, cz);
+            const uint32_t B = encode(a.lg, wrap_add(cx, ox, a.lg.n[0]), wrap_add(cy, oy, a.lg.n[1]),
+                                      wrap_add(cz, oz, a.lg.n[2]));
+            lo = a.start[B];
+            len = a.start[B + 1] - lo;
+        }
+        uint32_t end = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= (uint32_t)o) end += v;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, end, 31), base = lo - (end - len);
+        if (lane < kAdjLanes) found.count[lane] = 0u;
+        __syncwarp();
+        uint32_t m2 = 0;
+        for (uint32_t t0 = 0; t0 < total; t0 += 32 * kAhead) {  // every load before the tests
+            double4 pj[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const uint32_t t = t0 + 32u * u + lane;
+                uint32_t k = 0;  // the first cell whose scan exceeds t
+#pragma unroll
+                for (uint32_t step = 16; step > 0; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, end, k + step - 1) <= t) k += step;
+                const uint32_t q = __shfl_sync(0xffffffffu, base, k) + t;
+                pj[u] = make_double4(0.0, 0.0, 0.0, __longlong_as_double((long long)i));
+                if (t < total) pj[u] = load_slab(a.sorted, q);
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const uint32_t j = (uint32_t)__double_as_longlong(pj[u].w);
+                const double dx = list_image(a, pi.x - pj[u].x, 0), dy = list_image(a, pi.y - pj[u].y, 1),
+                             dz = list_image(a, pi.z - pj[u].z, 2);
+                const bool hit = j != i && dx * dx + dy * dy + dz * dz < a.rl2;
+                const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+                const uint32_t at = m2 + __popc(mask & ((1u << lane) - 1u));
+                if (hit && at < kAdjFound) {
+                    found.key[at] = lane_of(j) << 28 | j;
+                    atomicAdd(&found.count[lane_of(j)], 1u);
                 }
-                if (OBS && count) V = xadd(V, Vij);
-                if (GR && count) {
-                    int k0 = (int)ceil((d - gs.reach) / gs.dr - 0.5), k1 = (int)floor((d + gs.reach) / gs.dr - 0.5);
-                    k0 = k0 < 0 ? 0 : k0;
-                    k1 = k1 > gs.bins - 1 ? gs.bins - 1 : k1;
-                    for (int bb = k0; bb <= k1; ++bb) {
-                        double z = d - (bb + 0.5) * gs.dr;
-                        if (fabs(z) >= gs.reach) continue;
-                        double G = exp(z * z * gs.c2);
-                        atomicAdd(&wh[bb], (unsigned long long)llrint(G * kHistScale));
-                    }
-                }
-                if (!F32 && fmag != 0.0) {
-                    double inv = xdiv(1.0, d);
-                    ax = xadd(ax, xmul(xmul(xmul(dx, inv), fmag), inv_mi));
-                    ay = xadd(ay, xmul(xmul(xmul(dy, inv), fmag), inv_mi));
-                    az = xadd(az, xmul(xmul(xmul(dz, inv), fmag), inv_mi));
-                }
+                m2 += __popc(mask);
             }
         }
+        if (m2 <= kAdjFound) {
+            if (lane < 4) found.key[m2 + lane] = 0xffffffffu;
+            __syncwarp();
+            for (uint32_t k = lane; k < m2; k += 32) {  // the keys below this one, those of lower lanes aside
+                const uint32_t key = found.key[k], l = key >> 28;
+                uint32_t place = 0;
+                for (uint32_t q = 0; q < m2; q += 4) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(&found.key[q]);
+                    place += (v.x < key) + (v.y < key) + (v.z < key) + (v.w < key);
+                }
+                for (uint32_t q = 0; q < l; ++q) place -= found.count[q];
+                if (place < (uint32_t)a.cap_l) a.list[place * stride + i * kAdjLanes + l] = key & 0x0fffffffu;
+            }
+        }
+        // more than a warp can hold: every lane looks at all atoms
+        if (lane < kAdjLanes) a.cnt[i * kAdjLanes + lane] = m2 <= kAdjFound ? found.count[lane] : (uint32_t)a.cap_l + 1u;
+        __syncwarp();
     }
-    // every lane of an atom is in the same warp and takes part
-    if (F32) {
-        fx = lane_sum_ll(fx);
-        fy = lane_sum_ll(fy);
-        fz = lane_sum_ll(fz);
-        if (p < n) {
-            const double im = inv_mass[perm[p]];
-            ax = xmul(xmul(__ll2double_rn(fx), kFixInv), im);
-            ay = xmul(xmul(__ll2double_rn(fy), kFixInv), im);
-            az = xmul(xmul(__ll2double_rn(fz), kFixInv), im);
+    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;  // the lists are read by other threads
+    return true;
+}
+
+// Every partner of lane l of atom i in ascending slot order, with its slab
+// entry loaded one partner ahead; a lane whose list overflowed looks at all
+// atoms.
+template <class V>
+__device__ __forceinline__ void adj_partners(const AdjArgs& a, const double* X, uint32_t i, uint32_t l, V&& visit) {
+    const uint32_t e = i * kAdjLanes + l, m = a.cnt[e];
+    if (m <= (uint32_t)a.cap_l) {
+        if (m == 0) return;
+        const size_t stride = (size_t)kAdjLanes * a.cap;
+        const uint32_t* row = a.list + e;
+        uint32_t j = row[0], j1 = m > 1 ? row[stride] : j;
+        double4 p = load_slab(X, j);
+        for (uint32_t k = 0; k < m; ++k) {
+            const double4 p1 = load_slab(X, j1);
+            const uint32_t j2 = k + 2 < m ? row[(k + 2) * stride] : j1;
+            visit(j, p);
+            j = j1;
+            p = p1;
+            j1 = j2;
         }
     } else {
-        ax = lane_sum(ax);
-        ay = lane_sum(ay);
-        az = lane_sum(az);
+        for (uint32_t j = l; j < a.n; j += kAdjLanes)  // lane_of
+            if (j != i) visit(j, load_slab(X, j));
     }
-    if (p < n && lane == 0) {
-        uint32_t i = perm[p];
-        a.c(0, i) = ax;
-        a.c(1, i) = ay;
-        a.c(2, i) = az;
-        v.c(0, i) = xadd(v.c(0, i), xmul(ax, half_dt));
-        v.c(1, i) = xadd(v.c(1, i), xmul(ay, half_dt));
-        v.c(2, i) = xadd(v.c(2, i), xmul(az, half_dt));
+}
+
+// The minimum image of a difference of two positions: where both are wrapped
+// and every pair within the cutoff is seen once, without the division.
+__device__ __forceinline__ double adj_image(const AdjArgs& a, double d, int k) {
+    return a.plain ? min_image_near(d, a.L.box[k], a.half_box[k]) : near_image(d, a.L.box[k]);
+}
+
+// The bins within the kernel's reach of distance d: f(bin, G_bin) with
+// G = exp(c2 z^2), z = d - centre[bin].  Along the bins z changes by -dr, so G
+// follows from two exponentials by two products a bin (their rounding adds to
+// some 1e-15; the sums keep 2^-32).
+template <class F>
+__device__ __forceinline__ void gr_bins(const GrSpec& gs, const double* centre, double d, F&& f) {
+    int k0 = (int)ceil((d - gs.reach) / gs.dr - 0.5), k1 = (int)floor((d + gs.reach) / gs.dr - 0.5);
+    k0 = k0 < 0 ? 0 : k0;
+    k1 = k1 > gs.bins - 1 ? gs.bins - 1 : k1;
+    if (k0 <= k1 && !(fabs(d - centre[k0]) < gs.reach)) ++k0;  // within rounding of the reach
+    if (k0 <= k1 && !(fabs(d - centre[k1]) < gs.reach)) --k1;
+    if (k0 > k1) return;
+    const double z = d - centre[k0];
+    double G = exp(z * z * gs.c2), R = exp(gs.c2 * gs.dr * (gs.dr - 2.0 * z));
+    for (int b = k0; b <= k1; ++b) {
+        f(b, G);
+        G *= R;
+        R *= gs.step;
     }
-    if (OBS) {
-        V = block_sum<kAdjThreads>(V, shd);
-        if (threadIdx.x == 0) vpart[blockIdx.x] = V;
+}
+
+// Ticks first .. last.  With `obs` V_t and the smoothed histogram; with
+// `keep` the last tick stops after the drift (the reverse sweep needs its
+// positions only).  F32: the mixed method's pair law with the force summed
+// in 2^-32 fixed point and a = F 2^-32 / m as the list path's finish takes
+// it; the potential sums the FP32 pair energies in FP64.
+template <bool F32>
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_constant__ AdjArgs a) {
+    extern __shared__ uint32_t s_hist[];  // with obs a histogram per warp: low 16 bits' sums, then the rest's
+    __shared__ double s_sig[kNElem * kNElem], s_eps[kNElem * kNElem], s_e24[kNElem * kNElem];
+    __shared__ PairF s_tab[F32 ? kMaxKinds * kMaxKinds : 1];
+    __shared__ double sh[kAdjThreads / 32], s_r[kAdjMaxBins], s_queue[kAdjThreads / 32][kAdjQueue];
+    __shared__ uint32_t s_queued[kAdjThreads / 32];
+    __shared__ uint32_t s_warp[kAdjThreads / 32], s_off[kScanMaxTiles];
+    __shared__ AdjFound s_found[kAdjThreads / 32];
+    __shared__ int s_ok;
+    const uint32_t tid = threadIdx.x, n = a.n, lanes = n * kAdjLanes;
+    const uint32_t gt = blockIdx.x * kAdjThreads + tid, gs = gridDim.x * kAdjThreads;
+    const uint32_t pad = (lanes + 31u) & ~31u;  // whole warps
+    const size_t cap = a.cap;
+    const int bins = a.obs ? a.gs.bins : 0;
+    const double h3[3] = {xmul(0.5, a.L.box[0]), xmul(0.5, a.L.box[1]), xmul(0.5, a.L.box[2])};
+    const bool recorder = blockIdx.x == gridDim.x - 1;
+    uint32_t target = 0;
+    for (int k = tid; k < kNElem * kNElem; k += kAdjThreads) {
+        s_sig[k] = a.psig[k];
+        s_eps[k] = a.peps[k];
+        s_e24[k] = xdiv(xmul(24.0, a.peps[k]), a.psig[k]);
     }
-    if (GR) {
-        __syncthreads();
-        for (int k = threadIdx.x; k < gs.bins; k += kAdjThreads) {
-            unsigned long long s = 0ull;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) s += hist[w][k];
-            hpart[(size_t)blockIdx.x * gs.bins + k] = (double)s * kHistInv;
+    if (F32)
+        for (int k = tid; k < a.L32.nkinds * a.L32.nkinds; k += kAdjThreads) s_tab[k] = a.tabf[k];
+    for (int k = tid; k < (kAdjThreads / 32) * 2 * bins; k += kAdjThreads) s_hist[k] = 0u;
+    for (int k = tid; k < bins; k += kAdjThreads) s_r[k] = (k + 0.5) * a.gs.dr;
+    uint32_t* wh = s_hist + (tid / 32) * 2 * bins;
+    uint32_t held = 0;  // terms that a bin of this warp's histogram may hold
+    if (tid < kAdjThreads / 32) s_queued[tid] = 0u;
+    auto into_warp = [&](int b, unsigned long long v) {
+        atomicAdd(&wh[b], (uint32_t)v & 0xffffu);
+        atomicAdd(&wh[bins + b], (uint32_t)(v >> 16));
+    };
+    for (uint32_t c = gt; c < a.lg.ncell + 1; c += gs) a.count[c] = a.fill[c] = 0u;
+    // V_t and the histogram of a finished tick, by one block
+    auto record = [&](int t) {
+        const int turn = t & 1;
+        double s = 0.0;
+        for (uint32_t k = tid; k < gridDim.x; k += kAdjThreads) s = xadd(s, a.vpart[turn * gridDim.x + k]);
+        s = block_sum<kAdjThreads>(s, sh);
+        if (tid == 0) a.pot[t - 1] = s;
+        if (bins && t % a.every == 0)
+            for (int k = tid; k < bins; k += kAdjThreads) {
+                unsigned long long* g = a.ghist + turn * bins + k;
+                a.hacc[k] += (double)*g * kHistInv;
+                *g = 0ull;
+            }
+    };
+    int built = 0;  // the tick of the last rebuild
+    for (int t = a.first; t <= a.last; ++t) {
+        const int turn = t & 1, ask = t % 3;
+        double* X = a.slabs + (size_t)(a.keep ? t - a.first : turn) * 4 * cap;
+        const bool odd = a.wrap && ((t - built) & 1);
+        const bool ckpt = a.ck && (t - 1) % a.K == 0;
+        bool over = false;
+        for (uint32_t e = gt; e < pad; e += gs) {  // kick, drift, wrap (integrate.rs:39-43, 62-66; boundary.rs:28-34)
+            const uint32_t i = e / kAdjLanes, l = e % kAdjLanes;
+            const bool live = i < n;
+            double x = 0.0;
+            if (live && l < 3) {
+                double *sx = a.S + l * cap + i, *sv = sx + 3 * cap, *sa = sx + 6 * cap;
+                x = *sx;
+                double v = *sv;
+                const double acc = *sa;
+                if (ckpt) {
+                    double* c = a.ck + (size_t)((t - 1) / a.K) * 9 * cap + l * cap + i;
+                    c[0] = x;
+                    c[3 * cap] = v;
+                    c[6 * cap] = acc;
+                }
+                const double hb = l == 0 ? h3[0] : (l == 1 ? h3[1] : h3[2]);
+                v = xadd(v, xmul(acc, a.half_dt));
+                x = xadd(x, xmul(v, a.dt));
+                if (a.wrap) x = xsub(rem_euclid(x, xmul(2.0, hb)), hb);
+                *sv = v;
+                *sx = x;
+                X[4 * (size_t)i + l] = x;
+                if (!isfinite(x)) atomicOr(a.err, kErrNonFinite);
+            }
+            uint32_t cell = 0;
+            if (a.two) {
+                const double px = __shfl_sync(0xffffffffu, x, 0, kAdjLanes), py = __shfl_sync(0xffffffffu, x, 1, kAdjLanes),
+                             pz = __shfl_sync(0xffffffffu, x, 2, kAdjLanes);
+                cell = cell_of(a.fg, px, py, pz);
+            }
+            if (live && l == 3)
+                X[4 * (size_t)i + 3] = __longlong_as_double(
+                    (long long)((unsigned long long)cell << 32 | (uint32_t)a.kind[i] << 8 | a.elem[i]));
+            if (built) over |= !(moved2(a, i, l, live, x, odd) <= a.lim2);
+        }
+        if (t == a.last && a.keep) break;
+        if (__syncthreads_or(over) && tid == 0) a.sync->request[ask] = 1u;
+        if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
+        const bool rebuild = !built || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
+        if (recorder) {
+            if (a.obs && t > a.first) record(t - 1);
+            if (tid == 0) a.sync->request[(ask + 2) % 3] = 0u;  // every block has read it before this barrier
+        }
+        if (rebuild) {
+            if (!adj_rebuild(a, X, target, &s_ok, s_warp, s_off, s_found)) return;
+            built = t;
+        }
+        const bool gr = bins > 0 && t % a.every == 0;
+        double V = 0.0;
+        auto flush = [&](uint32_t* hist, int warps, int from, int by) {  // adds histograms to the tick's and clears them
+            for (int k = from; k < bins; k += by) {
+                unsigned long long s = 0ull;
+                for (int w = 0; w < warps; ++w) {
+                    uint32_t* hw = hist + w * 2 * bins + k;
+                    s += hw[0] + ((unsigned long long)hw[bins] << 16);
+                    hw[0] = hw[bins] = 0u;
+                }
+                if (s) atomicAdd(&a.ghist[turn * bins + k], s);
+            }
+        };
+        for (uint32_t e = gt; e < pad; e += gs) {  // pair pass and second kick
+            const uint32_t i = e / kAdjLanes, l = e % kAdjLanes;
+            bool direct = false;  // an overflowed lane's terms go to the tick's histogram one by one
+            if (gr) {  // 65,535 terms (of at most `two`'s eight visits of a pair) cannot overflow 32 bits
+                const uint32_t c = i < n ? a.cnt[e] : 0u;
+                direct = c > (uint32_t)a.cap_l;
+                const uint32_t terms = __reduce_add_sync(0xffffffffu, direct ? 0u : c);
+                const uint32_t most = a.two ? 65535u / 8u : 65535u;
+                if (held + terms > most) {
+                    __syncwarp();
+                    flush(wh, 1, (int)(tid & 31u), 32);
+                    __syncwarp();
+                    held = 0;
+                }
+                held += terms;
+            }
+            double ax = 0.0, ay = 0.0, az = 0.0;
+            long long fx = 0, fy = 0, fz = 0;
+            if (i < n) {
+                const double4 pi = load_slab(X, i);
+                const uint32_t ti = packed_elem(pi.w) * kNElem;
+                const uint32_t kti = F32 ? packed_kind(pi.w) * a.L32.nkinds : 0u;
+                const double qi = a.charge[i], mi = a.mass[i], inv_mi = a.inv_mass[i];
+                adj_partners(a, X, i, l, [&](uint32_t j, const double4& pj) {
+                    const double dx = adj_image(a, xsub(pi.x, pj.x), 0);
+                    const double dy = adj_image(a, xsub(pi.y, pj.y), 1);
+                    const double dz = adj_image(a, xsub(pi.z, pj.z), 2);
+                    const double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
+                    if (d2 >= a.L.rc2) return;
+                    const double d = xsqrt(d2);
+                    if (d <= kEpsF64) return;
+                    const int mult = a.two ? pair_multiplicity(a.fg, packed_cell(pi.w), packed_cell(pj.w)) : 1;
+                    const bool count = j > i;
+                    double Vij = 0.0;
+                    if (F32) {
+                        const float gx = (float)dx, gy = (float)dy, gz = (float)dz;
+                        float fs, vf;
+                        pair_f32(a.L32, s_tab[kti + packed_kind(pj.w)], dist2(gx, gy, gz), fs, vf);
+                        long long qx, qy, qz;
+                        quant3(fmul(gx, fs), fmul(gy, fs), fmul(gz, fs), qx, qy, qz, a.err);
+                        fx += mult * qx;
+                        fy += mult * qy;
+                        fz += mult * qz;
+                        Vij = (double)vf;
+                    } else {
+                        const uint32_t tt = ti + packed_elem(pj.w);
+                        const bool far = a.L.coul || a.L.grav;
+                        double fmag = 0.0;
+                        pair_f64_e24(a.L, d, s_sig[tt], s_eps[tt], s_e24[tt], qi, far ? a.charge[j] : 0.0, mi,
+                                     far ? a.mass[j] : 0.0, fmag, Vij);
+                        if (fmag != 0.0) {
+                            const double inv = xdiv(1.0, d);
+                            for (int r = 0; r < mult; ++r) {
+                                ax = xadd(ax, xmul(xmul(xmul(dx, inv), fmag), inv_mi));
+                                ay = xadd(ay, xmul(xmul(xmul(dy, inv), fmag), inv_mi));
+                                az = xadd(az, xmul(xmul(xmul(dz, inv), fmag), inv_mi));
+                            }
+                        }
+                    }
+                    if (!a.obs || !count) return;
+                    for (int r = 0; r < mult; ++r) V = xadd(V, Vij);
+                    if (!gr) return;
+                    // half of the partners count: the warp takes their distances together below
+                    if (!a.two && !direct) {
+                        const uint32_t at = atomicAdd(&s_queued[tid / 32], 1u);
+                        if (at < kAdjQueue) {
+                            s_queue[tid / 32][at] = d;
+                            return;
+                        }
+                    }
+                    gr_bins(a.gs, s_r, d, [&](int b, double G) {
+                        const unsigned long long v = (unsigned long long)(mult * llrint(G * kHistScale));
+                        if (direct) atomicAdd(&a.ghist[turn * bins + b], v);
+                        else into_warp(b, v);
+                    });
+                });
+            }
+            if (gr) {
+                __syncwarp();
+                const uint32_t queued = min(s_queued[tid / 32], kAdjQueue);
+                for (uint32_t k = tid & 31u; k < queued; k += 32)
+                    gr_bins(a.gs, s_r, s_queue[tid / 32][k],
+                            [&](int b, double G) { into_warp(b, (unsigned long long)llrint(G * kHistScale)); });
+                __syncwarp();
+                if ((tid & 31u) == 0) s_queued[tid / 32] = 0u;
+                __syncwarp();
+            }
+            // every lane of an atom is in the same warp and takes part
+            if (F32) {
+                fx = lane_sum_ll(fx);
+                fy = lane_sum_ll(fy);
+                fz = lane_sum_ll(fz);
+            } else {
+                ax = lane_sum(ax);
+                ay = lane_sum(ay);
+                az = lane_sum(az);
+            }
+            if (i < n && l < 3) {
+                double acc = l == 0 ? ax : (l == 1 ? ay : az);
+                if (F32) acc = xmul(xmul(__ll2double_rn(l == 0 ? fx : (l == 1 ? fy : fz)), kFixInv), a.inv_mass[i]);
+                double* sv = a.S + (3 + l) * cap + i;
+                sv[3 * cap] = acc;
+                *sv = xadd(*sv, xmul(acc, a.half_dt));
+            }
+        }
+        if (a.obs) {
+            V = block_sum<kAdjThreads>(V, sh);
+            if (tid == 0) a.vpart[turn * gridDim.x + blockIdx.x] = V;
+            if (gr) {
+                __syncthreads();
+                flush(s_hist, kAdjThreads / 32, (int)tid, kAdjThreads);
+                held = 0;
+            }
         }
     }
+    if (a.obs) {
+        if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
+        if (recorder) record(a.last);
+    }
+    grid_leave(a.sync);
 }
 
-// hacc[k] += sum over blocks of hpart[b][k], blocks in order.
-__global__ void k_adj_gr_finalize(int bins, int nblocks, const double* __restrict__ hpart, double* hacc) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= bins) return;
-    double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += hpart[(size_t)b * bins + k];
-    hacc[k] += s;
-}
-
-// Backward pass of one tick (see the file comment).  P rows: sigma, epsilon,
-// rc_lj, rc_coulomb, rc_gravity partials per atom.
-template <bool GR>
-__global__ void __launch_bounds__(kAdjThreads)
-    k_adj_back(GridGeom g, uint32_t n, LawF64 L, const double* __restrict__ psig, const double* __restrict__ peps,
-               const double* __restrict__ epsk, const uint32_t* __restrict__ start, const uint32_t* __restrict__ ks,
-               Vec3Field xs, Vec3Field ws, const uint8_t* __restrict__ es, const double* __restrict__ qs,
-               const double* __restrict__ ms, const uint32_t* __restrict__ perm, Vec3Field Lx, Vec3Field Lv,
-               Vec3Field La, double* __restrict__ P, size_t cap, const double* __restrict__ alpha_t, double dt,
-               double half_dt, GrSpec gs, const double* __restrict__ bw) {
-    const uint32_t t = blockIdx.x * kAdjThreads + threadIdx.x;
-    const uint32_t p = t / kAdjLanes;
-    const int lane = (int)(t % kAdjLanes);
-    double gx = 0.0, gy = 0.0, gz = 0.0;
-    double Ps = 0.0, Pe = 0.0, Pr0 = 0.0, Pr1 = 0.0, Pr2 = 0.0;
-    if (p < n) {
-    const double alpha = *alpha_t;
-    uint32_t c = ks[p], cx, cy, cz;
-    decode(g, c, cx, cy, cz);
-    double xi = xs.c(0, p), yi = xs.c(1, p), zi = xs.c(2, p);
-    double wxi = ws.c(0, p), wyi = ws.c(1, p), wzi = ws.c(2, p);
-    int ti = es[p];
-    double qi = qs[p], mi = ms[p];
-    double ehalf_base = 0.5 / epsk[ti];
-    for (int k = lane - 1; k < g.nfull; k += kAdjLanes) {
-        uint32_t B = visit_cell(g, c, cx, cy, cz, k);
-        uint32_t lo = start[B], hi = start[B + 1];
-        for (uint32_t q = lo; q < hi; ++q) {
-            if (q == p) continue;
-            double dx = near_image(xi - xs.c(0, q), L.box[0]);
-            double dy = near_image(yi - xs.c(1, q), L.box[1]);
-            double dz = near_image(zi - xs.c(2, q), L.box[2]);
-            double d2 = dx * dx + dy * dy + dz * dz;
-            if (d2 >= L.rc2) continue;
-            double d = sqrt(d2);
-            if (d <= kEpsF64) continue;
-            double inv = 1.0 / d;
-            double nx = dx * inv, ny = dy * inv, nz = dz * inv;
-            double ux = wxi - ws.c(0, q), uy = wyi - ws.c(1, q), uz = wzi - ws.c(2, q);
-            double rho = nx * ux + ny * uy + nz * uz;
-            int tj = es[q];
-            double sg = psig[ti * kNElem + tj], ep = peps[ti * kNElem + tj];
-            PairG G = pair_grad(L, d, sg, ep, qi, qs[q], mi, ms[q]);
-            double psi = 0.0;
-            if (GR) {
-                int k0 = (int)ceil((d - gs.reach) / gs.dr - 0.5), k1 = (int)floor((d + gs.reach) / gs.dr - 0.5);
-                k0 = k0 < 0 ? 0 : k0;
-                k1 = k1 > gs.bins - 1 ? gs.bins - 1 : k1;
-                for (int b = k0; b <= k1; ++b) {
-                    double z = d - (b + 0.5) * gs.dr;
-                    if (fabs(z) >= gs.reach) continue;
-                    psi += bw[b] * (2.0 * gs.c2 * z) * exp(z * z * gs.c2);
+// The reverse sweep of ticks last .. first (see the file comment), from the
+// positions that k_adj_ticks kept.  P rows: sigma, epsilon, rc_lj,
+// rc_coulomb, rc_gravity partials per atom.
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_constant__ AdjArgs a) {
+    __shared__ double s_sig[kNElem * kNElem], s_eps[kNElem * kNElem], s_is[kNElem * kNElem];
+    __shared__ double s_bw[kAdjMaxBins], s_r[kAdjMaxBins];
+    __shared__ uint32_t s_warp[kAdjThreads / 32], s_off[kScanMaxTiles];
+    __shared__ AdjFound s_found[kAdjThreads / 32];
+    __shared__ int s_ok;
+    const uint32_t tid = threadIdx.x, n = a.n, lanes = n * kAdjLanes;
+    const uint32_t gt = blockIdx.x * kAdjThreads + tid, gs = gridDim.x * kAdjThreads;
+    const uint32_t pad = (lanes + 31u) & ~31u;
+    const size_t cap = a.cap;
+    uint32_t target = 0;
+    for (int k = tid; k < kNElem * kNElem; k += kAdjThreads) {
+        s_sig[k] = a.psig[k];
+        s_eps[k] = a.peps[k];
+        s_is[k] = 1.0 / a.psig[k];
+    }
+    if (a.gr)
+        for (int k = tid; k < a.gs.bins; k += kAdjThreads) {
+            s_bw[k] = a.bw[k] * (2.0 * a.gs.c2);
+            s_r[k] = (k + 0.5) * a.gs.dr;
+        }
+    for (uint32_t c = gt; c < a.lg.ncell + 1; c += gs) a.count[c] = a.fill[c] = 0u;
+    for (uint32_t e = gt; e < lanes; e += gs) {  // W/m of the last tick
+        const uint32_t i = e / kAdjLanes, l = e % kAdjLanes;
+        if (l >= 3) continue;
+        const double *lv = a.Ladj + (3 + l) * cap + i, *la = lv + 3 * cap;
+        a.W[(size_t)(a.last & 1) * 4 * cap + 4 * (size_t)i + l] = (*la + a.half_dt * *lv) * a.inv_mass[i];
+    }
+    int built = 0;
+    for (int t = a.last; t >= a.first; --t) {
+        const double* X = a.slabs + (size_t)(t - a.first) * 4 * cap;
+        const double* W = a.W + (size_t)(t & 1) * 4 * cap;
+        const int ask = t % 3;
+        if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
+        const bool rebuild = !built || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
+        if (blockIdx.x == 0 && tid == 0) a.sync->request[(ask + 1) % 3] = 0u;  // tick t + 1's, read before this barrier
+        if (rebuild) {
+            if (!adj_rebuild(a, X, target, &s_ok, s_warp, s_off, s_found)) return;
+            built = t;
+        }
+        const bool gr = a.gr && t % a.every == 0;
+        const double alpha = a.alpha[t - 1];
+        const double* Xp = t > a.first ? X - 4 * cap : nullptr;  // the next tick of the sweep
+        const bool odd = a.wrap && ((built - (t - 1)) & 1);
+        bool over = false;
+        for (uint32_t e = gt; e < pad; e += gs) {
+            const uint32_t i = e / kAdjLanes, l = e % kAdjLanes;
+            double gx = 0.0, gy = 0.0, gz = 0.0;
+            double Ps = 0.0, Pe = 0.0, Pr0 = 0.0, Pr1 = 0.0, Pr2 = 0.0;
+            if (i < n) {
+                const double4 pi = load_slab(X, i), wi = load_slab(W, i);
+                const uint32_t ti = packed_elem(pi.w);
+                const double qi = a.charge[i], mi = a.mass[i];
+                const double ehalf = 0.5 / a.epsk[ti];
+                adj_partners(a, X, i, l, [&](uint32_t j, const double4& pj) {
+                    const double dx = adj_image(a, pi.x - pj.x, 0);
+                    const double dy = adj_image(a, pi.y - pj.y, 1);
+                    const double dz = adj_image(a, pi.z - pj.z, 2);
+                    const double d2 = dx * dx + dy * dy + dz * dz;
+                    if (d2 >= a.L.rc2) return;
+                    const double d = sqrt(d2);
+                    if (d <= kEpsF64) return;
+                    const double inv = 1.0 / d;
+                    const double nx = dx * inv, ny = dy * inv, nz = dz * inv;
+                    const double4 wj = load_slab(W, j);
+                    const double ux = wi.x - wj.x, uy = wi.y - wj.y, uz = wi.z - wj.z;
+                    const double rho = nx * ux + ny * uy + nz * uz;
+                    const uint32_t tt = ti * kNElem + packed_elem(pj.w);
+                    const bool far = a.L.coul || a.L.grav;
+                    const double ep = s_eps[tt];
+                    const PairG G = pair_grad(a.L, d, inv, s_sig[tt], s_is[tt], ep, qi, far ? a.charge[j] : 0.0, mi,
+                                              far ? a.mass[j] : 0.0);
+                    double psi = 0.0;
+                    if (gr)
+                        gr_bins(a.gs, s_r, d, [&](int b, double Gb) { psi += s_bw[b] * ((d - s_r[b]) * Gb); });
+                    const double mult =
+                        a.two ? (double)pair_multiplicity(a.fg, packed_cell(pi.w), packed_cell(pj.w)) : 1.0;
+                    const double c1 = mult * (rho * G.fd + alpha * G.Ud + psi), c2 = mult * (G.f * inv);
+                    gx += c1 * nx + c2 * (ux - rho * nx);
+                    gy += c1 * ny + c2 * (uy - rho * ny);
+                    gz += c1 * nz + c2 * (uz - rho * nz);
+                    Ps += mult * (0.5 * (rho * G.fs + alpha * G.Us));
+                    Pe += mult * (ep * ehalf * (rho * G.fe + alpha * G.Ue));
+                    Pr0 += mult * (0.5 * (rho * G.frc[0] + alpha * G.Urc[0]));
+                    if (a.L.coul) Pr1 += mult * (0.5 * (rho * G.frc[1] + alpha * G.Urc[1]));
+                    if (a.L.grav) Pr2 += mult * (0.5 * (rho * G.frc[2] + alpha * G.Urc[2]));
+                });
+            }
+            // every lane of an atom is in the same warp and takes part
+            gx = lane_sum(gx);
+            gy = lane_sum(gy);
+            gz = lane_sum(gz);
+            Ps = lane_sum(Ps);
+            Pe = lane_sum(Pe);
+            Pr0 = lane_sum(Pr0);
+            if (a.L.coul) Pr1 = lane_sum(Pr1);
+            if (a.L.grav) Pr2 = lane_sum(Pr2);
+            double xp = 0.0;
+            if (i < n && l < 3) {
+                double* Lx = a.Ladj + l * cap + i;
+                const double lx = Lx[0] + (l == 0 ? gx : (l == 1 ? gy : gz));
+                const double lv = Lx[3 * cap] + a.dt * lx, la = a.half_dt * lv;
+                Lx[0] = lx;
+                Lx[3 * cap] = lv;
+                Lx[6 * cap] = la;
+                if (Xp) {
+                    a.W[(size_t)((t - 1) & 1) * 4 * cap + 4 * (size_t)i + l] = (la + a.half_dt * lv) * a.inv_mass[i];
+                    xp = Xp[4 * (size_t)i + l];
                 }
             }
-            double c1 = rho * G.fd + alpha * G.Ud + psi;
-            double c2 = G.f * inv;
-            gx += c1 * nx + c2 * (ux - rho * nx);
-            gy += c1 * ny + c2 * (uy - rho * ny);
-            gz += c1 * nz + c2 * (uz - rho * nz);
-            Ps += 0.5 * (rho * G.fs + alpha * G.Us);
-            Pe += ep * ehalf_base * (rho * G.fe + alpha * G.Ue);
-            Pr0 += 0.5 * (rho * G.frc[0] + alpha * G.Urc[0]);
-            Pr1 += 0.5 * (rho * G.frc[1] + alpha * G.Urc[1]);
-            Pr2 += 0.5 * (rho * G.frc[2] + alpha * G.Urc[2]);
+            if (i < n && l < 5)
+                a.P[l * cap + i] += l == 0 ? Ps : (l == 1 ? Pe : (l == 2 ? Pr0 : (l == 3 ? Pr1 : Pr2)));
+            if (Xp) over |= !(moved2(a, i, l, i < n, xp, odd) <= a.lim2);
         }
+        if (Xp && __syncthreads_or(over) && tid == 0) a.sync->request[(ask + 2) % 3] = 1u;  // tick t - 1's
     }
-    }
-    // every lane of an atom is in the same warp and takes part
-    gx = lane_sum(gx);
-    gy = lane_sum(gy);
-    gz = lane_sum(gz);
-    Ps = lane_sum(Ps);
-    Pe = lane_sum(Pe);
-    Pr0 = lane_sum(Pr0);
-    Pr1 = lane_sum(Pr1);
-    Pr2 = lane_sum(Pr2);
-    if (p >= n || lane != 0) return;
-    uint32_t i = perm[p];
-    double g3[3] = {gx, gy, gz};
-    for (int k = 0; k < 3; ++k) {
-        double lx = Lx.c(k, i) + g3[k];
-        double lvh = Lv.c(k, i) + dt * lx;
-        Lx.c(k, i) = lx;
-        Lv.c(k, i) = lvh;
-        La.c(k, i) = half_dt * lvh;
-    }
-    P[0 * cap + i] += Ps;
-    P[1 * cap + i] += Pe;
-    P[2 * cap + i] += Pr0;
-    P[3 * cap + i] += Pr1;
-    P[4 * cap + i] += Pr2;
+    grid_leave(a.sync);
 }
 
 // out[e] = sum of sigma partials of element e, out[10 + e] epsilon partials,
@@ -535,23 +889,27 @@ struct AdjBuffers {
     double gr_rmax = 0, gr_width = 0, gr_support = 0;
     bool ready = false;
     bool f32 = false;  // the forward in the mixed method (a handle of mixed precision)
-    uint8_t *kind = nullptr, *kinds = nullptr;  // kind per slot, per sorted position (F32 forward)
-    double *S = nullptr, *Ladj = nullptr, *P = nullptr, *ck = nullptr, *seg = nullptr;
-    double *xs = nullptr, *ws = nullptr, *qs = nullptr, *ms = nullptr;
+    uint8_t *kind = nullptr, *elem = nullptr;
+    double *S = nullptr, *Ladj = nullptr, *P = nullptr, *ck = nullptr, *slabs = nullptr, *W = nullptr, *ref = nullptr;
     double *charge = nullptr, *mass = nullptr, *inv_mass = nullptr;
-    uint8_t *elem = nullptr, *es = nullptr;
-    uint32_t *key = nullptr, *perm = nullptr, *ks = nullptr;
-    double *vpart = nullptr, *dV = nullptr, *alpha = nullptr, *bw = nullptr, *hpart = nullptr, *hacc = nullptr;
+    double* sorted = nullptr;
+    uint32_t *key = nullptr, *count = nullptr, *start = nullptr, *fill = nullptr;
+    uint32_t *list = nullptr, *cnt = nullptr;
+    GridGeom lg{};
+    int cap_l = 0;
+    size_t cap_cells = 0;
+    int resident[3] = {0, 0, 0};  // blocks that fit: FP64 ticks, mixed ticks, the reverse sweep
+    size_t resident_smem = 0;
+    double *vpart = nullptr, *dV = nullptr, *alpha = nullptr, *bw = nullptr, *hacc = nullptr;
+    unsigned long long* ghist = nullptr;
+    GridSync* sync = nullptr;
     double *tab = nullptr;  // psig[100], peps[100], epsk[10], out[kNOut]
-    CellList cl;
     std::vector<void*> owned;
 };
 
 static void adj_release(AdjBuffers* A) {
     for (void* p : A->owned) cudaFree(p);
     A->owned.clear();
-    cells_free(A->cl);
-    A->cl = CellList();
 }
 
 void adjoint_free(gx_handle* h) {
@@ -564,14 +922,38 @@ void adjoint_free(gx_handle* h) {
 
 namespace {
 
+// The list grid (cells >= rc + skin, few enough for the scan's tiles) and a
+// lane's list length: four times its share of the mean neighbourhood.
+bool adj_grid(const gx_handle* h, GridGeom* g, int* cap_l) {
+    const double rl = h->fs.rc * (1.0 + kAdjSkin);
+    double cell = rl;
+    int ok = 0;
+    for (int k = 0; k < 64; ++k, cell *= 1.3) {
+        *g = make_grid(h->p.box, cell, &ok);
+        if (ok && g->ncell < kScanTileCells * kScanMaxTiles) break;
+        ok = 0;
+    }
+    const double vol = h->p.box[0] * h->p.box[1] * h->p.box[2];
+    const double mean = std::min((double)h->n / vol * (4.0 / 3.0) * 3.14159265358979 * rl * rl * rl, (double)h->n);
+    *cap_l = (int)std::min(4.0 * mean / kAdjLanes + 16.0, 256.0);
+    return ok != 0;
+}
+
 int adj_alloc(gx_handle* h, AdjBuffers* A, size_t n, int T, int K, int bins) {
     int nck = (T + K - 1) / K;
-    if (n <= A->cap && T <= A->cap_T && nck <= A->cap_ck && K <= A->cap_K && bins <= A->cap_bins && A->tab) return GX_OK;
-    for (void* p : A->owned) cudaFree(p);
-    A->owned.clear();
+    GridGeom lg;
+    int cap_l = 0;
+    if (!adj_grid(h, &lg, &cap_l)) return set_err(h, GX_ERR_ARG, "adjoint list grid is empty or too large");
+    A->lg = lg;
+    if (n <= A->cap && T <= A->cap_T && nck <= A->cap_ck && K <= A->cap_K && bins <= A->cap_bins &&
+        cap_l <= A->cap_l && lg.ncell + 1 <= A->cap_cells && A->tab)
+        return GX_OK;
+    adj_release(A);
+    A->tab = nullptr;
+    A->cap = 0;
     size_t cap = n < 1 ? 1 : n;
     cap = (cap + 31) & ~(size_t)31;
-    size_t nb = nblk(cap * kAdjLanes, kAdjThreads);
+    const size_t cells = (size_t)lg.ncell + 1;
     int binc = bins < 1 ? 1 : bins;
     auto get = [&](void** p, size_t bytes) -> int {
         cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
@@ -579,37 +961,37 @@ int adj_alloc(gx_handle* h, AdjBuffers* A, size_t n, int T, int K, int bins) {
         A->owned.push_back(*p);
         return GX_OK;
     };
+    const size_t slabs = (size_t)std::max(std::min(K, T), 2);
     int rc = 0;
     rc |= get((void**)&A->S, 9 * cap * sizeof(double));
     rc |= get((void**)&A->Ladj, 9 * cap * sizeof(double));
     rc |= get((void**)&A->P, 5 * cap * sizeof(double));
     rc |= get((void**)&A->ck, (size_t)nck * 9 * cap * sizeof(double));
-    rc |= get((void**)&A->seg, (size_t)K * 3 * cap * sizeof(double));
-    rc |= get((void**)&A->xs, 3 * cap * sizeof(double));
-    rc |= get((void**)&A->ws, 3 * cap * sizeof(double));
-    rc |= get((void**)&A->qs, cap * sizeof(double));
-    rc |= get((void**)&A->ms, cap * sizeof(double));
+    rc |= get((void**)&A->slabs, slabs * 4 * cap * sizeof(double));
+    rc |= get((void**)&A->W, 2 * 4 * cap * sizeof(double));
+    rc |= get((void**)&A->ref, 3 * cap * sizeof(double));
     rc |= get((void**)&A->charge, cap * sizeof(double));
     rc |= get((void**)&A->mass, cap * sizeof(double));
     rc |= get((void**)&A->inv_mass, cap * sizeof(double));
     rc |= get((void**)&A->elem, cap);
-    rc |= get((void**)&A->es, cap);
     rc |= get((void**)&A->kind, cap);
-    rc |= get((void**)&A->kinds, cap);
     rc |= get((void**)&A->key, cap * sizeof(uint32_t));
-    rc |= get((void**)&A->perm, cap * sizeof(uint32_t));
-    rc |= get((void**)&A->ks, cap * sizeof(uint32_t));
-    rc |= get((void**)&A->vpart, nb * sizeof(double));
+    rc |= get((void**)&A->sorted, 4 * cap * sizeof(double));
+    rc |= get((void**)&A->count, cells * sizeof(uint32_t));
+    rc |= get((void**)&A->start, cells * sizeof(uint32_t));
+    rc |= get((void**)&A->fill, cells * sizeof(uint32_t));
+    rc |= get((void**)&A->list, (size_t)cap_l * kAdjLanes * cap * sizeof(uint32_t));
+    rc |= get((void**)&A->cnt, kAdjLanes * cap * sizeof(uint32_t));
+    rc |= get((void**)&A->vpart, 2 * (nblk(cap * kAdjLanes, kAdjThreads) + 1) * sizeof(double));
     rc |= get((void**)&A->dV, (size_t)T * sizeof(double));
     rc |= get((void**)&A->alpha, (size_t)T * sizeof(double));
     rc |= get((void**)&A->bw, (size_t)binc * sizeof(double));
-    rc |= get((void**)&A->hpart, nb * (size_t)binc * sizeof(double));
+    rc |= get((void**)&A->ghist, 2 * (size_t)binc * sizeof(unsigned long long));
     rc |= get((void**)&A->hacc, (size_t)binc * sizeof(double));
+    rc |= get((void**)&A->sync, sizeof(GridSync));
     rc |= get((void**)&A->tab, (2 * kNElem * kNElem + kNElem + kNOut) * sizeof(double));
     if (rc) {
-        for (void* p : A->owned) cudaFree(p);
-        A->owned.clear();
-        A->cap = 0;
+        adj_release(A);
         A->tab = nullptr;
         return rc;
     }
@@ -618,6 +1000,8 @@ int adj_alloc(gx_handle* h, AdjBuffers* A, size_t n, int T, int K, int bins) {
     A->cap_ck = nck;
     A->cap_K = K;
     A->cap_bins = binc;
+    A->cap_l = cap_l;
+    A->cap_cells = cells;
     return GX_OK;
 }
 
@@ -630,45 +1014,88 @@ GrSpec gr_spec(const AdjBuffers* A) {
     g.width = A->gr_width;
     g.reach = A->gr_support * A->gr_width;
     g.c2 = A->gr_width > 0 ? -0.5 / (A->gr_width * A->gr_width) : 0.0;
+    g.step = std::exp(2.0 * g.c2 * g.dr * g.dr);
     return g;
 }
 
-// One forward tick in slot order.  obs: record V_t (and the histogram on
-// sampled ticks); xsave: keep x_t; with_force false stops after the drift.
-int adj_tick(gx_handle* h, AdjBuffers* A, int t, bool obs, double* xsave, bool with_force) {
-    const uint32_t n = (uint32_t)A->n;
-    const size_t cap = A->cap;
-    const GridGeom& g = h->fgrid;
-    Vec3Field x = field(A->S, cap), v = field(A->S + 3 * cap, cap), a = field(A->S + 6 * cap, cap);
-    double half_dt = 0.5 * h->p.dt;
-    GX_LAUNCH(h, k_adj_kick_drift, nblk(n, 256), 256, g, n, x, v, a, half_dt, h->p.dt, h->p.box[0] * 0.5,
-              h->p.box[1] * 0.5, h->p.box[2] * 0.5, h->p.enable_boundaries ? 1 : 0, A->key,
-              field(xsave, cap), h->derr);
-    if (!with_force) return GX_OK;
-    int rc = counting_sort(h, A->cl, g.ncell, A->key, n, A->perm);
-    if (rc) return rc;
-    Vec3Field xs = field(A->xs, cap), none = field(nullptr, cap);
-    GX_LAUNCH(h, k_adj_stage, nblk(n, 256), 256, n, A->perm, A->key, x, A->elem, A->charge, A->mass, A->inv_mass,
-              xs, A->es, A->qs, A->ms, A->ks, none, none, half_dt, none, A->kind, A->f32 ? A->kinds : nullptr);
-    LawF64 L = make_law64(h);
-    const double* psig = A->tab;
-    const double* peps = A->tab + kNElem * kNElem;
-    GrSpec gs = gr_spec(A);
-    unsigned nb = nblk((size_t)n * kAdjLanes, kAdjThreads);
-    bool gr = obs && A->bins > 0 && (t % A->every) == 0;
-    auto kern = A->f32 ? (!obs ? k_adj_force<false, false, true>
-                               : (gr ? k_adj_force<true, true, true> : k_adj_force<true, false, true>))
-                       : (!obs ? k_adj_force<false, false, false>
-                               : (gr ? k_adj_force<true, true, false> : k_adj_force<true, false, false>));
-    GX_LAUNCH(h, kern, nb, kAdjThreads, g, n, L, psig, peps, A->cl.start, A->ks, xs, A->es, A->qs, A->ms, A->perm,
-              A->inv_mass, v, a, half_dt, A->vpart, gs, A->hpart, make_law32(h), h->d_pairf, A->kinds, h->derr);
-    if (obs) {
-        launch_finalize_sum(h, A->vpart, (int)nb, A->dV + (t - 1));
-        if (gr) {
-            GX_LAUNCH(h, k_adj_gr_finalize, nblk(A->bins, 256), 256, A->bins, (int)nb, A->hpart, A->hacc);
-            A->samples++;
-        }
+AdjArgs adj_args(gx_handle* h, AdjBuffers* A) {
+    AdjArgs a{};
+    a.lg = A->lg;
+    a.fg = h->fgrid;
+    a.two = a.fg.n[0] == 2 || a.fg.n[1] == 2 || a.fg.n[2] == 2;
+    a.plain = a.fg.n[0] >= 3 && a.fg.n[1] >= 3 && a.fg.n[2] >= 3 && h->p.enable_boundaries;
+    for (int k = 0; k < 3; ++k) {
+        a.half_box[k] = 0.5 * h->p.box[k];
+        a.inv_box[k] = 1.0 / h->p.box[k];
     }
+    a.n = (uint32_t)A->n;
+    a.cap = A->cap;
+    a.L = make_law64(h);
+    if (A->f32) a.L32 = make_law32(h);
+    a.tabf = h->d_pairf;
+    a.psig = A->tab;
+    a.peps = A->tab + kNElem * kNElem;
+    a.epsk = A->tab + 2 * kNElem * kNElem;
+    a.elem = A->elem;
+    a.kind = A->kind;
+    a.charge = A->charge;
+    a.mass = A->mass;
+    a.inv_mass = A->inv_mass;
+    a.S = A->S;
+    a.slabs = A->slabs;
+    a.K = A->K;
+    a.list = A->list;
+    a.cnt = A->cnt;
+    a.cap_l = A->cap_l;
+    a.ref = A->ref;
+    a.key = A->key;
+    a.sorted = A->sorted;
+    a.count = A->count;
+    a.start = A->start;
+    a.fill = A->fill;
+    a.sync = A->sync;
+    a.err = h->derr;
+    a.vpart = A->vpart;
+    a.pot = A->dV;
+    a.ghist = A->ghist;
+    a.hacc = A->hacc;
+    a.gs = gr_spec(A);
+    a.every = A->every;
+    a.half_dt = 0.5 * h->p.dt;
+    a.dt = h->p.dt;
+    const double rl = h->fs.rc * (1.0 + kAdjSkin), lim = 0.5 * kAdjSkin * h->fs.rc * (1.0 - 1e-6);
+    a.rl2 = rl * rl;
+    a.lim2 = lim * lim;
+    a.wrap = h->p.enable_boundaries ? 1 : 0;
+    a.Ladj = A->Ladj;
+    a.P = A->P;
+    a.W = A->W;
+    a.alpha = A->alpha;
+    a.bw = A->bw;
+    return a;
+}
+
+// One cooperative launch of kernel `which` (AdjBuffers::resident).
+int adj_launch(gx_handle* h, AdjBuffers* A, int which, AdjArgs& a) {
+    const void* kern = which == 2 ? (const void*)k_adj_reverse
+                                  : (which == 1 ? (const void*)k_adj_ticks<true> : (const void*)k_adj_ticks<false>);
+    const size_t smem = which < 2 ? (size_t)(kAdjThreads / 32) * 2 * A->bins * sizeof(uint32_t) : 0;
+    if (smem != A->resident_smem && which < 2) {
+        A->resident[0] = A->resident[1] = 0;
+        A->resident_smem = smem;
+    }
+    int& resident = A->resident[which];
+    if (!resident) {
+        int per = 0, sms = 0;
+        if (smem) GX_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        GX_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kAdjThreads, smem));
+        GX_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->p.device));
+        resident = std::max(per * sms, 1);
+    }
+    const unsigned grid = std::min(nblk((size_t)a.n * kAdjLanes, kAdjThreads), (unsigned)resident);
+    void* args[] = {&a};
+    GX_CUDA(h, cudaLaunchCooperativeKernel(kern, grid, kAdjThreads, args, smem, h->stream));
+    ++h->launches;
     return GX_OK;
 }
 
@@ -687,6 +1114,11 @@ int check_err(gx_handle* h) {
     if (e & kErrNonFinite) {
         cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
         return set_err(h, GX_ERR_NONFINITE, "non-finite position in the adjoint trajectory");
+    }
+    if (e & kErrTimeout) {  // a block gave up at a barrier: the words are no longer zero
+        cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
+        cudaMemsetAsync(static_cast<AdjBuffers*>(h->adj)->sync, 0, sizeof(GridSync), h->stream);
+        return set_err(h, GX_ERR_TIMEOUT, "a bounded device wait timed out in the adjoint");
     }
     if (e & kErrSaturation) {  // the fixed-point force of the mixed forward
         cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
@@ -719,7 +1151,7 @@ int gx_adjoint_forward(gx_handle* h, const gx_adjoint_spec* spec, double* potent
         return set_err(h, GX_ERR_UNSUPPORTED, "the adjoint covers NVE ticks without the bond spring");
     for (int e = 0; e < kNElem; ++e)
         if (!(h->p.epsilon_k[e] > 0.0)) return set_err(h, GX_ERR_UNSUPPORTED, "the adjoint needs every epsilon_k > 0");
-    if (h->n >= (1u << 31)) return set_err(h, GX_ERR_CAPACITY, "too many atoms");
+    if (h->n >= (1u << 28)) return set_err(h, GX_ERR_CAPACITY, "too many atoms");
     if (h->precision == GX_MIXED && h->nkinds > kMaxKinds)
         return set_err(h, GX_ERR_UNSUPPORTED, "the mixed forward supports at most 16 distinct (element, charge) kinds");
     // NVE only, so no Berendsen scale can be pending on the handle's velocities.
@@ -750,13 +1182,19 @@ int gx_adjoint_forward(gx_handle* h, const gx_adjoint_spec* spec, double* potent
     StateBuf& b = h->buf[h->cur];
     GX_LAUNCH(h, k_adj_import, nblk(n, 256), 256, b, n, field(A->S, cap), field(A->S + 3 * cap, cap),
               field(A->S + 6 * cap, cap), A->elem, A->charge, A->mass, A->inv_mass, A->kind);
-    GX_CUDA(h, cudaMemcpyAsync(A->ck, A->S, 9 * cap * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    if (A->bins > 0) GX_CUDA(h, cudaMemsetAsync(A->hacc, 0, A->bins * sizeof(double), h->stream));
-    for (int t = 1; t <= T; ++t) {
-        if ((rc = adj_tick(h, A, t, true, nullptr, true))) return rc;
-        if (t % K == 0 && t / K < A->nck)
-            GX_CUDA(h, cudaMemcpyAsync(A->ck + (size_t)(t / K) * 9 * cap, A->S, 9 * cap * sizeof(double),
-                                       cudaMemcpyDeviceToDevice, h->stream));
+    GX_CUDA(h, cudaMemsetAsync(A->sync, 0, sizeof(GridSync), h->stream));
+    if (A->bins > 0) {
+        GX_CUDA(h, cudaMemsetAsync(A->hacc, 0, A->bins * sizeof(double), h->stream));
+        GX_CUDA(h, cudaMemsetAsync(A->ghist, 0, 2 * A->bins * sizeof(unsigned long long), h->stream));
+        A->samples = T / A->every;
+    }
+    AdjArgs args = adj_args(h, A);
+    args.ck = A->ck;
+    args.obs = 1;
+    for (int t0 = 0; t0 < T; t0 += kAdjTicksPerLaunch) {
+        args.first = t0 + 1;
+        args.last = std::min(t0 + kAdjTicksPerLaunch, T);
+        if ((rc = adj_launch(h, A, A->f32 ? 1 : 0, args))) return rc;
     }
     GX_CUDA(h, cudaMemcpyAsync(potential, A->dV, T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     std::vector<double> hacc(A->bins > 0 ? A->bins : 0);
@@ -782,8 +1220,6 @@ int gx_adjoint_backward(gx_handle* h, const double* dl_dpotential, const double*
     const uint32_t n = (uint32_t)A->n;
     const size_t cap = A->cap;
     const int T = A->T, K = A->K;
-    const GridGeom& g = h->fgrid;
-    double half_dt = 0.5 * h->p.dt;
     // cotangents
     std::vector<double> alpha(T, 0.0), bw(A->bins > 0 ? A->bins : 1, 0.0);
     if (dl_dpotential)
@@ -794,39 +1230,23 @@ int gx_adjoint_backward(gx_handle* h, const double* dl_dpotential, const double*
     GX_CUDA(h, cudaMemcpyAsync(A->bw, bw.data(), bw.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     GX_CUDA(h, cudaMemsetAsync(A->Ladj, 0, 9 * cap * sizeof(double), h->stream));
     GX_CUDA(h, cudaMemsetAsync(A->P, 0, 5 * cap * sizeof(double), h->stream));
-    Vec3Field Lx = field(A->Ladj, cap), Lv = field(A->Ladj + 3 * cap, cap), La = field(A->Ladj + 6 * cap, cap);
-    Vec3Field xs = field(A->xs, cap), ws = field(A->ws, cap);
-    LawF64 L = make_law64(h);
-    const double* psig = A->tab;
-    const double* peps = A->tab + kNElem * kNElem;
-    const double* epsk = A->tab + 2 * kNElem * kNElem;
     double* out = A->tab + 2 * kNElem * kNElem + kNElem;
-    GrSpec gs = gr_spec(A);
-    unsigned nb = nblk((size_t)n * kAdjLanes, kAdjThreads);
-    bool has_gr = dl_dgr && A->bins > 0;
+    AdjArgs args = adj_args(h, A);
+    args.gr = dl_dgr && A->bins > 0;
+    args.keep = 1;
     for (int s = A->nck - 1; s >= 0; --s) {
-        int t0 = s * K, t1 = t0 + K < T ? t0 + K : T;
+        args.first = s * K + 1;
+        args.last = std::min((s + 1) * K, T);
         GX_CUDA(h, cudaMemcpyAsync(A->S, A->ck + (size_t)s * 9 * cap, 9 * cap * sizeof(double),
                                    cudaMemcpyDeviceToDevice, h->stream));
-        for (int t = t0 + 1; t <= t1; ++t)
-            if ((rc = adj_tick(h, A, t, false, A->seg + (size_t)(t - t0 - 1) * 3 * cap, t < t1))) return rc;
-        for (int t = t1; t > t0; --t) {
-            Vec3Field xt = field(A->seg + (size_t)(t - t0 - 1) * 3 * cap, cap);
-            GX_LAUNCH(h, k_adj_keys, nblk(n, 256), 256, g, n, xt, A->key);
-            if ((rc = counting_sort(h, A->cl, g.ncell, A->key, n, A->perm))) return rc;
-            GX_LAUNCH(h, k_adj_stage, nblk(n, 256), 256, n, A->perm, A->key, xt, A->elem, A->charge, A->mass,
-                      A->inv_mass, xs, A->es, A->qs, A->ms, A->ks, Lv, La, half_dt, ws, A->kind, nullptr);
-            bool gr = has_gr && (t % A->every) == 0;
-            auto kern = gr ? k_adj_back<true> : k_adj_back<false>;
-            GX_LAUNCH(h, kern, nb, kAdjThreads, g, n, L, psig, peps, epsk, A->cl.start, A->ks, xs, ws, A->es, A->qs,
-                      A->ms, A->perm, Lx, Lv, La, A->P, cap, A->alpha + (t - 1), h->p.dt, half_dt, gs, A->bw);
-        }
+        if ((rc = adj_launch(h, A, A->f32 ? 1 : 0, args))) return rc;
+        if ((rc = adj_launch(h, A, 2, args))) return rc;
     }
     GX_LAUNCH(h, k_adj_reduce, kNOut, 256, n, A->elem, A->P, cap, out);
     double sums[kNOut];
     GX_CUDA(h, cudaMemcpyAsync(sums, out, sizeof sums, cudaMemcpyDeviceToHost, h->stream));
     double* dsts[3] = {grad_pos0, grad_vel0, grad_acc0};
-    double* stage = A->xs;  // 3 * cap, free once the sweep is done
+    double* stage = A->W;  // 8 * cap, free once the sweep is done
     for (int q = 0; q < 3; ++q) {
         if (!dsts[q] || !n) continue;
         GX_LAUNCH(h, k_adj_export, nblk(n, 256), 256, n, field(A->Ladj + (size_t)q * 3 * cap, cap), stage);

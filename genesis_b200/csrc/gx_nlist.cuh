@@ -3,16 +3,15 @@
 // small universes (gx_nltick.cu) share.
 #pragma once
 
+#include "gx_gridsync.cuh"
 #include "gx_pair_f32.cuh"
 
 namespace gx {
 
 // Device words of the one-launch ticks (gx_nltick.cu).
 struct TickSync {
-    uint32_t arrived, left;        // grid barrier arrivals, blocks that left the launch
-    uint32_t request[2];           // rebuild requested, by tick parity
+    GridSync grid;                 // rebuilds requested by tick parity
     unsigned long long acc[2][4];  // by tick parity: potential, pair count, bond energy
-    uint32_t tile[64];             // scan tile totals of a rebuild
 };
 
 struct NlState {

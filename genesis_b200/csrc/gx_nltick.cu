@@ -36,6 +36,7 @@
 // 54 us at 59,319 atoms, against 55 with three and 57 with five.
 #include <algorithm>
 
+#include "gx_gridsync.cuh"
 #include "gx_law64.cuh"
 #include "gx_nlist.cuh"
 
@@ -43,9 +44,6 @@ namespace gx {
 namespace {
 
 constexpr int kTickThreads = 256;           // as k_nl_finish's blocks: one partial per 256 atoms
-constexpr uint32_t kTickTile = 1024;        // cell counters per scan tile
-constexpr uint32_t kTickMaxTiles = 64;      // of at most 65,536 counters
-constexpr uint32_t kTickPolls = 1u << 22;   // polls of the grid barrier before giving up (seconds)
 constexpr uint32_t kPartRow = 2048;         // partials per parity (reduction rows hold at least 4,096)
 
 struct TickArgs {
@@ -80,71 +78,11 @@ struct TickArgs {
     int wrap, thermo, nticks;
 };
 
-__device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Grid barrier: arrivals only grow during a launch, and `target` is the count
-// at which every block has arrived.  The wait is bounded: a block that gives
-// up sets kErrTimeout and leaves, and the others follow as their waits end.
-__device__ __forceinline__ bool grid_barrier(const TickArgs& a, uint32_t& target, int* s_ok) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        target += gridDim.x;
-        __threadfence();
-        atomicAdd(&a.sync->arrived, 1u);
-        uint32_t polls = 0;
-        int ok = 1;
-        while ((int32_t)(load_acquire(&a.sync->arrived) - target) < 0)
-            if (++polls > kTickPolls) {
-                atomicOr(a.err, kErrTimeout);
-                ok = 0;
-                break;
-            }
-        __threadfence();
-        *s_ok = ok;
-    }
-    __syncthreads();
-    return *s_ok != 0;
-}
-
 // Sum of part[0 .. nb) in k_thermostat_lambda's order (valid in thread 0).
 __device__ __forceinline__ double part_sum(const double* part, int nb, double* sh) {
     double s = 0.0;
     for (int i = threadIdx.x; i < nb; i += kTickThreads) s = xadd(s, part[i]);
     return block_sum_d<kTickThreads>(s, sh);
-}
-
-// Exclusive scan of one tile of cell counts in place; its total to *total.
-__device__ __forceinline__ void scan_tile(uint32_t* count, uint32_t t, uint32_t m, uint32_t* total, uint32_t* s_warp) {
-    constexpr int kItems = kTickTile / kTickThreads;
-    const uint32_t base = t * kTickTile + threadIdx.x * kItems;
-    uint32_t v[kItems], local = 0;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        v[k] = base + k < m ? count[base + k] : 0u;
-        local += v[k];
-    }
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    uint32_t inc = local;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= (uint32_t)o) inc += u;
-    }
-    if (lane == 31) s_warp[w] = inc;
-    __syncthreads();
-    uint32_t run = inc - local;
-    for (uint32_t k = 0; k < w; ++k) run += s_warp[k];
-    if (threadIdx.x == kTickThreads - 1) *total = run + local;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        if (base + k < m) count[base + k] = run;
-        run += v[k];
-    }
-    __syncthreads();  // s_warp is reused by the next tile
 }
 
 // The record of one finished tick, by one block: K and the speed sum from its
@@ -176,12 +114,12 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
     __shared__ float4 s_shift[27];
     __shared__ double sh[kTickThreads / 32];
     __shared__ unsigned long long shu[kTickThreads / 32];
-    __shared__ uint32_t s_warp[kTickThreads / 32], s_off[kTickMaxTiles];
+    __shared__ uint32_t s_warp[kTickThreads / 32], s_off[kScanMaxTiles];
     __shared__ double s_lam;
     __shared__ int s_ok;
     const uint32_t tid = threadIdx.x, n = a.n;
     const uint32_t gt = blockIdx.x * kTickThreads + tid, gs = gridDim.x * kTickThreads;
-    const uint32_t m = a.g.ncell + 1, ntiles = (m + kTickTile - 1) / kTickTile;
+    const uint32_t m = a.g.ncell + 1, ntiles = (m + kScanTileCells - 1) / kScanTileCells;
     const int nb = (int)((n + kTickThreads - 1) / kTickThreads);
     const bool recorder = blockIdx.x == gridDim.x - 1;
     uint32_t target = 0;  // thread 0's count of barrier arrivals
@@ -209,14 +147,14 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
             over |= nl_advance_one(a.b, i, &s_lam, a.half_dt, a.dt, a.hx, a.hy, a.hz, a.wrap, a.g, a.home, a.pos4,
                                    a.ref, a.lim2, half, a.err);
         }
-        if (__syncthreads_or(over) && tid == 0) a.sync->request[par] = 1u;
-        if (!grid_barrier(a, target, &s_ok)) return;
-        const bool rebuild = (tick == 0 && asked) || *(volatile uint32_t*)&a.sync->request[par] != 0u;
+        if (__syncthreads_or(over) && tid == 0) a.sync->grid.request[par] = 1u;
+        if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+        const bool rebuild = (tick == 0 && asked) || *(volatile uint32_t*)&a.sync->grid.request[par] != 0u;
         if (recorder) {  // the other parity's words: every block has left that tick's pair pass
             if (REC && tick > 0) take_record(a, tick - 1, s_lam, nb, sh);
             __syncthreads();
             if (tid < 4) a.sync->acc[par ^ 1][tid] = 0ull;
-            if (tid == 4) a.sync->request[par ^ 1] = 0u;
+            if (tid == 4) a.sync->grid.request[par ^ 1] = 0u;
         }
         if (!a.thermo && tid == 0) s_lam = 1.0;
         if (rebuild) {
@@ -225,22 +163,22 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
                 a.key[i] = c;
                 atomicAdd(&a.count[c], 1u);
             }
-            if (!grid_barrier(a, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x)
-                scan_tile(a.count, t, m, &a.sync->tile[t], s_warp);
-            if (!grid_barrier(a, target, &s_ok)) return;
+                scan_tile<kTickThreads>(a.count, t, m, &a.sync->grid.tile[t], s_warp);
+            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             if (tid < ntiles) {  // tile offsets, in every block
                 uint32_t run = 0;
-                for (uint32_t t = 0; t < tid; ++t) run += a.sync->tile[t];
+                for (uint32_t t = 0; t < tid; ++t) run += a.sync->grid.tile[t];
                 s_off[tid] = run;
             }
             __syncthreads();
-            for (uint32_t c = gt; c < m; c += gs) a.start[c] = a.count[c] + s_off[c / kTickTile];
+            for (uint32_t c = gt; c < m; c += gs) a.start[c] = a.count[c] + s_off[c / kScanTileCells];
             for (uint32_t i = gt; i < n; i += gs) {
                 const uint32_t c = a.key[i];
-                a.tmp[a.count[c] + s_off[c / kTickTile] + atomicAdd(&a.fill[c], 1u)] = i;
+                a.tmp[a.count[c] + s_off[c / kScanTileCells] + atomicAdd(&a.fill[c], 1u)] = i;
             }
-            if (!grid_barrier(a, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             for (uint32_t i = gt; i < n; i += gs) {  // k_rank and k_gather: ascending source order within a cell
                 const uint32_t c = a.key[i], lo = a.start[c], hi = a.start[c + 1];
                 uint32_t p = lo;
@@ -264,7 +202,7 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
                 a.home[p] = c;
                 a.pos_of_slot[s] = p;
             }
-            if (!grid_barrier(a, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             for (uint32_t p = gt; p < n; p += gs) {
                 const double x = a.o.x[p], y = a.o.y[p], z = a.o.z[p];
                 a.b.x[p] = x;
@@ -287,10 +225,10 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
                 a.ref[p] = f;
             }
             for (uint32_t c = gt; c < m; c += gs) a.count[c] = a.fill[c] = 0u;
-            if (!grid_barrier(a, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             for (uint32_t p = gt / 32u; p < n; p += gs / 32u)
                 nl_build_warp_one<true>(a.g, a.pos4, a.home, a.start, p, a.rl2, a.list, a.stride, a.cap_nb, a.cnt);
-            if (!grid_barrier(a, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             parity = 0u;
             ++rebuilds;
         } else if (a.wrap) {
@@ -375,7 +313,7 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
                 }
             }
         }
-        if (!grid_barrier(a, target, &s_ok)) return;
+        if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
         for (uint32_t v = blockIdx.x; v < (uint32_t)nb; v += gridDim.x) {
             const uint32_t i = v * kTickThreads + tid;  // the thread that advances atom i
             double ks = 0.0, ss = 0.0;
@@ -394,13 +332,13 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
             }
         }
         if (a.thermo) {
-            if (!grid_barrier(a, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             const double K = part_sum(a.kpart + par * kPartRow, nb, sh);
             if (tid == 0) s_lam = berendsen_scale(K, n, a.k_thermal, a.target, a.tau);
             __syncthreads();
         }
     }
-    if (REC && !a.thermo && !grid_barrier(a, target, &s_ok)) return;  // the last partials
+    if (REC && !a.thermo && !grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;  // the last partials
     if (recorder) {
         if (REC) take_record(a, a.nticks - 1, s_lam, nb, sh);
         if (tid == 0) {
@@ -410,14 +348,7 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
             a.flag[2] = parity;
         }
     }
-    __syncthreads();
-    if (tid == 0) {  // the last block to leave clears the words for the next launch
-        __threadfence();
-        if (atomicAdd(&a.sync->left, 1u) == gridDim.x - 1) {
-            a.sync->arrived = a.sync->left = 0u;
-            a.sync->request[0] = a.sync->request[1] = 0u;
-        }
-    }
+    grid_leave(&a.sync->grid);
 }
 
 // Lanes per atom of the pair pass: as many as keep the chip filled, since a
@@ -437,7 +368,7 @@ bool nl_ticks_eligible(gx_handle* h) {
     if (h->p.enable_collisions || h->prof_on || h->pass_timing) return false;
     const NlState* s = static_cast<const NlState*>(h->nl);
     if (!s || 0.5 * s->expect * (double)h->n > kTickMaxEntries) return false;
-    return !s->shape_set && s->half == 1 && s->lg.ncell < kTickTile * kTickMaxTiles;
+    return !s->shape_set && s->half == 1 && s->lg.ncell < kScanTileCells * kScanMaxTiles;
 }
 
 // nticks ticks with the records (may be null) at rec[0 .. nticks).
