@@ -190,12 +190,6 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return v;
 }
 
-// min_image1 for |d| <= 0.49 L without the division: the rounded quotient
-// is zero there and d - L * 0 is d itself, sign of a zero included.
-__device__ __forceinline__ double near_image(double d, double L) {
-    return fabs(d) <= xmul(0.49, L) ? d : min_image1(d, L);
-}
-
 // Sum over the kAdjLanes lanes of one atom (a butterfly: every lane ends
 // with the same bits, and the association is fixed, so recomputed ticks
 // reproduce the forward pass exactly).
@@ -661,11 +655,11 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
                     } else {
                         const uint32_t tt = ti + packed_elem(pj.w);
                         const bool far = a.L.coul || a.L.grav;
+                        const double inv = __drcp_rn(d);
                         double fmag = 0.0;
-                        pair_f64_e24(a.L, d, s_sig[tt], s_eps[tt], s_e24[tt], qi, far ? a.charge[j] : 0.0, mi,
+                        pair_f64_e24(a.L, d, inv, s_sig[tt], s_eps[tt], s_e24[tt], qi, far ? a.charge[j] : 0.0, mi,
                                      far ? a.mass[j] : 0.0, fmag, Vij);
                         if (fmag != 0.0) {
-                            const double inv = xdiv(1.0, d);
                             for (int r = 0; r < mult; ++r) {
                                 ax = xadd(ax, xmul(xmul(xmul(dx, inv), fmag), inv_mi));
                                 ay = xadd(ay, xmul(xmul(xmul(dy, inv), fmag), inv_mi));

@@ -90,24 +90,24 @@ __global__ void __launch_bounds__(kForceThreads) k_force_f64(GridGeom g, StateBu
             uint32_t lo = start[B], hi = start[B + 1];
             for (uint32_t j = lo; j < hi; ++j) {
                 if (j == i) continue;
-                double dx = min_image1(xsub(xi, b.x[j]), L.box[0]);
-                double dy = min_image1(xsub(yi, b.y[j]), L.box[1]);
-                double dz = min_image1(xsub(zi, b.z[j]), L.box[2]);
+                double dx = near_image(xsub(xi, b.x[j]), L.box[0]);
+                double dy = near_image(xsub(yi, b.y[j]), L.box[1]);
+                double dz = near_image(xsub(zi, b.z[j]), L.box[2]);
                 double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
                 if (d2 >= L.rc2) continue;
                 double d = xsqrt(d2);
                 if (d <= kEpsF64) continue;
                 bool count = (k < 0) ? (j > i) : half;
-                int tj = b.elem[j];
+                const int tt = ti * kNElem + b.elem[j];
+                const double inv = __drcp_rn(d);
                 double fmag, Vij = 0.0;
-                pair_f64(L, d, psig[ti * kNElem + tj], peps[ti * kNElem + tj], qi, b.charge[j], mi, b.mass[j], fmag,
-                         Vij);
+                pair_f64_e24(L, d, inv, psig[tt], peps[tt], peps[kNElem * kNElem + tt], qi, b.charge[j], mi, b.mass[j],
+                             fmag, Vij);
                 if (count) {
                     V = xadd(V, Vij);
                     ++np;
                 }
                 if (fmag != 0.0) {
-                    double inv = xdiv(1.0, d);
                     ax = xadd(ax, xmul(xmul(xmul(dx, inv), fmag), inv_mi));
                     ay = xadd(ay, xmul(xmul(xmul(dy, inv), fmag), inv_mi));
                     az = xadd(az, xmul(xmul(xmul(dz, inv), fmag), inv_mi));

@@ -48,6 +48,11 @@ __device__ __forceinline__ double rem_euclid(double a, double b) {
 __device__ __forceinline__ double min_image1(double d, double L) {
     return xsub(d, xmul(L, round(xdiv(d, L))));
 }
+// min_image1 for |d| <= 0.49 L without the division: the rounded quotient
+// is zero there and d - L * 0 is d itself, sign of a zero included.
+__device__ __forceinline__ double near_image(double d, double L) {
+    return fabs(d) <= xmul(0.49, L) ? d : min_image1(d, L);
+}
 // min_image1 without the division, for the separation d of two wrapped
 // positions (|d| < L): round(d / L) is then 0 or +-1, and the sign test
 // below gives the same value except for |d| within rounding of L/2; the

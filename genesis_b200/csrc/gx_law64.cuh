@@ -14,65 +14,80 @@ struct LawF64 {
     double k_e, G;
     double box[3];
     int coul, grav;
+    double lj_iw, coul_iw, grav_iw;  // 1 / (rc - r_on), correctly rounded
+    int one_switch;                  // LJ and Coulomb have the same switch
 };
 
+// a / b, correctly rounded, from y = 1 / b correctly rounded (Markstein, IBM
+// J. Res. Dev. 34 (1990) 111): a y lies within two units of the last place,
+// one remainder step makes it faithful and a second one exact.  Quotients
+// near the ends of the range, zeros and non-finite ones take the division.
+// Five operations where a division takes over twenty; the reciprocal of a
+// distance or of a switch's width serves several quotients.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q0 = xmul(a, y);
+    if (!(fabs(q0) > 0x1p-900 && fabs(q0) < 0x1p900)) return xdiv(a, b);
+    const double q1 = fma(fma(-b, q0, a), y, q0);
+    return fma(fma(-b, q1, a), y, q1);
+}
+
 // smooth_cutoff, src/physics/forces.rs:302-318 (exact FP64).
-__device__ __forceinline__ void smooth_f64(double r, double ron, double rc, double& sw, double& dsw) {
+// iw = 1 / (rc - ron), correctly rounded.
+__device__ __forceinline__ void smooth_f64(double r, double ron, double rc, double iw, double& sw, double& dsw) {
     if (r <= ron) { sw = 1.0; dsw = 0.0; return; }
     if (r >= rc) { sw = 0.0; dsw = 0.0; return; }
     double w = xsub(rc, ron);
-    double u = xdiv(xsub(r, ron), w);
+    double u = div_by(xsub(r, ron), w, iw);
     double u2 = xmul(u, u);
     double u3 = xmul(u2, u);
     double u4 = xmul(u3, u);
     double u5 = xmul(u4, u);
     sw = xsub(xadd(xsub(1.0, xmul(10.0, u3)), xmul(15.0, u4)), xmul(6.0, u5));
     double omu = xsub(1.0, u);
-    dsw = xdiv(xmul(xmul(xmul(-30.0, u2), omu), omu), w);
+    dsw = div_by(xmul(xmul(xmul(-30.0, u2), omu), omu), w, iw);
 }
 
 // One pair's LJ + Coulomb + gravity scalar (systems/forces.rs:270-299), exact.
-// e24s = (24 ep) / sg, which depends on the element pair only: a caller may
-// pass it from a table computed with the same two IEEE operations (the same
-// bits) instead of dividing per pair.
-__device__ __forceinline__ void pair_f64_e24(const LawF64& L, double d, double sg, double ep, double e24s, double qa,
-                                             double qb, double ma, double mb, double& fmag, double& V) {
+// inv = 1 / d correctly rounded.  e24s = (24 ep) / sg, which depends on the
+// element pair only: it comes from a table computed with the same two IEEE
+// operations.  A term of no strength adds a zero and is left out.
+__device__ __forceinline__ void pair_f64_e24(const LawF64& L, double d, double inv, double sg, double ep, double e24s,
+                                             double qa, double qb, double ma, double mb, double& fmag, double& V) {
     fmag = 0.0;
-    double sw, dsw;
+    double sw = 0.0, dsw = 0.0;
+    const double half = xmul(0.5, sg);
     if (d < L.lj_rc) {  // force_switched_scalar, forces.rs:270-275; lj_raw :346-353
-        double r = fmax(d, xmul(0.5, sg));
-        double s = xdiv(sg, r);
-        double s6 = xmul(xmul(xmul(xmul(xmul(s, s), s), s), s), s);
-        double s12 = xmul(s6, s6);
-        double v = xmul(xmul(4.0, ep), xsub(s12, s6));
-        double m = xmul(xmul(e24s, s), xsub(xmul(2.0, s12), s6));
-        smooth_f64(r, L.lj_ron, L.lj_rc, sw, dsw);
+        const double r = fmax(d, half);
+        const double s = d >= half ? div_by(sg, d, inv) : xdiv(sg, r);
+        const double s6 = xmul(xmul(xmul(xmul(xmul(s, s), s), s), s), s);
+        const double s12 = xmul(s6, s6);
+        const double v = xmul(xmul(4.0, ep), xsub(s12, s6));
+        const double m = xmul(xmul(e24s, s), xsub(xmul(2.0, s12), s6));
+        smooth_f64(r, L.lj_ron, L.lj_rc, L.lj_iw, sw, dsw);
         fmag = xadd(fmag, xsub(xmul(m, sw), xmul(v, dsw)));
         V = xadd(V, xmul(v, sw));
     }
-    if (L.coul && d < L.coul_rc) {  // :282-289, coulomb_raw :330-333
-        double r = fmax(d, 0.5);
-        double q = xmul(xmul(L.k_e, qa), qb);
-        double m = xdiv(q, xmul(r, r));
-        double v = xdiv(q, r);
-        smooth_f64(d, L.coul_ron, L.coul_rc, sw, dsw);
+    const auto central = [&](double q) {  // coulomb_raw :330-333, gravity_raw :338-341
+        const double r = fmax(d, 0.5);
+        const double m = xdiv(q, xmul(r, r));
+        const double v = d >= 0.5 ? div_by(q, d, inv) : xdiv(q, r);
         fmag = xadd(fmag, xsub(xmul(m, sw), xmul(v, dsw)));
         V = xadd(V, xmul(v, sw));
+    };
+    if (L.coul && d < L.coul_rc) {  // :282-289
+        const double q = xmul(xmul(L.k_e, qa), qb);
+        if (q != 0.0) {
+            if (!(L.one_switch && d >= half)) smooth_f64(d, L.coul_ron, L.coul_rc, L.coul_iw, sw, dsw);
+            central(q);
+        }
     }
-    if (L.grav && d < L.grav_rc) {  // :292-299, gravity_raw :338-341
-        double r = fmax(d, 0.5);
-        double mm = xmul(xmul(L.G, ma), mb);
-        double m = xdiv(-mm, xmul(r, r));
-        double v = xdiv(-mm, r);
-        smooth_f64(d, L.grav_ron, L.grav_rc, sw, dsw);
-        fmag = xadd(fmag, xsub(xmul(m, sw), xmul(v, dsw)));
-        V = xadd(V, xmul(v, sw));
+    if (L.grav && d < L.grav_rc) {  // :292-299
+        const double mm = xmul(xmul(L.G, ma), mb);
+        if (mm != 0.0) {
+            smooth_f64(d, L.grav_ron, L.grav_rc, L.grav_iw, sw, dsw);
+            central(-mm);
+        }
     }
-}
-
-__device__ __forceinline__ void pair_f64(const LawF64& L, double d, double sg, double ep, double qa, double qb,
-                                         double ma, double mb, double& fmag, double& V) {
-    pair_f64_e24(L, d, sg, ep, xdiv(xmul(24.0, ep), sg), qa, qb, ma, mb, fmag, V);
 }
 
 // One observed bond's spring (src/systems/forces.rs:305-317,
@@ -98,7 +113,7 @@ __device__ __forceinline__ bool bond_f64(const LawF64& L, const StateBuf& b, uin
     const double m = xmul(-kk, dr);
     const double v = xmul(xmul(xmul(0.5, kk), dr), dr);
     double sw, dsw;
-    smooth_f64(d, r_eq, rc_bond, sw, dsw);
+    smooth_f64(d, r_eq, rc_bond, __drcp_rn(xsub(rc_bond, r_eq)), sw, dsw);
     fm = xsub(xmul(m, sw), xmul(v, dsw));
     vv = xmul(v, sw);
     const double inv = xdiv(1.0, d);
@@ -133,6 +148,10 @@ inline LawF64 make_law64(const gx_handle* h) {
     L.k_e = h->p.coulomb_constant;
     L.G = h->p.gravity_constant;
     for (int k = 0; k < 3; ++k) L.box[k] = h->p.box[k];
+    L.lj_iw = 1.0 / (L.lj_rc - L.lj_ron);
+    L.coul_iw = 1.0 / (L.coul_rc - L.coul_ron);
+    L.grav_iw = 1.0 / (L.grav_rc - L.grav_ron);
+    L.one_switch = L.lj_rc == L.coul_rc && L.lj_ron == L.coul_ron;
     L.coul = h->p.enable_electrostatics ? 1 : 0;
     L.grav = h->p.enable_gravity ? 1 : 0;
     return L;

@@ -1010,102 +1010,57 @@ __global__ void __launch_bounds__(kRedThreads) k_nl_finish(StateBuf b, const lon
     }
 }
 
-// Plain FP64 pass over the full list: one thread per atom visits every
-// neighbour of its list (within r_c + skin at the last rebuild) in the
-// build's order with the reference's exact per-pair arithmetic (the
-// minimum image of the FP64 positions, pair_f64) and sums its acceleration
-// in that order: no atomics, deterministic.  The list build used the FP32
-// staging; its radius exceeds r_c + skin by 1e-6 relative and the staging
-// error is ~1e-6 absolute, both far inside the skin/2 margin, so every pair
-// with d < r_c in FP64 is in the list.  V and the pair count take each
-// unordered pair once (q > p).
-__global__ void __launch_bounds__(kNlThreads) k_nl_force64(GridGeom g, StateBuf b, const uint32_t* __restrict__ home,
-                                                            const uint32_t* __restrict__ start, uint32_t n, LawF64 L,
-                                                            const double* __restrict__ psig,
+// Plain FP64 pass over the full list, nl_atom64's lanes per atom: no atomics,
+// deterministic.  The list build used the FP32 staging; its radius exceeds
+// r_c + skin by 1e-6 relative and the staging error is ~1e-6 absolute, both
+// far inside the skin/2 margin, so every pair with d < r_c in FP64 is in the
+// list.  The atom's potential goes to vat for the finish to sum.
+// Bound by the latency of the gathers and of the dependent FP64 operations:
+// eight blocks per SM (64 registers, a few spilled) take 217 us at 250,047
+// atoms where five take 260 and seven 219; with divisions for every quotient
+// and one thread per atom it was 399 us (215 M warp instructions, 134 M now).
+__global__ void __launch_bounds__(kNlThreads, 8) k_nl_force64(GridGeom g, StateBuf b, const uint32_t* __restrict__ home,
+                                                            const uint32_t* __restrict__ start, uint32_t n,
+                                                            uint32_t lanes, LawF64 L, const double* __restrict__ psig,
                                                             const double* __restrict__ peps,
                                                             const uint32_t* __restrict__ list, size_t stride,
                                                             int cap_nb, const uint32_t* __restrict__ cnt,
-                                                            double* __restrict__ vpart,
+                                                            double* __restrict__ vat,
                                                             unsigned long long* __restrict__ npairs) {
-    __shared__ double shd[kNlThreads / 32];
     __shared__ unsigned long long shu[kNlThreads / 32];
-    const uint32_t i = blockIdx.x * kNlThreads + threadIdx.x;
-    double V = 0.0;
-    unsigned long long np = 0;
-    if (i < n) {
-        const double xi = b.x[i], yi = b.y[i], zi = b.z[i];
-        const int ti = b.elem[i];
-        const double qi = b.charge[i], mi = b.mass[i], inv_mi = b.inv_mass[i];
-        double ax = 0.0, ay = 0.0, az = 0.0;
-        // the list grid has >= 3 cells per axis (min_image_near)
-        const double hx = xmul(0.5, L.box[0]), hy = xmul(0.5, L.box[1]), hz = xmul(0.5, L.box[2]);
-        auto visit = [&](uint32_t j) {
-            const double dx = min_image_near(xsub(xi, b.x[j]), L.box[0], hx);
-            const double dy = min_image_near(xsub(yi, b.y[j]), L.box[1], hy);
-            const double dz = min_image_near(xsub(zi, b.z[j]), L.box[2], hz);
-            const double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
-            if (d2 >= L.rc2) return;
-            const double d = xsqrt(d2);
-            if (d <= kEpsF64) return;
-            const int tj = b.elem[j];
-            double fmag, Vij = 0.0;
-            const int tt = ti * kNElem + tj;  // psig, then peps, then (24 eps) / sigma, each kNElem^2
-            pair_f64_e24(L, d, psig[tt], peps[tt], peps[kNElem * kNElem + tt], qi, b.charge[j], mi, b.mass[j], fmag,
-                         Vij);
-            if (j > i) {
-                V = xadd(V, Vij);
-                ++np;
-            }
-            if (fmag != 0.0) {
-                const double inv = xdiv(1.0, d);
-                ax = xadd(ax, xmul(xmul(xmul(dx, inv), fmag), inv_mi));
-                ay = xadd(ay, xmul(xmul(xmul(dy, inv), fmag), inv_mi));
-                az = xadd(az, xmul(xmul(xmul(dz, inv), fmag), inv_mi));
-            }
-        };
-        const uint32_t m = cnt[i];
-        if (m <= (uint32_t)cap_nb) {
-            const uint32_t* lp = list + i;
-            for (uint32_t e = 0; e < m; ++e) visit(__ldg(lp + (size_t)e * stride) & kIdxMask);
-        } else {  // overflowed list: every atom of the 27 home-grid cells
-            uint32_t cx, cy, cz;
-            decode(g, home[i], cx, cy, cz);
-            for (uint32_t code = 0; code < 27; ++code) {
-                const uint32_t B = cell_at(g, cx, cy, cz, code);
-                for (uint32_t q = start[B], hi = start[B + 1]; q < hi; ++q)
-                    if (q != i) visit(q);
-            }
-        }
-        b.ax[i] = ax;
-        b.ay[i] = ay;
-        b.az[i] = az;
+    const uint32_t t = blockIdx.x * kNlThreads + threadIdx.x;
+    const uint32_t i = t / lanes, sub = t % lanes;
+    Acc64 a;
+    if (i < n) nl_atom64(g, b, home, start, L, psig, peps, list, stride, cap_nb, cnt, i, sub, lanes, a);
+    nl_sum64(a, lanes);
+    if (i < n && sub == 0) {
+        b.ax[i] = a.ax;
+        b.ay[i] = a.ay;
+        b.az[i] = a.az;
+        vat[i] = a.V;
     }
-    V = block_sum_d<kNlThreads>(V, shd);
-    np = block_sum_u<kNlThreads>(np, shu);
-    if (threadIdx.x == 0) {
-        vpart[blockIdx.x] = V;
-        if (np) atomicAdd(npairs, np);
-    }
+    const unsigned long long np = block_sum_u<kNlThreads>(a.np, shu);
+    if (threadIdx.x == 0 && np) atomicAdd(npairs, np);
 }
 
 // FP64 second kick (as k_kick) and, with THERMO, the kinetic-energy partials
-// with k_nl_finish's block mapping and operation order.
+// with k_nl_finish's block mapping and operation order; THERMO = 2 also the
+// speed partials and those of the atoms' potentials.
 template <int THERMO>
 __global__ void __launch_bounds__(kRedThreads) k_nl_finish64(StateBuf b, uint32_t n, double half_dt,
-                                                             double* __restrict__ kpart, double* __restrict__ spart) {
+                                                             double* __restrict__ kpart, double* __restrict__ spart,
+                                                             const double* __restrict__ vat,
+                                                             double* __restrict__ vpart) {
     __shared__ double sh[kRedThreads / 32];
-    double ks = 0.0, ss = 0.0;
+    double ks = 0.0, ss = 0.0, vs = 0.0;
     for (uint32_t i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
-        const double vx = xadd(b.vx[i], xmul(b.ax[i], half_dt));
-        const double vy = xadd(b.vy[i], xmul(b.ay[i], half_dt));
-        const double vz = xadd(b.vz[i], xmul(b.az[i], half_dt));
-        b.vx[i] = vx;
-        b.vy[i] = vy;
-        b.vz[i] = vz;
+        const double l2 = nl_finish64_one(b, i, half_dt);
         if (THERMO) {
-            double l2 = xadd(xadd(xmul(vx, vx), xmul(vy, vy)), xmul(vz, vz));
             ks = xadd(ks, xmul(xmul(0.5, b.mass[i]), l2));
-            if (THERMO == 2) ss = xadd(ss, xsqrt(l2));
+            if (THERMO == 2) {
+                ss = xadd(ss, xsqrt(l2));
+                vs = xadd(vs, vat[i]);
+            }
         }
     }
     if (THERMO) {
@@ -1115,6 +1070,8 @@ __global__ void __launch_bounds__(kRedThreads) k_nl_finish64(StateBuf b, uint32_
     if (THERMO == 2) {
         ss = block_sum_d<kRedThreads>(ss, sh);
         if (threadIdx.x == 0) spart[blockIdx.x] = ss;
+        vs = block_sum_d<kRedThreads>(vs, sh);
+        if (threadIdx.x == 0) vpart[blockIdx.x] = vs;
     }
 }
 
@@ -1330,12 +1287,11 @@ int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, in
     LawF32 L = make_law32(h);
     prof_begin(h, "force_nl");
     if (f64) {
-        double* vpart = h->red;  // row 0 of the block partials
         const double* psig = d_psig(h);
-        const unsigned fb = nblk(n, kNlThreads);
-        GX_LAUNCH(h, k_nl_force64, fb, kNlThreads, g, b, h->key_sorted, s->cl.start, n, make_law64(h), psig,
-                  psig + kNElem * kNElem, s->list, s->cap, s->cap_nb, s->cnt, vpart, h->dcount + 0);
-        launch_sum_rows(h, vpart, (int)fb, h->dscal + 2);
+        const uint32_t lanes = nl_auto_lanes64(n);
+        GX_LAUNCH(h, k_nl_force64, nblk((size_t)n * lanes, kNlThreads), kNlThreads, g, b, h->key_sorted, s->cl.start, n,
+                  lanes, make_law64(h), psig, psig + kNElem * kNElem, s->list, s->cap, s->cap_nb, s->cnt,
+                  reinterpret_cast<double*>(h->F), h->dcount + 0);  // the fixed-point sums' room holds the potentials
     } else if (halfl) {
         launch_nl_force<true>(h, nl_lanes(s, n), g, s, n, L, energy);
     } else {
@@ -1354,7 +1310,9 @@ int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, in
     const int mode = kpart ? (spart ? 2 : 1) : 0;
     if (f64) {
         auto k = mode == 2 ? k_nl_finish64<2> : (mode == 1 ? k_nl_finish64<1> : k_nl_finish64<0>);
-        GX_LAUNCH(h, k, nb, kRedThreads, b, n, half_dt, kpart, spart);
+        double* vpart = h->red;  // row 0 of the block partials
+        GX_LAUNCH(h, k, nb, kRedThreads, b, n, half_dt, kpart, spart, reinterpret_cast<const double*>(h->F), vpart);
+        if (mode == 2) launch_sum_rows(h, vpart, nb, h->dscal + 2);
         if (!spring) GX_CUDA(h, cudaMemsetAsync(h->dscal + 3, 0, sizeof(double), h->stream));
     } else {
         auto k = mode == 2 ? k_nl_finish<2> : (mode == 1 ? k_nl_finish<1> : k_nl_finish<0>);

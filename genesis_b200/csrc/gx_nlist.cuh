@@ -4,6 +4,7 @@
 #pragma once
 
 #include "gx_gridsync.cuh"
+#include "gx_law64.cuh"
 #include "gx_pair_f32.cuh"
 
 namespace gx {
@@ -42,13 +43,14 @@ struct NlState {
     uint32_t body_runs_seen = 0;
     TickSync* tick_sync = nullptr;
     bool tick_sync_dirty = false;  // a launch gave up: clear the words before the next one
-    int tick_blocks[2] = {0, 0};   // resident blocks of the one-launch tick, without / with records
+    int tick_blocks[4] = {0, 0, 0, 0};  // resident blocks of the one-launch tick: without / with records, mixed then FP64
 };
 
 // Universes up to this many atoms and expected half-list entries run their
 // ticks in one launch (gx_nltick.cu, where both sides' times stand).
 constexpr size_t kTickMaxAtoms = 65536;
 constexpr double kTickMaxEntries = 1.7e6;
+constexpr size_t kTickMaxAtoms64 = 24576;  // FP64 ticks
 // Ticks of one launch at most, so that a long call stays a queue of launches.
 constexpr int kTicksPerLaunch = 256;
 
@@ -270,6 +272,106 @@ __device__ __forceinline__ double nl_finish_one(const StateBuf& b, const long lo
     const double vx = xadd(b.vx[i], xmul(ax, half_dt));
     const double vy = xadd(b.vy[i], xmul(ay, half_dt));
     const double vz = xadd(b.vz[i], xmul(az, half_dt));
+    b.vx[i] = vx;
+    b.vy[i] = vy;
+    b.vz[i] = vz;
+    return xadd(xadd(xmul(vx, vx), xmul(vy, vy)), xmul(vz, vz));
+}
+
+// The FP64 pass over one atom's full list, the reference's exact per-pair
+// arithmetic: lane `sub` of `lanes` takes entries sub, sub + lanes, ... in the
+// build's order, positions loaded one entry ahead.  V and the pair count take
+// each unordered pair once (the later sorted position's visit).
+struct Acc64 {
+    double ax = 0.0, ay = 0.0, az = 0.0, V = 0.0;
+    unsigned int np = 0;
+};
+
+__device__ __forceinline__ void nl_atom64(const GridGeom& g, const StateBuf& b, const uint32_t* home,
+                                          const uint32_t* start, const LawF64& L, const double* psig,
+                                          const double* peps, const uint32_t* list, size_t stride, int cap_nb,
+                                          const uint32_t* cnt, uint32_t i, uint32_t sub, uint32_t lanes, Acc64& a) {
+    const double xi = b.x[i], yi = b.y[i], zi = b.z[i];
+    const int ti = b.elem[i] * kNElem;
+    const double qi = b.charge[i], mi = b.mass[i], inv_mi = b.inv_mass[i];
+    // the list grid has >= 3 cells per axis (min_image_near)
+    const double hx = xmul(0.5, L.box[0]), hy = xmul(0.5, L.box[1]), hz = xmul(0.5, L.box[2]);
+    const auto visit = [&](uint32_t j, double xj, double yj, double zj) {
+        const double dx = min_image_near(xsub(xi, xj), L.box[0], hx);
+        const double dy = min_image_near(xsub(yi, yj), L.box[1], hy);
+        const double dz = min_image_near(xsub(zi, zj), L.box[2], hz);
+        const double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
+        if (d2 >= L.rc2) return;
+        const int tt = ti + b.elem[j];  // psig, then peps, then (24 eps) / sigma, each kNElem^2
+        const double qj = b.charge[j], mj = L.grav ? b.mass[j] : 0.0;
+        const double d = xsqrt(d2);
+        if (d <= kEpsF64) return;
+        const double inv = __drcp_rn(d);
+        double fmag, Vij = 0.0;
+        pair_f64_e24(L, d, inv, psig[tt], peps[tt], peps[kNElem * kNElem + tt], qi, qj, mi, mj, fmag, Vij);
+        if (j > i) {
+            a.V = xadd(a.V, Vij);
+            ++a.np;
+        }
+        if (fmag != 0.0) {
+            a.ax = xadd(a.ax, xmul(xmul(xmul(dx, inv), fmag), inv_mi));
+            a.ay = xadd(a.ay, xmul(xmul(xmul(dy, inv), fmag), inv_mi));
+            a.az = xadd(a.az, xmul(xmul(xmul(dz, inv), fmag), inv_mi));
+        }
+    };
+    const uint32_t m = cnt[i];
+    if (m <= (uint32_t)cap_nb) {
+        if (sub >= m) return;
+        const uint32_t* lp = list + i;
+        uint32_t j = lp[(size_t)sub * stride] & kIdxMask;
+        double xj = b.x[j], yj = b.y[j], zj = b.z[j];
+        for (uint32_t e = sub; e < m; e += lanes) {
+            const uint32_t next = e + lanes < m ? lp[(size_t)(e + lanes) * stride] & kIdxMask : j;
+            const double xn = b.x[next], yn = b.y[next], zn = b.z[next];
+            visit(j, xj, yj, zj);
+            j = next;
+            xj = xn;
+            yj = yn;
+            zj = zn;
+        }
+    } else {  // overflowed list: the lanes split the 27 home-grid cells
+        uint32_t cx, cy, cz;
+        decode(g, home[i], cx, cy, cz);
+        for (uint32_t code = sub; code < 27; code += lanes) {
+            const uint32_t B = cell_at(g, cx, cy, cz, code);
+            for (uint32_t q = start[B], hi = start[B + 1]; q < hi; ++q)
+                if (q != i) visit(q, b.x[q], b.y[q], b.z[q]);
+        }
+    }
+}
+
+// The lanes' sums of one atom, in a fixed association (every lane ends with
+// them).
+__device__ __forceinline__ void nl_sum64(Acc64& a, uint32_t lanes) {
+    for (uint32_t o = lanes >> 1; o > 0; o >>= 1) {
+        a.ax += __shfl_xor_sync(0xffffffffu, a.ax, o);
+        a.ay += __shfl_xor_sync(0xffffffffu, a.ay, o);
+        a.az += __shfl_xor_sync(0xffffffffu, a.az, o);
+        a.V += __shfl_xor_sync(0xffffffffu, a.V, o);
+    }
+}
+
+// Lanes per atom of the FP64 pass: enough that no lane's chain of dependent
+// operations sets the pass.  Microseconds per pass with 1 / 2 / 4 / 8 / 16 / 32
+// lanes: 64 / 37 / 23 / 14 / 12 / 10 at 512 atoms, 68 / 39 / 25 / 16 / 12 / 14
+// at 4,096, 70 / 39 / 25 / 27 / 27 / 31 at 13,824; with 1 / 2 / 4:
+// 86 / 53 / 39 at 32,768, 248 / 225 / 217 at 250,047, 876 / 805 / 811 at
+// 1,000,000.
+inline uint32_t nl_auto_lanes64(uint32_t n) {
+    if (n <= 8192) return n <= 2048 ? 32 : 16;
+    return n <= 400000 ? 4 : 2;
+}
+
+// FP64 second kick of one atom (as k_kick); returns |v|^2.
+__device__ __forceinline__ double nl_finish64_one(const StateBuf& b, uint32_t i, double half_dt) {
+    const double vx = xadd(b.vx[i], xmul(b.ax[i], half_dt));
+    const double vy = xadd(b.vy[i], xmul(b.ay[i], half_dt));
+    const double vz = xadd(b.vz[i], xmul(b.az[i], half_dt));
     b.vx[i] = vx;
     b.vy[i] = vy;
     b.vz[i] = vz;

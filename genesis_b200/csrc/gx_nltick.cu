@@ -33,7 +33,9 @@
 // from about 1.7 M list entries the kernels win (73 / 73 at 2.6 M, 98 / 93 at
 // 3.4 M, 202 / 143 at 7.1 M): their pair pass keeps more warps resident than
 // the one kernel that holds every phase.  Four blocks per SM (64 registers):
-// 54 us at 59,319 atoms, against 55 with three and 57 with five.
+// 54 us at 59,319 atoms, against 55 with three and 57 with five.  FP64, here /
+// as kernels: 21 / 36 at 512 atoms, 26 / 43 at 4,096, 46 / 62 at 13,824, 78 /
+// 74 at 32,768.
 #include <algorithm>
 
 #include "gx_gridsync.cuh"
@@ -63,7 +65,7 @@ struct TickArgs {
     uint32_t* cnt;
     long long* F;
     size_t fstride;
-    double *kpart, *spart, *dscal;
+    double *kpart, *spart, *vpart, *dscal;
     uint32_t* flag;
     uint32_t* err;
     TickSync* sync;
@@ -87,13 +89,15 @@ __device__ __forceinline__ double part_sum(const double* part, int nb, double* s
 
 // The record of one finished tick, by one block: K and the speed sum from its
 // partials, the potential, bond energy and pair count from its counters.
+template <bool F64>
 __device__ __forceinline__ void take_record(const TickArgs& a, int tick, double lam, int nb, double* sh) {
     const int par = tick & 1;
     const double K = part_sum(a.kpart + par * kPartRow, nb, sh);
     const double S = part_sum(a.spart + par * kPartRow, nb, sh);
+    const double V64 = F64 ? part_sum(a.vpart + par * kPartRow, nb, sh) : 0.0;
     if (threadIdx.x != 0) return;
     const unsigned long long* c = a.sync->acc[par];
-    const double V = xmul(__ll2double_rn((long long)c[0]), kFixInv);
+    const double V = F64 ? V64 : xmul(__ll2double_rn((long long)c[0]), kFixInv);
     const double Vb = xmul(__ll2double_rn((long long)c[2]), kFixInv);
     gx_tick_stats& r = a.rec[tick];
     r.kinetic = a.thermo ? xmul(xmul(K, lam), lam) : K;
@@ -108,9 +112,11 @@ __device__ __forceinline__ void take_record(const TickArgs& a, int tick, double 
     a.dscal[4] = S;
 }
 
-template <bool REC>
-__global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_constant__ TickArgs a) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
+// F64: the plain FP64 tick over the full list (nl_atom64); the atoms'
+// potentials lie in the room of the fixed-point sums until the finish.
+template <bool REC, bool F64>
+__global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __grid_constant__ TickArgs a) {
+    __shared__ PairF st[F64 ? 1 : kMaxKinds * kMaxKinds];
     __shared__ float4 s_shift[27];
     __shared__ double sh[kTickThreads / 32];
     __shared__ unsigned long long shu[kTickThreads / 32];
@@ -123,7 +129,8 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
     const int nb = (int)((n + kTickThreads - 1) / kTickThreads);
     const bool recorder = blockIdx.x == gridDim.x - 1;
     uint32_t target = 0;  // thread 0's count of barrier arrivals
-    const int nk2 = a.L.nkinds * a.L.nkinds;
+    const int nk2 = F64 ? 0 : a.L.nkinds * a.L.nkinds;
+    double* vat = reinterpret_cast<double*>(a.F);
     for (int t = tid; t < nk2; t += kTickThreads) st[t] = a.tab[t];
     if (tid < 27) {
         float sx, sy, sz;
@@ -141,9 +148,11 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
         const bool half = ((parity + (a.wrap ? 1u : 0u)) & 1u) != 0u;
         bool over = false;
         for (uint32_t i = gt; i < n; i += gs) {
-            a.F[i] = 0;
-            a.F[a.fstride + i] = 0;
-            a.F[2 * a.fstride + i] = 0;
+            if (!F64) {
+                a.F[i] = 0;
+                a.F[a.fstride + i] = 0;
+                a.F[2 * a.fstride + i] = 0;
+            }
             over |= nl_advance_one(a.b, i, &s_lam, a.half_dt, a.dt, a.hx, a.hy, a.hz, a.wrap, a.g, a.home, a.pos4,
                                    a.ref, a.lim2, half, a.err);
         }
@@ -151,7 +160,7 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
         if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
         const bool rebuild = (tick == 0 && asked) || *(volatile uint32_t*)&a.sync->grid.request[par] != 0u;
         if (recorder) {  // the other parity's words: every block has left that tick's pair pass
-            if (REC && tick > 0) take_record(a, tick - 1, s_lam, nb, sh);
+            if (REC && tick > 0) take_record<F64>(a, tick - 1, s_lam, nb, sh);
             __syncthreads();
             if (tid < 4) a.sync->acc[par ^ 1][tid] = 0ull;
             if (tid == 4) a.sync->grid.request[par ^ 1] = 0u;
@@ -227,14 +236,37 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
             for (uint32_t c = gt; c < m; c += gs) a.count[c] = a.fill[c] = 0u;
             if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             for (uint32_t p = gt / 32u; p < n; p += gs / 32u)
-                nl_build_warp_one<true>(a.g, a.pos4, a.home, a.start, p, a.rl2, a.list, a.stride, a.cap_nb, a.cnt);
+                nl_build_warp_one<!F64>(a.g, a.pos4, a.home, a.start, p, a.rl2, a.list, a.stride, a.cap_nb, a.cnt);
             if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             parity = 0u;
             ++rebuilds;
         } else if (a.wrap) {
             parity ^= 1u;
         }
-        {  // pair pass: k_nl_force_tpp's loop
+        if (F64) {  // pair pass: k_nl_force64
+            const uint32_t lanes = 1u << a.lanes_log2, sub = tid & (lanes - 1u);
+            const uint32_t end = ((n << a.lanes_log2) + 31u) & ~31u;  // whole warps
+            unsigned int np = 0;
+            for (uint32_t t = gt; t < end; t += gs) {
+                const uint32_t i = t >> a.lanes_log2;
+                Acc64 f;
+                if (i < n)
+                    nl_atom64(a.g, a.b, a.home, a.start, a.L64, a.psig, a.peps, a.list, a.stride, a.cap_nb, a.cnt, i,
+                              sub, lanes, f);
+                nl_sum64(f, lanes);
+                if (i < n && sub == 0) {
+                    a.b.ax[i] = f.ax;
+                    a.b.ay[i] = f.ay;
+                    a.b.az[i] = f.az;
+                    vat[i] = f.V;
+                }
+                np += f.np;
+            }
+            if (REC) {
+                const unsigned long long c = block_sum_u<kTickThreads>(np, shu);
+                if (tid == 0 && c) atomicAdd(&a.sync->acc[par][1], c);
+            }
+        } else {  // pair pass: k_nl_force_tpp's loop
             const uint32_t lanes = 1u << a.lanes_log2, sub = tid & (lanes - 1u);
             const uint32_t end = ((n << a.lanes_log2) + 31u) & ~31u;  // whole warps
             long long vq = 0;
@@ -316,11 +348,13 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
         if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
         for (uint32_t v = blockIdx.x; v < (uint32_t)nb; v += gridDim.x) {
             const uint32_t i = v * kTickThreads + tid;  // the thread that advances atom i
-            double ks = 0.0, ss = 0.0;
+            double ks = 0.0, ss = 0.0, vs = 0.0;
             if (i < n) {
-                const double l2 = nl_finish_one(a.b, a.F, a.fstride, i, a.half_dt);
+                const double l2 = F64 ? nl_finish64_one(a.b, i, a.half_dt)
+                                      : nl_finish_one(a.b, a.F, a.fstride, i, a.half_dt);
                 ks = xadd(0.0, xmul(xmul(0.5, a.b.mass[i]), l2));
                 if (REC) ss = xadd(0.0, xsqrt(l2));
+                if (REC && F64) vs = xadd(0.0, vat[i]);
             }
             if (REC || a.thermo) {
                 ks = block_sum_d<kTickThreads>(ks, sh);
@@ -329,6 +363,10 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
             if (REC) {
                 ss = block_sum_d<kTickThreads>(ss, sh);
                 if (tid == 0) a.spart[par * kPartRow + v] = ss;
+            }
+            if (REC && F64) {
+                vs = block_sum_d<kTickThreads>(vs, sh);
+                if (tid == 0) a.vpart[par * kPartRow + v] = vs;
             }
         }
         if (a.thermo) {
@@ -340,7 +378,7 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
     }
     if (REC && !a.thermo && !grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;  // the last partials
     if (recorder) {
-        if (REC) take_record(a, a.nticks - 1, s_lam, nb, sh);
+        if (REC) take_record<F64>(a, a.nticks - 1, s_lam, nb, sh);
         if (tid == 0) {
             a.dscal[0] = a.thermo ? s_lam : 1.0;
             a.flag[0] = 0u;
@@ -357,6 +395,8 @@ __global__ void __launch_bounds__(kTickThreads, 4) k_nl_ticks(const __grid_const
 // 22.0 / 20.1 / 22.1 / 31.7 at 4,096, 30.3 / 26.1 / 25.5 / 33.4 at 13,824,
 // 49.7 / 42.0 / 42.9 / 52.4 at 32,768 and - / 59.5 / 56.1 / 63.0 at 59,319.
 inline uint32_t tick_lanes(uint32_t n) { return n <= 2048 ? 32 : (n <= 8192 ? 16 : 8); }
+// The FP64 pass keeps the per-kernel tick's lanes: its sums depend on them.
+inline uint32_t tick_lanes64(uint32_t n) { return nl_auto_lanes64(n); }
 
 }  // namespace
 
@@ -364,11 +404,13 @@ inline uint32_t tick_lanes(uint32_t n) { return n <= 2048 ? 32 : (n <= 8192 ? 16
 // collision pass, no per-launch timing, and a size at which the launches and
 // not the work set the tick.
 bool nl_ticks_eligible(gx_handle* h) {
-    if (h->n == 0 || h->n > kTickMaxAtoms || h->precision != GX_MIXED || h->kernel_variant != 0) return false;
+    const bool mixed = h->precision == GX_MIXED;
+    if (h->n == 0 || h->n > (mixed ? kTickMaxAtoms : kTickMaxAtoms64)) return false;
+    if (mixed ? h->kernel_variant != 0 : bonds_on(h)) return false;  // the FP64 spring adds to finished accelerations
     if (h->p.enable_collisions || h->prof_on || h->pass_timing) return false;
     const NlState* s = static_cast<const NlState*>(h->nl);
-    if (!s || 0.5 * s->expect * (double)h->n > kTickMaxEntries) return false;
-    return !s->shape_set && s->half == 1 && s->lg.ncell < kScanTileCells * kScanMaxTiles;
+    if (!s || (mixed && 0.5 * s->expect * (double)h->n > kTickMaxEntries)) return false;
+    return !s->shape_set && s->half == (mixed ? 1 : 0) && s->lg.ncell < kScanTileCells * kScanMaxTiles;
 }
 
 // nticks ticks with the records (may be null) at rec[0 .. nticks).
@@ -383,8 +425,10 @@ int nl_ticks(gx_handle* h, int nticks, gx_tick_stats* rec, bool thermo, double t
         GX_CUDA(h, cudaMemsetAsync(s->tick_sync, 0, sizeof(TickSync), h->stream));
         s->tick_sync_dirty = false;
     }
-    auto kern = rec ? k_nl_ticks<true> : k_nl_ticks<false>;
-    int& resident = s->tick_blocks[rec ? 1 : 0];
+    const bool f64 = h->precision != GX_MIXED;
+    auto kern = f64 ? (rec ? k_nl_ticks<true, true> : k_nl_ticks<false, true>)
+                    : (rec ? k_nl_ticks<true, false> : k_nl_ticks<false, false>);
+    int& resident = s->tick_blocks[(f64 ? 2 : 0) + (rec ? 1 : 0)];
     if (!resident) {
         int per = 0, sms = 0;
         GX_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kTickThreads, 0));
@@ -396,11 +440,11 @@ int nl_ticks(gx_handle* h, int nticks, gx_tick_stats* rec, bool thermo, double t
     a.o = h->buf[h->cur ^ 1];
     a.g = s->lg;
     a.n = n;
-    const uint32_t lanes = tick_lanes(n);
+    const uint32_t lanes = f64 ? tick_lanes64(n) : tick_lanes(n);
     uint32_t log2 = 0;
     while ((1u << log2) < lanes) ++log2;
     a.lanes_log2 = log2;
-    a.L = make_law32(h);
+    if (!f64) a.L = make_law32(h);
     a.L64 = make_law64(h);
     a.tab = h->d_pairf;
     a.psig = d_psig(h);
@@ -422,6 +466,7 @@ int nl_ticks(gx_handle* h, int nticks, gx_tick_stats* rec, bool thermo, double t
     a.fstride = h->cap;
     a.kpart = kpart;
     a.spart = spart;
+    a.vpart = h->red;  // row 0 of the block partials
     a.dscal = h->dscal;
     a.flag = s->flag;
     a.err = h->derr;

@@ -36,12 +36,14 @@ def _pair(cfg, u, ticks, bonds=None, skin=None, precision="mixed"):
     return ra
 
 
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
 @pytest.mark.parametrize("n_side,coul,target", [(8, False, 0.0), (9, True, 40.0), (16, False, 0.0), (16, True, 40.0),
                                                 (25, True, 0.0), (40, True, 300.0)])
-def test_one_launch_ticks_match_the_per_kernel_ticks(gpu, n_side, coul, target):
+def test_one_launch_ticks_match_the_per_kernel_ticks(gpu, n_side, coul, target, precision):
     wl = W.Workload("tick check", n_side=n_side, temperature=200.0, steps=10, electrostatics=coul,
                     thermostat=target > 0.0, thermostat_temperature=target if target > 0.0 else 300.0)
-    rebuilds = _pair(wl.config(), wl.generate(), [(1, True), (2, False), (7, True), (1, False), (9, True)])
+    rebuilds = _pair(wl.config(), wl.generate(), [(1, True), (2, False), (7, True), (1, False), (9, True)],
+                     precision=precision)
     assert rebuilds >= 2
 
 
@@ -75,6 +77,7 @@ def test_one_launch_sparse_box_and_overflowing_clump(gpu):
     u.pos[300:] = rng.uniform(-0.5 * L, 0.5 * L, size=(700, 3))
     u.vel[:] *= 0.01
     _pair(cfg, u, [(3, True), (1, False)])
+    _pair(cfg, u, [(3, True), (1, False)], precision="fp64")
 
 
 def test_one_launch_tick_reports_and_recovers_from_a_non_finite_velocity(gpu):
