@@ -313,6 +313,16 @@ void free_arrays(gx_batch* b) {
 
 }  // namespace
 
+// The three columns of a vector as the caller's rows.
+__global__ void k_batch_aos(const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
+                            double* __restrict__ aos, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    aos[3 * (size_t)i] = x[i];
+    aos[3 * (size_t)i + 1] = y[i];
+    aos[3 * (size_t)i + 2] = z[i];
+}
+
 extern "C" {
 
 const char* gx_batch_last_error(const gx_batch* b) { return b ? b->err.c_str() : "null batch"; }
@@ -628,17 +638,17 @@ int gx_batch_get_state(gx_batch* b, double* pos, double* vel, double* acc) {
     if (!b) return GX_ERR_ARG;
     if (!b->has_state) return berr(b, GX_ERR_STATE, "no state uploaded");
     const size_t total = b->total;
-    std::vector<double> col(total);
     double* outs[3] = {pos, vel, acc};
     double* srcs[3][3] = {{b->A.x, b->A.y, b->A.z}, {b->A.vx, b->A.vy, b->A.vz}, {b->A.ax, b->A.ay, b->A.az}};
-    GXB_CUDA(b, cudaStreamSynchronize(b->stream));
+    double* stage = reinterpret_cast<double*>(b->A.F);  // zeroed by every tick before it is summed into
     for (int q = 0; q < 3; ++q) {
-        if (!outs[q]) continue;
-        for (int k = 0; k < 3; ++k) {
-            GXB_CUDA(b, cudaMemcpy(col.data(), srcs[q][k], total * sizeof(double), cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < total; ++i) outs[q][3 * i + k] = col[i];
-        }
+        if (!outs[q] || !total) continue;
+        k_batch_aos<<<(unsigned)((total + 255) / 256), 256, 0, b->stream>>>(srcs[q][0], srcs[q][1], srcs[q][2], stage,
+                                                                            (uint32_t)total);
+        GXB_CUDA(b, cudaGetLastError());
+        GXB_CUDA(b, cudaMemcpyAsync(outs[q], stage, 3 * total * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     }
+    GXB_CUDA(b, cudaStreamSynchronize(b->stream));
     return GX_OK;
 }
 
