@@ -496,7 +496,7 @@ template <bool F32>
 __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_constant__ AdjArgs a) {
     extern __shared__ uint32_t s_hist[];  // with obs a histogram per warp: low 16 bits' sums, then the rest's
     __shared__ double s_sig[kNElem * kNElem], s_eps[kNElem * kNElem], s_e24[kNElem * kNElem];
-    __shared__ PairF s_tab[F32 ? kMaxKinds * kMaxKinds : 1];
+    __shared__ PairTab s_tab;
     __shared__ double sh[kAdjThreads / 32], s_r[kAdjMaxBins], s_queue[kAdjThreads / 32][kAdjQueue];
     __shared__ uint32_t s_queued[kAdjThreads / 32];
     __shared__ uint32_t s_warp[kAdjThreads / 32], s_off[kScanMaxTiles];
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
         s_e24[k] = xdiv(xmul(24.0, a.peps[k]), a.psig[k]);
     }
     if (F32)
-        for (int k = tid; k < a.L32.nkinds * a.L32.nkinds; k += kAdjThreads) s_tab[k] = a.tabf[k];
+        for (int k = tid; k < a.L32.nkinds * a.L32.nkinds; k += kAdjThreads) s_tab.put(k, a.tabf[k]);
     for (int k = tid; k < (kAdjThreads / 32) * 2 * bins; k += kAdjThreads) s_hist[k] = 0u;
     for (int k = tid; k < bins; k += kAdjThreads) s_r[k] = (k + 0.5) * a.gs.dr;
     uint32_t* wh = s_hist + (tid / 32) * 2 * bins;

@@ -406,7 +406,6 @@ int upload_pairf(gx_handle* h) {
             double sg = h->fs.pair_sigma[ea * kNElem + eb], ep = h->fs.pair_eps[ea * kNElem + eb];
             PairF& t = tab[a * nk + b];
             t.sigma = (float)sg;
-            t.half_sigma = (float)(0.5 * sg);
             t.inv_half_sigma = (float)(2.0 / sg);
             t.eps4 = (float)(4.0 * ep);
             t.eps24 = (float)(24.0 * ep);

@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kBThreads, 2)
     __shared__ RepDesc R;
     __shared__ uint32_t s_cnt[kBMaxCells + 1];
     __shared__ uint32_t s_start[kBMaxCells + 1];
-    __shared__ PairF s_tab[kMaxKinds * kMaxKinds];
+    __shared__ PairTab s_tab;
     __shared__ double s_red[kBThreads / 32];
     __shared__ unsigned long long s_redu[kBThreads / 32][2];
     __shared__ uint32_t s_wsum[kBThreads / 32];
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kBThreads, 2)
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int r = order[blockIdx.x];
     if (tid == 0) R = reps[r];
-    for (int t = tid; t < L.nkinds * L.nkinds; t += kBThreads) s_tab[t] = tab[t];
+    for (int t = tid; t < L.nkinds * L.nkinds; t += kBThreads) s_tab.put(t, tab[t]);
     if (tid == 0) s_lambda = 1.0;
     __syncthreads();
     const GridGeom& g = R.g;
@@ -444,7 +444,6 @@ int gx_batch_set_state(gx_batch* b, const uint32_t* natoms, const double* pos, c
             double sg = b->pair_sigma[kel[a] * kNElem + kel[c]], ep = b->pair_eps[kel[a] * kNElem + kel[c]];
             PairF& t = tab[a * nk + c];
             t.sigma = (float)sg;
-            t.half_sigma = (float)(0.5 * sg);
             t.inv_half_sigma = (float)(2.0 / sg);
             t.eps4 = (float)(4.0 * ep);
             t.eps24 = (float)(24.0 * ep);

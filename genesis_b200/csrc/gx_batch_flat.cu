@@ -167,7 +167,7 @@ template <bool ENERGY>
 __device__ __forceinline__ void fb_force_one(uint32_t s, const RepGeo* __restrict__ geo,
                                              const float4* __restrict__ pos4, const uint32_t* __restrict__ skey,
                                              const uint32_t* __restrict__ srep, const uint32_t* __restrict__ start,
-                                             uint32_t total, const LawF32& L, const PairF* st,
+                                             uint32_t total, const LawF32& L, const PairTab& st,
                                              long long* __restrict__ F, size_t fstride,
                                              unsigned long long* __restrict__ racc, uint32_t* __restrict__ err) {
     long long vq = 0;
@@ -257,9 +257,9 @@ __global__ void __launch_bounds__(kFbThreads) k_fb_force(const RepGeo* __restric
                                                           const PairF* __restrict__ tab, long long* __restrict__ F,
                                                           size_t fstride, unsigned long long* __restrict__ racc,
                                                           uint32_t* __restrict__ err) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
+    __shared__ PairTab st;
     const int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kFbThreads) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kFbThreads) st.put(t, tab[t]);
     __syncthreads();
     fb_force_one<ENERGY>(blockIdx.x * kFbThreads + threadIdx.x, geo, pos4, skey, srep, start, total, L, st, F, fstride,
                          racc, err);
@@ -501,12 +501,12 @@ __device__ __forceinline__ void coop_scan_tiles(const CoopArgs& a, uint32_t ntil
 }
 
 __global__ void __launch_bounds__(kCoopThreads) k_fb_coop(CoopArgs a) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
+    __shared__ PairTab st;
     __shared__ double sh[kCoopThreads / 32];
     __shared__ uint32_t s_warp[kCoopThreads / 32 + 1];
     __shared__ int s_ok;
     const int nk2 = a.L.nkinds * a.L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kCoopThreads) st[t] = a.tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kCoopThreads) st.put(t, a.tab[t]);
     const uint32_t gt = blockIdx.x * kCoopThreads + threadIdx.x, gs = gridDim.x * kCoopThreads;
     const uint32_t n = a.total, m = a.ncell + 1;
     const uint32_t ntiles = (m + kCoopTile - 1) / kCoopTile;

@@ -296,16 +296,17 @@ __global__ void __launch_bounds__(kBnThreads) k_bn_force(const BnGeo* __restrict
                                                           long long* __restrict__ F, size_t fstride,
                                                           unsigned long long* __restrict__ racc,
                                                           uint32_t* __restrict__ err) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
-    __shared__ float4 s_shift[2][27];
+    __shared__ PairTab st;
+    __shared__ ShiftTab s_shift[2];
     const int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kBnThreads) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kBnThreads) st.put(t, tab[t]);
     const uint32_t first = blockIdx.x * kBnThreads;
     const uint32_t last = min(first + (uint32_t)kBnThreads, total) - 1u;
     const uint32_t r0 = srep[first], r1 = srep[last];
     if (threadIdx.x < 54) {
         const uint32_t w = threadIdx.x / 27, k = threadIdx.x % 27;
-        s_shift[w][k] = shift_tab[(size_t)(w ? r1 : r0) * 27 + k];
+        const float4 v = shift_tab[(size_t)(w ? r1 : r0) * 27 + k];
+        s_shift[w].put(k, v.x, v.y, v.z);
     }
     __syncthreads();
     const uint32_t s = first + threadIdx.x;
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kBnThreads) k_bn_force(const BnGeo* __restrict
     uint32_t r = 0xFFFFFFFFu;
     if (s < total) {
         r = srep[s];
-        const float4* sh_tab = s_shift[r == r0 ? 0 : 1];
+        const ShiftTab& sh_tab = s_shift[r == r0 ? 0 : 1];
         const float4 pi = pos4[s];
         const int ki = __float_as_int(pi.w);
         const uint32_t m = cnt[s];

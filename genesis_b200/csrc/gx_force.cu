@@ -136,10 +136,10 @@ __global__ void __launch_bounds__(kForceThreads) k_force_mixed(GridGeom g, const
                                                                 unsigned long long* __restrict__ vacc,
                                                                 unsigned long long* __restrict__ npairs,
                                                                 uint32_t* __restrict__ err) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
+    __shared__ PairTab st;
     __shared__ unsigned long long shu[kForceThreads / 32];
     int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kForceThreads) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kForceThreads) st.put(t, tab[t]);
     __syncthreads();
     uint32_t i = blockIdx.x * kForceThreads + threadIdx.x;
     long long vq = 0;

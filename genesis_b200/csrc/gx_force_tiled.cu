@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kTThreads, 4)
                         long long* __restrict__ F, size_t fstride, unsigned long long* __restrict__ vacc,
                         unsigned long long* __restrict__ npairs, uint32_t* __restrict__ err) {
     extern __shared__ __align__(128) float4 s_pos[];
-    __shared__ PairF s_tab[kMaxKinds * kMaxKinds];
+    __shared__ PairTab s_tab;
     __shared__ Stage<kTSlots> S;
     __shared__ TileInfo s_tile[kTWarps][kTiles];
     __shared__ uint2 s_q[kTWarps][kQ];
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kTThreads, 4)
     const uint32_t bx = blockIdx.x % nbx, yz = blockIdx.x / nbx;
     const uint32_t cy = yz % g.n[1], cz = yz / g.n[1];
     const int x0 = (int)bx * run;
-    for (int t = tid; t < L.nkinds * L.nkinds; t += kTThreads) s_tab[t] = tab[t];
+    for (int t = tid; t < L.nkinds * L.nkinds; t += kTThreads) s_tab.put(t, tab[t]);
     if (!stage_rows<kTSlots>(S, s_pos, kTStageCap, g, run, x0, cy, cz, pos4, start, err)) return;
     const bool staged = S.staged != 0;
     const float4* P = staged ? (const float4*)s_pos : pos4;
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kRThreads, 4)
                        long long* __restrict__ F, size_t fstride, unsigned long long* __restrict__ vacc,
                        unsigned long long* __restrict__ npairs, uint32_t* __restrict__ err) {
     extern __shared__ __align__(128) float4 s_pos[];
-    __shared__ PairF s_tab[kMaxKinds * kMaxKinds];
+    __shared__ PairTab s_tab;
     __shared__ Stage<kRSlots> S;
     __shared__ uint32_t s_list[kLCap][kRThreads];
     __shared__ uint32_t s_home[kRRunMax + 1];  // prefix of home atoms per own-row slot
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kRThreads, 4)
     const uint32_t bx = blockIdx.x % nbx, yz = blockIdx.x / nbx;
     const uint32_t cy = yz % g.n[1], cz = yz / g.n[1];
     const int x0 = (int)bx * run;
-    for (int t = tid; t < L.nkinds * L.nkinds; t += kRThreads) s_tab[t] = tab[t];
+    for (int t = tid; t < L.nkinds * L.nkinds; t += kRThreads) s_tab.put(t, tab[t]);
     if (!stage_rows<kRSlots>(S, s_pos, kRStageCap, g, run, x0, cy, cz, pos4, start, err)) return;
     const bool staged = S.staged != 0;
     const float4* P = staged ? (const float4*)s_pos : pos4;
@@ -473,12 +473,12 @@ __global__ void __launch_bounds__(kLThreads, 8)
                         const uint32_t* __restrict__ start, uint32_t n, LawF32 L, const PairF* __restrict__ tab,
                         long long* __restrict__ F, size_t fstride, unsigned long long* __restrict__ vacc,
                         unsigned long long* __restrict__ npairs, uint32_t* __restrict__ err) {
-    __shared__ PairF s_tab[kMaxKinds * kMaxKinds];
+    __shared__ PairTab s_tab;
     __shared__ float s_shift[kTiles][3];
     __shared__ uint32_t s_list[kL4Cap][kLThreads];
     __shared__ unsigned long long s_red[kLThreads / 32][2];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    for (int t = tid; t < L.nkinds * L.nkinds; t += kLThreads) s_tab[t] = tab[t];
+    for (int t = tid; t < L.nkinds * L.nkinds; t += kLThreads) s_tab.put(t, tab[t]);
     if (tid < kTiles) {
         float sx = 0.f, sy = 0.f, sz = 0.f;
         if (tid > 0 && tid - 1 < g.nhalf) {

@@ -151,8 +151,8 @@ struct ForceSetup {
 
 // Mixed-path pair table entry, one per (kind_i, kind_j).
 struct PairF {
-    float sigma, half_sigma, inv_half_sigma, eps4;
-    float eps24, qq, gm, pad1;  // qq = k_e q_i q_j, gm = G m_i m_j
+    float sigma, eps4, eps24, qq;  // qq = k_e q_i q_j
+    float inv_half_sigma, gm;      // gm = G m_i m_j
 };
 
 // Device buffers of one atom set in cell-sorted order.

@@ -215,16 +215,16 @@ __global__ void __launch_bounds__(BS) k_nl_force_local(GridGeom g, const float4*
                                                         unsigned long long* __restrict__ vacc,
                                                         unsigned long long* __restrict__ npairs,
                                                         uint32_t* __restrict__ err) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
-    __shared__ float4 s_shift[27];
+    __shared__ PairTab st;
+    __shared__ ShiftTab s_shift;
     __shared__ unsigned long long shu[BS / 32];
     __shared__ uint32_t s_lo[3][BS], s_hi[3][BS];
     const int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += BS) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += BS) st.put(t, tab[t]);
     if (threadIdx.x < 27) {
         float sx, sy, sz;
         code_shift(g, threadIdx.x, sx, sy, sz);
-        s_shift[threadIdx.x] = make_float4(sx, sy, sz, 0.f);
+        s_shift.put(threadIdx.x, sx, sy, sz);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -337,15 +337,15 @@ __global__ void __launch_bounds__(kNlThreads) k_nl_force(GridGeom g, const float
                                                           unsigned long long* __restrict__ vacc,
                                                           unsigned long long* __restrict__ npairs,
                                                           uint32_t* __restrict__ err) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
-    __shared__ float4 s_shift[27];
+    __shared__ PairTab st;
+    __shared__ ShiftTab s_shift;
     __shared__ unsigned long long shu[kNlThreads / 32];
     int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st.put(t, tab[t]);
     if (threadIdx.x < 27) {
         float sx, sy, sz;
         code_shift(g, threadIdx.x, sx, sy, sz);
-        s_shift[threadIdx.x] = make_float4(sx, sy, sz, 0.f);
+        s_shift.put(threadIdx.x, sx, sy, sz);
     }
     __syncthreads();
     uint32_t p = blockIdx.x * kNlThreads + threadIdx.x;
@@ -430,15 +430,15 @@ __global__ void __launch_bounds__(kNlThreads) k_nl_force_tpp(GridGeom g, const f
                                                               unsigned long long* __restrict__ npairs,
                                                               uint32_t* __restrict__ err) {
     static_assert(kNlThreads % TPP == 0 && 32 % TPP == 0, "TPP must divide the warp");
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
-    __shared__ float4 s_shift[27];
+    __shared__ PairTab st;
+    __shared__ ShiftTab s_shift;
     __shared__ unsigned long long shu[kNlThreads / 32];
     int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st.put(t, tab[t]);
     if (threadIdx.x < 27) {
         float sx, sy, sz;
         code_shift(g, threadIdx.x, sx, sy, sz);
-        s_shift[threadIdx.x] = make_float4(sx, sy, sz, 0.f);
+        s_shift.put(threadIdx.x, sx, sy, sz);
     }
     __syncthreads();
     const uint32_t gid = blockIdx.x * kNlThreads + threadIdx.x;
@@ -530,16 +530,16 @@ __global__ void __launch_bounds__(kNlThreads) k_nl_force_cmp(GridGeom g, const f
                                                               unsigned long long* __restrict__ vacc,
                                                               unsigned long long* __restrict__ npairs,
                                                               uint32_t* __restrict__ err) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
-    __shared__ float4 s_shift[27];
+    __shared__ PairTab st;
+    __shared__ ShiftTab s_shift;
     __shared__ unsigned long long shu[kNlThreads / 32];
     __shared__ float4 stash[S * kNlThreads];  // slot k of thread t at [k * kNlThreads + t]
     int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st.put(t, tab[t]);
     if (threadIdx.x < 27) {
         float sx, sy, sz;
         code_shift(g, threadIdx.x, sx, sy, sz);
-        s_shift[threadIdx.x] = make_float4(sx, sy, sz, 0.f);
+        s_shift.put(threadIdx.x, sx, sy, sz);
     }
     __syncthreads();
     const uint32_t p = blockIdx.x * kNlThreads + threadIdx.x;
@@ -795,16 +795,16 @@ __global__ void __launch_bounds__(kNlThreads) k_nl_force_brick(GridGeom g, const
                                                                 unsigned long long* __restrict__ npairs,
                                                                 uint32_t* __restrict__ err, uint32_t K,
                                                                 uint32_t nchunks) {
-    __shared__ PairF st[kMaxKinds * kMaxKinds];
-    __shared__ float4 s_shift[27];
+    __shared__ PairTab st;
+    __shared__ ShiftTab s_shift;
     __shared__ unsigned long long shu[kNlThreads / 32];
     __shared__ __align__(16) BrickSmem<CAP> S;
     const int nk2 = L.nkinds * L.nkinds;
-    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st[t] = tab[t];
+    for (int t = threadIdx.x; t < nk2; t += kNlThreads) st.put(t, tab[t]);
     if (threadIdx.x < 27) {
         float sx, sy, sz;
         code_shift(g, threadIdx.x, sx, sy, sz);
-        s_shift[threadIdx.x] = make_float4(sx, sy, sz, 0.f);
+        s_shift.put(threadIdx.x, sx, sy, sz);
     }
     uint32_t hlo, hhi;
     if (!brick_stage<CAP>(g, start, pos4, K, nchunks, S, err, hlo, hhi)) return;

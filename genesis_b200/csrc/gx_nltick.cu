@@ -116,8 +116,8 @@ __device__ __forceinline__ void take_record(const TickArgs& a, int tick, double 
 // potentials lie in the room of the fixed-point sums until the finish.
 template <bool REC, bool F64>
 __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __grid_constant__ TickArgs a) {
-    __shared__ PairF st[F64 ? 1 : kMaxKinds * kMaxKinds];
-    __shared__ float4 s_shift[27];
+    __shared__ PairTab st;
+    __shared__ ShiftTab s_shift;
     __shared__ double sh[kTickThreads / 32];
     __shared__ unsigned long long shu[kTickThreads / 32];
     __shared__ uint32_t s_warp[kTickThreads / 32], s_off[kScanMaxTiles];
@@ -131,11 +131,11 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
     uint32_t target = 0;  // thread 0's count of barrier arrivals
     const int nk2 = F64 ? 0 : a.L.nkinds * a.L.nkinds;
     double* vat = reinterpret_cast<double*>(a.F);
-    for (int t = tid; t < nk2; t += kTickThreads) st[t] = a.tab[t];
+    for (int t = tid; t < nk2; t += kTickThreads) st.put(t, a.tab[t]);
     if (tid < 27) {
         float sx, sy, sz;
         code_shift(a.g, tid, sx, sy, sz);
-        s_shift[tid] = make_float4(sx, sy, sz, 0.f);
+        s_shift.put(tid, sx, sy, sz);
     }
     for (uint32_t c = gt; c < m; c += gs) a.count[c] = a.fill[c] = 0u;  // counted into before the next use
     if (recorder && tid < 4) a.sync->acc[0][tid] = 0ull;
