@@ -460,14 +460,30 @@ __global__ void __launch_bounds__(kRThreads, 4)
 }
 
 // ------------------------------------------------------------------ variant 4
-// A thread per atom over the whole sorted array (like k_force_mixed), the
+// TPP lanes per atom over the whole sorted array (k_force_mixed has one), the
 // reference's canonical half shell, L1-cached loads, and the per-thread
 // candidate list of variant 3 so the pair law runs outside the filter loop.
+// Lane k of an atom's group walks cells k, k + TPP, ... of the shell; the
+// group's integer sums are combined with shuffles, the same bits for any TPP.
+
+// One lane leaves a small universe's pass to the latency of 127 candidates
+// in a row; many lanes cost a large one idle lanes in each cell.  1 / 2 / 4 /
+// 8 / 16 lanes, us: 51 / 32 / 24 / 18 / 14 at 4,096 atoms, 58 / 38 / 27 / 22 /
+// 26 at 13,824, 64 / 42 / 32 / 39 / 44 at 29,791, 72 / 48 / 52 / 63 / 77 at
+// 64,000, 79 / 78 / 80 / 110 / 137 at 125,000, 149 / 147 / 170 / 230 / 292 at
+// 262,144, 245 / 252 / 306 / 424 / 544 at 512,000.
+int lists_lanes(uint32_t n) {
+    if (n <= 8192) return 16;
+    if (n <= 20480) return 8;
+    if (n <= 45056) return 4;
+    return n <= 131072 ? 2 : 1;
+}
 
 constexpr int kLThreads = 128;
 constexpr int kL4Cap = 32;
 constexpr int kL4Step = 16;
 
+template <int TPP>
 __global__ void __launch_bounds__(kLThreads, 8)
     k_force_mixed_lists(GridGeom g, const float4* __restrict__ pos4, const uint32_t* __restrict__ key,
                         const uint32_t* __restrict__ start, uint32_t n, LawF32 L, const PairF* __restrict__ tab,
@@ -491,7 +507,8 @@ __global__ void __launch_bounds__(kLThreads, 8)
         s_shift[tid][2] = sz;
     }
     __syncthreads();
-    const uint32_t i = blockIdx.x * kLThreads + tid;
+    const uint32_t i = (blockIdx.x * kLThreads + tid) / TPP;
+    const int sub = tid % TPP;
     const bool act = i < n;
     float4 pi = act ? __ldg(pos4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     const int ki = __float_as_int(pi.w);
@@ -537,9 +554,10 @@ __global__ void __launch_bounds__(kLThreads, 8)
         cnt = 0;
     };
 
-    for (int t = 0; t <= g.nhalf; ++t) {
+    for (int t0 = 0; t0 <= g.nhalf; t0 += TPP) {
+        const int t = t0 + sub;
         uint32_t lo = 0, hi = 0;
-        if (act) {
+        if (act && t <= g.nhalf) {
             if (t == 0) {
                 lo = i + 1;
                 hi = start[c + 1];
@@ -550,7 +568,7 @@ __global__ void __launch_bounds__(kLThreads, 8)
                 hi = start[B + 1];
             }
         }
-        const float sx = s_shift[t][0], sy = s_shift[t][1], sz = s_shift[t][2];
+        const float sx = s_shift[t % kTiles][0], sy = s_shift[t % kTiles][1], sz = s_shift[t % kTiles][2];
         const int mine = (int)(hi > lo ? hi - lo : 0u);
         const int most = __reduce_max_sync(0xffffffffu, mine);
         for (int c0 = 0; c0 < most; c0 += kL4Step) {
@@ -575,7 +593,13 @@ __global__ void __launch_bounds__(kLThreads, 8)
         }
     }
     flush();
-    if (act) {
+#pragma unroll
+    for (int o = TPP / 2; o > 0; o >>= 1) {
+        fx += __shfl_down_sync(0xffffffffu, fx, o, TPP);
+        fy += __shfl_down_sync(0xffffffffu, fy, o, TPP);
+        fz += __shfl_down_sync(0xffffffffu, fz, o, TPP);
+    }
+    if (act && sub == 0) {
         if (fx) atomicAdd((unsigned long long*)&F[i], (unsigned long long)fx);
         if (fy) atomicAdd((unsigned long long*)&F[fstride + i], (unsigned long long)fy);
         if (fz) atomicAdd((unsigned long long*)&F[2 * fstride + i], (unsigned long long)fz);
@@ -607,8 +631,14 @@ __global__ void __launch_bounds__(kLThreads, 8)
 void launch_force_mixed_lists(gx_handle* h, const GridGeom& g, const float4* pos4, const uint32_t* key,
                               const uint32_t* start, uint32_t n, const LawF32& L, const PairF* tab, long long* F,
                               size_t fstride, unsigned long long* vacc, unsigned long long* npairs, uint32_t* err) {
-    k_force_mixed_lists<<<(n + kLThreads - 1) / kLThreads, kLThreads, 0, h->stream>>>(
-        g, pos4, key, start, n, L, tab, F, fstride, vacc, npairs, err);
+    const int tpp = lists_lanes(n);
+    auto k = tpp == 16  ? k_force_mixed_lists<16>
+             : tpp == 8 ? k_force_mixed_lists<8>
+             : tpp == 4 ? k_force_mixed_lists<4>
+             : tpp == 2 ? k_force_mixed_lists<2>
+                        : k_force_mixed_lists<1>;
+    const unsigned blocks = (unsigned)(((size_t)n * tpp + kLThreads - 1) / kLThreads);
+    k<<<blocks, kLThreads, 0, h->stream>>>(g, pos4, key, start, n, L, tab, F, fstride, vacc, npairs, err);
     ++h->launches;
 }
 

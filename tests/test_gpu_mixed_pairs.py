@@ -57,3 +57,25 @@ def test_isolated_pairs(gpu, coul, grav):
         if variant >= 5 or variant == 0:  # one frame of coordinates: the same bits
             first = got if first is None else first
             assert np.array_equal(got, first), variant
+
+
+@pytest.mark.parametrize("n_side", [3, 4, 20, 21, 27, 28, 35, 36, 50, 51])
+def test_lanes_of_the_per_tick_pass(gpu, n_side):
+    """The per-tick pass with 16, 8, 4, 2 and 1 lanes per atom (sizes on both
+    sides of each line, grids of one to three cells too) against one thread
+    per atom: the same integer sums."""
+    from genesis_b200._lib import Handle
+    wl = W.Workload("lanes", n_side=n_side, temperature=200.0, steps=10, electrostatics=True)
+    cfg, u = wl.config(), wl.generate()
+    out = []
+    for variant in (1, 0):
+        with Handle(cfg, "mixed") as h:
+            h.set_universe(u)
+            h.set_kernel_variant(variant)
+            h.half_kick()
+            h.drift()
+            h.wrap()
+            out.append((h.forces(), h.get_state()))
+    assert out[0][0] == out[1][0]
+    for a, b in zip(out[0][1], out[1][1]):
+        assert np.array_equal(a, b)
