@@ -484,6 +484,7 @@ int gx_create(const gx_params* p, gx_handle** out) {
     if (e == cudaSuccess) e = cudaMalloc(&h->dscal, 16 * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&h->dcount, 16 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&h->derr, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMallocHost(&h->page, sizeof(HostPage));
     if (e != cudaSuccess) {
         int rc = cuda_err(h, e, "gx_create");
         *out = h;
@@ -518,6 +519,7 @@ void gx_destroy(gx_handle* h) {
         if (e) cudaEventDestroy(e);
     cudaFree(h->io_stage);
     if (h->herr) cudaFreeHost(h->herr);
+    if (h->page) cudaFreeHost(h->page);
     free_buf(h->buf[0]);
     free_buf(h->buf[1]);
     cudaFree(h->key);
@@ -639,7 +641,6 @@ int gx_get_state(gx_handle* h, double* pos, double* vel, double* acc) {
         GX_LAUNCH(h, k_soa_to_aos, nblk(n, 256), 256, srcs[k][0], srcs[k][1], srcs[k][2], b.slot, h->host_stage, n);
         GX_CUDA(h, cudaMemcpyAsync(outs[k], h->host_stage, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost,
                                    h->stream));
-        GX_CUDA(h, cudaStreamSynchronize(h->stream));
     }
     GX_CUDA(h, cudaGetLastError());
     GX_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -740,14 +741,11 @@ int gx_thermostat(gx_handle* h, double* kinetic, double* lambda) {
     launch_kinetic(h, h->buf[h->cur], (uint32_t)h->n, nullptr, kpart, nullptr, &nb);
     launch_thermostat_lambda(h, kpart, nb, h->p.thermal_constant, h->p.thermostat_temperature, tau,
                              (uint32_t)h->n, h->dscal + 0, h->dscal + 1);
-    double out[2];
-    GX_CUDA(h, cudaMemcpyAsync(out, h->dscal, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    launch_apply_lambda(h, h->buf[h->cur], (uint32_t)h->n, h->dscal + 0, false);
+    launch_page(h, nullptr, nullptr, true);
     GX_CUDA(h, cudaStreamSynchronize(h->stream));
-    h->lambda_pending = true;
-    commit_lambda(h);
-    GX_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (kinetic) *kinetic = out[1];
-    if (lambda) *lambda = out[0];
+    if (kinetic) *kinetic = h->page->scal[1];
+    if (lambda) *lambda = h->page->scal[0];
     GX_CUDA(h, cudaGetLastError());
     return GX_OK;
 }
@@ -760,13 +758,11 @@ int gx_stats(gx_handle* h, double* kinetic, double* speed_sum) {
     double* spart = h->red + 3 * rows;
     int nb = 0;
     launch_kinetic(h, h->buf[h->cur], (uint32_t)h->n, h->lambda_pending ? h->dscal + 0 : nullptr, kpart, spart, &nb);
-    launch_finalize_sum(h, kpart, nb, h->dscal + 1);
-    launch_finalize_sum(h, spart, nb, h->dscal + 4);
-    double out[5];
-    GX_CUDA(h, cudaMemcpyAsync(out, h->dscal, 5 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    launch_finalize_two(h, kpart, spart, nb, h->dscal + 1, h->dscal + 4);
+    launch_page(h);
     GX_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (kinetic) *kinetic = out[1];
-    if (speed_sum) *speed_sum = out[4];
+    if (kinetic) *kinetic = h->page->scal[1];
+    if (speed_sum) *speed_sum = h->page->scal[4];
     GX_CUDA(h, cudaGetLastError());
     return GX_OK;
 }
@@ -866,14 +862,15 @@ int step_impl(gx_handle* h, int nsteps, gx_tick_stats* stats, int use_graph, boo
         if (drec) {
             int nb = 0;
             launch_kinetic(h, h->buf[h->cur], n, h->lambda_pending ? h->dscal + 0 : nullptr, kpart, spart, &nb);
-            launch_finalize_sum(h, kpart, nb, h->dscal + 1);
-            launch_finalize_sum(h, spart, nb, h->dscal + 4);
+            launch_finalize_two(h, kpart, spart, nb, h->dscal + 1, h->dscal + 4);
             GX_LAUNCH(h, k_record, 1, 1, drec, h->dscal, h->dcount, thermo ? 1 : 0, 0);
         }
         return GX_OK;
     };
-    if (drec) GX_CUDA(h, cudaMemsetAsync(h->dcount + 5, 0, sizeof(unsigned long long), h->stream));
     const bool graph = use_graph && n && !h->prof_on;
+    const bool one_launch = graph && use_nl && nl_ticks_eligible(h);  // a small universe: no graph at all
+    if (drec && !one_launch)  // the records' cursor
+        GX_CUDA(h, cudaMemsetAsync(h->dcount + 5, 0, sizeof(unsigned long long), h->stream));
     const uint64_t key = ((uint64_t)n << 20) ^ ((uint64_t)h->precision << 1) ^ ((uint64_t)h->kernel_variant << 3) ^
                          ((uint64_t)bonds_on(h) << 6) ^ ((uint64_t)thermo << 7) ^ ((uint64_t)h->cap << 8) ^
                          ((uint64_t)use_nl << 62) ^ 1u;
@@ -905,7 +902,6 @@ int step_impl(gx_handle* h, int nsteps, gx_tick_stats* stats, int use_graph, boo
         h->launches = l0;
         return GX_OK;
     };
-    const bool one_launch = graph && use_nl && nl_ticks_eligible(h);  // a small universe: no graph at all
     if (one_launch && nsteps > 0 && (rc = nl_ticks(h, nsteps, drec, thermo, tau, kpart, spart))) return rc;
     for (int s = one_launch ? nsteps : 0; s < nsteps; ++s) {
         if (!graph) {
@@ -973,11 +969,13 @@ int step_impl(gx_handle* h, int nsteps, gx_tick_stats* stats, int use_graph, boo
     h->nl_fresh = nsteps > 0 ? (use_nl && h->nl_valid) : fresh0;
     h->last_tick_nl = use_nl && !one_launch;  // whether the tick recorded io_ev[3]
     if (defer) return GX_OK;
+    const bool later = h->step_async && !drec && h->herr;
+    if (!later) launch_page(h);
     if (drec) {
         GX_CUDA(h, cudaMemcpyAsync(stats, drec, (size_t)nsteps * sizeof(gx_tick_stats), cudaMemcpyDeviceToHost,
                                    h->stream));
     }
-    if (h->step_async && !drec && h->herr) {
+    if (later) {
         // no wait: the error word follows in stream order, read by the next waiting call
         GX_CUDA(h, cudaMemcpyAsync(h->herr, h->derr, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
         GX_CUDA(h, cudaGetLastError());
@@ -987,9 +985,7 @@ int step_impl(gx_handle* h, int nsteps, gx_tick_stats* stats, int use_graph, boo
     GX_CUDA(h, cudaStreamSynchronize(h->stream));
     GX_CUDA(h, cudaGetLastError());
     h->step_errs_pending = false;
-    uint32_t e = 0;
-    GX_CUDA(h, cudaMemcpy(&e, h->derr, sizeof e, cudaMemcpyDeviceToHost));
-    return step_error(h, e);
+    return step_error(h, h->page->err);
 }
 }  // namespace
 
@@ -1377,18 +1373,14 @@ int gx_tick_host(gx_handle* h, double* pos, double* vel, double* acc, gx_tick_st
             GX_IO(cudaMemcpyAsync(outs[k], st[k + 1], bytes, cudaMemcpyDeviceToHost, io));
         }
     }
+    launch_page(h, stats ? (const gx_tick_stats*)(h->red + 4 * (h->cap / 64 + kRedCap)) : nullptr);
     GX_IO(cudaGetLastError());
     GX_IO(cudaStreamSynchronize(io));
     GX_IO(cudaStreamSynchronize(ms));
-    if (stats) {
-        size_t rows = h->cap / 64 + kRedCap;
-        GX_IO(cudaMemcpy(stats, h->red + 4 * rows, sizeof(gx_tick_stats), cudaMemcpyDeviceToHost));
-    }
 #undef GX_IO
+    if (stats) *stats = h->page->rec;
     h->step_errs_pending = false;
-    uint32_t e = 0;
-    GX_CUDA(h, cudaMemcpy(&e, h->derr, sizeof e, cudaMemcpyDeviceToHost));
-    return step_error(h, e);
+    return step_error(h, h->page->err);
 }
 
 int gx_synchronize(gx_handle* h) {

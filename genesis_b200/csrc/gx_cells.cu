@@ -254,6 +254,34 @@ __global__ void __launch_bounds__(kRedThreads) k_finalize_sum(const double* __re
     if (threadIdx.x == 0) *out = s;
 }
 
+// Two such sums, one per block.
+__global__ void __launch_bounds__(kRedThreads) k_finalize_two(const double* __restrict__ a, const double* __restrict__ b,
+                                                              int nb, double* out_a, double* out_b) {
+    __shared__ double sh[kRedThreads / 32];
+    const double* part = blockIdx.x ? b : a;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < nb; i += kRedThreads) s = xadd(s, part[i]);
+    s = block_sum<kRedThreads>(s, sh);
+    if (threadIdx.x == 0) *(blockIdx.x ? out_b : out_a) = s;
+}
+
+__global__ void k_page(HostPage* page, double* dscal, const unsigned long long* dcount, const uint32_t* derr,
+                       const gx_tick_stats* rec, const unsigned long long* vfix, int reset_scale) {
+    const int t = threadIdx.x;
+    if (t < 8) {
+        double v = dscal[t];
+        if (t == 2 && vfix) dscal[2] = v = xmul(__ll2double_rn((long long)*vfix), kFixInv);
+        page->scal[t] = v;
+        if (t == 0 && reset_scale) dscal[0] = 1.0;
+    } else if (t == 8) {
+        page->pairs = dcount[0];
+    } else if (t == 9) {
+        page->err = *derr;
+    } else if (t == 10 && rec) {
+        page->rec = *rec;
+    }
+}
+
 // ThermostatSystem::run tail (src/systems/thermostat.rs:58-71): lambda from K.
 __global__ void __launch_bounds__(kRedThreads) k_thermostat_lambda(const double* __restrict__ part, int nb, double k,
                                                                    double target, double tau, uint32_t n,
@@ -415,9 +443,9 @@ void launch_wrap(gx_handle* h, const StateBuf& b, uint32_t n) {
     GX_LAUNCH(h, k_wrap, nblk(n, 256), 256, b, n, 0.5 * h->p.box[0], 0.5 * h->p.box[1], 0.5 * h->p.box[2]);
     prof_end(h, "wrap");
 }
-void launch_apply_lambda(gx_handle* h, const StateBuf& b, uint32_t n, double* lambda) {
+void launch_apply_lambda(gx_handle* h, const StateBuf& b, uint32_t n, double* lambda, bool reset) {
     if (n) GX_LAUNCH(h, k_apply_lambda, nblk(n, 256), 256, b, n, lambda);
-    GX_LAUNCH(h, k_set_one, 1, 1, lambda);
+    if (reset) GX_LAUNCH(h, k_set_one, 1, 1, lambda);
 }
 void launch_kinetic(gx_handle* h, const StateBuf& b, uint32_t n, const double* lambda, double* kpart,
                     double* spart, int* nblocks) {
@@ -428,6 +456,12 @@ void launch_kinetic(gx_handle* h, const StateBuf& b, uint32_t n, const double* l
     GX_LAUNCH(h, k_kinetic, nb, kRedThreads, b, n, lambda, kpart, spart);
     prof_end(h, "kinetic");
     *nblocks = nb;
+}
+void launch_finalize_two(gx_handle* h, const double* a, const double* b, int nblocks, double* out_a, double* out_b) {
+    GX_LAUNCH(h, k_finalize_two, 2, kRedThreads, a, b, nblocks, out_a, out_b);
+}
+void launch_page(gx_handle* h, const gx_tick_stats* rec, const unsigned long long* vfix, bool reset_scale) {
+    GX_LAUNCH(h, k_page, 1, 32, h->page, h->dscal, h->dcount, h->derr, rec, vfix, reset_scale ? 1 : 0);
 }
 void launch_finalize_sum(gx_handle* h, const double* partials, int nblocks, double* out) {
     GX_LAUNCH(h, k_finalize_sum, 1, kRedThreads, partials, nblocks, out);

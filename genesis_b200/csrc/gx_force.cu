@@ -346,21 +346,17 @@ int force_pass(gx_handle* h, bool finalize_acc, double* V, double* Vb, uint64_t*
     if (rc) return rc;
     if (mixed) {
         if (finalize_acc && n) GX_LAUNCH(h, k_fix_to_acc, nblk(n, 256), 256, b, h->F, h->cap, n);
-        GX_LAUNCH(h, k_fix_to_double, 1, 1, h->dcount + 1, h->dscal + 2);
+        if (!sync_out) GX_LAUNCH(h, k_fix_to_double, 1, 1, h->dcount + 1, h->dscal + 2);
     } else {
         GX_LAUNCH(h, k_sum_rows, 1, 256, vpart, (int)fb, h->dscal + 2);
     }
     if (sync_out) {
-        double vv[2];
-        unsigned long long cnt;
-        GX_CUDA(h, cudaMemcpyAsync(vv, h->dscal + 2, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        GX_CUDA(h, cudaMemcpyAsync(&cnt, h->dcount, sizeof(cnt), cudaMemcpyDeviceToHost, h->stream));
-        uint32_t e = 0;
-        GX_CUDA(h, cudaMemcpyAsync(&e, h->derr, sizeof(e), cudaMemcpyDeviceToHost, h->stream));
+        launch_page(h, nullptr, mixed ? h->dcount + 1 : nullptr);
         GX_CUDA(h, cudaStreamSynchronize(h->stream));
-        if (V) *V = vv[0];
-        if (Vb) *Vb = vv[1];
-        if (npairs_out) *npairs_out = cnt;
+        const uint32_t e = h->page->err;
+        if (V) *V = h->page->scal[2];
+        if (Vb) *Vb = h->page->scal[3];
+        if (npairs_out) *npairs_out = h->page->pairs;
         if (e) {
             GX_CUDA(h, cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream));
             if (e & kErrNonFinite) return set_err(h, GX_ERR_NONFINITE, "non-finite force in the pair pass");
