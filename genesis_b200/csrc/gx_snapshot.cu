@@ -98,37 +98,65 @@ __device__ __forceinline__ unsigned char* put_vec3(unsigned char* p, double x, d
 }
 
 // One record per ECS slot at 8 + 115 s + 8 off[s]; the state is read through
-// pos_of_slot (the device keeps it in cell order).
-__global__ void __launch_bounds__(kSnapThreads) k_snap_write(StateBuf b, const uint32_t* __restrict__ pos_of_slot,
-                                                             const uint32_t* __restrict__ entity,
-                                                             const uint32_t* __restrict__ gen, uint32_t n,
-                                                             const unsigned long long* __restrict__ off,
-                                                             const uint32_t* __restrict__ adj,
-                                                             unsigned char* __restrict__ out) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+// pos_of_slot (the device keeps it in cell order).  A record's bytes are odd in
+// number and in place, so stored one by one they reach L2 as 115 scattered
+// stores an atom (255 us for 250,047 atoms, 15 staged): a block's records,
+// contiguous in the output, are put together in shared memory, at the output's
+// offset modulo 16, and leave in 16-byte words.  A block whose records do not
+// fit (more than some 16 bonds an atom on average) stores them directly.
+constexpr int kSnapWriteThreads = 128;
+constexpr uint32_t kSnapStage = 32 * 1024;
+
+__global__ void __launch_bounds__(kSnapWriteThreads) k_snap_write(StateBuf b, const uint32_t* __restrict__ pos_of_slot,
+                                                                  const uint32_t* __restrict__ entity,
+                                                                  const uint32_t* __restrict__ gen, uint32_t n,
+                                                                  const unsigned long long* __restrict__ off,
+                                                                  const uint32_t* __restrict__ adj,
+                                                                  unsigned char* __restrict__ out) {
+    __shared__ __align__(16) unsigned char stage[kSnapStage];
+    const uint32_t s0 = blockIdx.x * kSnapWriteThreads, s1 = min(s0 + (uint32_t)kSnapWriteThreads, n);
+    const uint32_t s = s0 + threadIdx.x;
+    const unsigned long long first = 8 + kSnapFixed * (unsigned long long)s0 + 8ull * off[s0];
+    const unsigned long long bytes = 8 + kSnapFixed * (unsigned long long)s1 + 8ull * off[s1] - first;
+    const uint32_t skew = (uint32_t)(first & 15u);  // out itself is 256-byte aligned
+    const bool staged = skew + bytes <= kSnapStage;
     if (s == 0) put_u64(out, (unsigned long long)n);  // Vec<EntitySnapshot> length
-    if (s >= n) return;
-    const uint32_t i = pos_of_slot[s];
-    const unsigned long long lo = off[s], hi = off[s + 1];
-    unsigned char* p = out + 8 + kSnapFixed * (unsigned long long)s + 8ull * lo;
-    p = put_u32(p, entity ? entity[s] : s);
-    p = put_u32(p, gen ? gen[s] : 0u);
-    p = put_vec3(p, b.x[i], b.y[i], b.z[i]);
-    p = put_vec3(p, b.vx[i], b.vy[i], b.vz[i]);
-    *p++ = 1;
-    p = put_f64(p, b.mass[i]);
-    *p++ = 1;
-    p = put_f64(p, b.charge[i]);
-    *p++ = 1;
-    p = put_u32(p, (uint32_t)b.elem[i]);
-    *p++ = 1;
-    p = put_u64(p, hi - lo);
-    for (unsigned long long k = lo; k < hi; ++k) {
-        const uint32_t q = adj[k];
-        p = put_u32(p, entity ? entity[q] : q);
-        p = put_u32(p, gen ? gen[q] : 0u);
+    if (s < n) {
+        const uint32_t i = pos_of_slot[s];
+        const unsigned long long lo = off[s], hi = off[s + 1];
+        const unsigned long long at = 8 + kSnapFixed * (unsigned long long)s + 8ull * lo;
+        unsigned char* p = staged ? stage + skew + (at - first) : out + at;
+        p = put_u32(p, entity ? entity[s] : s);
+        p = put_u32(p, gen ? gen[s] : 0u);
+        p = put_vec3(p, b.x[i], b.y[i], b.z[i]);
+        p = put_vec3(p, b.vx[i], b.vy[i], b.vz[i]);
+        *p++ = 1;
+        p = put_f64(p, b.mass[i]);
+        *p++ = 1;
+        p = put_f64(p, b.charge[i]);
+        *p++ = 1;
+        p = put_u32(p, (uint32_t)b.elem[i]);
+        *p++ = 1;
+        p = put_u64(p, hi - lo);
+        for (unsigned long long k = lo; k < hi; ++k) {
+            const uint32_t q = adj[k];
+            p = put_u32(p, entity ? entity[q] : q);
+            p = put_u32(p, gen ? gen[q] : 0u);
+        }
+        put_vec3(p, b.ax[i], b.ay[i], b.az[i]);
     }
-    put_vec3(p, b.ax[i], b.ay[i], b.az[i]);
+    if (!staged) return;
+    __syncthreads();
+    unsigned char* base = out + (first - skew);  // stage[0]'s place, 16-byte aligned
+    const uint32_t end = skew + (uint32_t)bytes;
+    const uint32_t w0 = (skew + 15u) / 16u, w1 = end / 16u;  // whole words; a block holds 115 bytes or more
+    for (uint32_t w = w0 + threadIdx.x; w < w1; w += kSnapWriteThreads)
+        reinterpret_cast<uint4*>(base)[w] = reinterpret_cast<const uint4*>(stage)[w];
+    if (threadIdx.x < 16) {  // the ragged first and last word, a byte each
+        const uint32_t k0 = skew + threadIdx.x, k1 = 16u * w1 + threadIdx.x;
+        if (k0 < 16u * w0) base[k0] = stage[k0];
+        if (k1 < end) base[k1] = stage[k1];
+    }
 }
 
 struct SnapState {
@@ -239,12 +267,12 @@ extern "C" int gx_snapshot_world(gx_handle* h, const uint32_t* generation, uint8
                   S.adj);
         GX_LAUNCH(h, k_snap_sort_rows, nblk(n, kSnapThreads), kSnapThreads, S.off, n, S.adj);
     }
-    GX_LAUNCH(h, k_snap_write, nblk(n, kSnapThreads), kSnapThreads, h->buf[h->cur], h->pos_of_slot,
+    GX_LAUNCH(h, k_snap_write, nblk(n, kSnapWriteThreads), kSnapWriteThreads, h->buf[h->cur], h->pos_of_slot,
               h->has_entity ? h->entity : nullptr, generation ? S.gen : nullptr, n, S.off, S.adj, S.bytes);
     prof_end(h, "snapshot");
     uint32_t herr = 0;
-    GX_CUDA(h, cudaMemcpyAsync(&herr, S.err, sizeof herr, cudaMemcpyDeviceToHost, h->stream));
     GX_CUDA(h, cudaMemcpyAsync(out, S.bytes, total, cudaMemcpyDeviceToHost, h->stream));
+    GX_CUDA(h, cudaMemcpyAsync(&herr, S.err, sizeof herr, cudaMemcpyDeviceToHost, h->stream));
     GX_CUDA(h, cudaStreamSynchronize(h->stream));
     GX_CUDA(h, cudaGetLastError());
     if (herr) return set_err(h, GX_ERR_STATE, "gx_snapshot_world: a bond names a slot beyond the atom count");

@@ -50,3 +50,26 @@ def test_world_bytes_of_the_quench_lattice(gpu):
     assert len(got) == 8 + S.RECORD_FIXED * u.n
     want = S.encode_world(pos, vel, acc, u.mass, u.charge, u.elem)
     assert got == want
+
+
+@pytest.mark.parametrize("n,per_atom", [(1, 0), (127, 0), (128, 3), (129, 12), (300, 15), (300, 16), (300, 17),
+                                        (300, 40)])
+def test_world_bytes_at_the_edges_of_a_block(gpu, n, per_atom):
+    """Blocks of 128 records that are staged, and those whose bonds do not fit."""
+    from genesis_b200._lib import Handle
+    rng = np.random.default_rng(n + per_atom)
+    cfg = W.C2.scaled(8).config()
+    L = cfg.size[0]
+    pos, vel = rng.uniform(-0.5 * L, 0.5 * L, (n, 3)), rng.normal(size=(n, 3))
+    elem = rng.integers(0, 10, n).astype(np.uint8)
+    charge, mass = rng.normal(size=n), rng.uniform(1.0, 9.0, n)
+    k = rng.permutation(n)
+    bonds = np.concatenate([np.stack([k, np.roll(k, s)], 1) for s in range(1, per_atom + 1)]
+                           or [np.zeros((0, 2), int)])[: n * per_atom // 2]
+    bonds = np.sort(bonds, 1).astype(np.uint32)
+    with Handle(cfg, "fp64") as h:
+        h.set_state(pos, vel, elem, charge=charge, mass=mass)
+        h.set_bonds(bonds)
+        p, v, a = h.get_state()
+        got = h.snapshot_world()
+    assert got == S.encode_world(p, v, a, mass, charge, elem, None, None, bonds)
