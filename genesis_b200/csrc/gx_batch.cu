@@ -359,6 +359,9 @@ int gx_batch_create(const gx_params* p, int nrep, const double* box, const doubl
     L.coul_ron = (float)(0.9 * coul_rc);
     L.inv_coul_w = L.coul ? (float)(1.0 / (coul_rc - 0.9 * coul_rc)) : 0.f;
     L.nkinds = 0;
+    L.one_switch = L.coul && L.coul_rc == L.lj_rc && L.coul_ron == L.lj_ron && L.inv_coul_w == L.inv_lj_w &&
+                   0.5 * max_sigma <= L.lj_ron;
+    L.fq_max = (float)(8.9e18 / rc);
     b->reps.resize(nrep);
     for (int r = 0; r < nrep; ++r) {
         int ok = 0;

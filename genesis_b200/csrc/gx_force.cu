@@ -382,6 +382,9 @@ LawF32 make_law32(const gx_handle* h) {
     L.grav_ron = (float)h->fs.grav_ron;
     L.inv_grav_w = L.grav ? (float)(1.0 / (h->fs.grav_rc - h->fs.grav_ron)) : 0.f;
     L.nkinds = h->nkinds;
+    L.one_switch = L.coul && L.coul_rc == L.lj_rc && L.coul_ron == L.lj_ron && L.inv_coul_w == L.inv_lj_w &&
+                   0.5 * h->fs.max_sigma <= L.lj_ron;
+    L.fq_max = (float)(8.9e18 / h->fs.rc);
     return L;
 }
 

@@ -57,10 +57,10 @@ constexpr int kTicksPerLaunch = 256;
 // Lanes per atom of the half-list pass where none were set: enough to fill
 // the chip and to share the long lists of a condensed state, one where the
 // gathers of a homogeneous one set the time.  Microseconds per pass with
-// 1 / 2 / 4 / 8 lanes on the lattice: 31 / 22 / 14 / 12 at 4,096 atoms,
-// 31 / 23 / 19 / 20 at 32,768, 35 / 27 / 27 / 27 at 59,319, 46 / 44 / 43 / 46
-// at 125,000, 78 / 74 / 77 / 91 at 262,144, 131 / 132 / 145 / 177 at 512,000,
-// 232 / 242 / 274 / 369 at 1,000,000, 460 / 486 / 563 / 726 at 2,097,152; per
+// 1 / 2 / 4 / 8 lanes on the lattice: 31 / 21 / 15 / 10 at 4,096 atoms,
+// 31 / 23 / 17 / 19 at 32,768, 34 / 25 / 27 / 27 at 59,319, 44 / 42 / 41 / 45
+// at 125,000, 76 / 71 / 76 / 90 at 262,144, 124 / 129 / 146 / 177 at 512,000,
+// 221 / 236 / 274 / 357 at 1,000,000, 435 / 477 / 563 / 709 at 2,097,152; per
 // tick after 1,000 ticks of condensation with charges and gravity:
 // 96 / 73 / 60 / 59 at 32,768, 107 / 89 / 82 / 77 at 59,319,
 // 263 / 234 / 223 / 232 at 262,144.

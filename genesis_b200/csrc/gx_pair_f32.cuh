@@ -24,6 +24,8 @@ struct LawF32 {
     int coul, nkinds;
     int grav = 0;
     float grav_rc = 0.f, grav_ron = 0.f, inv_grav_w = 0.f;
+    int one_switch = 0;   // Coulomb has LJ's cutoff and switch, the cores lie below them
+    float fq_max = 0.f;  // below it, 2^32 |F| / d times any displacement within the cutoff fits a fixed-point sum
 };
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
@@ -34,6 +36,23 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float delta1(float a, float b, float s) { return fadd(fsub(a, b), s); }
 __device__ __forceinline__ float dist2(float dx, float dy, float dz) {
     return fmaf(dz, dz, fmaf(dy, dy, fmul(dx, dx)));
+}
+
+// min(max(a * b, 0), 1) in one instruction (0 for a NaN, as fmaxf gives).
+__device__ __forceinline__ float fmul_sat(float a, float b) {
+    float r;
+    asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// rsqrtf without the scaling of subnormal arguments, and with it only for those.
+__device__ __forceinline__ float rsqrt_normal(float d2) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d2));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_any(float d2) {
+    return d2 < 1.17549435e-38f ? rsqrtf(d2) : rsqrt_normal(d2);
 }
 
 // quintic switch 1 - 10u^3 + 15u^4 - 6u^5 and its derivative (per unit u)
@@ -52,9 +71,12 @@ __device__ __forceinline__ void switch5(float u, float& sw, float& dsw_du) {
 // takes (sigma, 4 eps, 24 eps, the charges' product) is one 16-byte word, and
 // the core's 2 / sigma and the masses' product are read where a pair needs
 // them (sigma / 2 is exact).  With the shifts below one bank per axis, the
-// half-list pass of 2,097,152 atoms takes 465 us (527 with 32-byte rows and
+// half-list pass of 2,097,152 atoms took 465 us (527 with 32-byte rows and
 // 16-byte shifts), 131 at 512,000 (145), and the 256-replica batch's 290
-// (300).
+// (300).  What bounds it since is the number of instructions (79 % issue), so
+// the law below spends none twice: one switch for two terms of the same
+// cutoff, one range check for a force's three components, clamps folded into
+// products (436 us, 123 at 512,000).
 struct PairTab {
     float4 main[kMaxKinds * kMaxKinds];
     float2 rest[kMaxKinds * kMaxKinds];
@@ -81,8 +103,8 @@ struct ShiftTab {
     }
 };
 
-__device__ __forceinline__ void pair_f32(const LawF32& L, PairTab::Ref ref, float d2, float& fs, float& v) {
-    float inv_d = rsqrtf(d2);
+__device__ __forceinline__ void pair_f32(const LawF32& L, PairTab::Ref ref, float d2, float inv_d, float& fs,
+                                         float& v) {
     float d = fmul(d2, inv_d);
     float f = 0.f;
     v = 0.f;
@@ -104,18 +126,25 @@ __device__ __forceinline__ void pair_f32(const LawF32& L, PairTab::Ref ref, floa
         // give f = fmaf(ml, 1, +-0) = ml and v = vl exactly, S(1) = 0 gives
         // zeros, so the result is bit-identical to skipping the switch
         // outside (r_on, r_c) -- and no lane of a warp diverges on it.
-        float u = fminf(fmaxf(fmul(fsub(r, L.lj_ron), L.inv_lj_w), 0.f), 1.f);
+        float u = fmul_sat(fsub(r, L.lj_ron), L.inv_lj_w);
         float sw, dsdu;
         switch5(u, sw, dsdu);
         float dsw = fmul(dsdu, L.inv_lj_w);
         f = fmaf(ml, sw, -fmul(vl, dsw));
         v = fmul(vl, sw);
+        if (L.one_switch) {  // in the core too: S(0) and S'(0) for r = sigma / 2 and for d
+            float inv_c = d < 0.5f ? 2.f : inv_d;
+            float vc = fmul(qq, inv_c);
+            float mc = fmul(vc, inv_c);
+            f = fadd(f, fmaf(mc, sw, -fmul(vc, dsw)));
+            v = fadd(v, fmul(vc, sw));
+        }
     }
-    if (L.coul && d < L.coul_rc) {
+    if (L.coul && !L.one_switch && d < L.coul_rc) {
         float inv_r = d < 0.5f ? 2.f : inv_d;
         float vc = fmul(qq, inv_r);
         float mc = fmul(vc, inv_r);
-        float u = fminf(fmaxf(fmul(fsub(d, L.coul_ron), L.inv_coul_w), 0.f), 1.f);  // as above
+        float u = fmul_sat(fsub(d, L.coul_ron), L.inv_coul_w);  // as above
         float sw, dsdu;
         switch5(u, sw, dsdu);
         float dsw = fmul(dsdu, L.inv_coul_w);
@@ -126,7 +155,7 @@ __device__ __forceinline__ void pair_f32(const LawF32& L, PairTab::Ref ref, floa
         float inv_r = d < 0.5f ? 2.f : inv_d;
         float vg = -fmul(ref.t->rest[ref.i].y, inv_r);  // attractive
         float mg = fmul(vg, inv_r);
-        float u = fminf(fmaxf(fmul(fsub(d, L.grav_ron), L.inv_grav_w), 0.f), 1.f);  // as above
+        float u = fmul_sat(fsub(d, L.grav_ron), L.inv_grav_w);  // as above
         float sw, dsdu;
         switch5(u, sw, dsdu);
         float dsw = fmul(dsdu, L.inv_grav_w);
@@ -134,6 +163,10 @@ __device__ __forceinline__ void pair_f32(const LawF32& L, PairTab::Ref ref, floa
         v = fadd(v, fmul(vg, sw));
     }
     fs = fmul(f, inv_d);
+}
+
+__device__ __forceinline__ void pair_f32(const LawF32& L, PairTab::Ref ref, float d2, float& fs, float& v) {
+    pair_f32(L, ref, d2, rsqrt_any(d2), fs, v);
 }
 
 // One FP32 value to 2^-32 fixed point; flags saturation / non-finite.
@@ -190,26 +223,37 @@ __device__ __forceinline__ void nl_pair(const LawF32& L, const PairTab& st, int 
                                         long long* far = nullptr, uint32_t q = 0, size_t fstride = 0) {
     float dx = delta1(pi.x, pj.x, sx), dy = delta1(pi.y, pj.y, sy), dz = delta1(pi.z, pj.z, sz);
     float d2 = dist2(dx, dy, dz);
-    if (!(d2 < L.rc2) || d2 == 0.f) return;
+    if (!(d2 < L.rc2)) return;
+    float inv_d;
+    if (d2 >= 1.17549435e-38f) {
+        inv_d = rsqrt_normal(d2);
+    } else {
+        if (d2 == 0.f) return;
+        inv_d = rsqrtf(d2);
+    }
     float fs, v;
-    pair_f32(L, st[ki * L.nkinds + __float_as_int(pj.w)], d2, fs, v);
+    pair_f32(L, st[ki * L.nkinds + __float_as_int(pj.w)], d2, inv_d, fs, v);
+    // The force quantised with 2^32 folded into its magnitude (a power of two:
+    // the same integers) and one range check for the three components; what
+    // fails it takes quant3's checks of each.  The far end's share is
+    // quantised: the conversion rounds to nearest even, symmetric in sign, so
+    // this end's is exactly its negative.
+    const float fq = fmul(fs, -kFixScaleF);
     long long qx, qy, qz;
-    if (far) {
-        // The far end's share quantised directly: the conversion rounds to
-        // nearest even, which is symmetric in sign, so these are exactly
-        // -quant(f) (flags included), and this end subtracts them.
+    if (fabsf(fq) < L.fq_max) {
+        qx = __float2ll_rn(fmul(dx, fq));
+        qy = __float2ll_rn(fmul(dy, fq));
+        qz = __float2ll_rn(fmul(dz, fq));
+    } else {
         quant3(-fmul(dx, fs), -fmul(dy, fs), -fmul(dz, fs), qx, qy, qz, err);
-        a.fx -= qx;
-        a.fy -= qy;
-        a.fz -= qz;
+    }
+    a.fx -= qx;
+    a.fy -= qy;
+    a.fz -= qz;
+    if (far) {
         atomicAdd((unsigned long long*)&far[q], (unsigned long long)qx);
         atomicAdd((unsigned long long*)&far[fstride + q], (unsigned long long)qy);
         atomicAdd((unsigned long long*)&far[2 * fstride + q], (unsigned long long)qz);
-    } else {
-        quant3(fmul(dx, fs), fmul(dy, fs), fmul(dz, fs), qx, qy, qz, err);
-        a.fx += qx;
-        a.fy += qy;
-        a.fz += qz;
     }
     if (once) {
         a.vq += quant(v, err);
