@@ -246,15 +246,7 @@ __global__ void __launch_bounds__(kRedThreads) k_kinetic(StateBuf b, uint32_t n,
     }
 }
 
-__global__ void __launch_bounds__(kRedThreads) k_finalize_sum(const double* __restrict__ part, int nb, double* out) {
-    __shared__ double sh[kRedThreads / 32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += kRedThreads) s = xadd(s, part[i]);
-    s = block_sum<kRedThreads>(s, sh);
-    if (threadIdx.x == 0) *out = s;
-}
-
-// Two such sums, one per block.
+// The sums of two rows of block partials, one per block.
 __global__ void __launch_bounds__(kRedThreads) k_finalize_two(const double* __restrict__ a, const double* __restrict__ b,
                                                               int nb, double* out_a, double* out_b) {
     __shared__ double sh[kRedThreads / 32];
@@ -462,9 +454,6 @@ void launch_finalize_two(gx_handle* h, const double* a, const double* b, int nbl
 }
 void launch_page(gx_handle* h, const gx_tick_stats* rec, const unsigned long long* vfix, bool reset_scale) {
     GX_LAUNCH(h, k_page, 1, 32, h->page, h->dscal, h->dcount, h->derr, rec, vfix, reset_scale ? 1 : 0);
-}
-void launch_finalize_sum(gx_handle* h, const double* partials, int nblocks, double* out) {
-    GX_LAUNCH(h, k_finalize_sum, 1, kRedThreads, partials, nblocks, out);
 }
 void launch_thermostat_lambda(gx_handle* h, const double* partials, int nblocks, double k, double target,
                               double tau, uint32_t n, double* lambda_out, double* K_out) {

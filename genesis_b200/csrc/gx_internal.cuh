@@ -357,7 +357,6 @@ int bond_spring(gx_handle* h, bool unit_mult);
 // FP64 pair table on the device: sigma_ij then eps_ij, kNElem^2 each (gx_force.cu).
 double* d_psig(gx_handle* h);
 // out = the sum of part[0..nb) in a fixed order, one block (gx_force.cu).
-void launch_sum_rows(gx_handle* h, const double* part, int nb, double* out);
 inline bool bonds_on(const gx_handle* h) { return h->p.enable_bond_interaction && h->bonds_cap > 0; }
 inline unsigned long long* dnbonds(gx_handle* h) { return h->dcount + 8; }
 void adjoint_free(gx_handle* h);
@@ -366,6 +365,8 @@ void adjoint_free(gx_handle* h);
 bool nl_eligible(gx_handle* h);
 int nl_prepare(gx_handle* h, bool* graphs_stale);
 int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, int* nblocks, bool energy);
+void nl_close(gx_handle* h, const double* kpart, const double* spart, int nblocks, gx_tick_stats* rec, bool thermo,
+              double tau, bool reset_scale);
 int nl_rebuilds(gx_handle* h, uint64_t* out);
 // The ticks of a small universe in one cooperative launch (gx_nltick.cu).
 bool nl_ticks_eligible(gx_handle* h);
@@ -425,8 +426,7 @@ void launch_wrap(gx_handle* h, const StateBuf& b, uint32_t n);
 void launch_apply_lambda(gx_handle* h, const StateBuf& b, uint32_t n, double* lambda, bool reset = true);
 void launch_kinetic(gx_handle* h, const StateBuf& b, uint32_t n, const double* lambda, double* partials,
                     double* speed_partials, int* nblocks);
-void launch_finalize_sum(gx_handle* h, const double* partials, int nblocks, double* out);
-// out_a = the sum of partials a, out_b = that of b, each as launch_finalize_sum sums it.
+// out_a = the sum of partials a, out_b = that of b.
 void launch_finalize_two(gx_handle* h, const double* a, const double* b, int nblocks, double* out_a, double* out_b);
 // Queues the write of h->page.  vfix: the potential's fixed-point sum, converted into dscal[2] first; reset_scale:
 // the pending scale's slot back to 1 afterwards.

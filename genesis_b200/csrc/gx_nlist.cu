@@ -23,15 +23,16 @@
 // One tick (all launches captured in one CUDA graph; the rebuild launches
 // read a device flag and do nothing when it is clear):
 //   k_nl_advance   kick (with the pending Berendsen scale), drift, wrap,
-//                  home-frame FP32 staging, displacement check -> flag;
-//                  zeroes the force sums of the half-list pass
+//                  home-frame FP32 staging, displacement check -> flag and
+//                  the rebuild's condition; zeroes the energy counters and
+//                  the force sums of the half-list pass
 //   [rebuild]      cell keys, counting sort, gather, copy back, staging,
 //                  list build
-//   k_nl_end       rebuild count, frame parity, zeroed energy counters
 //   k_nl_force     one thread per atom over its full list: FP32 pair law,
 //                  fixed-point sums in registers, plain stores (no atomics);
 //                  the potential and pair count take each pair once (q > p)
 //   k_nl_finish    a = F 2^-32 / m, second kick, kinetic-energy partials
+//   k_nl_close     the thermostat's scale, the record, rebuild count, parity
 // An atom whose list overflowed scans its 27 home-grid cells directly, so
 // the pair set stays exact whatever the local density.
 #include <algorithm>
@@ -64,8 +65,14 @@ __global__ void __launch_bounds__(256) k_nl_advance(StateBuf b, uint32_t n, cons
                                                      float4* __restrict__ pos4, const float4* __restrict__ ref,
                                                      float lim2, uint32_t* __restrict__ flag,
                                                      uint32_t* __restrict__ err, long long* __restrict__ F,
-                                                     size_t fstride) {
+                                                     size_t fstride, unsigned long long* __restrict__ counts,
+                                                     cudaGraphConditionalHandle body, int has_body) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        // the force pass's potential, pair and bond-energy counters start at zero
+        counts[0] = counts[1] = counts[2] = counts[3] = 0ull;
+        if (has_body && *(volatile uint32_t*)flag != 0u) cudaGraphSetConditional(body, 1u);  // asked for beforehand
+    }
     if (F && i < n) {  // the half-list pass accumulates into F: zero it here, not in a separate memset
         F[i] = 0;
         F[fstride + i] = 0;
@@ -75,7 +82,8 @@ __global__ void __launch_bounds__(256) k_nl_advance(StateBuf b, uint32_t n, cons
     const bool half = ((flag[2] + (wrap ? 1u : 0u)) & 1u) != 0u;
     const bool over =
         i < n && nl_advance_one(b, i, lambda, half_dt, dt, hx, hy, hz, wrap, g, home, pos4, ref, lim2, half, err);
-    if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0) atomicOr(flag, 1u);
+    if (__any_sync(0xffffffffu, over) && (threadIdx.x & 31) == 0 && atomicOr(flag, 1u) == 0u && has_body)
+        cudaGraphSetConditional(body, 1u);
 }
 
 // buf[cur ^ 1] (just gathered) back into buf[cur], so the live state never
@@ -174,22 +182,61 @@ __global__ void __launch_bounds__(kNlBuildThreads) k_nl_build_warp(GridGeom g, c
     if (p < n) nl_build_warp_one<HALF>(g, pos4, home, start, p, rl2, list, stride, cap_nb, cnt);  // whole warps
 }
 
-// The rebuild body's condition: the flag k_nl_advance raised.
-__global__ void k_nl_set_cond(cudaGraphConditionalHandle hc, const uint32_t* __restrict__ flag) {
-    cudaGraphSetConditional(hc, flag[0] != 0u ? 1u : 0u);
-}
-
 __global__ void k_nl_body_done(uint32_t* flag) { flag[3] += 1u; }
 
-__global__ void k_nl_end(uint32_t* flag, int wrap, unsigned long long* __restrict__ counts) {
-    // the force pass's potential, pair and bond-energy counters start at zero
-    counts[0] = counts[1] = counts[2] = counts[3] = 0ull;
-    if (flag[0]) {
-        flag[1] += 1u;
-        flag[0] = 0u;
-        flag[2] = 0u;
-    } else if (wrap) {
-        flag[2] ^= 1u;
+// What ends a tick, in one block: the FP64 pass's potential, K and the
+// Berendsen scale (thermostat.rs:58-71), the record, the scale slot back to 1
+// where a scale was applied and none follows, and the rebuild bookkeeping
+// (count a rebuild and restart the parity, or toggle it with this tick's
+// wrap).  The sums are k_thermostat_lambda's and k_finalize_two's.  One launch
+// instead of up to five, with the rebuild's condition set by k_nl_advance:
+// some 2.5 us each of a tick of 93 us at 59,319 atoms.
+struct CloseArgs {
+    const double *kpart, *spart, *vpart;  // vpart: FP64 potentials, or null
+    int nb;
+    uint32_t n;
+    int thermo, reset;
+    double k_thermal, target, tau;
+    double* dscal;
+    unsigned long long* dcount;
+    gx_tick_stats* rec;
+    uint32_t* flag;
+    int wrap;
+};
+__global__ void __launch_bounds__(kRedThreads) k_nl_close(CloseArgs a) {
+    __shared__ double sh[kRedThreads / 32];
+    auto sum = [&](const double* part) {
+        double v = 0.0;
+        for (int i = threadIdx.x; i < a.nb; i += kRedThreads) v = xadd(v, part[i]);
+        return block_sum_d<kRedThreads>(v, sh);
+    };
+    const double V = a.vpart ? sum(a.vpart) : 0.0;
+    const double K = a.kpart ? sum(a.kpart) : 0.0;
+    const double S = a.rec ? sum(a.spart) : 0.0;
+    if (threadIdx.x != 0) return;
+    if (a.vpart) a.dscal[2] = V;
+    const double l = a.thermo ? berendsen_scale(K, a.n, a.k_thermal, a.target, a.tau) : 1.0;
+    if (a.thermo || a.reset) a.dscal[0] = l;
+    if (a.rec) {
+        a.dscal[1] = K;
+        a.dscal[4] = S;
+        const unsigned long long k = a.dcount[5];
+        gx_tick_stats& r = a.rec[k];
+        // of the scaled v: lambda^2 K and lambda S (equal to the sums over the scaled components up to rounding)
+        r.kinetic = a.thermo ? xmul(xmul(K, l), l) : K;
+        r.speed_sum = a.thermo ? xmul(S, l) : S;
+        r.potential = a.dscal[2];
+        r.bond_energy = a.dscal[3];
+        r.lambda = l;
+        r.pairs = a.dcount[0];
+        a.dcount[5] = k + 1;
+    }
+    if (a.flag[0]) {
+        a.flag[1] += 1u;
+        a.flag[0] = 0u;
+        a.flag[2] = 0u;
+    } else if (a.wrap) {
+        a.flag[2] ^= 1u;
     }
 }
 
@@ -1050,8 +1097,9 @@ template <int THERMO>
 __global__ void __launch_bounds__(kRedThreads) k_nl_finish64(StateBuf b, uint32_t n, double half_dt,
                                                              double* __restrict__ kpart, double* __restrict__ spart,
                                                              const double* __restrict__ vat,
-                                                             double* __restrict__ vpart) {
+                                                             double* __restrict__ vpart, double* __restrict__ bzero) {
     __shared__ double sh[kRedThreads / 32];
+    if (bzero && blockIdx.x == 0 && threadIdx.x == 0) *bzero = 0.0;  // no spring
     double ks = 0.0, ss = 0.0, vs = 0.0;
     for (uint32_t i = blockIdx.x * kRedThreads + threadIdx.x; i < n; i += gridDim.x * kRedThreads) {
         const double l2 = nl_finish64_one(b, i, half_dt);
@@ -1199,27 +1247,29 @@ int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, in
     StateBuf& o = h->buf[h->cur ^ 1];
     const double half_dt = 0.5 * h->p.dt;
     const float lim = (float)(0.5 * s->skin_used * (1.0 - 1e-4));
-    prof_begin(h, "nl_advance");
-    GX_LAUNCH(h, k_nl_advance, nblk(n, 256), 256, b, n, lambda, half_dt, h->p.dt, 0.5 * h->p.box[0],
-              0.5 * h->p.box[1], 0.5 * h->p.box[2], h->p.enable_boundaries ? 1 : 0, g, h->key_sorted, h->pos4, s->ref,
-              lim * lim, s->flag, h->derr, s->half == 1 ? h->F : nullptr, h->cap);
-    prof_end(h, "nl_advance");
-    // inside a capture: the rebuild goes into the body of an IF node
+    // inside a capture: the rebuild goes into the body of an IF node, whose
+    // condition is 0 at each launch until k_nl_advance sets it
     cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
     GX_CUDA(h, cudaStreamIsCapturing(h->stream, &cst));
     const bool cond = cst == cudaStreamCaptureStatusActive;
+    cudaStreamCaptureStatus st;
+    unsigned long long id = 0;
+    cudaGraph_t gr = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t nd = 0;
+    cudaGraphConditionalHandle hc = 0;
+    if (cond) {
+        GX_CUDA(h, cudaStreamGetCaptureInfo(h->stream, &st, &id, &gr, &deps, &nd));
+        GX_CUDA(h, cudaGraphConditionalHandleCreate(&hc, gr, 0, cudaGraphCondAssignDefault));
+    }
+    prof_begin(h, "nl_advance");
+    GX_LAUNCH(h, k_nl_advance, nblk(n, 256), 256, b, n, lambda, half_dt, h->p.dt, 0.5 * h->p.box[0],
+              0.5 * h->p.box[1], 0.5 * h->p.box[2], h->p.enable_boundaries ? 1 : 0, g, h->key_sorted, h->pos4, s->ref,
+              lim * lim, s->flag, h->derr, s->half == 1 ? h->F : nullptr, h->cap, h->dcount, hc, cond ? 1 : 0);
+    prof_end(h, "nl_advance");
     cudaStream_t main_stream = h->stream;
     uint64_t body_l0 = 0;
     if (cond) {
-        cudaStreamCaptureStatus st;
-        unsigned long long id = 0;
-        cudaGraph_t gr = nullptr;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t nd = 0;
-        GX_CUDA(h, cudaStreamGetCaptureInfo(h->stream, &st, &id, &gr, &deps, &nd));
-        cudaGraphConditionalHandle hc;
-        GX_CUDA(h, cudaGraphConditionalHandleCreate(&hc, gr, 0, cudaGraphCondAssignDefault));
-        GX_LAUNCH(h, k_nl_set_cond, 1, 1, hc, s->flag);
         GX_CUDA(h, cudaStreamGetCaptureInfo(h->stream, &st, &id, &gr, &deps, &nd));
         cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
         cp.conditional.handle = hc;
@@ -1275,7 +1325,6 @@ int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, in
         if (!rc && ce != cudaSuccess) rc = cuda_err(h, ce, "cudaStreamEndCapture (rebuild body)");
     }
     if (rc) return rc;
-    GX_LAUNCH(h, k_nl_end, 1, 1, s->flag, h->p.enable_boundaries ? 1 : 0, h->dcount);
     prof_end(h, "nl_rebuild");
     // Positions and the slot map are final here (the pair pass, the spring,
     // the collision pass and the finish write only forces and velocities).
@@ -1311,9 +1360,8 @@ int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, in
     if (f64) {
         auto k = mode == 2 ? k_nl_finish64<2> : (mode == 1 ? k_nl_finish64<1> : k_nl_finish64<0>);
         double* vpart = h->red;  // row 0 of the block partials
-        GX_LAUNCH(h, k, nb, kRedThreads, b, n, half_dt, kpart, spart, reinterpret_cast<const double*>(h->F), vpart);
-        if (mode == 2) launch_sum_rows(h, vpart, nb, h->dscal + 2);
-        if (!spring) GX_CUDA(h, cudaMemsetAsync(h->dscal + 3, 0, sizeof(double), h->stream));
+        GX_LAUNCH(h, k, nb, kRedThreads, b, n, half_dt, kpart, spart, reinterpret_cast<const double*>(h->F), vpart,
+                  spring ? nullptr : h->dscal + 3);
     } else {
         auto k = mode == 2 ? k_nl_finish<2> : (mode == 1 ? k_nl_finish<1> : k_nl_finish<0>);
         GX_LAUNCH(h, k, nb, kRedThreads, b, h->F, h->cap, n, half_dt, kpart, spart, vsum, h->dscal + 2, h->dscal + 3);
@@ -1321,6 +1369,28 @@ int nl_tick(gx_handle* h, const double* lambda, double* kpart, double* spart, in
     prof_end(h, "nl_finish");
     if (nb_out) *nb_out = nb;
     return GX_OK;
+}
+
+// The end of a tick, after nl_tick's kernels (kpart, spart, nb as it had them).
+void nl_close(gx_handle* h, const double* kpart, const double* spart, int nb, gx_tick_stats* rec, bool thermo, double tau,
+              bool reset_scale) {
+    CloseArgs a{};
+    a.kpart = kpart;
+    a.spart = spart;
+    a.vpart = h->precision != GX_MIXED && rec ? h->red : nullptr;  // row 0 of the block partials
+    a.nb = nb;
+    a.n = (uint32_t)h->n;
+    a.thermo = thermo ? 1 : 0;
+    a.reset = reset_scale ? 1 : 0;
+    a.k_thermal = h->p.thermal_constant;
+    a.target = h->p.thermostat_temperature;
+    a.tau = tau;
+    a.dscal = h->dscal;
+    a.dcount = h->dcount;
+    a.rec = rec;
+    a.flag = nl_of(h)->flag;
+    a.wrap = h->p.enable_boundaries ? 1 : 0;
+    GX_LAUNCH(h, k_nl_close, 1, kRedThreads, a);
 }
 
 // Rebuilds performed so far (reads the device counter; synchronises).
