@@ -45,7 +45,10 @@ BYTES_PER_ATOM = {
     # scatter: read key, read the cell's start, write the slot; the per-cell
     # ranking: read key, the cell's start and end, write the slot (the cell's
     # segment it scans is an L1/L2 hit)
-    "cell_scatter": 12, "cell_rank": 16, "reorder": 220, "stage_pos4": 45, "kinetic": 32,
+    # the per-tick sort's rank, move and staging in one launch: read the
+    # scatter's order 4, key 4, the state 106; write the state, key, slot map
+    # 114 and the float4 16
+    "cell_scatter": 12, "cell_rank": 16, "reorder": 220, "sort_move": 244, "kinetic": 32,
     # list path: fused kick + drift + wrap + FP32 staging + displacement test
     # (read x v a 72, kind 1, home cell 4, reference float4 16; write x v 48,
     # float4 16, and zero the int64 force sums 24 for the half-list pass),
@@ -854,7 +857,7 @@ def ours_arm(args, dist):
     hbm, hbm_src = hbm_peak()
     epa = entries / u.n if u.n else 0.0
     mem = {}
-    for src, keys in ((prof, ("nl_advance", "nl_finish", "kick", "drift", "wrap", "kinetic", "stage_pos4")),
+    for src, keys in ((prof, ("nl_advance", "nl_finish", "kick", "drift", "wrap", "kinetic", "sort_move")),
                       (prof_rb, REBUILD_KERNELS)):
         for k in keys:
             if k not in src or not src[k][0]:

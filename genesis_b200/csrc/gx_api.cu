@@ -343,14 +343,12 @@ int require_state(gx_handle* h) {
 int rebuild_cells(gx_handle* h) {
     uint32_t n = (uint32_t)h->n;
     StateBuf& src = h->buf[h->cur];
-    launch_cell_keys(h, h->fgrid, src, n, h->key);
-    int rc = counting_sort(h, h->cl, h->fgrid.ncell, h->key, n, h->perm);
+    int rc = sort_by_cell(h, h->cl, h->fgrid, src, h->buf[h->cur ^ 1], n, h->key, h->key_sorted, h->pos_of_slot,
+                          h->precision == GX_MIXED ? h->pos4 : nullptr);
     if (rc) return rc;
-    launch_gather(h, src, h->buf[h->cur ^ 1], h->perm, h->key, h->key_sorted, n, h->pos_of_slot);
     h->cur ^= 1;
     h->sorted = true;
     h->nl_valid = false;
-    if (h->precision == GX_MIXED) launch_build_pos4(h, h->fgrid, h->buf[h->cur], h->key_sorted, n, h->pos4);
     return GX_OK;
 }
 

@@ -104,15 +104,19 @@ __global__ void k_rank(const uint32_t* __restrict__ key, uint32_t n, const uint3
     perm[lo + r] = i;
 }
 
+// With count: also k_count's counts.
 __global__ void k_cell_keys(GridGeom g, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, uint32_t n, uint32_t* __restrict__ key,
-                            uint32_t* __restrict__ err, const uint32_t* __restrict__ gate) {
+                            uint32_t* __restrict__ err, const uint32_t* __restrict__ gate,
+                            uint32_t* __restrict__ count) {
     if (gated_off(gate)) return;
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double px = x[i], py = y[i], pz = z[i];
     if (!isfinite(px) || !isfinite(py) || !isfinite(pz)) atomicOr(err, kErrNonFinite);
-    key[i] = cell_of(g, px, py, pz);
+    const uint32_t c = cell_of(g, px, py, pz);
+    key[i] = c;
+    if (count) atomicAdd(&count[c], 1u);
 }
 
 __global__ void k_gather(StateBuf s, StateBuf d, const uint32_t* __restrict__ perm,
@@ -142,17 +146,48 @@ __global__ void k_gather(StateBuf s, StateBuf d, const uint32_t* __restrict__ pe
     pos_of_slot[sl] = p;
 }
 
-// Cell-local FP32 coordinates (u - i*cell, u as in cell_of) + kind in w.
-__global__ void k_build_pos4(GridGeom g, StateBuf b, const uint32_t* __restrict__ key, uint32_t n,
-                             float4* __restrict__ pos4) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// The per-tick sort's last step in one launch: k_rank's place of each atom
+// (thread t takes the t-th of the scatter's order, whose place is near t),
+// k_gather's move, and with pos4 the mixed pass's staging: cell-local FP32
+// coordinates (u - i*cell, u as in cell_of) + kind in w.  With k_cell_keys
+// counting, a re-sort is four launches instead of seven (22 -> 14 us of
+// kernels at 29,791 atoms).
+__global__ void k_rank_gather(GridGeom g, StateBuf s, StateBuf d, const uint32_t* __restrict__ key,
+                              const uint32_t* __restrict__ start, const uint32_t* __restrict__ scattered, uint32_t n,
+                              uint32_t* __restrict__ key_out, uint32_t* __restrict__ pos_of_slot,
+                              float4* __restrict__ pos4) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const uint32_t q = scattered[t], c = key[q];
+    const uint32_t lo = start[c], hi = start[c + 1];
+    uint32_t r = 0;
+    for (uint32_t b = lo; b < hi; ++b) r += __ldg(scattered + b) < q ? 1u : 0u;
+    const uint32_t p = lo + r;
+    const double x = s.x[q], y = s.y[q], z = s.z[q];
+    const uint8_t kind = s.kind[q];
+    d.x[p] = x;
+    d.y[p] = y;
+    d.z[p] = z;
+    d.vx[p] = s.vx[q];
+    d.vy[p] = s.vy[q];
+    d.vz[p] = s.vz[q];
+    d.ax[p] = s.ax[q];
+    d.ay[p] = s.ay[q];
+    d.az[p] = s.az[q];
+    d.charge[p] = s.charge[q];
+    d.mass[p] = s.mass[q];
+    d.inv_mass[p] = s.inv_mass[q];
+    d.elem[p] = s.elem[q];
+    d.kind[p] = kind;
+    const uint32_t sl = s.slot[q];
+    d.slot[p] = sl;
+    key_out[p] = c;
+    pos_of_slot[sl] = p;
+    if (!pos4) return;
     uint32_t ix, iy, iz;
-    decode(g, key[i], ix, iy, iz);
-    double ux = cell_local(b.x[i], g.L[0], g.cell[0], ix);
-    double uy = cell_local(b.y[i], g.L[1], g.cell[1], iy);
-    double uz = cell_local(b.z[i], g.L[2], g.cell[2], iz);
-    pos4[i] = make_float4((float)ux, (float)uy, (float)uz, __int_as_float((int)b.kind[i]));
+    decode(g, c, ix, iy, iz);
+    pos4[p] = make_float4((float)cell_local(x, g.L[0], g.cell[0], ix), (float)cell_local(y, g.L[1], g.cell[1], iy),
+                          (float)cell_local(z, g.L[2], g.cell[2], iz), __int_as_float((int)kind));
 }
 
 // VelocityHalfKick (src/systems/integrate.rs:38-45), with the pending
@@ -396,7 +431,7 @@ void launch_cell_keys(gx_handle* h, const GridGeom& g, const StateBuf& b, uint32
                       const uint32_t* gate) {
     if (!n) return;
     prof_begin(h, "cell_keys");
-    GX_LAUNCH(h, k_cell_keys, nblk(n, 256), 256, g, b.x, b.y, b.z, n, key, h->derr, gate);
+    GX_LAUNCH(h, k_cell_keys, nblk(n, 256), 256, g, b.x, b.y, b.z, n, key, h->derr, gate, nullptr);
     prof_end(h, "cell_keys");
 }
 
@@ -409,12 +444,26 @@ void launch_gather(gx_handle* h, const StateBuf& src, const StateBuf& dst, const
     prof_end(h, "reorder");
 }
 
-void launch_build_pos4(gx_handle* h, const GridGeom& g, const StateBuf& b, const uint32_t* key, uint32_t n,
-                       float4* pos4) {
-    if (!n) return;
-    prof_begin(h, "stage_pos4");
-    GX_LAUNCH(h, k_build_pos4, nblk(n, 256), 256, g, b, key, n, pos4);
-    prof_end(h, "stage_pos4");
+int sort_by_cell(gx_handle* h, CellList& cl, const GridGeom& g, const StateBuf& src, const StateBuf& dst, uint32_t n,
+                 uint32_t* key, uint32_t* key_out, uint32_t* pos_of_slot, float4* pos4) {
+    int rc = ensure_cells(h, cl, g.ncell);
+    if (rc) return rc;
+    if ((rc = ensure_sort_tmp(h, cl, n))) return rc;  // allocated before any capture by the callers that capture
+    prof_begin(h, "cell_keys");
+    GX_CUDA(h, cudaMemsetAsync(cl.count, 0, ((size_t)g.ncell + 1) * sizeof(uint32_t), h->stream));
+    GX_CUDA(h, cudaMemsetAsync(cl.fill, 0, (size_t)g.ncell * sizeof(uint32_t), h->stream));
+    if (n)
+        GX_LAUNCH(h, k_cell_keys, nblk(n, 256), 256, g, src.x, src.y, src.z, n, key, h->derr, nullptr, cl.count);
+    prof_end(h, "cell_keys");
+    cell_scan(h, cl, g.ncell);
+    if (!n) return GX_OK;
+    prof_begin(h, "cell_scatter");
+    GX_LAUNCH(h, k_scatter, nblk(n, 256), 256, key, n, cl.start, cl.fill, cl.tmp, nullptr);
+    prof_end(h, "cell_scatter");
+    prof_begin(h, "sort_move");
+    GX_LAUNCH(h, k_rank_gather, nblk(n, 128), 128, g, src, dst, key, cl.start, cl.tmp, n, key_out, pos_of_slot, pos4);
+    prof_end(h, "sort_move");
+    return GX_OK;
 }
 
 void launch_kick(gx_handle* h, const StateBuf& b, uint32_t n, double half_dt, const double* lambda) {

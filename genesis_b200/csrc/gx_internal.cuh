@@ -345,8 +345,10 @@ void launch_cell_keys(gx_handle* h, const GridGeom& g, const StateBuf& b, uint32
 void launch_gather(gx_handle* h, const StateBuf& src, const StateBuf& dst, const uint32_t* perm,
                    const uint32_t* key_in, uint32_t* key_out, uint32_t n, uint32_t* pos_of_slot,
                    const uint32_t* gate = nullptr);
-void launch_build_pos4(gx_handle* h, const GridGeom& g, const StateBuf& b, const uint32_t* key,
-                       uint32_t n, float4* pos4);
+// Cell keys, a deterministic counting sort (each cell in ascending source order) and the move from src to dst; with
+// pos4 also the mixed pass's staging.
+int sort_by_cell(gx_handle* h, CellList& cl, const GridGeom& g, const StateBuf& src, const StateBuf& dst, uint32_t n,
+                 uint32_t* key, uint32_t* key_out, uint32_t* pos_of_slot, float4* pos4);
 
 int force_pass(gx_handle* h, bool finalize_acc, double* V, double* Vb, uint64_t* npairs, bool sync_out);
 // The observed-bond spring over the device bond list (count in dcount[8])
