@@ -41,29 +41,26 @@ FLOP_PER_PAIR_LJC_NOV = 71
 # Algorithmic bytes per atom of each memory-bound kernel (reads + writes of
 # the arrays the kernel must touch; FP64 state, u8 element/kind, u32 ids).
 BYTES_PER_ATOM = {
-    "kick": 72, "drift": 72, "wrap": 48, "cell_keys": 28, "cell_count": 4, "cell_scan": 0,
-    # scatter: read key, read the cell's start, write the slot; the per-cell
-    # ranking: read key, the cell's start and end, write the slot (the cell's
-    # segment it scans is an L1/L2 hit)
-    # the per-tick sort's rank, move and staging in one launch: read the
-    # scatter's order 4, key 4, the state 106; write the state, key, slot map
-    # 114 and the float4 16
-    "cell_scatter": 12, "cell_rank": 16, "reorder": 220, "sort_move": 244, "kinetic": 32,
+    # keys: read x y z 24, write the key 4, count 4; scatter: read key, read
+    # the cell's start, write the slot; the sort's last step: read the
+    # scatter's order 4, key 4 and the state, write the state, key, slot map
+    # (with the accelerations and the float4 staging for the per-tick pass)
+    "kick": 72, "drift": 72, "wrap": 48, "cell_keys": 32, "cell_scan": 0,
+    "cell_scatter": 12, "sort_stage": 244, "sort_move": 172, "kinetic": 32,
     # list path: fused kick + drift + wrap + FP32 staging + displacement test
     # (read x v a 72, kind 1, home cell 4, reference float4 16; write x v 48,
     # float4 16, and zero the int64 force sums 24 for the half-list pass),
     # and fused F -> a + kick + K (read F 24, v 24, 1/m 8, m 8; write a 24,
     # v 24)
     "nl_advance": 181, "nl_finish": 112,
-    # list rebuild: the sorted state copied back (12 f64 columns, 2 u8, 1 u32,
-    # read and written), the staging (read x y z 24, kind 1, home 4; write
-    # the float4 and its reference copy 32); the list build's own bytes
-    # depend on the entries it writes (list_build_bytes_per_atom)
-    "nl_copy": 204, "nl_stage": 61,
+    # list rebuild: the sorted state copied back (9 f64 columns, 2 u8, 1 u32,
+    # read and written) and staged (read home 4; write the float4 and its
+    # reference copy 32); the list build's own bytes depend on the entries it
+    # writes (list_build_bytes_per_atom)
+    "nl_copy": 192,
 }
 # kernels that run only on ticks that rebuild the neighbour list
-REBUILD_KERNELS = ("cell_keys", "cell_count", "cell_scan", "cell_scatter", "cell_rank", "reorder", "nl_copy",
-                   "nl_stage", "nl_build")
+REBUILD_KERNELS = ("cell_keys", "cell_scan", "cell_scatter", "sort_move", "nl_copy", "nl_build")
 
 
 def list_build_bytes_per_atom(entries_per_atom: float) -> float:
@@ -857,7 +854,7 @@ def ours_arm(args, dist):
     hbm, hbm_src = hbm_peak()
     epa = entries / u.n if u.n else 0.0
     mem = {}
-    for src, keys in ((prof, ("nl_advance", "nl_finish", "kick", "drift", "wrap", "kinetic", "sort_move")),
+    for src, keys in ((prof, ("nl_advance", "nl_finish", "kick", "drift", "wrap", "kinetic", "sort_stage")),
                       (prof_rb, REBUILD_KERNELS)):
         for k in keys:
             if k not in src or not src[k][0]:

@@ -173,11 +173,10 @@ int ensure_capacity(gx_handle* h, size_t n) {
     cudaFree(h->F);
     cudaFree(h->host_stage);
     cudaFree(h->red);
-    GX_CUDA(h, cudaMalloc(&h->key, 5 * cap * sizeof(uint32_t)));
+    GX_CUDA(h, cudaMalloc(&h->key, 4 * cap * sizeof(uint32_t)));
     h->key_sorted = h->key + cap;
-    h->perm = h->key + 2 * cap;
-    h->pos_of_slot = h->key + 3 * cap;
-    h->entity = h->key + 4 * cap;
+    h->pos_of_slot = h->key + 2 * cap;
+    h->entity = h->key + 3 * cap;
     GX_CUDA(h, cudaMalloc(&h->pos4, cap * sizeof(float4)));
     GX_CUDA(h, cudaMalloc(&h->F, 3 * cap * sizeof(long long)));
     GX_CUDA(h, cudaMalloc(&h->host_stage, 3 * cap * sizeof(double) + cap * sizeof(uint32_t)));

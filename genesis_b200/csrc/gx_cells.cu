@@ -104,7 +104,7 @@ __global__ void k_rank(const uint32_t* __restrict__ key, uint32_t n, const uint3
     perm[lo + r] = i;
 }
 
-// With count: also k_count's counts.
+// Also k_count's counts.
 __global__ void k_cell_keys(GridGeom g, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, uint32_t n, uint32_t* __restrict__ key,
                             uint32_t* __restrict__ err, const uint32_t* __restrict__ gate,
@@ -116,46 +116,23 @@ __global__ void k_cell_keys(GridGeom g, const double* __restrict__ x, const doub
     if (!isfinite(px) || !isfinite(py) || !isfinite(pz)) atomicOr(err, kErrNonFinite);
     const uint32_t c = cell_of(g, px, py, pz);
     key[i] = c;
-    if (count) atomicAdd(&count[c], 1u);
+    atomicAdd(&count[c], 1u);
 }
 
-__global__ void k_gather(StateBuf s, StateBuf d, const uint32_t* __restrict__ perm,
-                         const uint32_t* __restrict__ key_in, uint32_t* __restrict__ key_out, uint32_t n,
-                         uint32_t* __restrict__ pos_of_slot, const uint32_t* __restrict__ gate) {
-    if (gated_off(gate)) return;
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    uint32_t q = perm[p];
-    d.x[p] = s.x[q];
-    d.y[p] = s.y[q];
-    d.z[p] = s.z[q];
-    d.vx[p] = s.vx[q];
-    d.vy[p] = s.vy[q];
-    d.vz[p] = s.vz[q];
-    d.ax[p] = s.ax[q];
-    d.ay[p] = s.ay[q];
-    d.az[p] = s.az[q];
-    d.charge[p] = s.charge[q];
-    d.mass[p] = s.mass[q];
-    d.inv_mass[p] = s.inv_mass[q];
-    d.elem[p] = s.elem[q];
-    d.kind[p] = s.kind[q];
-    uint32_t sl = s.slot[q];
-    d.slot[p] = sl;
-    key_out[p] = key_in[q];
-    pos_of_slot[sl] = p;
-}
-
-// The per-tick sort's last step in one launch: k_rank's place of each atom
-// (thread t takes the t-th of the scatter's order, whose place is near t),
-// k_gather's move, and with pos4 the mixed pass's staging: cell-local FP32
-// coordinates (u - i*cell, u as in cell_of) + kind in w.  With k_cell_keys
+// The last step of a universe's sort in one launch: k_rank's place of each
+// atom (thread t takes the t-th of the scatter's order, whose place is near
+// t), the move, and with pos4 the mixed pass's staging: cell-local FP32
+// coordinates (u - i*cell, u as in cell_of) + kind in w.  Without ACC the
+// accelerations stay behind (a list rebuild sits between the kick that used
+// them and the force pass that replaces them).  With k_cell_keys
 // counting, a re-sort is four launches instead of seven (22 -> 14 us of
 // kernels at 29,791 atoms).
+template <bool ACC>
 __global__ void k_rank_gather(GridGeom g, StateBuf s, StateBuf d, const uint32_t* __restrict__ key,
                               const uint32_t* __restrict__ start, const uint32_t* __restrict__ scattered, uint32_t n,
                               uint32_t* __restrict__ key_out, uint32_t* __restrict__ pos_of_slot,
-                              float4* __restrict__ pos4) {
+                              float4* __restrict__ pos4, const uint32_t* __restrict__ gate) {
+    if (gated_off(gate)) return;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const uint32_t q = scattered[t], c = key[q];
@@ -171,9 +148,11 @@ __global__ void k_rank_gather(GridGeom g, StateBuf s, StateBuf d, const uint32_t
     d.vx[p] = s.vx[q];
     d.vy[p] = s.vy[q];
     d.vz[p] = s.vz[q];
-    d.ax[p] = s.ax[q];
-    d.ay[p] = s.ay[q];
-    d.az[p] = s.az[q];
+    if (ACC) {
+        d.ax[p] = s.ax[q];
+        d.ay[p] = s.ay[q];
+        d.az[p] = s.az[q];
+    }
     d.charge[p] = s.charge[q];
     d.mass[p] = s.mass[q];
     d.inv_mass[p] = s.inv_mass[q];
@@ -427,25 +406,9 @@ int counting_sort(gx_handle* h, CellList& cl, uint32_t ncell, const uint32_t* ke
     return GX_OK;
 }
 
-void launch_cell_keys(gx_handle* h, const GridGeom& g, const StateBuf& b, uint32_t n, uint32_t* key,
-                      const uint32_t* gate) {
-    if (!n) return;
-    prof_begin(h, "cell_keys");
-    GX_LAUNCH(h, k_cell_keys, nblk(n, 256), 256, g, b.x, b.y, b.z, n, key, h->derr, gate, nullptr);
-    prof_end(h, "cell_keys");
-}
-
-void launch_gather(gx_handle* h, const StateBuf& src, const StateBuf& dst, const uint32_t* perm,
-                   const uint32_t* key_in, uint32_t* key_out, uint32_t n, uint32_t* pos_of_slot,
-                   const uint32_t* gate) {
-    if (!n) return;
-    prof_begin(h, "reorder");
-    GX_LAUNCH(h, k_gather, nblk(n, 256), 256, src, dst, perm, key_in, key_out, n, pos_of_slot, gate);
-    prof_end(h, "reorder");
-}
-
 int sort_by_cell(gx_handle* h, CellList& cl, const GridGeom& g, const StateBuf& src, const StateBuf& dst, uint32_t n,
-                 uint32_t* key, uint32_t* key_out, uint32_t* pos_of_slot, float4* pos4) {
+                 uint32_t* key, uint32_t* key_out, uint32_t* pos_of_slot, float4* pos4, bool acc,
+                 const uint32_t* gate) {
     int rc = ensure_cells(h, cl, g.ncell);
     if (rc) return rc;
     if ((rc = ensure_sort_tmp(h, cl, n))) return rc;  // allocated before any capture by the callers that capture
@@ -453,16 +416,20 @@ int sort_by_cell(gx_handle* h, CellList& cl, const GridGeom& g, const StateBuf& 
     GX_CUDA(h, cudaMemsetAsync(cl.count, 0, ((size_t)g.ncell + 1) * sizeof(uint32_t), h->stream));
     GX_CUDA(h, cudaMemsetAsync(cl.fill, 0, (size_t)g.ncell * sizeof(uint32_t), h->stream));
     if (n)
-        GX_LAUNCH(h, k_cell_keys, nblk(n, 256), 256, g, src.x, src.y, src.z, n, key, h->derr, nullptr, cl.count);
+        GX_LAUNCH(h, k_cell_keys, nblk(n, 256), 256, g, src.x, src.y, src.z, n, key, h->derr, gate, cl.count);
     prof_end(h, "cell_keys");
-    cell_scan(h, cl, g.ncell);
+    prof_begin(h, "cell_scan");
+    scan_rec(h, cl, cl.count, cl.start, g.ncell + 1, 0, gate);
+    prof_end(h, "cell_scan");
     if (!n) return GX_OK;
     prof_begin(h, "cell_scatter");
-    GX_LAUNCH(h, k_scatter, nblk(n, 256), 256, key, n, cl.start, cl.fill, cl.tmp, nullptr);
+    GX_LAUNCH(h, k_scatter, nblk(n, 256), 256, key, n, cl.start, cl.fill, cl.tmp, gate);
     prof_end(h, "cell_scatter");
-    prof_begin(h, "sort_move");
-    GX_LAUNCH(h, k_rank_gather, nblk(n, 128), 128, g, src, dst, key, cl.start, cl.tmp, n, key_out, pos_of_slot, pos4);
-    prof_end(h, "sort_move");
+    const char* phase = acc ? "sort_stage" : "sort_move";
+    prof_begin(h, phase);
+    auto move = acc ? k_rank_gather<true> : k_rank_gather<false>;
+    GX_LAUNCH(h, move, nblk(n, 128), 128, g, src, dst, key, cl.start, cl.tmp, n, key_out, pos_of_slot, pos4, gate);
+    prof_end(h, phase);
     return GX_OK;
 }
 

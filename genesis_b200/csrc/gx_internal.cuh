@@ -216,7 +216,6 @@ struct gx_handle {
     // per-atom scratch
     uint32_t* key = nullptr;       // cell key per atom (current order)
     uint32_t* key_sorted = nullptr;
-    uint32_t* perm = nullptr;      // sorted position -> previous position
     uint32_t* pos_of_slot = nullptr;  // ECS slot -> sorted position
     uint32_t* entity = nullptr;    // EntityId::index per ECS slot
     bool has_entity = false;
@@ -340,15 +339,11 @@ void cell_scan(gx_handle* h, CellList& cl, uint32_t ncell);
 // `gate` (may be null): a device word; the launches do nothing while it is 0.
 int counting_sort(gx_handle* h, CellList& cl, uint32_t ncell, const uint32_t* key, uint32_t n,
                   uint32_t* perm, const uint32_t* gate = nullptr);
-void launch_cell_keys(gx_handle* h, const GridGeom& g, const StateBuf& b, uint32_t n, uint32_t* key,
-                      const uint32_t* gate = nullptr);
-void launch_gather(gx_handle* h, const StateBuf& src, const StateBuf& dst, const uint32_t* perm,
-                   const uint32_t* key_in, uint32_t* key_out, uint32_t n, uint32_t* pos_of_slot,
-                   const uint32_t* gate = nullptr);
 // Cell keys, a deterministic counting sort (each cell in ascending source order) and the move from src to dst; with
-// pos4 also the mixed pass's staging.
+// pos4 also the mixed pass's staging, without acc all but the accelerations.
 int sort_by_cell(gx_handle* h, CellList& cl, const GridGeom& g, const StateBuf& src, const StateBuf& dst, uint32_t n,
-                 uint32_t* key, uint32_t* key_out, uint32_t* pos_of_slot, float4* pos4);
+                 uint32_t* key, uint32_t* key_out, uint32_t* pos_of_slot, float4* pos4, bool acc = true,
+                 const uint32_t* gate = nullptr);
 
 int force_pass(gx_handle* h, bool finalize_acc, double* V, double* Vb, uint64_t* npairs, bool sync_out);
 // The observed-bond spring over the device bond list (count in dcount[8])
