@@ -1249,7 +1249,12 @@ int gx_tick_host(gx_handle* h, double* pos, double* vel, double* acc, gx_tick_st
                                                             "acceleration columns");
     if ((rc = settle_step_errors(h))) return rc;
     if (!h->io_stream) {
-        GX_CUDA(h, cudaStreamCreateWithFlags(&h->io_stream, cudaStreamNonBlocking));
+        // high priority: the positions' gather runs beside the pair pass, whose blocks fill every SM; queued behind
+        // them its copy starts a pass late (790 us a tick at 262,144 atoms, 795 to 840 from run to run at
+        // the default priority)
+        int least = 0, greatest = 0;
+        GX_CUDA(h, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        GX_CUDA(h, cudaStreamCreateWithPriority(&h->io_stream, cudaStreamNonBlocking, greatest));
         for (cudaEvent_t& e : h->io_ev) GX_CUDA(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     if (!h->io_events) {
