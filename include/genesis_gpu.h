@@ -105,8 +105,9 @@ const char* gx_last_error(const gx_handle* h);
 const char* gx_status_string(int status);
 int gx_set_precision(gx_handle* h, int precision);
 /* Tuning knob of the mixed pair pass: 0 = automatic (6 where it applies,
- * else 4; up to 65,536 atoms with no work shape set, the ticks of a gx_step
- * call with use_graph run in one launch, the same bits), 1 = one thread per atom over the canonical half shell,
+ * else 4; up to 65,536 atoms, 24,576 in FP64, with no work shape set, the
+ * ticks of a gx_step call with use_graph run in one launch, the same bits),
+ * 1 = one thread per atom over the canonical half shell,
  * 2 = warp-tiled cell pairs with ballot compaction, 3 = thread per atom with
  * staged rows, 4 = thread per atom with per-thread candidate lists (all
  * four re-sort the atoms by the force grid every tick, as the reference
