@@ -40,7 +40,7 @@
 // the launch, on the ticks on which an atom may have moved skin/2 since.
 // What bounds a tick is latency: 13 warps per SM walk lists of ten to twenty
 // partners, each a chain of dependent FP64 operations.  8,000 atoms, 200
-// ticks, mixed forward, both losses: 29.4 ms, where a sort, a staging and a
+// ticks, mixed forward, both losses: 34.6 ms, where a sort, a staging and a
 // pair pass over 27 cells per tick, one kernel each, took 143 ms; per tick
 // 13 us for the recomputed pair pass, 17 / 30 for the reverse pass without /
 // with g(r), 40 for a list rebuild every ten ticks.  Lists of rc + 0.2 rc:
@@ -86,7 +86,6 @@ struct Vec3Field {
 struct GrSpec {
     int bins;
     double dr, width, reach, c2;  // bin width, kernel width, truncation radius, -1/(2 w^2)
-    double step;                  // exp(2 c2 dr^2): how the ratio of neighbouring bins' kernels changes per bin
 };
 
 // Switch S(r) of smooth_cutoff (forces.rs:302-318) with its first two
@@ -466,24 +465,21 @@ __device__ __forceinline__ double adj_image(const AdjArgs& a, double d, int k) {
     return a.plain ? min_image_near(d, a.L.box[k], a.half_box[k]) : near_image(d, a.L.box[k]);
 }
 
-// The bins within the kernel's reach of distance d: f(bin, G_bin) with
-// G = exp(c2 z^2), z = d - centre[bin].  Along the bins z changes by -dr, so G
-// follows from two exponentials by two products a bin (their rounding adds to
-// some 1e-15; the sums keep 2^-32).
+// The bins within the kernel's reach of distance d: f(bin, z, G) with
+// z = d - centre and G = exp(c2 z^2).  An exponential per bin: a recurrence
+// over the bins loses all of them where the one it starts from underflows
+// (supports of some 38 widths), and its rounding grows with the square of
+// their number (8,000 atoms, 200 ticks, both losses: 29.5 ms so, 34.6 with the
+// exponentials).
 template <class F>
-__device__ __forceinline__ void gr_bins(const GrSpec& gs, const double* centre, double d, F&& f) {
+__device__ __forceinline__ void gr_bins(const GrSpec& gs, double d, F&& f) {
     int k0 = (int)ceil((d - gs.reach) / gs.dr - 0.5), k1 = (int)floor((d + gs.reach) / gs.dr - 0.5);
     k0 = k0 < 0 ? 0 : k0;
     k1 = k1 > gs.bins - 1 ? gs.bins - 1 : k1;
-    if (k0 <= k1 && !(fabs(d - centre[k0]) < gs.reach)) ++k0;  // within rounding of the reach
-    if (k0 <= k1 && !(fabs(d - centre[k1]) < gs.reach)) --k1;
-    if (k0 > k1) return;
-    const double z = d - centre[k0];
-    double G = exp(z * z * gs.c2), R = exp(gs.c2 * gs.dr * (gs.dr - 2.0 * z));
-    for (int b = k0; b <= k1; ++b) {
-        f(b, G);
-        G *= R;
-        R *= gs.step;
+    double at = k0 + 0.5;
+    for (int b = k0; b <= k1; ++b, at += 1.0) {
+        const double z = d - at * gs.dr;
+        if (fabs(z) < gs.reach) f(b, z, exp(z * z * gs.c2));
     }
 }
 
@@ -497,7 +493,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
     extern __shared__ uint32_t s_hist[];  // with obs a histogram per warp: low 16 bits' sums, then the rest's
     __shared__ double s_sig[kNElem * kNElem], s_eps[kNElem * kNElem], s_e24[kNElem * kNElem];
     __shared__ PairTab s_tab;
-    __shared__ double sh[kAdjThreads / 32], s_r[kAdjMaxBins], s_queue[kAdjThreads / 32][kAdjQueue];
+    __shared__ double sh[kAdjThreads / 32], s_queue[kAdjThreads / 32][kAdjQueue];
     __shared__ uint32_t s_queued[kAdjThreads / 32];
     __shared__ uint32_t s_warp[kAdjThreads / 32], s_off[kScanMaxTiles];
     __shared__ AdjFound s_found[kAdjThreads / 32];
@@ -518,7 +514,6 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
     if (F32)
         for (int k = tid; k < a.L32.nkinds * a.L32.nkinds; k += kAdjThreads) s_tab.put(k, a.tabf[k]);
     for (int k = tid; k < (kAdjThreads / 32) * 2 * bins; k += kAdjThreads) s_hist[k] = 0u;
-    for (int k = tid; k < bins; k += kAdjThreads) s_r[k] = (k + 0.5) * a.gs.dr;
     uint32_t* wh = s_hist + (tid / 32) * 2 * bins;
     uint32_t held = 0;  // terms that a bin of this warp's histogram may hold
     if (tid < kAdjThreads / 32) s_queued[tid] = 0u;
@@ -678,7 +673,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
                             return;
                         }
                     }
-                    gr_bins(a.gs, s_r, d, [&](int b, double G) {
+                    gr_bins(a.gs, d, [&](int b, double, double G) {
                         const unsigned long long v = (unsigned long long)(mult * llrint(G * kHistScale));
                         if (direct) atomicAdd(&a.ghist[turn * bins + b], v);
                         else into_warp(b, v);
@@ -689,8 +684,8 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
                 __syncwarp();
                 const uint32_t queued = min(s_queued[tid / 32], kAdjQueue);
                 for (uint32_t k = tid & 31u; k < queued; k += 32)
-                    gr_bins(a.gs, s_r, s_queue[tid / 32][k],
-                            [&](int b, double G) { into_warp(b, (unsigned long long)llrint(G * kHistScale)); });
+                    gr_bins(a.gs, s_queue[tid / 32][k],
+                            [&](int b, double, double G) { into_warp(b, (unsigned long long)llrint(G * kHistScale)); });
                 __syncwarp();
                 if ((tid & 31u) == 0) s_queued[tid / 32] = 0u;
                 __syncwarp();
@@ -735,7 +730,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
 // rc_coulomb, rc_gravity partials per atom.
 __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_constant__ AdjArgs a) {
     __shared__ double s_sig[kNElem * kNElem], s_eps[kNElem * kNElem], s_is[kNElem * kNElem];
-    __shared__ double s_bw[kAdjMaxBins], s_r[kAdjMaxBins];
+    __shared__ double s_bw[kAdjMaxBins];
     __shared__ uint32_t s_warp[kAdjThreads / 32], s_off[kScanMaxTiles];
     __shared__ AdjFound s_found[kAdjThreads / 32];
     __shared__ int s_ok;
@@ -750,10 +745,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_con
         s_is[k] = 1.0 / a.psig[k];
     }
     if (a.gr)
-        for (int k = tid; k < a.gs.bins; k += kAdjThreads) {
-            s_bw[k] = a.bw[k] * (2.0 * a.gs.c2);
-            s_r[k] = (k + 0.5) * a.gs.dr;
-        }
+        for (int k = tid; k < a.gs.bins; k += kAdjThreads) s_bw[k] = a.bw[k];
     for (uint32_t c = gt; c < a.lg.ncell + 1; c += gs) a.count[c] = a.fill[c] = 0u;
     for (uint32_t e = gt; e < lanes; e += gs) {  // W/m of the last tick
         const uint32_t i = e / kAdjLanes, l = e % kAdjLanes;
@@ -807,7 +799,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_con
                                               far ? a.mass[j] : 0.0);
                     double psi = 0.0;
                     if (gr)
-                        gr_bins(a.gs, s_r, d, [&](int b, double Gb) { psi += s_bw[b] * ((d - s_r[b]) * Gb); });
+                        gr_bins(a.gs, d, [&](int b, double z, double Gb) { psi += s_bw[b] * (2.0 * a.gs.c2 * z) * Gb; });
                     const double mult =
                         a.two ? (double)pair_multiplicity(a.fg, packed_cell(pi.w), packed_cell(pj.w)) : 1.0;
                     const double c1 = mult * (rho * G.fd + alpha * G.Ud + psi), c2 = mult * (G.f * inv);
@@ -1008,7 +1000,6 @@ GrSpec gr_spec(const AdjBuffers* A) {
     g.width = A->gr_width;
     g.reach = A->gr_support * A->gr_width;
     g.c2 = A->gr_width > 0 ? -0.5 / (A->gr_width * A->gr_width) : 0.0;
-    g.step = std::exp(2.0 * g.c2 * g.dr * g.dr);
     return g;
 }
 

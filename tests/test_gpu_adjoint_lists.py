@@ -86,3 +86,39 @@ def test_many_bins_long_horizon_and_far_atoms(gpu):
         V, g = h.adjoint_forward(3, checkpoint_every=2, gr_bins=16, gr_rmax=4.8, gr_width=0.1)
         gs, ge = h.adjoint_backward(dl_dpotential=np.ones(3), dl_dgr=np.ones(16))
     assert not V.any() and not g.any() and not gs.any() and not ge.any()
+
+
+@pytest.mark.parametrize("bins,rmax,width,support", [(50, 4.0, 0.02, 6.0), (50, 4.0, 0.02, 30.0), (50, 4.0, 0.02, 40.0),
+                                                     (512, 3.5, 0.015, 100.0)])
+def test_wide_supports_of_the_bins_kernel(gpu, orc, bins, rmax, width, support):
+    """A bin's kernel of its own value, however far away its row of bins begins: no weight is lost where the first
+    bins' underflow."""
+    cfg, u = _case(7, coul=True)
+    _against_dual(orc, cfg, u, 6, 3, dict(gr_bins=bins, gr_every=2, gr_rmax=rmax, gr_width=width, gr_support=support))
+
+
+def test_weights_of_one_pair(gpu):
+    """g(r) of a single pair is a row of kernel values in 2^-32 steps, and the initial positions' gradient one term of
+    them: no further off than the few roundings of a bin's own exponential."""
+    from genesis_b200._lib import Handle
+    cfg, _ = _case(8)
+    L = cfg.size[0]
+    bins, rmax, width, support = 512, 4.0, 0.1, 6.0
+    d = 147.0 / 64.0  # exact through the wrap, as d - r is for centres in 256ths
+    pos = np.array([[0.0, 0.0, 0.0], [d, 0.0, 0.0]])
+    r = (np.arange(bins) + 0.5) * (rmax / bins)
+    z = d - r
+    c = L ** 3 / (4.0 * np.pi * r ** 2 * np.sqrt(2.0 * np.pi) * width)
+    G = np.where(np.abs(z) < support * width, np.exp(-0.5 * (z / width) ** 2), 0.0)
+    with Handle(cfg, "fp64") as h:
+        h.set_state(pos, np.zeros_like(pos), np.zeros(2, np.uint8))  # at rest: the first drift leaves them in place
+        _, g = h.adjoint_forward(1, checkpoint_every=1, gr_bins=bins, gr_rmax=rmax, gr_width=width, gr_support=support)
+        assert np.max(np.abs(g / c - G)) <= 2.0 ** -33 * (1.0 + 2.0 ** -10)
+        for k in np.flatnonzero(G)[::5]:
+            w = np.zeros(bins)
+            w[k] = 1.0
+            _, _, (gx, _, _) = h.adjoint_backward(dl_dgr=w, initial_state=True)
+            want = -c[k] * z[k] / width ** 2 * G[k]
+            # three roundings of the exponent on each side, relative to it, and a dozen of the factors
+            rel = 2.0 ** -50 * (4.0 + 0.5 * (z[k] / width) ** 2)
+            assert abs(gx[1, 0] - want) <= rel * abs(want)
