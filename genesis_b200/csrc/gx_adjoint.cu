@@ -1060,11 +1060,14 @@ AdjArgs adj_args(gx_handle* h, AdjBuffers* A) {
     return a;
 }
 
+// k_adj_ticks' histograms: one per warp, two words a bin.
+constexpr size_t hist_bytes(int bins) { return (size_t)(kAdjThreads / 32) * 2 * bins * sizeof(uint32_t); }
+
 // One cooperative launch of kernel `which` (AdjBuffers::resident).
 int adj_launch(gx_handle* h, AdjBuffers* A, int which, AdjArgs& a) {
     const void* kern = which == 2 ? (const void*)k_adj_reverse
                                   : (which == 1 ? (const void*)k_adj_ticks<true> : (const void*)k_adj_ticks<false>);
-    const size_t smem = which < 2 ? (size_t)(kAdjThreads / 32) * 2 * A->bins * sizeof(uint32_t) : 0;
+    const size_t smem = which < 2 ? hist_bytes(A->bins) : 0;
     if (smem != A->resident_smem && which < 2) {
         A->resident[0] = A->resident[1] = 0;
         A->resident_smem = smem;
@@ -1072,7 +1075,9 @@ int adj_launch(gx_handle* h, AdjBuffers* A, int which, AdjArgs& a) {
     int& resident = A->resident[which];
     if (!resident) {
         int per = 0, sms = 0;
-        if (smem) GX_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the limit belongs to the kernel, not to this handle: the most that any handle asks for
+        if (which < 2)
+            GX_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hist_bytes(kAdjMaxBins)));
         GX_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kAdjThreads, smem));
         GX_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->p.device));
         resident = std::max(per * sms, 1);

@@ -122,3 +122,31 @@ def test_weights_of_one_pair(gpu):
             # three roundings of the exponent on each side, relative to it, and a dozen of the factors
             rel = 2.0 ** -50 * (4.0 + 0.5 * (z[k] / width) ** 2)
             assert abs(gx[1, 0] - want) <= rel * abs(want)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_handles_of_different_bins_side_by_side(gpu, precision):
+    """The many bins' launch after another handle's few: each handle as if it were alone."""
+    from genesis_b200._lib import Handle
+    cfg, u = _case(8)
+
+    def forward(h, bins):
+        h.set_universe(u)
+        return h.adjoint_forward(6, checkpoint_every=2, gr_bins=bins, gr_rmax=4.5, gr_width=0.08)
+
+    def backward(h, bins):
+        return h.adjoint_backward(dl_dpotential=np.ones(6), dl_dgr=np.ones(bins))
+
+    alone = []
+    for bins in (512, 16):
+        with Handle(cfg, precision) as h:
+            alone.append((forward(h, bins), backward(h, bins)))
+    with Handle(cfg, precision) as a, Handle(cfg, precision) as b:
+        fa, fb = forward(a, 512), forward(b, 16)
+        ba, bb = backward(a, 512), backward(b, 16)
+        again = a.adjoint_forward(6, checkpoint_every=2, gr_bins=512, gr_rmax=4.5, gr_width=0.08)
+    for (f, g), fwd, back in zip(alone, (fa, fb), (ba, bb)):
+        for x, y in zip(f + g, fwd + back):
+            assert np.array_equal(x, y)
+    for x, y in zip(alone[0][0], again):
+        assert np.array_equal(x, y)
