@@ -40,7 +40,7 @@
 // the launch, on the ticks on which an atom may have moved skin/2 since.
 // What bounds a tick is latency: 13 warps per SM walk lists of ten to twenty
 // partners, each a chain of dependent FP64 operations.  8,000 atoms, 200
-// ticks, mixed forward, both losses: 34.6 ms, where a sort, a staging and a
+// ticks, mixed forward, both losses: 36.2 ms, where a sort, a staging and a
 // pair pass over 27 cells per tick, one kernel each, took 143 ms; per tick
 // 13 us for the recomputed pair pass, 17 / 30 for the reverse pass without /
 // with g(r), 40 for a list rebuild every ten ticks.  Lists of rc + 0.2 rc:
@@ -229,21 +229,28 @@ __global__ void k_adj_import(StateBuf b, uint32_t n, Vec3Field x, Vec3Field v, V
     kind[s] = b.kind[p];
 }
 
-// The lane that visits partner j: neighbours in space are mostly runs of
-// neighbouring slots, which this deals out evenly.
-__device__ __forceinline__ uint32_t lane_of(uint32_t j) { return j % kAdjLanes; }
-constexpr uint32_t kAdjFound = 256;  // partners of one atom that a rebuild can hold
+// The lane that visits partner j: a multiplicative hash, so that no pattern of
+// slots puts a neighbourhood on one lane.  With j % 8 the longest lane of an
+// atom of a lattice whose side is a multiple of 8 holds 21 of 65 partners, and
+// of slots a multiple of 8 apart all of them; with this multiplier, searched
+// for lattices of side 8 to 80 and strides up to 65, 12 on average and at most
+// 16.  Gradients of 262,144 atoms (side 64) take 62 ms instead of 81, those of
+// 8,000 (side 20, which j % 8 deals out well) 36.2 instead of 35.5.
+static_assert(kAdjLanes == 8, "three bits of the hash");
+__device__ __forceinline__ uint32_t lane_of(uint32_t j) { return (j * 3192787907u) >> 29; }
+constexpr uint32_t kAdjFound = 512;  // partners of one atom that a rebuild sorts at a time
 constexpr uint32_t kAdjQueue = 128;  // distances that a warp collects for the histogram
 
-// A rebuild's words of one warp: the partners found, as (lane, slot) keys
-// padded to whole vectors, and how many each lane has.
+// A rebuild's words of one warp: the partners found by a pass, as (lane, slot)
+// keys padded to whole vectors; by lane, how many they are, how many earlier
+// passes wrote, and where in the pool the lane's entries beyond its row go.
 struct __align__(16) AdjFound {
     uint32_t key[kAdjFound + 4];
-    uint32_t count[kAdjLanes];
+    uint32_t count[kAdjLanes], have[kAdjLanes], pool[kAdjLanes];
 };
 
 struct AdjArgs {
-    GridGeom lg;  // list grid: cells >= rc + skin
+    GridGeom lg;  // list grid: cells >= rc + skin (with `walk` >= rc)
     GridGeom fg;  // force grid: its axes of two cells repeat pairs
     int two;      // the force grid has such an axis
     int plain;    // at least three force cells per axis, positions wrapped
@@ -265,9 +272,14 @@ struct AdjArgs {
     int obs;              // record the observables
     uint32_t* list;       // entry k of lane e = i * kAdjLanes + l at [k * kAdjLanes * cap + e], ascending slots
     uint32_t* cnt;
-    int cap_l;
+    uint32_t cap_l;
+    uint32_t *pool, *off; // entry k >= cap_l of lane e at pool[off[e] + k - cap_l]
+    unsigned long long* pool_used;  // words of the pool that the last rebuild asked for
+    unsigned long long pool_cap;
+    int walk;             // no lists: a sort and a walk over the cells every tick
     double* ref;          // positions at the last rebuild, three rows
-    double* sorted;       // a rebuild's cell-sorted (x, y, z, slot)
+    double* sorted;       // a rebuild's cell-sorted (x, y, z, slot); with `walk` slots in the scatter's order
+    uint32_t* order;      // with `walk`: slots by cell, ascending in each
     uint32_t *key, *count, *start, *fill;
     GridSync* sync;
     uint32_t* err;
@@ -315,8 +327,89 @@ __device__ __forceinline__ double list_image(const AdjArgs& a, double d, int k) 
     return d - a.L.box[k] * rint(d * a.inv_box[k]);
 }
 
+// Neighbour cell k < 27 of cell (cx, cy, cz), every distinct one once (both
+// sides of an axis only from three cells on); false for a repeated one.
+__device__ __forceinline__ bool adj_cell(const GridGeom& g, uint32_t cx, uint32_t cy, uint32_t cz, uint32_t k,
+                                         uint32_t& B) {
+    const int ox = (int)(k % 3u) - 1, oy = (int)((k / 3u) % 3u) - 1, oz = (int)(k / 9u) - 1;
+    if (!((ox == 0 || g.n[0] >= 3 || (ox > 0 && g.n[0] == 2)) && (oy == 0 || g.n[1] >= 3 || (oy > 0 && g.n[1] == 2)) &&
+          (oz == 0 || g.n[2] >= 3 || (oz > 0 && g.n[2] == 2))))
+        return false;
+    B = encode(g, wrap_add(cx, ox, g.n[0]), wrap_add(cy, oy, g.n[1]), wrap_add(cz, oz, g.n[2]));
+    return true;
+}
+
+// One pass over the candidates of atom i (position pi) for its list: 32 at a
+// time out of the run that the scan `end` of the cells' counts makes of them
+// (`base`: first candidate less the counts before it).  The partners with
+// slots in [from, to) are counted by lane, the first kAdjFound of them kept.
+__device__ __forceinline__ uint32_t adj_collect(const AdjArgs& a, const double4& pi, uint32_t i, uint32_t end,
+                                                uint32_t base, uint32_t total, uint32_t from, uint32_t to,
+                                                AdjFound& found) {
+    constexpr int kAhead = 4;  // candidates of a lane in flight
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    if (lane < kAdjLanes) found.count[lane] = 0u;
+    __syncwarp();
+    uint32_t m2 = 0;
+    for (uint32_t t0 = 0; t0 < total; t0 += 32 * kAhead) {  // every load before the tests
+        double4 pj[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const uint32_t t = t0 + 32u * u + lane;
+            uint32_t k = 0;  // the first cell whose scan exceeds t
+#pragma unroll
+            for (uint32_t step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(0xffffffffu, end, k + step - 1) <= t) k += step;
+            const uint32_t q = __shfl_sync(0xffffffffu, base, k) + t;
+            pj[u] = make_double4(0.0, 0.0, 0.0, __longlong_as_double((long long)i));
+            if (t < total) pj[u] = load_slab(a.sorted, q);
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const uint32_t j = (uint32_t)__double_as_longlong(pj[u].w);
+            const double dx = list_image(a, pi.x - pj[u].x, 0), dy = list_image(a, pi.y - pj[u].y, 1),
+                         dz = list_image(a, pi.z - pj[u].z, 2);
+            const bool hit = j != i && j - from < to - from && dx * dx + dy * dy + dz * dz < a.rl2;
+            const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+            const uint32_t at = m2 + __popc(mask & ((1u << lane) - 1u));
+            if (hit) {
+                if (at < kAdjFound) found.key[at] = lane_of(j) << 28 | j;
+                atomicAdd(&found.count[lane_of(j)], 1u);
+            }
+            m2 += __popc(mask);
+        }
+    }
+    __syncwarp();
+    return m2;
+}
+
+// The pass's m2 <= kAdjFound partners into their lanes' lists, after those of
+// earlier passes: a partner's place is the number of its lane's partners with
+// smaller slots.
+__device__ __forceinline__ void adj_emit(const AdjArgs& a, uint32_t i, uint32_t m2, AdjFound& found) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const size_t stride = (size_t)kAdjLanes * a.cap;
+    if (lane < 4) found.key[m2 + lane] = 0xffffffffu;
+    __syncwarp();
+    for (uint32_t k = lane; k < m2; k += 32) {  // the keys below this one, those of lower lanes aside
+        const uint32_t key = found.key[k], l = key >> 28;
+        uint32_t place = found.have[l];
+        for (uint32_t q = 0; q < m2; q += 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(&found.key[q]);
+            place += (v.x < key) + (v.y < key) + (v.z < key) + (v.w < key);
+        }
+        for (uint32_t q = 0; q < l; ++q) place -= found.count[q];
+        if (place < a.cap_l) a.list[place * stride + i * kAdjLanes + l] = key & 0x0fffffffu;
+        else a.pool[found.pool[l] + (place - a.cap_l)] = key & 0x0fffffffu;
+    }
+    __syncwarp();
+}
+
 // Lists of the pairs within rc + skin of the positions X, by lane; their
-// reference positions.  False when a barrier gave up.
+// reference positions.  With `walk` the cells' slots in ascending order
+// instead.  False when the launch is over: a barrier gave up, or the lists
+// need more room than the pool has (kErrCapacity; the host repeats the call).
 __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target, int* s_ok, uint32_t* s_warp,
                             uint32_t* s_off, AdjFound* s_found) {
     const uint32_t tid = threadIdx.x, gt = blockIdx.x * kAdjThreads + tid, gs = gridDim.x * kAdjThreads;
@@ -330,6 +423,7 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
     if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
     for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x)
         scan_tile<kAdjThreads>(a.count, t, m, &a.sync->tile[t], s_warp);
+    if (gt == 0 && !a.walk) *a.pool_used = 0ull;  // last read before this rebuild began
     if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
     if (tid < ntiles) {
         uint32_t run = 0;
@@ -340,38 +434,44 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
     for (uint32_t c = gt; c < m; c += gs) a.start[c] = a.count[c] + s_off[c / kScanTileCells];
     for (uint32_t i = gt; i < n; i += gs) {
         const uint32_t c = a.key[i];
+        const uint32_t at = a.count[c] + s_off[c / kScanTileCells] + atomicAdd(&a.fill[c], 1u);
+        if (a.walk) {
+            reinterpret_cast<uint32_t*>(a.sorted)[at] = i;
+            continue;
+        }
         const double4 p = load_slab(X, i);
-        double2* to = reinterpret_cast<double2*>(a.sorted) +
-                      2 * (size_t)(a.count[c] + s_off[c / kScanTileCells] + atomicAdd(&a.fill[c], 1u));
+        double2* to = reinterpret_cast<double2*>(a.sorted) + 2 * (size_t)at;
         to[0] = make_double2(p.x, p.y);
         to[1] = make_double2(p.z, __longlong_as_double((long long)i));
     }
     if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
     for (uint32_t c = gt; c < m; c += gs) a.count[c] = a.fill[c] = 0u;  // for the next rebuild
-    // A warp per atom: lane k < 27 looks up neighbour cell k (every distinct
-    // one: both sides of an axis only from three cells on), a scan of the
-    // counts turns the candidates into one run taken 32 at a time, and the
-    // partners found go to shared memory.  A partner's place in its lane's
-    // list is the number of that lane's partners with smaller slots.
-    constexpr int kAhead = 4;  // candidates of a lane in flight
-    const size_t stride = (size_t)kAdjLanes * a.cap;
+    if (a.walk) {
+        const uint32_t* tmp = reinterpret_cast<const uint32_t*>(a.sorted);
+        for (uint32_t i = gt; i < n; i += gs) {
+            const uint32_t lo = a.start[a.key[i]], hi = a.start[a.key[i] + 1];
+            uint32_t p = lo;
+            for (uint32_t q = lo; q < hi; ++q) p += tmp[q] < i ? 1u : 0u;
+            a.order[p] = i;
+        }
+        return grid_barrier(a.sync, a.err, target, s_ok);
+    }
+    // A warp per atom: lane k < 27 looks up neighbour cell k, and a scan of the
+    // counts turns the candidates into one run.  Atoms of more partners than a
+    // pass can sort take them by ranges of slots.
     const uint32_t lane = tid & 31u;
     AdjFound& found = s_found[tid / 32];
-    const int ox = (int)(lane % 3u) - 1, oy = (int)((lane / 3u) % 3u) - 1, oz = (int)(lane / 9u) - 1;
-    const bool distinct = lane < 27 && (ox == 0 || a.lg.n[0] >= 3 || (ox > 0 && a.lg.n[0] == 2)) &&
-                          (oy == 0 || a.lg.n[1] >= 3 || (oy > 0 && a.lg.n[1] == 2)) &&
-                          (oz == 0 || a.lg.n[2] >= 3 || (oz > 0 && a.lg.n[2] == 2));
     for (uint32_t i = gt / 32u; i < n; i += gs / 32u) {
         const double4 pi = load_slab(X, i);
         if (lane < 3) a.ref[lane * a.cap + i] = lane == 0 ? pi.x : (lane == 1 ? pi.y : pi.z);
         uint32_t lo = 0, len = 0;
-        if (distinct) {
-            uint32_t cx, cy, cz;
+        if (lane < 27) {
+            uint32_t cx, cy, cz, B;
             decode(a.lg, a.key[i], cx, cy, cz);
-            const uint32_t B = encode(a.lg, wrap_add(cx, ox, a.lg.n[0]), wrap_add(cy, oy, a.lg.n[1]),
-                                      wrap_add(cz, oz, a.lg.n[2]));
-            lo = a.start[B];
-            len = a.start[B + 1] - lo;
+            if (adj_cell(a.lg, cx, cy, cz, lane, B)) {
+                lo = a.start[B];
+                len = a.start[B + 1] - lo;
+            }
         }
         uint32_t end = len;
 #pragma unroll
@@ -380,82 +480,86 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
             if (lane >= (uint32_t)o) end += v;
         }
         const uint32_t total = __shfl_sync(0xffffffffu, end, 31), base = lo - (end - len);
-        if (lane < kAdjLanes) found.count[lane] = 0u;
-        __syncwarp();
-        uint32_t m2 = 0;
-        for (uint32_t t0 = 0; t0 < total; t0 += 32 * kAhead) {  // every load before the tests
-            double4 pj[kAhead];
-#pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
-                const uint32_t t = t0 + 32u * u + lane;
-                uint32_t k = 0;  // the first cell whose scan exceeds t
-#pragma unroll
-                for (uint32_t step = 16; step > 0; step >>= 1)
-                    if (__shfl_sync(0xffffffffu, end, k + step - 1) <= t) k += step;
-                const uint32_t q = __shfl_sync(0xffffffffu, base, k) + t;
-                pj[u] = make_double4(0.0, 0.0, 0.0, __longlong_as_double((long long)i));
-                if (t < total) pj[u] = load_slab(a.sorted, q);
-            }
-#pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
-                const uint32_t j = (uint32_t)__double_as_longlong(pj[u].w);
-                const double dx = list_image(a, pi.x - pj[u].x, 0), dy = list_image(a, pi.y - pj[u].y, 1),
-                             dz = list_image(a, pi.z - pj[u].z, 2);
-                const bool hit = j != i && dx * dx + dy * dy + dz * dz < a.rl2;
-                const uint32_t mask = __ballot_sync(0xffffffffu, hit);
-                const uint32_t at = m2 + __popc(mask & ((1u << lane) - 1u));
-                if (hit && at < kAdjFound) {
-                    found.key[at] = lane_of(j) << 28 | j;
-                    atomicAdd(&found.count[lane_of(j)], 1u);
-                }
-                m2 += __popc(mask);
-            }
+        uint32_t m2 = adj_collect(a, pi, i, end, base, total, 0u, n, found);
+        const uint32_t mine = lane < kAdjLanes ? found.count[lane] : 0u;
+        const uint32_t beyond = mine > a.cap_l ? mine - a.cap_l : 0u;
+        if (lane < kAdjLanes) {
+            a.cnt[i * kAdjLanes + lane] = mine;
+            found.have[lane] = 0u;
         }
+        bool room = true;
+        if (__any_sync(0xffffffffu, beyond != 0u)) {
+            uint32_t run = beyond;  // inclusive scan of the lanes' needs
+#pragma unroll
+            for (int o = 1; o < kAdjLanes; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, run, o);
+                if (lane >= (uint32_t)o) run += v;
+            }
+            const uint32_t need = __shfl_sync(0xffffffffu, run, kAdjLanes - 1);
+            unsigned long long at = lane == 0 ? atomicAdd(a.pool_used, (unsigned long long)need) : 0ull;
+            at = __shfl_sync(0xffffffffu, at, 0);
+            room = at + need <= a.pool_cap;
+            if (room && lane < kAdjLanes) a.off[i * kAdjLanes + lane] = found.pool[lane] = (uint32_t)at + run - beyond;
+        }
+        if (!room) continue;  // the lists will not be read
         if (m2 <= kAdjFound) {
-            if (lane < 4) found.key[m2 + lane] = 0xffffffffu;
-            __syncwarp();
-            for (uint32_t k = lane; k < m2; k += 32) {  // the keys below this one, those of lower lanes aside
-                const uint32_t key = found.key[k], l = key >> 28;
-                uint32_t place = 0;
-                for (uint32_t q = 0; q < m2; q += 4) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(&found.key[q]);
-                    place += (v.x < key) + (v.y < key) + (v.z < key) + (v.w < key);
-                }
-                for (uint32_t q = 0; q < l; ++q) place -= found.count[q];
-                if (place < (uint32_t)a.cap_l) a.list[place * stride + i * kAdjLanes + l] = key & 0x0fffffffu;
-            }
+            adj_emit(a, i, m2, found);
+            continue;
         }
-        // more than a warp can hold: every lane looks at all atoms
-        if (lane < kAdjLanes) a.cnt[i * kAdjLanes + lane] = m2 <= kAdjFound ? found.count[lane] : (uint32_t)a.cap_l + 1u;
-        __syncwarp();
+        uint32_t width = n / (2 * m2 / kAdjFound + 1) + 1;
+        for (uint32_t from = 0; from < n;) {
+            const uint32_t to = min(from + width, n);
+            m2 = adj_collect(a, pi, i, end, base, total, from, to, found);
+            if (m2 > kAdjFound) {  // kAdjFound slots and fewer always fit
+                width = (width + 1) / 2;
+                continue;
+            }
+            adj_emit(a, i, m2, found);
+            if (lane < kAdjLanes) found.have[lane] += found.count[lane];
+            from = to;
+            if (m2 < kAdjFound / 4) width = min(2 * width, n);
+        }
     }
     if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;  // the lists are read by other threads
-    return true;
+    if (*(volatile unsigned long long*)a.pool_used <= a.pool_cap) return true;
+    if (gt == 0) atomicOr(a.err, kErrCapacity);
+    grid_leave(a.sync);
+    return false;
 }
 
-// Every partner of lane l of atom i in ascending slot order, with its slab
-// entry loaded one partner ahead; a lane whose list overflowed looks at all
-// atoms.
+// Every partner of lane l of atom i, in an order that depends on the pairs in
+// range alone: its list's ascending slots, with the slab entry loaded one
+// partner ahead, or this tick's cells.
 template <class V>
 __device__ __forceinline__ void adj_partners(const AdjArgs& a, const double* X, uint32_t i, uint32_t l, V&& visit) {
-    const uint32_t e = i * kAdjLanes + l, m = a.cnt[e];
-    if (m <= (uint32_t)a.cap_l) {
+    if (!a.walk) {
+        const uint32_t e = i * kAdjLanes + l, m = a.cnt[e];
         if (m == 0) return;
         const size_t stride = (size_t)kAdjLanes * a.cap;
         const uint32_t* row = a.list + e;
+        const uint32_t in_row = min(m, a.cap_l);
         uint32_t j = row[0], j1 = m > 1 ? row[stride] : j;
         double4 p = load_slab(X, j);
         for (uint32_t k = 0; k < m; ++k) {
             const double4 p1 = load_slab(X, j1);
-            const uint32_t j2 = k + 2 < m ? row[(k + 2) * stride] : j1;
+            uint32_t j2 = j1;
+            if (k + 2 < in_row) j2 = row[(k + 2) * stride];
+            else if (k + 2 < m) j2 = a.pool[a.off[e] + (k + 2 - a.cap_l)];
             visit(j, p);
             j = j1;
             p = p1;
             j1 = j2;
         }
     } else {
-        for (uint32_t j = l; j < a.n; j += kAdjLanes)  // lane_of
-            if (j != i) visit(j, load_slab(X, j));
+        uint32_t cx, cy, cz, B;
+        decode(a.lg, a.key[i], cx, cy, cz);
+        for (uint32_t k = 0; k < 27; ++k) {
+            if (!adj_cell(a.lg, cx, cy, cz, k, B)) continue;
+            for (uint32_t q = a.start[B] + l, hi = a.start[B + 1]; q < hi; q += kAdjLanes) {
+                const uint32_t j = a.order[q];
+                if (j != i) visit(j, load_slab(X, j));
+            }
+        }
     }
 }
 
@@ -490,7 +594,8 @@ __device__ __forceinline__ void gr_bins(const GrSpec& gs, double d, F&& f) {
 // it; the potential sums the FP32 pair energies in FP64.
 template <bool F32>
 __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_constant__ AdjArgs a) {
-    extern __shared__ uint32_t s_hist[];  // with obs a histogram per warp: low 16 bits' sums, then the rest's
+    // with obs a histogram per warp: low 16 bits' sums, then the rest's; with `walk`, whose terms nobody counted, 64-bit sums
+    extern __shared__ __align__(16) uint32_t s_hist[];
     __shared__ double s_sig[kNElem * kNElem], s_eps[kNElem * kNElem], s_e24[kNElem * kNElem];
     __shared__ PairTab s_tab;
     __shared__ double sh[kAdjThreads / 32], s_queue[kAdjThreads / 32][kAdjQueue];
@@ -506,6 +611,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
     const double h3[3] = {xmul(0.5, a.L.box[0]), xmul(0.5, a.L.box[1]), xmul(0.5, a.L.box[2])};
     const bool recorder = blockIdx.x == gridDim.x - 1;
     uint32_t target = 0;
+    if (*a.err & kErrCapacity) return;  // an earlier launch of the call ended early
     for (int k = tid; k < kNElem * kNElem; k += kAdjThreads) {
         s_sig[k] = a.psig[k];
         s_eps[k] = a.peps[k];
@@ -518,6 +624,10 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
     uint32_t held = 0;  // terms that a bin of this warp's histogram may hold
     if (tid < kAdjThreads / 32) s_queued[tid] = 0u;
     auto into_warp = [&](int b, unsigned long long v) {
+        if (a.walk) {
+            atomicAdd(reinterpret_cast<unsigned long long*>(wh) + b, v);
+            return;
+        }
         atomicAdd(&wh[b], (uint32_t)v & 0xffffu);
         atomicAdd(&wh[bins + b], (uint32_t)(v >> 16));
     };
@@ -576,12 +686,12 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
             if (live && l == 3)
                 X[4 * (size_t)i + 3] = __longlong_as_double(
                     (long long)((unsigned long long)cell << 32 | (uint32_t)a.kind[i] << 8 | a.elem[i]));
-            if (built) over |= !(moved2(a, i, l, live, x, odd) <= a.lim2);
+            if (built && !a.walk) over |= !(moved2(a, i, l, live, x, odd) <= a.lim2);
         }
         if (t == a.last && a.keep) break;
         if (__syncthreads_or(over) && tid == 0) a.sync->request[ask] = 1u;
         if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
-        const bool rebuild = !built || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
+        const bool rebuild = !built || a.walk || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
         if (recorder) {
             if (a.obs && t > a.first) record(t - 1);
             if (tid == 0) a.sync->request[(ask + 2) % 3] = 0u;  // every block has read it before this barrier
@@ -597,6 +707,12 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
                 unsigned long long s = 0ull;
                 for (int w = 0; w < warps; ++w) {
                     uint32_t* hw = hist + w * 2 * bins + k;
+                    if (a.walk) {
+                        unsigned long long* h64 = reinterpret_cast<unsigned long long*>(hist + w * 2 * bins) + k;
+                        s += *h64;
+                        *h64 = 0ull;
+                        continue;
+                    }
                     s += hw[0] + ((unsigned long long)hw[bins] << 16);
                     hw[0] = hw[bins] = 0u;
                 }
@@ -605,12 +721,12 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
         };
         for (uint32_t e = gt; e < pad; e += gs) {  // pair pass and second kick
             const uint32_t i = e / kAdjLanes, l = e % kAdjLanes;
-            bool direct = false;  // an overflowed lane's terms go to the tick's histogram one by one
-            if (gr) {  // 65,535 terms (of at most `two`'s eight visits of a pair) cannot overflow 32 bits
-                const uint32_t c = i < n ? a.cnt[e] : 0u;
-                direct = c > (uint32_t)a.cap_l;
-                const uint32_t terms = __reduce_add_sync(0xffffffffu, direct ? 0u : c);
+            bool direct = false;  // terms that may overflow the warp's histogram go to the tick's one by one
+            if (gr && !a.walk) {  // 65,535 terms (of at most `two`'s eight visits of a pair) cannot overflow 32 bits
                 const uint32_t most = a.two ? 65535u / 8u : 65535u;
+                uint32_t terms = __reduce_add_sync(0xffffffffu, i < n ? min(a.cnt[e], 65536u) : 0u);
+                direct = terms > most;
+                if (direct) terms = 0u;
                 if (held + terms > most) {
                     __syncwarp();
                     flush(wh, 1, (int)(tid & 31u), 32);
@@ -739,6 +855,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_con
     const uint32_t pad = (lanes + 31u) & ~31u;
     const size_t cap = a.cap;
     uint32_t target = 0;
+    if (*a.err & kErrCapacity) return;  // an earlier launch of the call ended early
     for (int k = tid; k < kNElem * kNElem; k += kAdjThreads) {
         s_sig[k] = a.psig[k];
         s_eps[k] = a.peps[k];
@@ -759,7 +876,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_con
         const double* W = a.W + (size_t)(t & 1) * 4 * cap;
         const int ask = t % 3;
         if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
-        const bool rebuild = !built || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
+        const bool rebuild = !built || a.walk || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
         if (blockIdx.x == 0 && tid == 0) a.sync->request[(ask + 1) % 3] = 0u;  // tick t + 1's, read before this barrier
         if (rebuild) {
             if (!adj_rebuild(a, X, target, &s_ok, s_warp, s_off, s_found)) return;
@@ -837,7 +954,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_con
             }
             if (i < n && l < 5)
                 a.P[l * cap + i] += l == 0 ? Ps : (l == 1 ? Pe : (l == 2 ? Pr0 : (l == 3 ? Pr1 : Pr2)));
-            if (Xp) over |= !(moved2(a, i, l, i < n, xp, odd) <= a.lim2);
+            if (Xp && !a.walk) over |= !(moved2(a, i, l, i < n, xp, odd) <= a.lim2);
         }
         if (Xp && __syncthreads_or(over) && tid == 0) a.sync->request[(ask + 2) % 3] = 1u;  // tick t - 1's
     }
@@ -880,9 +997,14 @@ struct AdjBuffers {
     double *charge = nullptr, *mass = nullptr, *inv_mass = nullptr;
     double* sorted = nullptr;
     uint32_t *key = nullptr, *count = nullptr, *start = nullptr, *fill = nullptr;
-    uint32_t *list = nullptr, *cnt = nullptr;
-    GridGeom lg{};
-    int cap_l = 0;
+    uint32_t *order = nullptr;
+    uint32_t *list = nullptr, *cnt = nullptr, *off = nullptr, *pool = nullptr;  // one block, not in `owned`
+    uint32_t* large_pool = nullptr;  // in place of the block's, once that was too small
+    unsigned long long* pool_used = nullptr;
+    size_t pool_cap = 0;  // words
+    bool walk = false;    // this forward's ticks go without lists
+    GridGeom lg{}, wg{};  // of the lists, and without them
+    uint32_t cap_l = 0;
     size_t cap_cells = 0;
     int resident[3] = {0, 0, 0};  // blocks that fit: FP64 ticks, mixed ticks, the reverse sweep
     size_t resident_smem = 0;
@@ -893,9 +1015,18 @@ struct AdjBuffers {
     std::vector<void*> owned;
 };
 
+static void adj_free_lists(AdjBuffers* A) {
+    cudaFree(A->list);
+    cudaFree(A->large_pool);
+    A->list = A->cnt = A->off = A->pool = A->large_pool = nullptr;
+    A->pool_cap = 0;
+    A->cap_l = 0;
+}
+
 static void adj_release(AdjBuffers* A) {
     for (void* p : A->owned) cudaFree(p);
     A->owned.clear();
+    adj_free_lists(A);
 }
 
 void adjoint_free(gx_handle* h) {
@@ -908,38 +1039,93 @@ void adjoint_free(gx_handle* h) {
 
 namespace {
 
-// The list grid (cells >= rc + skin, few enough for the scan's tiles) and a
-// lane's list length: four times its share of the mean neighbourhood.
-bool adj_grid(const gx_handle* h, GridGeom* g, int* cap_l) {
-    const double rl = h->fs.rc * (1.0 + kAdjSkin);
-    double cell = rl;
+// Lists hold up to this many partners an atom on average; above, and where
+// their rows would take more than half of what memory is free, every tick
+// sorts the atoms and walks their cells.  Twenty ticks and their gradient, ms,
+// with lists / without: 27,000 atoms of 900 partners 66 / 76, of 2,130 260 /
+// 245; 8,000 of 266 6.6 / 14.3, of 65 2.6 / 6.8.
+constexpr double kAdjMostPartners = 1024.0;
+constexpr size_t kAdjPoolMost = (size_t)1 << 28;  // words
+
+// Cells >= min_cell, few enough for the scan's tiles.
+bool adj_grid(const gx_handle* h, double min_cell, GridGeom* g) {
     int ok = 0;
-    for (int k = 0; k < 64; ++k, cell *= 1.3) {
-        *g = make_grid(h->p.box, cell, &ok);
-        if (ok && g->ncell < kScanTileCells * kScanMaxTiles) break;
-        ok = 0;
+    for (int k = 0; k < 64; ++k, min_cell *= 1.3) {
+        *g = make_grid(h->p.box, min_cell, &ok);
+        if (ok && g->ncell < kScanTileCells * kScanMaxTiles) return true;
     }
-    const double vol = h->p.box[0] * h->p.box[1] * h->p.box[2];
-    const double mean = std::min((double)h->n / vol * (4.0 / 3.0) * 3.14159265358979 * rl * rl * rl, (double)h->n);
-    *cap_l = (int)std::min(4.0 * mean / kAdjLanes + 16.0, 256.0);
-    return ok != 0;
+    return false;
+}
+
+// The mean neighbourhood of a list.
+double adj_mean(const gx_handle* h) {
+    const double rl = h->fs.rc * (1.0 + kAdjSkin), vol = h->p.box[0] * h->p.box[1] * h->p.box[2];
+    return std::min((double)h->n / vol * (4.0 / 3.0) * 3.14159265358979 * rl * rl * rl, (double)h->n);
+}
+
+// Rows of twice a lane's share of the mean neighbourhood, and a pool for what
+// is denser (64,000 atoms, a cube at four times the mean density: 43 ms for
+// twenty ticks and their gradient, 117 with a walk of 27 cells every tick, 427
+// with a look at all atoms for the denser lanes).  Without lists when they
+// cannot be had.
+int adj_alloc_lists(gx_handle* h, AdjBuffers* A, double mean) {
+    A->walk = mean > kAdjMostPartners;
+    const uint32_t cap_l = (uint32_t)std::ceil(2.0 * mean / kAdjLanes) + 8u;
+    if (A->walk || (A->list && cap_l <= A->cap_l)) return GX_OK;
+    adj_free_lists(A);
+    const size_t lanes = kAdjLanes * A->cap, rows = cap_l * lanes, pool = 16 * A->cap;
+    const size_t bytes = (rows + 2 * lanes + pool) * sizeof(uint32_t);
+    size_t free_bytes = ~(size_t)0, all = 0;
+    if (bytes >> 30) GX_CUDA(h, cudaMemGetInfo(&free_bytes, &all));
+    if (bytes > free_bytes / 2 || cudaMalloc((void**)&A->list, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        A->list = nullptr;
+        A->walk = true;
+        return GX_OK;
+    }
+    A->cnt = A->list + rows;
+    A->off = A->cnt + lanes;
+    A->pool = A->off + lanes;
+    A->cap_l = cap_l;
+    A->pool_cap = pool;
+    return GX_OK;
+}
+
+// The pool as large as the lists asked for, and as much again; without lists
+// where that is too much.
+int adj_more_pool(gx_handle* h, AdjBuffers* A) {
+    unsigned long long need = 0;
+    GX_CUDA(h, cudaMemcpy(&need, A->pool_used, sizeof need, cudaMemcpyDeviceToHost));
+    cudaFree(A->large_pool);
+    A->pool = A->large_pool = nullptr;
+    A->pool_cap = 0;
+    const size_t words = (size_t)std::min<unsigned long long>(2 * need, kAdjPoolMost);
+    if (words < need || cudaMalloc((void**)&A->large_pool, words * sizeof(uint32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        A->large_pool = nullptr;
+        adj_free_lists(A);
+        A->walk = true;
+    } else {
+        A->pool = A->large_pool;
+        A->pool_cap = words;
+    }
+    return GX_OK;
 }
 
 int adj_alloc(gx_handle* h, AdjBuffers* A, size_t n, int T, int K, int bins) {
     int nck = (T + K - 1) / K;
-    GridGeom lg;
-    int cap_l = 0;
-    if (!adj_grid(h, &lg, &cap_l)) return set_err(h, GX_ERR_ARG, "adjoint list grid is empty or too large");
-    A->lg = lg;
+    if (!adj_grid(h, h->fs.rc * (1.0 + kAdjSkin), &A->lg) || !adj_grid(h, h->fs.rc, &A->wg))
+        return set_err(h, GX_ERR_ARG, "adjoint list grid is empty or too large");
+    const double mean = adj_mean(h);
+    const size_t cells = (size_t)std::max(A->lg.ncell, A->wg.ncell) + 1;
     if (n <= A->cap && T <= A->cap_T && nck <= A->cap_ck && K <= A->cap_K && bins <= A->cap_bins &&
-        cap_l <= A->cap_l && lg.ncell + 1 <= A->cap_cells && A->tab)
-        return GX_OK;
+        cells <= A->cap_cells && A->tab)
+        return adj_alloc_lists(h, A, mean);
     adj_release(A);
     A->tab = nullptr;
     A->cap = 0;
     size_t cap = n < 1 ? 1 : n;
     cap = (cap + 31) & ~(size_t)31;
-    const size_t cells = (size_t)lg.ncell + 1;
     int binc = bins < 1 ? 1 : bins;
     auto get = [&](void** p, size_t bytes) -> int {
         cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
@@ -961,20 +1147,20 @@ int adj_alloc(gx_handle* h, AdjBuffers* A, size_t n, int T, int K, int bins) {
     rc |= get((void**)&A->inv_mass, cap * sizeof(double));
     rc |= get((void**)&A->elem, cap);
     rc |= get((void**)&A->kind, cap);
-    rc |= get((void**)&A->key, cap * sizeof(uint32_t));
+    rc |= get((void**)&A->key, 2 * cap * sizeof(uint32_t));
+    A->order = A->key + cap;
     rc |= get((void**)&A->sorted, 4 * cap * sizeof(double));
     rc |= get((void**)&A->count, cells * sizeof(uint32_t));
     rc |= get((void**)&A->start, cells * sizeof(uint32_t));
     rc |= get((void**)&A->fill, cells * sizeof(uint32_t));
-    rc |= get((void**)&A->list, (size_t)cap_l * kAdjLanes * cap * sizeof(uint32_t));
-    rc |= get((void**)&A->cnt, kAdjLanes * cap * sizeof(uint32_t));
     rc |= get((void**)&A->vpart, 2 * (nblk(cap * kAdjLanes, kAdjThreads) + 1) * sizeof(double));
     rc |= get((void**)&A->dV, (size_t)T * sizeof(double));
     rc |= get((void**)&A->alpha, (size_t)T * sizeof(double));
     rc |= get((void**)&A->bw, (size_t)binc * sizeof(double));
     rc |= get((void**)&A->ghist, 2 * (size_t)binc * sizeof(unsigned long long));
     rc |= get((void**)&A->hacc, (size_t)binc * sizeof(double));
-    rc |= get((void**)&A->sync, sizeof(GridSync));
+    rc |= get((void**)&A->pool_used, sizeof(unsigned long long) + sizeof(GridSync));
+    A->sync = reinterpret_cast<GridSync*>(A->pool_used + 1);
     rc |= get((void**)&A->tab, (2 * kNElem * kNElem + kNElem + kNOut) * sizeof(double));
     if (rc) {
         adj_release(A);
@@ -986,9 +1172,8 @@ int adj_alloc(gx_handle* h, AdjBuffers* A, size_t n, int T, int K, int bins) {
     A->cap_ck = nck;
     A->cap_K = K;
     A->cap_bins = binc;
-    A->cap_l = cap_l;
     A->cap_cells = cells;
-    return GX_OK;
+    return adj_alloc_lists(h, A, mean);
 }
 
 Vec3Field field(double* base, size_t cap) { return Vec3Field{base, cap}; }
@@ -1005,7 +1190,7 @@ GrSpec gr_spec(const AdjBuffers* A) {
 
 AdjArgs adj_args(gx_handle* h, AdjBuffers* A) {
     AdjArgs a{};
-    a.lg = A->lg;
+    a.lg = A->walk ? A->wg : A->lg;
     a.fg = h->fgrid;
     a.two = a.fg.n[0] == 2 || a.fg.n[1] == 2 || a.fg.n[2] == 2;
     a.plain = a.fg.n[0] >= 3 && a.fg.n[1] >= 3 && a.fg.n[2] >= 3 && h->p.enable_boundaries;
@@ -1032,6 +1217,12 @@ AdjArgs adj_args(gx_handle* h, AdjBuffers* A) {
     a.list = A->list;
     a.cnt = A->cnt;
     a.cap_l = A->cap_l;
+    a.pool = A->pool;
+    a.off = A->off;
+    a.pool_used = A->pool_used;
+    a.pool_cap = A->pool_cap;
+    a.walk = A->walk ? 1 : 0;
+    a.order = A->order;
     a.ref = A->ref;
     a.key = A->key;
     a.sorted = A->sorted;
@@ -1097,22 +1288,25 @@ double gr_norm(const gx_handle* h, const AdjBuffers* A, int k) {
     return vol / (npair * 4.0 * pi * r * r * std::sqrt(2.0 * pi) * A->gr_width);
 }
 
-int check_err(gx_handle* h) {
+// The outcome of a call's launches; *again: the lists needed more room and
+// have it now, or do without.
+int check_err(gx_handle* h, AdjBuffers* A, bool* again) {
     uint32_t e = 0;
+    *again = false;
     GX_CUDA(h, cudaMemcpyAsync(&e, h->derr, sizeof e, cudaMemcpyDeviceToHost, h->stream));
     GX_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (e & kErrNonFinite) {
-        cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
-        return set_err(h, GX_ERR_NONFINITE, "non-finite position in the adjoint trajectory");
-    }
+    if (!e) return GX_OK;
+    cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
+    if (e & kErrNonFinite) return set_err(h, GX_ERR_NONFINITE, "non-finite position in the adjoint trajectory");
     if (e & kErrTimeout) {  // a block gave up at a barrier: the words are no longer zero
-        cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
-        cudaMemsetAsync(static_cast<AdjBuffers*>(h->adj)->sync, 0, sizeof(GridSync), h->stream);
+        cudaMemsetAsync(A->sync, 0, sizeof(GridSync), h->stream);
         return set_err(h, GX_ERR_TIMEOUT, "a bounded device wait timed out in the adjoint");
     }
-    if (e & kErrSaturation) {  // the fixed-point force of the mixed forward
-        cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
+    if (e & kErrSaturation)  // the fixed-point force of the mixed forward
         return set_err(h, GX_ERR_SATURATION, "fixed-point force saturated in the adjoint trajectory");
+    if (e & kErrCapacity) {
+        *again = true;
+        return adj_more_pool(h, A);
     }
     return GX_OK;
 }
@@ -1170,29 +1364,31 @@ int gx_adjoint_forward(gx_handle* h, const gx_adjoint_spec* spec, double* potent
     for (int e = 0; e < kNElem; ++e) tab[2 * kNElem * kNElem + e] = h->p.epsilon_k[e];
     GX_CUDA(h, cudaMemcpyAsync(A->tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     StateBuf& b = h->buf[h->cur];
-    GX_LAUNCH(h, k_adj_import, nblk(n, 256), 256, b, n, field(A->S, cap), field(A->S + 3 * cap, cap),
-              field(A->S + 6 * cap, cap), A->elem, A->charge, A->mass, A->inv_mass, A->kind);
     GX_CUDA(h, cudaMemsetAsync(A->sync, 0, sizeof(GridSync), h->stream));
-    if (A->bins > 0) {
-        GX_CUDA(h, cudaMemsetAsync(A->hacc, 0, A->bins * sizeof(double), h->stream));
-        GX_CUDA(h, cudaMemsetAsync(A->ghist, 0, 2 * A->bins * sizeof(unsigned long long), h->stream));
-        A->samples = T / A->every;
-    }
-    AdjArgs args = adj_args(h, A);
-    args.ck = A->ck;
-    args.obs = 1;
-    for (int t0 = 0; t0 < T; t0 += kAdjTicksPerLaunch) {
-        args.first = t0 + 1;
-        args.last = std::min(t0 + kAdjTicksPerLaunch, T);
-        if ((rc = adj_launch(h, A, A->f32 ? 1 : 0, args))) return rc;
-    }
-    GX_CUDA(h, cudaMemcpyAsync(potential, A->dV, T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    if (A->bins > 0) A->samples = T / A->every;
     std::vector<double> hacc(A->bins > 0 ? A->bins : 0);
-    if (A->bins > 0)
-        GX_CUDA(h, cudaMemcpyAsync(hacc.data(), A->hacc, A->bins * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    GX_CUDA(h, cudaStreamSynchronize(h->stream));
-    GX_CUDA(h, cudaGetLastError());
-    if ((rc = check_err(h))) return rc;
+    for (bool again = true; again;) {
+        GX_LAUNCH(h, k_adj_import, nblk(n, 256), 256, b, n, field(A->S, cap), field(A->S + 3 * cap, cap),
+                  field(A->S + 6 * cap, cap), A->elem, A->charge, A->mass, A->inv_mass, A->kind);
+        if (A->bins > 0) {
+            GX_CUDA(h, cudaMemsetAsync(A->hacc, 0, A->bins * sizeof(double), h->stream));
+            GX_CUDA(h, cudaMemsetAsync(A->ghist, 0, 2 * A->bins * sizeof(unsigned long long), h->stream));
+        }
+        AdjArgs args = adj_args(h, A);
+        args.ck = A->ck;
+        args.obs = 1;
+        for (int t0 = 0; t0 < T; t0 += kAdjTicksPerLaunch) {
+            args.first = t0 + 1;
+            args.last = std::min(t0 + kAdjTicksPerLaunch, T);
+            if ((rc = adj_launch(h, A, A->f32 ? 1 : 0, args))) return rc;
+        }
+        GX_CUDA(h, cudaMemcpyAsync(potential, A->dV, T * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        if (A->bins > 0)
+            GX_CUDA(h, cudaMemcpyAsync(hacc.data(), A->hacc, A->bins * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+        GX_CUDA(h, cudaStreamSynchronize(h->stream));
+        GX_CUDA(h, cudaGetLastError());
+        if ((rc = check_err(h, A, &again))) return rc;
+    }
     if (gr)
         for (int k = 0; k < A->bins; ++k) gr[k] = A->samples ? hacc[k] * gr_norm(h, A, k) / A->samples : 0.0;
     A->ready = true;
@@ -1218,34 +1414,36 @@ int gx_adjoint_backward(gx_handle* h, const double* dl_dpotential, const double*
         for (int k = 0; k < A->bins; ++k) bw[k] = dl_dgr[k] * gr_norm(h, A, k) / A->samples;
     GX_CUDA(h, cudaMemcpyAsync(A->alpha, alpha.data(), T * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     GX_CUDA(h, cudaMemcpyAsync(A->bw, bw.data(), bw.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    GX_CUDA(h, cudaMemsetAsync(A->Ladj, 0, 9 * cap * sizeof(double), h->stream));
-    GX_CUDA(h, cudaMemsetAsync(A->P, 0, 5 * cap * sizeof(double), h->stream));
     double* out = A->tab + 2 * kNElem * kNElem + kNElem;
-    AdjArgs args = adj_args(h, A);
-    args.gr = dl_dgr && A->bins > 0;
-    args.keep = 1;
-    for (int s = A->nck - 1; s >= 0; --s) {
-        args.first = s * K + 1;
-        args.last = std::min((s + 1) * K, T);
-        GX_CUDA(h, cudaMemcpyAsync(A->S, A->ck + (size_t)s * 9 * cap, 9 * cap * sizeof(double),
-                                   cudaMemcpyDeviceToDevice, h->stream));
-        if ((rc = adj_launch(h, A, A->f32 ? 1 : 0, args))) return rc;
-        if ((rc = adj_launch(h, A, 2, args))) return rc;
-    }
-    GX_LAUNCH(h, k_adj_reduce, kNOut, 256, n, A->elem, A->P, cap, out);
     double sums[kNOut];
-    GX_CUDA(h, cudaMemcpyAsync(sums, out, sizeof sums, cudaMemcpyDeviceToHost, h->stream));
-    double* dsts[3] = {grad_pos0, grad_vel0, grad_acc0};
-    double* stage = A->W;  // 8 * cap, free once the sweep is done
-    for (int q = 0; q < 3; ++q) {
-        if (!dsts[q] || !n) continue;
-        GX_LAUNCH(h, k_adj_export, nblk(n, 256), 256, n, field(A->Ladj + (size_t)q * 3 * cap, cap), stage);
-        GX_CUDA(h, cudaMemcpyAsync(dsts[q], stage, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    for (bool again = true; again;) {
+        GX_CUDA(h, cudaMemsetAsync(A->Ladj, 0, 9 * cap * sizeof(double), h->stream));
+        GX_CUDA(h, cudaMemsetAsync(A->P, 0, 5 * cap * sizeof(double), h->stream));
+        AdjArgs args = adj_args(h, A);
+        args.gr = dl_dgr && A->bins > 0;
+        args.keep = 1;
+        for (int s = A->nck - 1; s >= 0; --s) {
+            args.first = s * K + 1;
+            args.last = std::min((s + 1) * K, T);
+            GX_CUDA(h, cudaMemcpyAsync(A->S, A->ck + (size_t)s * 9 * cap, 9 * cap * sizeof(double),
+                                       cudaMemcpyDeviceToDevice, h->stream));
+            if ((rc = adj_launch(h, A, A->f32 ? 1 : 0, args))) return rc;
+            if ((rc = adj_launch(h, A, 2, args))) return rc;
+        }
+        GX_LAUNCH(h, k_adj_reduce, kNOut, 256, n, A->elem, A->P, cap, out);
+        GX_CUDA(h, cudaMemcpyAsync(sums, out, sizeof sums, cudaMemcpyDeviceToHost, h->stream));
+        double* dsts[3] = {grad_pos0, grad_vel0, grad_acc0};
+        double* stage = A->W;  // 8 * cap, free once the sweep is done
+        for (int q = 0; q < 3; ++q) {
+            if (!dsts[q] || !n) continue;
+            GX_LAUNCH(h, k_adj_export, nblk(n, 256), 256, n, field(A->Ladj + (size_t)q * 3 * cap, cap), stage);
+            GX_CUDA(h, cudaMemcpyAsync(dsts[q], stage, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+            GX_CUDA(h, cudaStreamSynchronize(h->stream));
+        }
         GX_CUDA(h, cudaStreamSynchronize(h->stream));
+        GX_CUDA(h, cudaGetLastError());
+        if ((rc = check_err(h, A, &again))) return rc;
     }
-    GX_CUDA(h, cudaStreamSynchronize(h->stream));
-    GX_CUDA(h, cudaGetLastError());
-    if ((rc = check_err(h))) return rc;
     // The cutoffs: lj_rc = max(lj_cutoff_factor, 1) * max pair sigma (LjTable::new,
     // forces.rs:223-237), coulomb/gravity rc = max(factor, 1) * max sigma
     // (systems/forces.rs:108-116); the derivative goes to the first element

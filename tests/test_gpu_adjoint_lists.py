@@ -150,3 +150,65 @@ def test_handles_of_different_bins_side_by_side(gpu, precision):
             assert np.array_equal(x, y)
     for x, y in zip(alone[0][0], again):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n_side", [10, 11])  # 999 partners: lists sorted by ranges of slots; 1,330: cells every tick
+def test_every_atom_within_the_cutoff_matches_dual_oracle(gpu, orc, n_side):
+    cfg, u = _case(n_side, coul=True)
+    cfg.coulomb_cutoff = 8.0
+    _against_dual(orc, cfg, u, 3, 2, dict(gr_bins=30, gr_every=1, gr_rmax=6.0, gr_width=0.15, gr_support=6.0))
+
+
+def _clump(n, radius, L=200.0):
+    rng = np.random.default_rng(4)
+    d = rng.normal(size=(n, 3))
+    d *= (radius * rng.random(n) ** (1 / 3) / np.linalg.norm(d, axis=1))[:, None]
+    return d + 0.25 * L, rng.integers(0, 10, n).astype(np.uint8)
+
+
+@pytest.mark.parametrize("n,radius,slots", [(600, 2.0, 1), (3000, 4.0, 8), (20000, 3.0, 1)])
+def test_clumps_for_any_checkpoint_spacing(gpu, n, radius, slots):
+    """Rows, the pool beyond them (repeated calls, as it grows), and what no pool holds; slots of one residue in a
+    clump.  The potential is the plain FP64 tick's, and the checkpoint spacing changes no bit."""
+    from genesis_b200._lib import Handle
+    cfg, _ = _case(8)
+    cfg.size, cfg.dt = (200.0, 200.0, 200.0), 1e-7
+    pos, elem = _clump(n, radius)
+    if slots > 1:  # a clump's slots are those divisible by `slots`, the others spread over the box
+        far = np.random.default_rng(5).uniform(-100.0, 100.0, size=(n * slots, 3))
+        far[::slots] = pos
+        pos, elem = far, np.repeat(elem, slots)
+    T = 2
+    with Handle(cfg, "fp64") as h:
+        h.set_state(pos, np.zeros_like(pos), elem)
+        want = h.step(T)["potential"]
+    out = []
+    for K in (1, 2):
+        with Handle(cfg, "fp64") as h:
+            h.set_state(pos, np.zeros_like(pos), elem)
+            V, g = h.adjoint_forward(T, checkpoint_every=K, gr_bins=40, gr_rmax=3.0, gr_width=0.05)
+            grad = h.adjoint_backward(dl_dpotential=np.ones(T), dl_dgr=np.ones(40), initial_state=True)
+        assert np.max(np.abs(V - want) / np.abs(want)) <= 1e-10
+        out.append((V, g, *grad[:2], *grad[2]))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+def test_slots_eight_apart_cost_no_look_at_all_atoms(gpu):
+    """A lattice whose neighbours' slots are eight apart against the same lattice in its own order: a lane that fell
+    back to all 8,000 atoms took fifteen times as long."""
+    import time
+    from genesis_b200._lib import Handle
+    cfg, u = _case(20)
+    k = np.arange(u.n)
+    best = []
+    for order in (k, np.argsort((k % (u.n // 8)) * 8 + k // (u.n // 8))):
+        with Handle(cfg, "mixed") as h:
+            h.set_state(u.pos[order], u.vel[order], u.elem[order])
+            took = []
+            for _ in range(5):
+                t = time.perf_counter()
+                h.adjoint_forward(20, checkpoint_every=10)
+                took.append(time.perf_counter() - t)
+        best.append(min(took))
+    assert best[1] <= 4.0 * best[0]
