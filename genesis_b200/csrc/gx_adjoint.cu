@@ -281,6 +281,7 @@ struct AdjArgs {
     double* sorted;       // a rebuild's cell-sorted (x, y, z, slot); with `walk` slots in the scatter's order
     uint32_t* order;      // with `walk`: slots by cell, ascending in each
     uint32_t *key, *count, *start, *fill;
+    uint32_t tile_log2;   // cells of one of the scan's tiles
     GridSync* sync;
     uint32_t* err;
     double *vpart, *pot;  // block partials (two turns), V_t
@@ -413,7 +414,8 @@ __device__ __forceinline__ void adj_emit(const AdjArgs& a, uint32_t i, uint32_t 
 __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target, int* s_ok, uint32_t* s_warp,
                             uint32_t* s_off, AdjFound* s_found) {
     const uint32_t tid = threadIdx.x, gt = blockIdx.x * kAdjThreads + tid, gs = gridDim.x * kAdjThreads;
-    const uint32_t n = a.n, m = a.lg.ncell + 1, ntiles = (m + kScanTileCells - 1) / kScanTileCells;
+    const uint32_t n = a.n, m = a.lg.ncell + 1, log2 = a.tile_log2, per = (1u << log2) / kScanTileCells;
+    const uint32_t ntiles = (m - 1) / (1u << log2) + 1;  // of 1 << log2 cells, `per` scans in a row
     for (uint32_t i = gt; i < n; i += gs) {
         const double4 p = load_slab(X, i);
         const uint32_t c = cell_of(a.lg, p.x, p.y, p.z);
@@ -421,8 +423,11 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
         atomicAdd(&a.count[c], 1u);
     }
     if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x)
-        scan_tile<kAdjThreads>(a.count, t, m, &a.sync->tile[t], s_warp);
+    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        uint32_t total = 0;
+        for (uint32_t u = 0; u < per; ++u) total = scan_tile<kAdjThreads>(a.count, t * per + u, m, total, s_warp);
+        if (tid == 0) a.sync->tile[t] = total;
+    }
     if (gt == 0 && !a.walk) *a.pool_used = 0ull;  // last read before this rebuild began
     if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
     if (tid < ntiles) {
@@ -431,10 +436,10 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
         s_off[tid] = run;
     }
     __syncthreads();
-    for (uint32_t c = gt; c < m; c += gs) a.start[c] = a.count[c] + s_off[c / kScanTileCells];
+    for (uint32_t c = gt; c < m; c += gs) a.start[c] = a.count[c] + s_off[c >> log2];
     for (uint32_t i = gt; i < n; i += gs) {
         const uint32_t c = a.key[i];
-        const uint32_t at = a.count[c] + s_off[c / kScanTileCells] + atomicAdd(&a.fill[c], 1u);
+        const uint32_t at = a.count[c] + s_off[c >> log2] + atomicAdd(&a.fill[c], 1u);
         if (a.walk) {
             reinterpret_cast<uint32_t*>(a.sorted)[at] = i;
             continue;
@@ -1047,12 +1052,15 @@ namespace {
 constexpr double kAdjMostPartners = 1024.0;
 constexpr size_t kAdjPoolMost = (size_t)1 << 28;  // words
 
-// Cells >= min_cell, few enough for the scan's tiles.
+// Cells >= min_cell, no more of them than atoms or one scan's tiles of 1,024
+// cells.  (A limit of 65,536 cells whatever the atoms: 8,000,000 atoms, 122 in
+// a cell, took 3.6 s for twenty ticks and their gradient, 2.0 so.)
 bool adj_grid(const gx_handle* h, double min_cell, GridGeom* g) {
+    const size_t most = std::max((size_t)kScanTileCells * kScanMaxTiles - 1, (size_t)h->n);
     int ok = 0;
     for (int k = 0; k < 64; ++k, min_cell *= 1.3) {
         *g = make_grid(h->p.box, min_cell, &ok);
-        if (ok && g->ncell < kScanTileCells * kScanMaxTiles) return true;
+        if (ok && g->ncell <= most) return true;
     }
     return false;
 }
@@ -1191,6 +1199,8 @@ GrSpec gr_spec(const AdjBuffers* A) {
 AdjArgs adj_args(gx_handle* h, AdjBuffers* A) {
     AdjArgs a{};
     a.lg = A->walk ? A->wg : A->lg;
+    a.tile_log2 = 10;
+    static_assert(kScanTileCells == 1u << 10, "");
     a.fg = h->fgrid;
     a.two = a.fg.n[0] == 2 || a.fg.n[1] == 2 || a.fg.n[2] == 2;
     a.plain = a.fg.n[0] >= 3 && a.fg.n[1] >= 3 && a.fg.n[2] >= 3 && h->p.enable_boundaries;
@@ -1229,6 +1239,7 @@ AdjArgs adj_args(gx_handle* h, AdjBuffers* A) {
     a.count = A->count;
     a.start = A->start;
     a.fill = A->fill;
+    while (a.tile_log2 < 32 && (a.lg.ncell >> a.tile_log2) >= kScanMaxTiles) ++a.tile_log2;
     a.sync = A->sync;
     a.err = h->derr;
     a.vpart = A->vpart;

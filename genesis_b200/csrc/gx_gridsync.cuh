@@ -59,10 +59,11 @@ __device__ __forceinline__ void grid_leave(GridSync* s) {
     }
 }
 
-// Exclusive scan of tile t of the m cell counts in place; its total to *total.
-// BS threads; s_warp holds BS / 32 words.
+// Exclusive scan of tile t of the m cell counts in place, from `carry` on;
+// returns what the next tile would carry.  BS threads; s_warp holds BS / 32
+// words.
 template <int BS>
-__device__ __forceinline__ void scan_tile(uint32_t* count, uint32_t t, uint32_t m, uint32_t* total, uint32_t* s_warp) {
+__device__ __forceinline__ uint32_t scan_tile(uint32_t* count, uint32_t t, uint32_t m, uint32_t carry, uint32_t* s_warp) {
     constexpr int kItems = kScanTileCells / BS;
     const uint32_t base = t * kScanTileCells + threadIdx.x * kItems;
     uint32_t v[kItems], local = 0;
@@ -80,15 +81,18 @@ __device__ __forceinline__ void scan_tile(uint32_t* count, uint32_t t, uint32_t 
     }
     if (lane == 31) s_warp[w] = inc;
     __syncthreads();
-    uint32_t run = inc - local;
-    for (uint32_t k = 0; k < w; ++k) run += s_warp[k];
-    if (threadIdx.x == BS - 1) *total = run + local;
+    uint32_t run = carry + inc - local, total = carry;
+    for (uint32_t k = 0; k < BS / 32; ++k) {
+        if (k < w) run += s_warp[k];
+        total += s_warp[k];
+    }
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
         if (base + k < m) count[base + k] = run;
         run += v[k];
     }
     __syncthreads();  // s_warp is reused by the next tile
+    return total;
 }
 
 }  // namespace gx

@@ -173,8 +173,10 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                 atomicAdd(&a.count[c], 1u);
             }
             if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
-            for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x)
-                scan_tile<kTickThreads>(a.count, t, m, &a.sync->grid.tile[t], s_warp);
+            for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+                const uint32_t total = scan_tile<kTickThreads>(a.count, t, m, 0u, s_warp);
+                if (tid == 0) a.sync->grid.tile[t] = total;
+            }
             if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
             if (tid < ntiles) {  // tile offsets, in every block
                 uint32_t run = 0;

@@ -212,3 +212,22 @@ def test_slots_eight_apart_cost_no_look_at_all_atoms(gpu):
                 took.append(time.perf_counter() - t)
         best.append(min(took))
     assert best[1] <= 4.0 * best[0]
+
+
+def test_more_cells_than_one_scan_of_tiles(gpu):
+    """68,921 atoms on as many list cells: several scans in a row per tile, the last one ragged."""
+    from genesis_b200._lib import Handle
+    cfg, _ = _case(8)
+    n, L = 41 ** 3, 41.5 * 1.2 * W.lattice_rc()
+    cfg.size, cfg.dt = (L, L, L), 1e-7
+    rng = np.random.default_rng(9)
+    pos, elem = rng.uniform(-0.5 * L, 0.5 * L, size=(n, 3)), rng.integers(0, 10, n).astype(np.uint8)
+    with Handle(cfg, "fp64") as h:
+        h.set_state(pos, np.zeros_like(pos), elem)
+        want = h.step(2)["potential"]
+        h.set_state(pos, np.zeros_like(pos), elem)
+        V, _ = h.adjoint_forward(2, checkpoint_every=1)
+        gs, ge = h.adjoint_backward(dl_dpotential=np.array([0.0, 1.0]))
+    assert np.max(np.abs(V - want) / np.abs(want)) <= 1e-10
+    # V is linear in one factor on all epsilons but for the two ticks' drift at this step
+    assert abs(ge @ np.asarray(cfg.epsilon_k) - V[1]) <= 1e-6 * abs(V[1])
