@@ -70,7 +70,7 @@ EXPORTS = (
     "gx_set_list_skin", "gx_list_rebuilds", "gx_list_stats", "gx_batch_set_mode", "gx_batch_get_mode", "gx_batch_autotune", "gx_batch_set_list_skin", "gx_batch_list_rebuilds", "gx_batch_list_stats",
     "gx_get_list_config", "gx_set_list_threads", "gx_set_list_stash", "gx_set_list_brick", "gx_set_list_block", "gx_get_list_shape", "gx_set_pass_timing", "gx_pass_ms", "gx_bond_observe", "gx_bond_tracker_reset", "gx_get_bonds",
     "gx_bond_components", "gx_collisions", "gx_collision_count", "gx_xyz_frame", "gx_snapshot_world",
-    "gx_set_step_async", "gx_tick_host",
+    "gx_set_step_async", "gx_set_wait_polls", "gx_tick_host",
 )
 
 _lib = None
@@ -146,6 +146,7 @@ def load(path: str | Path | None = None) -> C.CDLL:
         "gx_xyz_frame": (C.c_int, [vp, C.c_uint64, C.c_char_p, sz, C.POINTER(sz)]),
         "gx_snapshot_world": (C.c_int, [vp, u32p, C.c_void_p, sz, C.POINTER(sz)]),
         "gx_set_step_async": (C.c_int, [vp, C.c_int]),
+        "gx_set_wait_polls": (C.c_int, [vp, C.c_uint32]),
         "gx_adjoint_backward": (C.c_int, [vp, dp, dp, dp, dp, dp, dp, dp]),
     }
     for name, (res, args) in proto.items():
@@ -547,6 +548,11 @@ class Handle:
         """gx_step without records returns without waiting; its errors come
         back from the next call that waits (gx_set_step_async)."""
         self._check(self.lib.gx_set_step_async(self.h, int(on)))
+
+    def set_wait_polls(self, polls: int):
+        """Polls of a device-wide barrier before a launch of several ticks
+        gives up (gx_set_wait_polls); 0 gives up at once."""
+        self._check(self.lib.gx_set_wait_polls(self.h, int(polls)))
 
     def xyz_frame(self, tick: int) -> bytes:
         """The XYZ frame of the current state as export::write_frame writes

@@ -284,6 +284,7 @@ struct AdjArgs {
     uint32_t tile_log2;   // cells of one of the scan's tiles
     GridSync* sync;
     uint32_t* err;
+    uint32_t polls;       // of a barrier before it gives up
     double *vpart, *pot;  // block partials (two turns), V_t
     unsigned long long* ghist;  // two turns of bins
     double* hacc;
@@ -422,14 +423,14 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
         a.key[i] = c;
         atomicAdd(&a.count[c], 1u);
     }
-    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
+    if (!grid_barrier(a.sync, a.err, a.polls, target, s_ok)) return false;
     for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         uint32_t total = 0;
         for (uint32_t u = 0; u < per; ++u) total = scan_tile<kAdjThreads>(a.count, t * per + u, m, total, s_warp);
         if (tid == 0) a.sync->tile[t] = total;
     }
     if (gt == 0 && !a.walk) *a.pool_used = 0ull;  // last read before this rebuild began
-    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
+    if (!grid_barrier(a.sync, a.err, a.polls, target, s_ok)) return false;
     if (tid < ntiles) {
         uint32_t run = 0;
         for (uint32_t t = 0; t < tid; ++t) run += a.sync->tile[t];
@@ -449,7 +450,7 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
         to[0] = make_double2(p.x, p.y);
         to[1] = make_double2(p.z, __longlong_as_double((long long)i));
     }
-    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;
+    if (!grid_barrier(a.sync, a.err, a.polls, target, s_ok)) return false;
     for (uint32_t c = gt; c < m; c += gs) a.count[c] = a.fill[c] = 0u;  // for the next rebuild
     if (a.walk) {
         const uint32_t* tmp = reinterpret_cast<const uint32_t*>(a.sorted);
@@ -459,7 +460,7 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
             for (uint32_t q = lo; q < hi; ++q) p += tmp[q] < i ? 1u : 0u;
             a.order[p] = i;
         }
-        return grid_barrier(a.sync, a.err, target, s_ok);
+        return grid_barrier(a.sync, a.err, a.polls, target, s_ok);
     }
     // A warp per atom: lane k < 27 looks up neighbour cell k, and a scan of the
     // counts turns the candidates into one run.  Atoms of more partners than a
@@ -525,7 +526,7 @@ __device__ bool adj_rebuild(const AdjArgs& a, const double* X, uint32_t& target,
             if (m2 < kAdjFound / 4) width = min(2 * width, n);
         }
     }
-    if (!grid_barrier(a.sync, a.err, target, s_ok)) return false;  // the lists are read by other threads
+    if (!grid_barrier(a.sync, a.err, a.polls, target, s_ok)) return false;  // the lists are read by other threads
     if (*(volatile unsigned long long*)a.pool_used <= a.pool_cap) return true;
     if (gt == 0) atomicOr(a.err, kErrCapacity);
     grid_leave(a.sync);
@@ -616,7 +617,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
     const double h3[3] = {xmul(0.5, a.L.box[0]), xmul(0.5, a.L.box[1]), xmul(0.5, a.L.box[2])};
     const bool recorder = blockIdx.x == gridDim.x - 1;
     uint32_t target = 0;
-    if (*a.err & kErrCapacity) return;  // an earlier launch of the call ended early
+    if (*a.err & (kErrCapacity | kErrBarrier)) return;  // an earlier launch of the call ended early
     for (int k = tid; k < kNElem * kNElem; k += kAdjThreads) {
         s_sig[k] = a.psig[k];
         s_eps[k] = a.peps[k];
@@ -695,7 +696,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
         }
         if (t == a.last && a.keep) break;
         if (__syncthreads_or(over) && tid == 0) a.sync->request[ask] = 1u;
-        if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
+        if (!grid_barrier(a.sync, a.err, a.polls, target, &s_ok)) return;
         const bool rebuild = !built || a.walk || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
         if (recorder) {
             if (a.obs && t > a.first) record(t - 1);
@@ -840,7 +841,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_ticks(const __grid_const
         }
     }
     if (a.obs) {
-        if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
+        if (!grid_barrier(a.sync, a.err, a.polls, target, &s_ok)) return;
         if (recorder) record(a.last);
     }
     grid_leave(a.sync);
@@ -860,7 +861,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_con
     const uint32_t pad = (lanes + 31u) & ~31u;
     const size_t cap = a.cap;
     uint32_t target = 0;
-    if (*a.err & kErrCapacity) return;  // an earlier launch of the call ended early
+    if (*a.err & (kErrCapacity | kErrBarrier)) return;  // an earlier launch of the call ended early
     for (int k = tid; k < kNElem * kNElem; k += kAdjThreads) {
         s_sig[k] = a.psig[k];
         s_eps[k] = a.peps[k];
@@ -880,7 +881,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_reverse(const __grid_con
         const double* X = a.slabs + (size_t)(t - a.first) * 4 * cap;
         const double* W = a.W + (size_t)(t & 1) * 4 * cap;
         const int ask = t % 3;
-        if (!grid_barrier(a.sync, a.err, target, &s_ok)) return;
+        if (!grid_barrier(a.sync, a.err, a.polls, target, &s_ok)) return;
         const bool rebuild = !built || a.walk || *(volatile uint32_t*)&a.sync->request[ask] != 0u;
         if (blockIdx.x == 0 && tid == 0) a.sync->request[(ask + 1) % 3] = 0u;  // tick t + 1's, read before this barrier
         if (rebuild) {
@@ -1242,6 +1243,7 @@ AdjArgs adj_args(gx_handle* h, AdjBuffers* A) {
     while (a.tile_log2 < 32 && (a.lg.ncell >> a.tile_log2) >= kScanMaxTiles) ++a.tile_log2;
     a.sync = A->sync;
     a.err = h->derr;
+    a.polls = h->wait_polls;
     a.vpart = A->vpart;
     a.pot = A->dV;
     a.ghist = A->ghist;
@@ -1308,11 +1310,11 @@ int check_err(gx_handle* h, AdjBuffers* A, bool* again) {
     GX_CUDA(h, cudaStreamSynchronize(h->stream));
     if (!e) return GX_OK;
     cudaMemsetAsync(h->derr, 0, sizeof(uint32_t), h->stream);
-    if (e & kErrNonFinite) return set_err(h, GX_ERR_NONFINITE, "non-finite position in the adjoint trajectory");
-    if (e & kErrTimeout) {  // a block gave up at a barrier: the words are no longer zero
+    if (e & kErrBarrier) {  // a block gave up at a barrier: the words are no longer zero
         cudaMemsetAsync(A->sync, 0, sizeof(GridSync), h->stream);
         return set_err(h, GX_ERR_TIMEOUT, "a bounded device wait timed out in the adjoint");
     }
+    if (e & kErrNonFinite) return set_err(h, GX_ERR_NONFINITE, "non-finite position in the adjoint trajectory");
     if (e & kErrSaturation)  // the fixed-point force of the mixed forward
         return set_err(h, GX_ERR_SATURATION, "fixed-point force saturated in the adjoint trajectory");
     if (e & kErrCapacity) {
@@ -1330,7 +1332,7 @@ using namespace gx;
 int gx_adjoint_forward(gx_handle* h, const gx_adjoint_spec* spec, double* potential, double* gr) {
     if (!h || !spec || !potential) return GX_ERR_ARG;
     int rc = GX_OK;
-    if (!h->cap) return set_err(h, GX_ERR_STATE, "no state uploaded (call gx_set_state first)");
+    if ((rc = check_state(h))) return rc;
     if (h->n == 0) return set_err(h, GX_ERR_ARG, "the adjoint needs at least one atom");
     if ((rc = settle_step_errors(h))) return rc;  // a queued step's error first: the word is cleared below
     h->nl_fresh = false;  // conservative: the passes below may reorder or move the resident state

@@ -307,7 +307,11 @@ int commit_lambda(gx_handle* h) {
 int step_error(gx_handle* h, uint32_t e) {
     if (!e) return GX_OK;
     cudaMemset(h->derr, 0, sizeof(uint32_t));
-    if (e & kErrTimeout) nl_after_timeout(h);
+    if (e & kErrBarrier) {  // the launch left its ticks half done, whatever else it met
+        nl_after_timeout(h);
+        h->state_lost = true;
+        return set_err(h, GX_ERR_TIMEOUT, "a bounded device wait timed out (the state is lost: call gx_set_state)");
+    }
     if (e & kErrNonFinite) return set_err(h, GX_ERR_NONFINITE, "non-finite force in the pair pass");
     if (e & kErrSaturation) return set_err(h, GX_ERR_SATURATION, "fixed-point force saturated");
     if (e & kErrTimeout) return set_err(h, GX_ERR_TIMEOUT, "a bounded device wait timed out");
@@ -317,6 +321,11 @@ int step_error(gx_handle* h, uint32_t e) {
 }  // namespace
 
 namespace gx {
+int check_state(gx_handle* h) {
+    if (!h->cap) return set_err(h, GX_ERR_STATE, "no state uploaded (call gx_set_state first)");
+    if (h->state_lost) return set_err(h, GX_ERR_STATE, "the state was lost in a launch that timed out (call gx_set_state)");
+    return GX_OK;
+}
 int commit_pending_lambda(gx_handle* h) { return commit_lambda(h); }
 int take_step_errors(gx_handle* h) {
     if (!h->step_errs_pending) return GX_OK;
@@ -334,8 +343,7 @@ namespace {
 
 int require_state(gx_handle* h) {
     if (!h) return GX_ERR_ARG;
-    if (!h->cap) return set_err(h, GX_ERR_STATE, "no state uploaded (call gx_set_state first)");
-    return GX_OK;
+    return check_state(h);
 }
 
 // Cell list of the force grid: keys, counting sort, reorder (double buffer).
@@ -521,8 +529,17 @@ int gx_set_state(gx_handle* h, size_t n, const double* pos, const double* vel, c
     for (size_t i = 0; i < n; ++i)
         if (elem[i] >= kNElem) return set_err(h, GX_ERR_ARG, "element index out of range (0..9)");
     GX_CUDA(h, cudaSetDevice(h->p.device));
+    if (h->step_errs_pending) {  // a queued step that gave up lost the atoms before these
+        GX_CUDA(h, cudaStreamSynchronize(h->stream));
+        if (*h->herr & kErrBarrier) {
+            nl_after_timeout(h);
+            *h->herr &= ~kErrBarrier;  // still reported as a timeout
+            GX_CUDA(h, cudaMemcpy(h->derr, h->herr, sizeof(uint32_t), cudaMemcpyHostToDevice));
+        }
+    }
     int rc = ensure_capacity(h, n);
     if (rc) return rc;
+    h->state_lost = false;
     h->n = n;
     h->cur = 0;
     h->sorted = false;
@@ -1356,6 +1373,12 @@ int gx_set_step_async(gx_handle* h, int on) {
         return rc;
     }
     h->step_async = true;
+    return GX_OK;
+}
+
+int gx_set_wait_polls(gx_handle* h, uint32_t polls) {
+    if (!h) return GX_ERR_ARG;
+    h->wait_polls = polls;
     return GX_OK;
 }
 

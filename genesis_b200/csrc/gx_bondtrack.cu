@@ -529,7 +529,7 @@ int gx_bond_observe(gx_handle* h, double k_bind, double min_periods, int debounc
                     gx_bond_observation* out) {
     if (!h || !out || debounce < 1 || !(k_bind > 0.0)) return GX_ERR_ARG;
     if ((uint32_t)debounce > kMaxDebounce) return set_err(h, GX_ERR_ARG, "debounce above 65535 ticks");
-    if (!h->cap) return set_err(h, GX_ERR_STATE, "no state uploaded (call gx_set_state first)");
+    if (const int rs = check_state(h)) return rs;
     if (!h->tracker) h->tracker = new BondTracker();
     BondTracker* t = static_cast<BondTracker*>(h->tracker);
     int rc = tracker_init(h, t);

@@ -284,8 +284,7 @@ struct ExportState {
 
 int require_state(gx_handle* h) {
     if (!h) return GX_ERR_ARG;
-    if (!h->cap) return set_err(h, GX_ERR_STATE, "no state uploaded (call gx_set_state first)");
-    return GX_OK;
+    return check_state(h);
 }
 
 ExportState& export_of(gx_handle* h) {

@@ -6,7 +6,6 @@
 
 namespace gx {
 
-constexpr uint32_t kSyncPolls = 1u << 22;  // polls of the grid barrier before giving up (seconds)
 constexpr uint32_t kScanTileCells = 1024;  // cell counters per scan tile
 constexpr uint32_t kScanMaxTiles = 64;     // of at most 65,536 counters
 
@@ -24,23 +23,28 @@ __device__ __forceinline__ uint32_t load_acquire(const uint32_t* p) {
 }
 
 // Grid barrier: arrivals only grow during a launch, and `target` (thread 0's)
-// is the count at which every block has arrived.  The wait is bounded: a
-// block that gives up sets kErrTimeout and leaves (false), and the others
-// follow as their waits end.
-__device__ __forceinline__ bool grid_barrier(GridSync* s, uint32_t* err, uint32_t& target, int* s_ok) {
+// is the count at which every block has arrived.  The wait is bounded by
+// `limit` polls: a block that gives up sets kErrBarrier and leaves (false),
+// and the others follow as they see that word or their waits end.  The words
+// are no longer zero then, so a launch that finds kErrBarrier set when it
+// starts (one queued behind, before the host has read the error) does nothing.
+__device__ __forceinline__ bool grid_barrier(GridSync* s, uint32_t* err, uint32_t limit, uint32_t& target, int* s_ok) {
     __syncthreads();
     if (threadIdx.x == 0) {
         target += gridDim.x;
         __threadfence();
         atomicAdd(&s->arrived, 1u);
-        uint32_t polls = 0;
         int ok = 1;
-        while ((int32_t)(load_acquire(&s->arrived) - target) < 0)
-            if (++polls > kSyncPolls) {
-                atomicOr(err, kErrTimeout);
+        for (uint32_t polls = 0; ok; ++polls) {
+            if (polls >= limit) {
+                atomicOr(err, kErrTimeout | kErrBarrier);
                 ok = 0;
+            } else if ((int32_t)(load_acquire(&s->arrived) - target) >= 0) {
                 break;
+            } else if ((polls & 1023u) == 1023u && (load_acquire(err) & kErrBarrier)) {
+                ok = 0;
             }
+        }
         __threadfence();
         *s_ok = ok;
     }

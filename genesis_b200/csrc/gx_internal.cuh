@@ -25,6 +25,7 @@ enum : uint32_t {
     kErrCapacity = 4u,
     kErrBinRange = 8u,
     kErrTimeout = 16u,
+    kErrBarrier = 32u,  // with kErrTimeout: a grid barrier gave up and its launch left its work half done
 };
 
 // ---------------------------------------------------------------------------
@@ -231,6 +232,8 @@ struct gx_handle {
     unsigned long long* dcount = nullptr;  // [0]=pairs, [1..3]=fixed V, Vb, ..., [8]=bond count
     uint32_t* derr = nullptr;      // device error word
     gx::HostPage* page = nullptr;  // pinned: what a waiting call reads back (launch_page)
+    uint32_t wait_polls = 1u << 22;  // polls of a grid barrier before it gives up (some seconds)
+    bool state_lost = false;         // a launch of several ticks gave up: the atoms may be half moved
     // gx_set_step_async: gx_step returns without waiting; its error word is
     // copied to pinned host memory and reported by the next call that waits
     bool step_async = false;
@@ -398,6 +401,9 @@ int take_step_errors(gx_handle* h);
 // call that clears or consumes the device error word runs this first, so a
 // step's error is never cleared before it is reported.
 int settle_step_errors(gx_handle* h);
+// GX_ERR_STATE without an uploaded state, or with one that a timed-out launch
+// left half moved.
+int check_state(gx_handle* h);
 
 // Read-only view of the persistent neighbour list (gx_nlist.cu) for the
 // passes that can take their candidates from it.  Entry e of atom p (sorted

@@ -837,8 +837,7 @@ int build_aux(gx_handle* h, AuxPool& P, const GridGeom& g, const uint32_t* sel, 
 
 int require(gx_handle* h) {
     if (!h) return GX_ERR_ARG;
-    if (!h->cap) return set_err(h, GX_ERR_STATE, "no state uploaded (call gx_set_state first)");
-    return GX_OK;
+    return check_state(h);
 }
 
 int gr_common(gx_handle* h, int ta, int tb, double r_max_in, size_t nbins_in, size_t sample_cap, uint64_t* counts,

@@ -1573,6 +1573,7 @@ int nl_set_skin(gx_handle* h, double skin) {
 
 void nl_after_timeout(gx_handle* h) {
     if (h->nl) static_cast<NlState*>(h->nl)->tick_sync_dirty = true;
+    h->nl_valid = h->nl_fresh = false;
 }
 
 bool nl_view(const gx_handle* h, NlView* v) {

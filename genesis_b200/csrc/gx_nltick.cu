@@ -78,6 +78,7 @@ struct TickArgs {
     double k_thermal, target, tau;
     float lim2, rl2;
     int wrap, thermo, nticks;
+    uint32_t polls;  // of a barrier before it gives up
 };
 
 // Sum of part[0 .. nb) in k_thermostat_lambda's order (valid in thread 0).
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
     const int nb = (int)((n + kTickThreads - 1) / kTickThreads);
     const bool recorder = blockIdx.x == gridDim.x - 1;
     uint32_t target = 0;  // thread 0's count of barrier arrivals
+    if (*a.err & kErrBarrier) return;  // the launch before this one gave up
     const int nk2 = F64 ? 0 : a.L.nkinds * a.L.nkinds;
     double* vat = reinterpret_cast<double*>(a.F);
     for (int t = tid; t < nk2; t += kTickThreads) st.put(t, a.tab[t]);
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                                    a.ref, a.lim2, half, a.err);
         }
         if (__syncthreads_or(over) && tid == 0) a.sync->grid.request[par] = 1u;
-        if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+        if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
         const bool rebuild = (tick == 0 && asked) || *(volatile uint32_t*)&a.sync->grid.request[par] != 0u;
         if (recorder) {  // the other parity's words: every block has left that tick's pair pass
             if (REC && tick > 0) take_record<F64>(a, tick - 1, s_lam, nb, sh);
@@ -172,12 +174,12 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                 a.key[i] = c;
                 atomicAdd(&a.count[c], 1u);
             }
-            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
             for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
                 const uint32_t total = scan_tile<kTickThreads>(a.count, t, m, 0u, s_warp);
                 if (tid == 0) a.sync->grid.tile[t] = total;
             }
-            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
             if (tid < ntiles) {  // tile offsets, in every block
                 uint32_t run = 0;
                 for (uint32_t t = 0; t < tid; ++t) run += a.sync->grid.tile[t];
@@ -189,7 +191,7 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                 const uint32_t c = a.key[i];
                 a.tmp[a.count[c] + s_off[c / kScanTileCells] + atomicAdd(&a.fill[c], 1u)] = i;
             }
-            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
             for (uint32_t i = gt; i < n; i += gs) {  // k_rank and k_gather: ascending source order within a cell
                 const uint32_t c = a.key[i], lo = a.start[c], hi = a.start[c + 1];
                 uint32_t p = lo;
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                 a.home[p] = c;
                 a.pos_of_slot[s] = p;
             }
-            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
             for (uint32_t p = gt; p < n; p += gs) {
                 const double x = a.o.x[p], y = a.o.y[p], z = a.o.z[p];
                 a.b.x[p] = x;
@@ -236,10 +238,10 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                 a.ref[p] = f;
             }
             for (uint32_t c = gt; c < m; c += gs) a.count[c] = a.fill[c] = 0u;
-            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
             for (uint32_t p = gt / 32u; p < n; p += gs / 32u)
                 nl_build_warp_one<!F64>(a.g, a.pos4, a.home, a.start, p, a.rl2, a.list, a.stride, a.cap_nb, a.cnt);
-            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
             parity = 0u;
             ++rebuilds;
         } else if (a.wrap) {
@@ -347,7 +349,7 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                 }
             }
         }
-        if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+        if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
         for (uint32_t v = blockIdx.x; v < (uint32_t)nb; v += gridDim.x) {
             const uint32_t i = v * kTickThreads + tid;  // the thread that advances atom i
             double ks = 0.0, ss = 0.0, vs = 0.0;
@@ -372,13 +374,13 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
             }
         }
         if (a.thermo) {
-            if (!grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;
+            if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
             const double K = part_sum(a.kpart + par * kPartRow, nb, sh);
             if (tid == 0) s_lam = berendsen_scale(K, n, a.k_thermal, a.target, a.tau);
             __syncthreads();
         }
     }
-    if (REC && !a.thermo && !grid_barrier(&a.sync->grid, a.err, target, &s_ok)) return;  // the last partials
+    if (REC && !a.thermo && !grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;  // the last partials
     if (recorder) {
         if (REC) take_record<F64>(a, a.nticks - 1, s_lam, nb, sh);
         if (tid == 0) {
@@ -495,6 +497,7 @@ int nl_ticks(gx_handle* h, int nticks, gx_tick_stats* rec, bool thermo, double t
     a.rl2 = rl * rl;
     a.wrap = h->p.enable_boundaries ? 1 : 0;
     a.thermo = thermo ? 1 : 0;
+    a.polls = h->wait_polls;
     const size_t blocks = ((size_t)n * lanes + kTickThreads - 1) / kTickThreads;
     const unsigned grid = (unsigned)std::min<size_t>(blocks, (size_t)resident);
     for (int done = 0; done < nticks; done += kTicksPerLaunch) {

@@ -202,8 +202,8 @@ using namespace gx;
 
 extern "C" int gx_snapshot_world(gx_handle* h, const uint32_t* generation, uint8_t* out, size_t cap, size_t* len) {
     if (!h || !len) return GX_ERR_ARG;
-    if (!h->cap) return set_err(h, GX_ERR_STATE, "no state uploaded (call gx_set_state first)");
-    int rc = settle_step_errors(h);
+    int rc = check_state(h);
+    if (!rc) rc = settle_step_errors(h);
     if (rc) return rc;
     rc = commit_pending_lambda(h);  // v as the host would read it
     if (rc) return rc;

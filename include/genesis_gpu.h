@@ -513,6 +513,12 @@ int gx_synchronize(gx_handle* h);
  * Lets a host scheduler queue the force systems and the observation of one
  * tick behind a single wait.  Default 0: gx_step waits and reports. */
 int gx_set_step_async(gx_handle* h, int on);
+/* Polls of a device-wide barrier inside a launch of several ticks (gx_step,
+ * gx_tick_host, gx_adjoint_*) before the launch gives up with GX_ERR_TIMEOUT:
+ * by default 4,194,304, some seconds; 0 gives up at once.  A gx_step or
+ * gx_tick_host that gave up leaves the atoms half moved: every call on the
+ * state fails with GX_ERR_STATE until gx_set_state. */
+int gx_set_wait_polls(gx_handle* h, uint32_t polls);
 /* Records CUDA event `slot` (0..15) on the handle's stream. */
 int gx_timer_mark(gx_handle* h, int slot);
 /* Milliseconds between two recorded events (waits for the second). */
