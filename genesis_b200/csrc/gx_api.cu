@@ -995,7 +995,6 @@ int gx_autotune(gx_handle* h, int reps, int* best, double* ms) {
     // passes leave the state bit-identical whichever variant runs.
     const int cand[4] = {4, 1, 3, 2};
     int pick = 4;
-    bool automatic = false;  // the one-launch tick of a small universe won
     double best_ms = 1e300;
     const int saved = h->kernel_variant;
     for (int v : cand) {
@@ -1118,16 +1117,22 @@ int gx_autotune(gx_handle* h, int reps, int* best, double* ms) {
                     int r2 = tick_ms(&best_t);  // restores the snapshot after the tick above
                     if (!rc) rc = r2;
                 }
-                // a small universe's automatic tick is one launch (gx_nltick.cu)
+                // a small universe's half-list tick without a shape is one launch (gx_nltick.cu)
                 if (!rc && n <= kTickMaxAtoms) {
                     int lanes = 0, block = 0, slots = 0, brick = 0;
                     nl_shape(h, &lanes, &block, &slots, &brick);
                     double t = 1e300;
-                    h->kernel_variant = 0;
+                    bool stale = false, one_launch = false;
+                    h->kernel_variant = 6;
                     nl_clear_shape(h);
-                    rc = tick_ms(&t);
-                    automatic = !rc && t < best_t;
-                    if (!automatic) {
+                    if (!(rc = nl_prepare(h, &stale)) && nl_ticks_eligible(h)) {
+                        rc = tick_ms(&t);
+                        one_launch = !rc && t < best_t;
+                    }
+                    if (one_launch) {
+                        pick = 6;
+                    } else {
+                        h->kernel_variant = pick;
                         nl_set_tpp(h, lanes);
                         nl_set_block(h, block);
                     }
@@ -1136,9 +1141,9 @@ int gx_autotune(gx_handle* h, int reps, int* best, double* ms) {
             cudaFree(snap);
         }
     }
-    h->kernel_variant = rc ? saved : (automatic ? 0 : pick);
+    h->kernel_variant = rc ? saved : pick;
     invalidate_graphs(h);
-    if (best) *best = automatic ? 6 : h->kernel_variant;  // the automatic variant walks the half list of 6
+    if (best) *best = h->kernel_variant;
     return rc;
 }
 

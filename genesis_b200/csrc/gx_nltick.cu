@@ -404,13 +404,13 @@ inline uint32_t tick_lanes64(uint32_t n) { return nl_auto_lanes64(n); }
 
 }  // namespace
 
-// One launch covers the plain half-list tick of the automatic variant: no
-// collision pass, no per-launch timing, and a size at which the launches and
-// not the work set the tick.
+// One launch covers the plain half-list tick (variant 6, which the automatic
+// one is here): no work shape set, no collision pass, no per-launch timing,
+// and a size at which the launches and not the work set the tick.
 bool nl_ticks_eligible(gx_handle* h) {
     const bool mixed = h->precision == GX_MIXED;
     if (h->n == 0 || h->n > (mixed ? kTickMaxAtoms : kTickMaxAtoms64)) return false;
-    if (mixed ? h->kernel_variant != 0 : bonds_on(h)) return false;  // the FP64 spring adds to finished accelerations
+    if (mixed ? h->kernel_variant != 0 && h->kernel_variant != 6 : bonds_on(h)) return false;  // the FP64 spring adds to finished accelerations
     if (h->p.enable_collisions || h->prof_on || h->pass_timing) return false;
     const NlState* s = static_cast<const NlState*>(h->nl);
     if (!s || (mixed && 0.5 * s->expect * (double)h->n > kTickMaxEntries)) return false;

@@ -105,8 +105,9 @@ const char* gx_last_error(const gx_handle* h);
 const char* gx_status_string(int status);
 int gx_set_precision(gx_handle* h, int precision);
 /* Tuning knob of the mixed pair pass: 0 = automatic (6 where it applies,
- * else 4; up to 65,536 atoms, 24,576 in FP64, with no work shape set, the
- * ticks of a gx_step call with use_graph run in one launch, the same bits),
+ * else 4; with either, up to 65,536 atoms, 24,576 in FP64, with no work
+ * shape set, the ticks of a gx_step call with use_graph run in one launch,
+ * the same bits),
  * 1 = one thread per atom over the canonical half shell,
  * 2 = warp-tiled cell pairs with ballot compaction, 3 = thread per atom with
  * staged rows, 4 = thread per atom with per-thread candidate lists (all
@@ -144,7 +145,8 @@ int gx_set_kernel_variant(gx_handle* h, int variant);
  * 0.2 r_c (the list-grid cell is r_c + skin; gx_get_list_config reports
  * the choice), and the lanes per atom (the stash size of 7, the brick
  * length of 8) over passes
- * on a list of that skin.  The state is left as it was. */
+ * on a list of that skin; a universe small enough for one launch is also
+ * timed so, which is 6 with no shape set.  The state is left as it was. */
 int gx_autotune(gx_handle* h, int reps, int* best, double* ms);
 /* No counterpart in the reference.  Skin of the variant-5/6 neighbour list
  * (default 0.1 r_c); 0 rebuilds every tick. */

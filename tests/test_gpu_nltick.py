@@ -98,3 +98,23 @@ def test_one_launch_tick_reports_and_recovers_from_a_non_finite_velocity(gpu):
         h.set_universe(u)
         want = h.step(3, graph=True)
     assert np.array_equal(st["potential"], want["potential"])
+
+
+def test_autotuned_variant_is_the_same_tick_on_another_handle(gpu):
+    """A small universe's autotuner keeps the one-launch tick, and the variant it reports gives it elsewhere."""
+    from genesis_b200._lib import Handle
+    wl = W.Workload("tick check", n_side=8, temperature=100.0, steps=10)
+    cfg, u = wl.config(), wl.generate()
+    out = []
+    with Handle(cfg, "mixed") as a, Handle(cfg, "mixed") as b:
+        for h in (a, b):
+            h.set_universe(u)
+        best, _ = a.autotune(reps=20)
+        b.set_kernel_variant(best)
+        b.set_list_skin(a.list_config()[0])
+        for h in (a, b):
+            h.step(1, graph=True)
+            l0 = h.launches
+            h.step(20, graph=True)
+            out.append(h.launches - l0)
+    assert out == [2, 2]  # the ticks, and the words read back
