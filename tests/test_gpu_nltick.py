@@ -118,3 +118,37 @@ def test_autotuned_variant_is_the_same_tick_on_another_handle(gpu):
             h.step(20, graph=True)
             out.append(h.launches - l0)
     assert out == [2, 2]  # the ticks, and the words read back
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("target", [0.0, 150.0])
+def test_ticks_across_launches(gpu, precision, target):
+    """Calls of more ticks than one launch takes (256): the records' places, the pending scale, the frame's parity."""
+    wl = W.Workload("tick check", n_side=8, temperature=200.0, steps=10, thermostat=target > 0.0,
+                    thermostat_temperature=target if target > 0.0 else 300.0)
+    _pair(wl.config(), wl.generate(), [(257, True), (513, True), (258, False), (3, True)], precision=precision)
+
+
+@pytest.mark.parametrize("precision,n_side,one", [("mixed", 8, True), ("mixed", 40, True), ("mixed", 41, False),
+                                                  ("fp64", 8, True), ("fp64", 29, True), ("fp64", 30, False)])
+def test_sizes_that_run_in_one_launch(gpu, precision, n_side, one):
+    """The exact launches of a call on both sides of each limit: one per 256 ticks and the read-back's."""
+    from genesis_b200._lib import Handle
+    wl = W.Workload("tick check", n_side=n_side, temperature=100.0, steps=10)
+    with Handle(wl.config(), precision) as h:
+        h.set_universe(wl.generate())
+        h.step(1, graph=True)
+        for ticks in (5,) if n_side > 8 else (1, 5, 256, 257, 513):
+            l0 = h.launches
+            h.step(ticks, graph=True)
+            assert (h.launches - l0 == -(-ticks // 256) + 1) == one
+        if precision == "mixed" and one:  # a work shape is the per-kernel tick's, as is any other variant
+            l0 = h.launches
+            h.set_kernel_variant(5)
+            h.step(5, graph=True)
+            assert h.launches - l0 > 2
+            h.set_kernel_variant(6)
+            h.set_list_threads(4)
+            l0 = h.launches
+            h.step(5, graph=True)
+            assert h.launches - l0 > 2
