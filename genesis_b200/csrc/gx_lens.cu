@@ -907,7 +907,9 @@ int gr_common(gx_handle* h, int ta, int tb, double r_max_in, size_t nbins_in, si
         const float reach2 = (float)(r_max * r_max * (1.0 + 1e-4));
         const bool wide = m >= kGrWideAtoms;
         const size_t warps = wide ? (m + 7) / 8 : (m + 1) / 2;
-        const unsigned grid = (unsigned)std::min<size_t>(nblk(warps, kGrThreads / 32), kGrBlocks);
+        // blocks enough that m / grid + 32 atoms of one, each with all the others in one bin, fit its 32-bit counts
+        const size_t least = ((unsigned long long)m * m >> 31) + 1;
+        const unsigned grid = (unsigned)std::min<size_t>(nblk(warps, kGrThreads / 32), std::max<size_t>(kGrBlocks, least));
         auto kern = ta >= 0 ? (wide ? k_gr<8, true> : k_gr<2, true>) : (wide ? k_gr<8, false> : k_gr<2, false>);
         GX_LAUNCH(h, kern, grid, kGrThreads, g, sub, a, box[0], box[1], box[2], r_max * r_max, reach2,
                   (float)(1.0 / dr), slack, v);
