@@ -41,8 +41,9 @@ struct AuxPool {
     double* xyz = nullptr;  // 6 * cap: staging xyz + sorted xyz
     uint8_t* elem = nullptr;  // 2 * cap
     uint32_t* u32 = nullptr;  // 6 * cap: slot, slot_sorted, key, key_sorted, perm, sel
-    float4* loc = nullptr;    // cap
     size_t cap = 0;
+    float4* loc = nullptr;    // loc_cap, for k_gr alone
+    size_t loc_cap = 0;
     CellList cl;
     uint32_t* parent = nullptr;
     uint32_t* size = nullptr;
@@ -74,12 +75,10 @@ int ensure_pool(gx_handle* h, AuxPool& P, size_t m, size_t natoms) {
         cudaFree(P.xyz);
         cudaFree(P.elem);
         cudaFree(P.u32);
-        cudaFree(P.loc);
         size_t cap = m < 1024 ? 1024 : m;
         GX_CUDA(h, cudaMalloc(&P.xyz, 6 * cap * sizeof(double)));
         GX_CUDA(h, cudaMalloc(&P.elem, 2 * cap));
         GX_CUDA(h, cudaMalloc(&P.u32, 6 * cap * sizeof(uint32_t)));
-        GX_CUDA(h, cudaMalloc(&P.loc, cap * sizeof(float4)));
         P.cap = cap;
     }
     if (natoms > P.ucap) {
@@ -894,6 +893,13 @@ int gr_common(gx_handle* h, int ta, int tb, double r_max_in, size_t nbins_in, si
             g = f;
             break;
         }
+    }
+    if (fast && m > P.loc_cap) {
+        cudaFree(P.loc);
+        P.loc = nullptr;
+        P.loc_cap = 0;
+        GX_CUDA(h, cudaMalloc(&P.loc, P.cap * sizeof(float4)));
+        P.loc_cap = P.cap;
     }
     if ((rc = build_aux(h, P, g, sel, (uint32_t)m, a, fast))) return rc;
     GX_CUDA(h, cudaMemsetAsync(P.counts, 0, nbins * sizeof(uint64_t), h->stream));
