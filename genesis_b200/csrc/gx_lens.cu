@@ -295,7 +295,7 @@ struct GrVisit {
 // (134 M pairs in range).  Instruction issue bounds it: about 30 warp
 // instructions per 32 candidate pairs, of which a third lie in range.
 constexpr int kGrThreads = 128;
-constexpr unsigned kGrBlocks = 148 * 12;
+constexpr unsigned kGrBlocksPerSm = 12;
 constexpr size_t kGrWideAtoms = 65536;  // atoms from which a warp takes 8 at a time, 2 below
 constexpr int kGrMaxSub = 3;            // 25 rows of the half space: one per lane
 
@@ -914,8 +914,10 @@ int gr_common(gx_handle* h, int ta, int tb, double r_max_in, size_t nbins_in, si
         const bool wide = m >= kGrWideAtoms;
         const size_t warps = wide ? (m + 7) / 8 : (m + 1) / 2;
         // blocks enough that m / grid + 32 atoms of one, each with all the others in one bin, fit its 32-bit counts
+        int sms = 0;
+        GX_CUDA(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->p.device));
         const size_t least = ((unsigned long long)m * m >> 31) + 1;
-        const unsigned grid = (unsigned)std::min<size_t>(nblk(warps, kGrThreads / 32), std::max<size_t>(kGrBlocks, least));
+        const unsigned grid = (unsigned)std::min<size_t>(nblk(warps, kGrThreads / 32), std::max<size_t>((size_t)kGrBlocksPerSm * sms, least));
         auto kern = ta >= 0 ? (wide ? k_gr<8, true> : k_gr<2, true>) : (wide ? k_gr<8, false> : k_gr<2, false>);
         GX_LAUNCH(h, kern, grid, kGrThreads, g, sub, a, box[0], box[1], box[2], r_max * r_max, reach2,
                   (float)(1.0 / dr), slack, v);
