@@ -8,7 +8,7 @@
 //
 // Forward.  The trajectory is recomputed in slot order (atoms never move
 // between arrays) in FP64 with the reference's per-pair arithmetic
-// (pair_f64).  On a handle of mixed precision the forward is the mixed method
+// (pair_f64_e24).  On a handle of mixed precision the forward is the mixed method
 // instead: the FP32 pair law of the list passes (pair_f32) on the FP64
 // minimum-image displacement rounded to FP32, the per-atom force summed in
 // 2^-32 fixed point, and FP64 positions, velocities and observables; the

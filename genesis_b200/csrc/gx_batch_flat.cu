@@ -131,7 +131,7 @@ __global__ void k_fb_advance(const RepGeo* __restrict__ geo, const uint32_t* __r
     if (i < total) fb_advance_one(i, geo, rep_of, A, lam, half_dt, dt, wrap, key, err);
 }
 
-// Sorted staging: cell-local FP32 position + kind (as k_build_pos4), the
+// Sorted staging: cell-local FP32 position + kind (as k_rank_gather), the
 // local cell and replica of each sorted position, zeroed forces.
 __device__ __forceinline__ void fb_stage_one(uint32_t s, const RepGeo* __restrict__ geo,
                                              const uint32_t* __restrict__ rep_of, const BatchArrays& A,

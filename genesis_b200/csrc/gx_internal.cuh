@@ -50,7 +50,8 @@ __device__ __forceinline__ double min_image1(double d, double L) {
     return xsub(d, xmul(L, round(xdiv(d, L))));
 }
 // min_image1 for |d| <= 0.49 L without the division: the rounded quotient
-// is zero there and d - L * 0 is d itself, sign of a zero included.
+// is zero there and d - L * 0 is d itself (for d = -0 it is +0: no square or
+// sum of forces sees the difference).
 __device__ __forceinline__ double near_image(double d, double L) {
     return fabs(d) <= xmul(0.49, L) ? d : min_image1(d, L);
 }
@@ -356,7 +357,6 @@ int force_pass(gx_handle* h, bool finalize_acc, double* V, double* Vb, uint64_t*
 int bond_spring(gx_handle* h, bool unit_mult);
 // FP64 pair table on the device: sigma_ij then eps_ij, kNElem^2 each (gx_force.cu).
 double* d_psig(gx_handle* h);
-// out = the sum of part[0..nb) in a fixed order, one block (gx_force.cu).
 inline bool bonds_on(const gx_handle* h) { return h->p.enable_bond_interaction && h->bonds_cap > 0; }
 inline unsigned long long* dnbonds(gx_handle* h) { return h->dcount + 8; }
 void adjoint_free(gx_handle* h);

@@ -169,13 +169,6 @@ __global__ void k_place(StateBuf b, uint32_t m, const uint32_t* __restrict__ key
 
 // Canonical half-shell enumeration with the exact check_pair test
 // (src/physics/grid.rs:201-225).  V::operator()(i, j, d) sees aux indices.
-// min_image1 for a difference of which only the length is used: within
-// 0.49 L the rounded quotient is below one half, round() gives zero and the
-// reference's d - L * 0 is d itself (up to the sign of a zero).
-__device__ __forceinline__ double near_image1(double d, double L) {
-    return fabs(d) <= xmul(0.49, L) ? d : min_image1(d, L);
-}
-
 template <class V>
 __global__ void k_pairs(GridGeom g, AuxSet a, double box0, double box1, double box2, double cd2, V visit) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -197,9 +190,9 @@ __global__ void k_pairs(GridGeom g, AuxSet a, double box0, double box1, double b
             }
             uint32_t hi = a.start[B + 1];
             for (uint32_t j = lo; j < hi; ++j) {
-                double dx = near_image1(xsub(xi, a.x[j]), box0);
-                double dy = near_image1(xsub(yi, a.y[j]), box1);
-                double dz = near_image1(xsub(zi, a.z[j]), box2);
+                double dx = near_image(xsub(xi, a.x[j]), box0);
+                double dy = near_image(xsub(yi, a.y[j]), box1);
+                double dz = near_image(xsub(zi, a.z[j]), box2);
                 double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
                 if (d2 >= cd2) continue;
                 double d = xsqrt(d2);
@@ -406,9 +399,9 @@ __global__ void __launch_bounds__(kGrThreads, 8) k_gr(GridGeom g, int sub, AuxSe
                         }
                         for (; edge; edge &= edge - 1u) {
                             const uint32_t i = r0 + (uint32_t)__ffs(edge) - 1u;
-                            const double ex = near_image1(xsub(a.x[i], a.x[j]), box0);
-                            const double ey = near_image1(xsub(a.y[i], a.y[j]), box1);
-                            const double ez = near_image1(xsub(a.z[i], a.z[j]), box2);
+                            const double ex = near_image(xsub(a.x[i], a.x[j]), box0);
+                            const double ey = near_image(xsub(a.y[i], a.y[j]), box1);
+                            const double ez = near_image(xsub(a.z[i], a.z[j]), box2);
                             const double e2 = xadd(xadd(xmul(ex, ex), xmul(ey, ey)), xmul(ez, ez));
                             if (e2 >= cd2) continue;
                             const double d = xsqrt(e2);
@@ -658,9 +651,9 @@ struct BucketArgs {
 __device__ __forceinline__ void bound_candidate(double xi, double yi, double zi, double si, uint32_t slot_i, double xj,
                                                 double yj, double zj, double sj, uint32_t slot_j, double box0,
                                                 double box1, double box2, double cd2, const BucketArgs& v) {
-    double dx = near_image1(xsub(xi, xj), box0);
-    double dy = near_image1(xsub(yi, yj), box1);
-    double dz = near_image1(xsub(zi, zj), box2);
+    double dx = near_image(xsub(xi, xj), box0);
+    double dy = near_image(xsub(yi, yj), box1);
+    double dz = near_image(xsub(zi, zj), box2);
     double d2 = xadd(xadd(xmul(dx, dx), xmul(dy, dy)), xmul(dz, dz));
     if (d2 >= cd2) return;
     double threshold = xmul(v.k_bind, xmul(0.5, xadd(si, sj)));  // pairs.rs:163

@@ -54,16 +54,21 @@ constexpr size_t kTickMaxAtoms64 = 24576;  // FP64 ticks
 // Ticks of one launch at most, so that a long call stays a queue of launches.
 constexpr int kTicksPerLaunch = 256;
 
-// Lanes per atom of the half-list pass where none were set: enough to fill
+// Lanes per atom of the list pass where none were set: enough to fill
 // the chip and to share the long lists of a condensed state, one where the
-// gathers of a homogeneous one set the time.  Microseconds per pass with
-// 1 / 2 / 4 / 8 lanes on the lattice: 31 / 21 / 15 / 10 at 4,096 atoms,
+// gathers of a homogeneous one set the time.  Microseconds per half-list pass
+// with 1 / 2 / 4 / 8 lanes on the lattice: 31 / 21 / 15 / 10 at 4,096 atoms,
 // 31 / 23 / 17 / 19 at 32,768, 34 / 25 / 27 / 27 at 59,319, 44 / 42 / 41 / 45
 // at 125,000, 76 / 71 / 76 / 90 at 262,144, 124 / 129 / 146 / 177 at 512,000,
 // 221 / 236 / 274 / 357 at 1,000,000, 435 / 477 / 563 / 709 at 2,097,152; per
 // tick after 1,000 ticks of condensation with charges and gravity:
 // 96 / 73 / 60 / 59 at 32,768, 107 / 89 / 82 / 77 at 59,319,
-// 263 / 234 / 223 / 232 at 262,144.
+// 263 / 234 / 223 / 232 at 262,144.  The full list (variant 5) has the same
+// lines: per captured tick, 1 / 2 / 4 / 8 lanes, 43 / 35 / 29 / 26 at 4,096,
+// 49 / 41 / 36 / 38 at 32,768, 56 / 49 / 50 / 48 at 59,319, 79 / 80 / 77 / 78
+// at 125,000, 133 / 129 / 133 / 141 at 262,144, 218 / 217 / 225 / 240 at
+// 512,000, 382 / 387 / 404 / 437 at 1,000,000, 819 / 829 / 875 / 947 at
+// 2,097,152.
 inline int nl_auto_lanes(uint32_t n) {
     if (n <= 98304) return 8;
     if (n <= 327680) return 4;

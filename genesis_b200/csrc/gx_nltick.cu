@@ -12,8 +12,8 @@
 //   [rebuild]        keys and counts, scan, scatter, rank and gather, copy
 //                    back and staging, lists by one warp per atom (six
 //                    barriers), only on the ticks that ask for it
-//   pair pass        2 .. 32 lanes per atom over its half list, and the
-//                    observed-bond spring
+//   pair pass        8 .. 32 lanes per atom over its half list (FP64: 4 .. 32
+//                    over its full list), and the observed-bond spring
 //   -- barrier --    the force sums are final
 //   finish           a = F 2^-32 / m, kick, kinetic-energy partials
 //   -- barrier --    with the thermostat: every block sums the partials and
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                 a.tmp[a.count[c] + s_off[c / kScanTileCells] + atomicAdd(&a.fill[c], 1u)] = i;
             }
             if (!grid_barrier(&a.sync->grid, a.err, a.polls, target, &s_ok)) return;
-            for (uint32_t i = gt; i < n; i += gs) {  // k_rank and k_gather: ascending source order within a cell
+            for (uint32_t i = gt; i < n; i += gs) {  // as k_rank_gather: ascending source order within a cell
                 const uint32_t c = a.key[i], lo = a.start[c], hi = a.start[c + 1];
                 uint32_t p = lo;
                 for (uint32_t q = lo; q < hi; ++q) p += a.tmp[q] < i ? 1u : 0u;

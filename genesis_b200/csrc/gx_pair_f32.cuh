@@ -45,7 +45,8 @@ __device__ __forceinline__ float fmul_sat(float a, float b) {
     return r;
 }
 
-// rsqrtf without the scaling of subnormal arguments, and with it only for those.
+// The PTX instruction flushes subnormal arguments to zero (its manual's .ftz),
+// so those take rsqrtf; normal ones kept the bits of every mixed trajectory.
 __device__ __forceinline__ float rsqrt_normal(float d2) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d2));
