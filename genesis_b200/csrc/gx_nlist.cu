@@ -513,16 +513,16 @@ __global__ void __launch_bounds__(kNlThreads) k_nl_force_tpp(GridGeom g, const f
                 nl_pair(L, st, ki, pi, __ldg(pos4 + q), sh.x, sh.y, sh.z, ENERGY && (HALF || q > p), a, err,
                         HALF ? F : nullptr, q, fstride);
             }
-        } else {  // overflowed list: the group splits the 27 home-grid cells
+        } else {  // overflowed list: the group splits each of the 27 home-grid cells
             uint32_t cx, cy, cz;
             decode(g, home[p], cx, cy, cz);
             const uint32_t c = home[p];
-            for (uint32_t code = sub; code < 27; code += TPP) {
+            for (uint32_t code = 0; code < 27; ++code) {
                 uint32_t B = cell_at(g, cx, cy, cz, code);
                 if (HALF && B < c) continue;
                 float sx, sy, sz;
                 code_shift(g, code, sx, sy, sz);
-                for (uint32_t q = start[B], hi = start[B + 1]; q < hi; ++q)
+                for (uint32_t q = start[B] + sub, hi = start[B + 1]; q < hi; q += TPP)
                     if (HALF ? q > p : q != p)
                         nl_pair(L, st, ki, pi, pos4[q], sx, sy, sz, ENERGY && q > p, a, err, HALF ? F : nullptr, q, fstride);
             }

@@ -339,12 +339,12 @@ __device__ __forceinline__ void nl_atom64(const GridGeom& g, const StateBuf& b, 
             yj = yn;
             zj = zn;
         }
-    } else {  // overflowed list: the lanes split the 27 home-grid cells
+    } else {  // overflowed list: the lanes split each of the 27 home-grid cells
         uint32_t cx, cy, cz;
         decode(g, home[i], cx, cy, cz);
-        for (uint32_t code = sub; code < 27; code += lanes) {
+        for (uint32_t code = 0; code < 27; ++code) {
             const uint32_t B = cell_at(g, cx, cy, cz, code);
-            for (uint32_t q = start[B], hi = start[B + 1]; q < hi; ++q)
+            for (uint32_t q = start[B] + sub, hi = start[B + 1]; q < hi; q += lanes)
                 if (q != i) visit(q, b.x[q], b.y[q], b.z[q]);
         }
     }

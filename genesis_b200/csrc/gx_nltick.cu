@@ -298,15 +298,15 @@ __global__ void __launch_bounds__(kTickThreads, F64 ? 3 : 4) k_nl_ticks(const __
                             const float4 s0 = s_shift[w >> 27];
                             nl_pair(a.L, st, ki, pi, a.pos4[q], s0.x, s0.y, s0.z, REC, f, a.err, a.F, q, a.fstride);
                         }
-                    } else {  // overflowed list: the group splits the 27 home-grid cells
+                    } else {  // overflowed list: the group splits each of the 27 home-grid cells
                         const uint32_t c = a.home[p];
                         uint32_t cx, cy, cz;
                         decode(a.g, c, cx, cy, cz);
-                        for (uint32_t code = sub; code < 27; code += lanes) {
+                        for (uint32_t code = 0; code < 27; ++code) {
                             const uint32_t B = cell_at(a.g, cx, cy, cz, code);
                             if (B < c) continue;
                             const float4 s0 = s_shift[code];
-                            for (uint32_t q = a.start[B], hi = a.start[B + 1]; q < hi; ++q)
+                            for (uint32_t q = a.start[B] + sub, hi = a.start[B + 1]; q < hi; q += lanes)
                                 if (q > p)
                                     nl_pair(a.L, st, ki, pi, a.pos4[q], s0.x, s0.y, s0.z, REC, f, a.err, a.F, q,
                                             a.fstride);

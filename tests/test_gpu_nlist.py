@@ -317,3 +317,36 @@ def test_pass_timing_inside_captured_ticks(gpu):
     assert 0.0 < t_graph < 50.0 and 0.0 < t_eager < 50.0
     st = h.step(2, graph=True)  # timing off again: the ticks re-capture without the events
     assert len(st["pairs"]) == 2
+
+
+def test_lanes_of_an_overflowed_list_share_its_cells(gpu):
+    """20,000 atoms in one or two cells, all of them beyond their rows: the same bits from any number of lanes, and the
+    lanes share the work (a cell per lane left one of them all of it, and took longer than one lane)."""
+    import time
+    from genesis_b200._lib import Handle
+    rng = np.random.default_rng(4)
+    n, L = 20000, 150.0
+    d = rng.normal(size=(n, 3))
+    d *= (3.0 * rng.random(n) ** (1 / 3) / np.linalg.norm(d, axis=1))[:, None]
+    pos = np.concatenate([d + 0.25 * L, rng.uniform(-0.5 * L, 0.5 * L, size=(5000, 3))])
+    elem = rng.integers(0, 10, len(pos)).astype(np.uint8)
+    cfg = W.C1.config()
+    cfg.size, cfg.dt = (L, L, L), 1e-9
+    out, best = [], []
+    for lanes in (1, 2, 8):
+        with Handle(cfg, "mixed") as h:
+            h.set_list_threads(lanes)
+            h.set_state(pos, np.zeros_like(pos), elem)
+            out.append((h.step(2, graph=True), h.get_state()))
+            assert h.list_stats()[1] > 19000
+            took = []
+            for _ in range(3):
+                t = time.perf_counter()
+                h.step(4, graph=True)
+                took.append(time.perf_counter() - t)
+            best.append(min(took))
+    for st, state in out[1:]:
+        assert np.array_equal(out[0][0], st)
+        for x, y in zip(out[0][1], state):
+            assert np.array_equal(x, y)
+    assert best[2] <= 0.7 * best[0]
