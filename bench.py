@@ -840,9 +840,9 @@ def ours_arm(args, dist):
             "frac": achieved / peak, "peak_source": peak_src, "traffic": traffic,
             "limiter": None if l1 is None else {
                 "unit": "L1/TEX throughput, fraction of peak (ncu)", "frac": l1,
-                "note": "as captured at 262,144 atoms (profiles/k_nl_force__c3_262144_atoms.txt); since the pair "
-                        "table left L1 the pass is bound by issue with idle lanes, then by its gathers and far-end "
-                        "reductions in L1/TEX, not by the FP32 pipe (profiles/k_nl_force__quench_512000_atoms.txt)"},
+                "note": "as captured at 1,404,928 atoms (profiles/k_nl_force__quench_1404928_atoms.txt): the pass is bound "
+                        "by issue with idle lanes, then by its gathers and far-end reductions in L1/TEX, not by the "
+                        "FP32 pipe"},
             "flop_per_launch": pairs * flop_pp, "flop_per_pair": flop_pp, "pairs_per_launch": pairs,
             "launch_ms": force_ms, "share_of_step": force_ms / tick_ms_here, "tick_ms_at_these_ticks": tick_ms_here,
             "launch_ms_min_max": [float(np.min(pass_ms)), float(np.max(pass_ms))],
