@@ -38,14 +38,16 @@
 // built: recomputed ticks reproduce the forward pass for any checkpoint
 // spacing.  The lists hold the pairs within rc + skin and are rebuilt, inside
 // the launch, on the ticks on which an atom may have moved skin/2 since.
+// Where lists do not pay or do not fit, every tick sorts the atoms and walks
+// their cells: the order then follows from the tick's positions.
 // What bounds a tick is latency: 13 warps per SM walk lists of ten to twenty
 // partners, each a chain of dependent FP64 operations.  8,000 atoms, 200
 // ticks, mixed forward, both losses: 36.2 ms, where a sort, a staging and a
-// pair pass over 27 cells per tick, one kernel each, took 143 ms; per tick
-// 13 us for the recomputed pair pass, 17 / 30 for the reverse pass without /
-// with g(r), 40 for a list rebuild every ten ticks.  Lists of rc + 0.2 rc:
-// 31.4 ms where 0.1 takes 33.8, 0.15 32.3 and 0.25 33.5; sixteen lanes per
-// atom 36.3 where eight take 34.7.
+// pair pass over 27 cells per tick, one kernel each, took 143 ms; per tick,
+// rebuilds included, 22 us for the recomputed ticks, 43 with the observables,
+// 28 / 68 for the reverse sweep without / with g(r).  Lists of rc + 0.2 rc, as
+// they were built: 31.4 ms where 0.1 takes 33.8, 0.15 32.3 and 0.25 33.5;
+// sixteen lanes per atom 36.3 where eight take 34.7.
 //
 // The cutoffs are multiples of max sigma; their derivative goes to the
 // lowest-index element attaining the max.  The hard-core clamp
