@@ -1541,7 +1541,6 @@ int nl_set_block(gx_handle* h, int block) {
     if (block != 0 && block != 128 && block != 256)
         return set_err(h, GX_ERR_ARG, "list block must be 0 (far ends in global memory), 128 or 256");
     nl_of(h)->block = block;
-    nl_of(h)->shape_set = true;
     return GX_OK;
 }
 
@@ -1554,14 +1553,12 @@ int nl_set_slots(gx_handle* h, int slots) {
 int nl_set_tpp(gx_handle* h, int tpp) {
     if (tpp != 1 && tpp != 2 && tpp != 4 && tpp != 8) return set_err(h, GX_ERR_ARG, "threads per atom must be 1, 2, 4 or 8");
     nl_of(h)->tpp = tpp;
-    nl_of(h)->shape_set = true;
     return GX_OK;
 }
 
 void nl_clear_shape(gx_handle* h) {
     NlState* s = nl_of(h);
     s->tpp = s->block = 0;
-    s->shape_set = false;
 }
 
 int nl_set_skin(gx_handle* h, double skin) {

@@ -20,8 +20,8 @@ struct NlState {
     double skin = -1.0;       // < 0: default (0.1 r_c)
     double skin_used = 0.0;
     int half = -1;            // list kind built: 0 full, 1 half (variant 6)
-    int tpp = 0;              // threads per atom in the list pass (1, 2, 4, 8; 0: nl_auto_lanes)
-    bool shape_set = false;   // the work shape was set or tuned: it is the per-kernel tick's
+    int tpp = 0;              // threads per atom in the list pass (1, 2, 4, 8; 0: nl_auto_lanes);
+                              // with it or `block` set, the work shape is the per-kernel tick's
     int slots = 16;           // variant 7: stash slots per thread (8 or 16)
     int brick = 1;            // variant 8: 0 = bricks of 4 cells (1024 staged atoms), 1 = 8 cells (2048)
     int block = 0;            // variant 6, one lane per atom: 0 = far ends always global, 128 or 256 = far

@@ -414,7 +414,7 @@ bool nl_ticks_eligible(gx_handle* h) {
     if (h->p.enable_collisions || h->prof_on || h->pass_timing) return false;
     const NlState* s = static_cast<const NlState*>(h->nl);
     if (!s || (mixed && 0.5 * s->expect * (double)h->n > kTickMaxEntries)) return false;
-    return !s->shape_set && s->half == (mixed ? 1 : 0) && s->lg.ncell < kScanTileCells * kScanMaxTiles;
+    return s->tpp == 0 && s->block == 0 && s->half == (mixed ? 1 : 0) && s->lg.ncell < kScanTileCells * kScanMaxTiles;
 }
 
 // nticks ticks with the records (may be null) at rec[0 .. nticks).

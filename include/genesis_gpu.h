@@ -153,7 +153,8 @@ int gx_autotune(gx_handle* h, int reps, int* best, double* ms);
 int gx_set_list_skin(gx_handle* h, double skin);
 /* Threads per atom of the variant-5/6 list pass: 1, 2, 4 or 8 lanes share
  * one atom's list (default: by the atom count; the autotuner picks the
- * fastest).  Every
+ * fastest).  A choice made here is the launched ticks' (see
+ * gx_set_kernel_variant).  Every
  * choice gives the same bits (integer sums).  No counterpart in the
  * reference. */
 int gx_set_list_threads(gx_handle* h, int threads_per_atom);

@@ -152,3 +152,17 @@ def test_sizes_that_run_in_one_launch(gpu, precision, n_side, one):
             l0 = h.launches
             h.step(5, graph=True)
             assert h.launches - l0 > 2
+
+
+def test_the_default_block_is_no_shape(gpu):
+    """Far ends in global memory is the default: setting it, or going back to it, keeps the one-launch tick."""
+    from genesis_b200._lib import Handle
+    wl = W.Workload("tick check", n_side=8, temperature=100.0, steps=10)
+    with Handle(wl.config(), "mixed") as h:
+        h.set_universe(wl.generate())
+        for block, one in ((0, True), (128, False), (0, True)):
+            h.set_list_block(block)
+            h.step(1, graph=True)
+            l0 = h.launches
+            h.step(5, graph=True)
+            assert (h.launches - l0 == 2) == one
