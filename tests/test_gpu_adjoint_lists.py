@@ -231,3 +231,10 @@ def test_more_cells_than_one_scan_of_tiles(gpu):
     assert np.max(np.abs(V - want) / np.abs(want)) <= 1e-10
     # V is linear in one factor on all epsilons but for the two ticks' drift at this step
     assert abs(ge @ np.asarray(cfg.epsilon_k) - V[1]) <= 1e-6 * abs(V[1])
+
+
+@pytest.mark.parametrize("n_side,cutoff", [(10, 5.9), (11, 6.5)])  # two force cells an axis: lists of 860; cells
+def test_wide_cutoffs_on_two_cells_match_dual_oracle(gpu, orc, n_side, cutoff):
+    cfg, u = _case(n_side, coul=True)
+    cfg.coulomb_cutoff = cutoff
+    _against_dual(orc, cfg, u, 3, 2, dict(gr_bins=30, gr_every=1, gr_rmax=6.0, gr_width=0.15, gr_support=6.0))
