@@ -350,3 +350,23 @@ def test_lanes_of_an_overflowed_list_share_its_cells(gpu):
         for x, y in zip(out[0][1], state):
             assert np.array_equal(x, y)
     assert best[2] <= 0.7 * best[0]
+
+
+@pytest.mark.parametrize("lanes", [1, 8])
+def test_captured_half_list_ticks_of_a_set_shape(gpu, lanes):
+    """A work shape keeps variant 6 on captured ticks at any size: the same ticks and rebuilds as eager execution."""
+    cfg, u = _lattice(14, temperature=300.0, coul=True)
+    out = []
+    for graph in (False, True):
+        h = _handle(cfg, 6)
+        h.set_list_threads(lanes)
+        h.set_universe(u)
+        l0 = h.launches
+        st = h.step(40, graph=graph)
+        out.append((h.get_state(), st, h.list_rebuilds(), h.launches - l0))
+    (s0, t0, r0, n0), (s1, t1, r1, n1) = out
+    for x, y in zip(s0, s1):
+        assert np.array_equal(x, y)
+    assert np.array_equal(t0, t1)
+    assert r0 == r1 and 3 <= r0 < 40
+    assert 3 * 40 < n1 < n0  # a few launches a tick, and a rebuild's only where one ran
